@@ -38,7 +38,7 @@ struct DGrid {
   const float *u0, *v0;       // base-state winds, full u-/v-arrays (Rayleigh damping)
   // launch shapes (cm1g_set_tune / cm1g_autotune): index into the tile-shape
   // table of the scalar and momentum passes, and the acoustic kernel's form
-  // (-1: chosen by the number of columns)
+  // (-1: the default, form 0)
   int tile_adv, tile_mom, sound_cfg;
 };
 
@@ -52,9 +52,9 @@ constexpr int kTileShapes[kNumTileShapes][3] = {{32, 8, 16}, {32, 8, 8}, {32, 4,
 // row of TX threads than the tile has cell rows (the row that evaluates the
 // tile's north and east faces), so a block is TX x (TY + 1) threads.
 constexpr int kScalShapes[kNumTileShapes][3] = {{32, 7, 16}, {32, 7, 8}, {32, 3, 16}, {64, 3, 16}, {32, 7, 32}};
-// Forms of the acoustic kernel: 0 tile (32 columns x 8 warps over the
-// levels), 1 tile with 4 warps, 2 column sweep 32 x 4 columns, 3 column
-// sweep 32 x 2 columns.
+// Forms of the acoustic kernel: 0 tile (32 columns, the warps over the levels
+// chosen by the grid's size), 1 tile with 16 explicit warps, 2 column sweep
+// 32 x 4 columns, 3 column sweep 32 x 2 columns.
 constexpr int kNumSoundCfgs = 4;
 
 // Fortran-layout offsets.  s and w arrays share the plane (NI*NJ); u arrays
@@ -78,6 +78,9 @@ __host__ __device__ __forceinline__ long nV(const DGrid &g) { return (long)g.NI 
 __host__ __device__ __forceinline__ long nW(const DGrid &g) { return (long)g.NI * g.NJ * (g.NK + 1); }
 
 #define LDG(p) __ldg(p)
+
+// brings the line of p into L2; the marching kernels call it for the levels ahead
+__device__ __forceinline__ void prefetch_l2(const float *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 // ---------------------------------------------------------------------
 // Face values (binary32 arithmetic in the reference's evaluation order;
@@ -232,6 +235,15 @@ struct EnerIn {
   const float *zh, *rho, *ua, *va, *wa, *ppi, *tha, *qv, *ql, *qi, *vr;
   float lv1, ls1;
 };
+
+// Levels that a block of a marching tile kernel owns, given the tiles of a
+// level: as many as still leave two blocks for each of the 148 SMs twice over
+// (a block loads the level below its first one again), at least 8.
+inline int tile_levels(long tiles, int nk) {
+  int kc = nk;
+  while (kc > 8 && tiles * ((nk + kc - 1) / kc) < 4L * 148) kc = (kc + 1) / 2;
+  return kc < 8 ? 8 : kc;
+}
 
 // Records a message for cm1g_last_error() and returns code (C++ linkage,
 // not part of the C-ABI).

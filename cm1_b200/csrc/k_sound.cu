@@ -1,19 +1,34 @@
 // k_sound.cu -- acoustic substeps of sound.F (psolver=3, no terrain).
 //
-// One kernel launch per small step.  A block owns a tile of TX consecutive
-// columns (i) of one row (j), all levels, and works in three phases:
+// One kernel launch per small step.  A block owns a tile of 32 consecutive
+// columns (i) of one row (j), all levels:
 //
-//  1. point-parallel (warp w takes levels w+1, w+1+NW, ...; lanes run along
-//     i so every global access is a coalesced row segment): new u and v by
-//     the pressure-gradient update (sound.F:321-341) with the open-boundary
+//  1. its explicit warps take interleaved levels (lanes run along i so every
+//     global access is a coalesced row segment): new u and v by the
+//     pressure-gradient update (sound.F:321-341) with the open-boundary
 //     updates of bc.F:2392-2686 folded in, the running sums of u and v
 //     (sound.F:806-835), the explicit pi' forcing fpk (sound.F:479-502), and
 //     the per-level pieces of the implicit w equation, kept in shared memory;
-//  2. column-sequential (one thread per column): the Thomas forward
-//     elimination and back substitution of sound.F:659-733, entirely in
-//     shared memory, with the reference's operation order;
-//  3. point-parallel again: pi' update with divergence damping
+//  2. its solver warp (one thread per column) follows them up the column with
+//     the Thomas forward elimination of sound.F:659-733 as groups of levels
+//     become complete, and then substitutes back, entirely in shared memory
+//     and with the reference's operation order;
+//  3. the explicit warps again: pi' update with divergence damping
 //     (sound.F:746-760), new w and the averaged w.
+//
+// What bounds it: latency and instruction issue, not bytes.  At 256x256x80 a
+// launch takes 0.141 ms = 3.4 TB/s of its 92 B a cell (0.53 of the measured
+// HBM copy rate); it executes about 430 warp instructions per 32 cells and
+// issues in half of the cycles.  Before (8 warps, the solve on one of them
+// after a block barrier, 64-bit indices, profiles read per level): 0.184 ms,
+// 558 instructions; at 512x512x128 2.27 ms against 0.86 now.  What made the
+// difference: the solver warp hidden behind the loads, 32-bit byte offsets,
+// the level constants formed once per block, the edge code (open boundaries,
+// mapped ppd reads, last faces) kept out of the interior blocks' level body,
+// and each warp's next level prefetched to L2 (4 to 8 %).  Measured and not
+// kept: two or four rows a block (more shared memory, less L1: 15 to 50 %
+// slower), four blocks an SM (L1 too small: 1.4 times), bulk prefetches of the
+// whole column by the solver warp (1,100 small requests a block: 2 times).
 //
 // Neighbour columns read u, v and ppd from the previous small step, so u, v
 // and ppd are double-buffered; w and pi' are read only by their own column
@@ -22,6 +37,7 @@
 // reproduces the stored value exactly.
 #include <cstdlib>
 #include <cstring>
+#include <type_traits>
 #include "cm1g_common.cuh"
 
 namespace cm1g {
@@ -196,20 +212,26 @@ __global__ void k_openbc_restrict(DGrid g, SoundIO io, float dts, float *ubw, fl
   }
 }
 
-static const int SND_TX = 32;     // columns per tile (one warp wide)
-static const int SND_NW = 8;      // warps per block
-static const int SND_KPT = 16;    // max levels per thread: nk <= SND_NW*SND_KPT
+constexpr int SND_TX = 32;        // columns per tile (one warp wide)
+constexpr int SND_MAXNK = 128;    // levels the tile forms hold
+constexpr int SND_NARR = 5;       // column arrays in shared memory
 
-#ifndef CM1G_SND_MINB
-#define CM1G_SND_MINB 3      // resident blocks per SM the tile kernel is compiled for
-#endif
-#ifndef CM1G_SND_UNROLL
-#define CM1G_SND_UNROLL 1    // phase-1 levels a warp keeps in flight
-#endif
-constexpr int kSndUnroll = CM1G_SND_UNROLL;
+// Per-level constants of a stage (sound.F:117-135, 188-189), formed once per
+// block: temq, r1, r2 and temm; c1, c2 of the level's lower and upper face.
+struct SndLev { float temq, r1, r2, temm, c1a, c2a, c1b, c2b; };
 
-template <int TX, int NW, int KPT>
-__global__ void __launch_bounds__(TX * NW, CM1G_SND_MINB) k_sound_tile(DGrid g, SoundIO io, SoundStep p) {
+__device__ __forceinline__ void bar_arrive(int id, int n) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+__device__ __forceinline__ void bar_wait(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+
+// NW explicit warps and one solver warp per block.  The explicit warps take
+// interleaved levels (w+1, w+1+NW, ...); after each GS rounds (GS*NW levels)
+// they arrive at a named barrier on which only the solver warp waits, so the
+// forward elimination runs while the levels above are still being loaded.
+template <int NW, int KPT, int MINB>
+__global__ void __launch_bounds__(SND_TX *(NW + 1), MINB) k_sound_tile(DGrid g, SoundIO io, SoundStep p) {
+  constexpr int TX = SND_TX;
+  constexpr int GS = (KPT + 13) / 14;         // rounds per barrier: at most 14 barrier ids
+  constexpr int NBT = TX * (NW + 1);
   extern __shared__ float sm[];
   const int lane = threadIdx.x, w = threadIdx.y;
   const int i = 1 + (int)blockIdx.x * TX + lane;
@@ -222,99 +244,126 @@ __global__ void __launch_bounds__(TX * NW, CM1G_SND_MINB) k_sound_tile(DGrid g, 
   float *P2 = sm + 2 * L * TX;  // pk2 - qk
   float *MM = sm + 3 * L * TX;  // mm, then the LU factor dum1
   float *DD = sm + 4 * L * TX;  // w_old + fwk, then dum2, then the new w (DD(1) = w(1))
+  SndLev *LV = reinterpret_cast<SndLev *>(sm + SND_NARR * L * TX);
 #define S(a, k) a[(k) * TX + lane]
 
   const float dts = p.dts, alph = g.alph, beta = 1.0f - alph, asq = alph * alph;
   const float cp = g.c.cp, rdx = g.rdx, rdy = g.rdy, rdz = g.rdz;
 
-  // ---------------- phase 1 ----------------
-  if (active) {
+  for (int k = 1 + lane + TX * w; k <= nk; k += NBT) {
+    const float mhk = LDG(&g.mh[k]), rr0k = LDG(&g.rr0[k]);
+    SndLev v;
+    v.temq = dts * rdz * mhk;
+    v.r2 = dts * rdz * mhk * rr0k * LDG(&g.rf0[k + 1]);
+    v.r1 = dts * rdz * mhk * rr0k * LDG(&g.rf0[k]);
+    v.temm = dts * rdz * cp * LDG(&g.mf[k]);
+    v.c1a = LDG(&g.c1[k]); v.c2a = LDG(&g.c2[k]);
+    v.c1b = LDG(&g.c1[k + 1]); v.c2b = LDG(&g.c2[k + 1]);
+    LV[k] = v;
+  }
+  __syncthreads();
+
+  // 32-bit byte offsets (sound_tall keeps larger arrays out): one 64-bit
+  // addition per access, 4 % faster over a step than element offsets
+  const uint32_t rowS = (uint32_t)g.NI * 4u, planeS = rowS * (uint32_t)g.NJ;
+  const uint32_t planeU = planeS + 4u * (uint32_t)g.NJ, planeV = planeS + rowS;
+  auto F = [](const float *a, uint32_t o) -> const float * { return reinterpret_cast<const float *>(reinterpret_cast<const char *>(a) + o); };
+  auto G = [](float *a, uint32_t o) -> float * { return reinterpret_cast<float *>(reinterpret_cast<char *>(a) + o); };
+  const uint32_t oc = (uint32_t)(i - g.ib) * 4u + rowS * (uint32_t)(j - g.jb);
+  const uint32_t ocu = oc + 4u * (uint32_t)(j - g.jb);
+
+  if (w < NW) {
+    // ---------------- phase 1: explicit updates of the warp's levels ----------------
     const float tem1pg = rdx * cp * 0.5f, tem2pg = rdy * cp * 0.5f;      // sound.F:321-322
     const float temx = dts * 0.5f * rdx, temy = dts * 0.5f * rdy;        // sound.F:479-480
-    const float uh_i = LDG(&g.uh[i - g.ib]), vh_j = LDG(&g.vh[j - g.jb]);
-    const float uf_i = LDG(&g.uf[i - g.ib]), uf_ip = LDG(&g.uf[i + 1 - g.ib]);
-    const float vf_j = LDG(&g.vf[j - g.jb]), vf_jp = LDG(&g.vf[j + 1 - g.jb]);
-    const float dtu_i = dts * LDG(&g.dtu0[i2(g, i, j)]), dtu_ip = dts * LDG(&g.dtu0[i2(g, i + 1, j)]);
-    const float dtv_j = dts * LDG(&g.dtv0[i2(g, i, j)]), dtv_jp = dts * LDG(&g.dtv0[i2(g, i, j + 1)]);
-    const bool openw = (g.wbc == 2 && g.ibw && i == 1), opene = (g.ebc == 2 && g.ibe && i == ni);
-    const bool opens = (g.sbc == 2 && g.ibs && j == 1), openn = (g.nbc == 2 && g.ibn && j == nj);
-    const PpdNbr pn_ = ppd_nbr(g, p.ppd_mapped, i, j);
-    // warps take interleaved levels (w+1, w+1+NW, ...): at any time the
-    // block's warps work on adjacent levels and share their vertical
-    // neighbours through L1
-    const long plane = (long)g.NI * g.NJ;
-#pragma unroll kSndUnroll
-    for (int m = 0; m < KPT; m++) {
-      const int k = 1 + w + m * NW;
-      if (k > nk) break;
-      const long o = iS(g, i, j, k);
-      const long ou = iU(g, i, j, k), oup = ou + 1;
-      const long ov = iV(g, i, j, k), ovp = ov + g.NI;
+    float uh_i = 0, vh_j = 0, uf_i = 0, uf_ip = 0, vf_j = 0, vf_jp = 0, dtu_i = 0, dtu_ip = 0, dtv_j = 0, dtv_jp = 0;
+    if (active) {
+      uh_i = LDG(&g.uh[i - g.ib]); vh_j = LDG(&g.vh[j - g.jb]);
+      uf_i = LDG(&g.uf[i - g.ib]); uf_ip = LDG(&g.uf[i + 1 - g.ib]);
+      vf_j = LDG(&g.vf[j - g.jb]); vf_jp = LDG(&g.vf[j + 1 - g.jb]);
+      dtu_i = dts * LDG(&g.dtu0[i2(g, i, j)]); dtu_ip = dts * LDG(&g.dtu0[i2(g, i + 1, j)]);
+      dtv_j = dts * LDG(&g.dtv0[i2(g, i, j)]); dtv_jp = dts * LDG(&g.dtv0[i2(g, i, j + 1)]);
+    }
+    // blocks away from the domain's edges run the level body without the
+    // open-boundary updates, the mapped ppd reads and the last faces' stores
+    const bool edge = blockIdx.x == 0 || (int)(blockIdx.x + 1) * TX >= ni || j == 1 || j == nj;
+    auto level = [&](auto edge_tag, int k) {
+      constexpr bool EDGE = decltype(edge_tag)::value;
+      const uint32_t o = oc + (uint32_t)k * planeS, ou = ocu + (uint32_t)k * planeU, ov = oc + (uint32_t)k * planeV;
+      const uint32_t om = o - planeS, op = o + planeS, ovp = ov + rowS;
+      // the warp's next level towards L2: the loads below then wait for L2 only
+      if (k + NW <= nk) {
+        const uint32_t qo = o + NW * planeS, qu = ou + NW * planeU, qv = ov + NW * planeV;
+        const float *next[] = {F(io.piadv, qo), F(io.thv, qo), F(io.ppd_in, qo), F(io.u_in, qu), F(io.v_in, qv), F(io.uten, qu),
+                               F(io.vten, qv), F(io.ppten, qo), F(io.ppterm, qo), F(io.w_in, qo), F(io.pp_in, qo), F(io.wten, qo)};
+#pragma unroll
+        for (const float *q : next) prefetch_l2(q);
+        if (!p.first) { prefetch_l2(F(io.rru, qu)); prefetch_l2(F(io.rrv, qv)); }
+      }
       // ---- loads (all independent)
-      const float pia = LDG(&io.piadv[o]);
-      const float pid = (k > 1) ? LDG(&io.piadv[o - plane]) : 0.0f;
-      const float thd = (k > 1) ? LDG(&io.thv[o - plane]) : 0.0f;
-      const float ppm = (k > 1) ? io.pp_in[o - plane] : 0.0f;
-      const float wk = io.w_in[o];
-      const float piw = LDG(&io.piadv[o - 1]), pie = LDG(&io.piadv[o + 1]);
-      const float pis = LDG(&io.piadv[o - g.NI]), pin = LDG(&io.piadv[o + g.NI]);
-      const float piu = (k < nk) ? LDG(&io.piadv[o + plane]) : 0.0f;
-      const float thc = LDG(&io.thv[o]), thw = LDG(&io.thv[o - 1]), the = LDG(&io.thv[o + 1]);
-      const float ths = LDG(&io.thv[o - g.NI]), thn = LDG(&io.thv[o + g.NI]);
-      const float ppc = LDG(&io.ppd_in[o]), ppw = LDG(&io.ppd_in[o + pn_.w]), ppe = LDG(&io.ppd_in[o + pn_.e]);
-      const float pps = LDG(&io.ppd_in[o + pn_.s]), ppn = LDG(&io.ppd_in[o + pn_.n]);
-      const float u0v = LDG(&io.u_in[ou]), u1v = LDG(&io.u_in[oup]);
-      const float v0v = LDG(&io.v_in[ov]), v1v = LDG(&io.v_in[ovp]);
-      const float ut0 = LDG(&io.uten[ou]), ut1 = LDG(&io.uten[oup]);
-      const float vt0 = LDG(&io.vten[ov]), vt1 = LDG(&io.vten[ovp]);
-      const float pptn = LDG(&io.ppten[o]), pptm = LDG(&io.ppterm[o]);
-      const float wkp = (k < nk) ? io.w_in[o + plane] : 0.0f;
-      const float pp = io.pp_in[o];
-      const float wtn = LDG(&io.wten[o]);
-      const float accu0 = p.first ? 0.0f : io.rru[ou];
-      const float accv0 = p.first ? 0.0f : io.rrv[ov];
-      // ---- u at faces i, i+1 and v at faces j, j+1
-      float uo = u0v;
-      if (openw) uo = g.roflux ? RJK(g, io.ubw, j, k) : uo + dts * (-radbc_in(g, RJK(g, io.radbcw, j, k), u0v) * (u1v - u0v) * rdx * LDG(&g.uh[1 - g.ib]) + ut0);
-      const float un0 = uo + dtu_i * (ut0 - tem1pg * (ppc - ppw) * uf_i * (thc + thw));
-      float uop = u1v;
-      if (opene) uop = g.roflux ? RJK(g, io.ube, j, k) : uop + dts * (-radbc_out(g, RJK(g, io.radbce, j, k), u1v) * (u1v - u0v) * rdx * LDG(&g.uh[ni - g.ib]) + ut1);
-      const float unp = uop + dtu_ip * (ut1 - tem1pg * (ppe - ppc) * uf_ip * (the + thc));
-      float vo = v0v;
-      if (opens) vo = g.roflux ? RIK(g, io.vbs, i, k) : vo + dts * (-radbc_in(g, RIK(g, io.radbcs, i, k), v0v) * (v1v - v0v) * rdy * LDG(&g.vh[1 - g.jb]) + vt0);
-      const float vn0 = vo + dtv_j * (vt0 - tem2pg * (ppc - pps) * vf_j * (thc + ths));
-      float vop = v1v;
-      if (openn) vop = g.roflux ? RIK(g, io.vbn, i, k) : vop + dts * (-radbc_out(g, RIK(g, io.radbcn, i, k), v1v) * (v1v - v0v) * rdy * LDG(&g.vh[nj - g.jb]) + vt1);
-      const float vnp = vop + dtv_jp * (vt1 - tem2pg * (ppn - ppc) * vf_jp * (thn + thc));
-      io.u_out[ou] = un0;
-      io.v_out[ov] = vn0;
-      if (p.last) {
-        io.rru[ou] = (accu0 + un0) * p.tavg;
-        io.rrv[ov] = (accv0 + vn0) * p.tavg;
+      const float pia = LDG(F(io.piadv, o)), piw = LDG(F(io.piadv, o) - 1), pie = LDG(F(io.piadv, o) + 1);
+      const float pis = LDG(F(io.piadv, o - rowS)), pin = LDG(F(io.piadv, o + rowS));
+      const float thc = LDG(F(io.thv, o)), thw = LDG(F(io.thv, o) - 1), the = LDG(F(io.thv, o) + 1);
+      const float ths = LDG(F(io.thv, o - rowS)), thn = LDG(F(io.thv, o + rowS));
+      float ppc, ppw, ppe, pps, ppn;
+      ppc = LDG(F(io.ppd_in, o));
+      if (EDGE) {
+        const PpdNbr pn_ = ppd_nbr(g, p.ppd_mapped, i, j);
+        ppw = LDG(F(io.ppd_in, o) + pn_.w); ppe = LDG(F(io.ppd_in, o) + pn_.e);
+        pps = LDG(F(io.ppd_in, o) + pn_.s); ppn = LDG(F(io.ppd_in, o) + pn_.n);
       } else {
-        io.rru[ou] = accu0 + un0;
-        io.rrv[ov] = accv0 + vn0;
+        ppw = LDG(F(io.ppd_in, o) - 1); ppe = LDG(F(io.ppd_in, o) + 1);
+        pps = LDG(F(io.ppd_in, o - rowS)); ppn = LDG(F(io.ppd_in, o + rowS));
       }
-      if (i == ni) {
-        io.u_out[oup] = unp;
-        const float a1 = p.first ? 0.0f : io.rru[oup];
-        io.rru[oup] = p.last ? (a1 + unp) * p.tavg : a1 + unp;
+      const float u0v = LDG(F(io.u_in, ou)), u1v = LDG(F(io.u_in, ou) + 1);
+      const float v0v = LDG(F(io.v_in, ov)), v1v = LDG(F(io.v_in, ovp));
+      const float ut0 = LDG(F(io.uten, ou)), ut1 = LDG(F(io.uten, ou) + 1);
+      const float vt0 = LDG(F(io.vten, ov)), vt1 = LDG(F(io.vten, ovp));
+      const float pptn = LDG(F(io.ppten, o)), pptm = LDG(F(io.ppterm, o));
+      const float wk = *F(io.w_in, o), pp = *F(io.pp_in, o), wtn = LDG(F(io.wten, o));
+      float pid = 0.0f, thd = 0.0f, ppm = 0.0f, piu = 0.0f, wkp = 0.0f;
+      if (k > 1) { pid = LDG(F(io.piadv, om)); thd = LDG(F(io.thv, om)); ppm = *F(io.pp_in, om); }
+      if (k < nk) { piu = LDG(F(io.piadv, op)); wkp = *F(io.w_in, op); }
+      float accu0 = 0.0f, accv0 = 0.0f;
+      if (!p.first) { accu0 = *F(io.rru, ou); accv0 = *F(io.rrv, ov); }
+      const SndLev lv = LV[k];
+      // ---- u at faces i, i+1 and v at faces j, j+1
+      float uo = u0v, uop = u1v, vo = v0v, vop = v1v;
+      if (EDGE) {
+        if (g.wbc == 2 && g.ibw && i == 1)
+          uo = g.roflux ? RJK(g, io.ubw, j, k) : uo + dts * (-radbc_in(g, RJK(g, io.radbcw, j, k), u0v) * (u1v - u0v) * rdx * LDG(&g.uh[1 - g.ib]) + ut0);
+        if (g.ebc == 2 && g.ibe && i == ni)
+          uop = g.roflux ? RJK(g, io.ube, j, k) : uop + dts * (-radbc_out(g, RJK(g, io.radbce, j, k), u1v) * (u1v - u0v) * rdx * LDG(&g.uh[ni - g.ib]) + ut1);
+        if (g.sbc == 2 && g.ibs && j == 1)
+          vo = g.roflux ? RIK(g, io.vbs, i, k) : vo + dts * (-radbc_in(g, RIK(g, io.radbcs, i, k), v0v) * (v1v - v0v) * rdy * LDG(&g.vh[1 - g.jb]) + vt0);
+        if (g.nbc == 2 && g.ibn && j == nj)
+          vop = g.roflux ? RIK(g, io.vbn, i, k) : vop + dts * (-radbc_out(g, RIK(g, io.radbcn, i, k), v1v) * (v1v - v0v) * rdy * LDG(&g.vh[nj - g.jb]) + vt1);
       }
-      if (j == nj) {
-        io.v_out[ovp] = vnp;
-        const float a1 = p.first ? 0.0f : io.rrv[ovp];
-        io.rrv[ovp] = p.last ? (a1 + vnp) * p.tavg : a1 + vnp;
+      const float un0 = uo + dtu_i * (ut0 - tem1pg * (ppc - ppw) * uf_i * (thc + thw));
+      const float unp = uop + dtu_ip * (ut1 - tem1pg * (ppe - ppc) * uf_ip * (the + thc));
+      const float vn0 = vo + dtv_j * (vt0 - tem2pg * (ppc - pps) * vf_j * (thc + ths));
+      const float vnp = vop + dtv_jp * (vt1 - tem2pg * (ppn - ppc) * vf_jp * (thn + thc));
+      *G(io.u_out, ou) = un0;
+      *G(io.v_out, ov) = vn0;
+      float ru = accu0 + un0, rv = accv0 + vn0;
+      if (p.last) { ru = ru * p.tavg; rv = rv * p.tavg; }
+      *G(io.rru, ou) = ru;
+      *G(io.rrv, ov) = rv;
+      if (EDGE) {
+        if (i == ni) {
+          *(G(io.u_out, ou) + 1) = unp;
+          const float a1 = p.first ? 0.0f : *(F(io.rru, ou) + 1);
+          *(G(io.rru, ou) + 1) = p.last ? (a1 + unp) * p.tavg : a1 + unp;
+        }
+        if (j == nj) {
+          *G(io.v_out, ovp) = vnp;
+          const float a1 = p.first ? 0.0f : *F(io.rrv, ovp);
+          *G(io.rrv, ovp) = p.last ? (a1 + vnp) * p.tavg : a1 + vnp;
+        }
       }
-      // ---- stage coefficients (sound.F:117-135, 188-189)
-      const float mhk = LDG(&g.mh[k]), rr0k = LDG(&g.rr0[k]);
-      const float temq = dts * rdz * mhk;
-      const float r2 = dts * rdz * mhk * rr0k * LDG(&g.rf0[k + 1]);
-      const float r1 = dts * rdz * mhk * rr0k * LDG(&g.rf0[k]);
-      const float temm = dts * rdz * cp * LDG(&g.mf[k]);
-      const float c1a = LDG(&g.c1[k]), c1b = LDG(&g.c1[k + 1]), c2a = LDG(&g.c2[k]), c2b = LDG(&g.c2[k + 1]);
-      const float qk = temq * pptm;
-      const float pk2 = (k == nk) ? 0.0f : r2 * (-c2b * piu + (1.0f - c1b) * pia);
-      const float pk1 = (k == 1) ? 0.0f : r1 * (+c1a * pid + (c2a - 1.0f) * pia);
+      const float qk = lv.temq * pptm;
+      const float pk2 = (k == nk) ? 0.0f : lv.r2 * (-lv.c2b * piu + (1.0f - lv.c1b) * pia);
+      const float pk1 = (k == 1) ? 0.0f : lv.r1 * (+lv.c1a * pid + (lv.c2a - 1.0f) * pia);
       const float p1 = pk1 + qk, p2 = pk2 - qk;
       // ---- fpk (sound.F:486-498)
       float div = (unp - un0) * rdx * uh_i + (vnp - vn0) * rdy * vh_j;
@@ -328,75 +377,68 @@ __global__ void __launch_bounds__(TX * NW, CM1G_SND_MINB) k_sound_tile(DGrid g, 
       S(PF, k) = pp + fpk;
       S(P1, k) = p1;
       S(P2, k) = p2;
-      if (k >= 2) {
-        const float mm = temm * (c2a * thc + c1a * thd);
-        const float fwk = dts * wtn + beta * (-mm * (pp - ppm));
-        S(MM, k) = mm;
-        S(DD, k) = wk + fwk;
+      const float mm = lv.temm * (lv.c2a * thc + lv.c1a * thd);
+      const float fwk = dts * wtn + beta * (-mm * (pp - ppm));
+      S(MM, k) = mm;                                  // level 1's mm is not read
+      S(DD, k) = (k == 1) ? wk : wk + fwk;
+    };
+#pragma unroll 1
+    for (int m = 0; m < KPT; m++) {
+      const int k = 1 + w + m * NW;
+      if (m * NW >= nk) break;
+      if (k <= nk && active) {
+        if (edge) level(std::true_type{}, k);
+        else level(std::false_type{}, k);
       }
-      if (k == 1) S(DD, 1) = wk;
+      __syncwarp();
+      if ((m + 1) % GS == 0 || (m + 1) * NW >= nk) bar_arrive(1 + m / GS, NBT);
     }
   }
-  __syncthreads();
 
   // phase 3's global inputs of this warp's levels (pi' before the step and
   // the running sum of w; the column's own points), loaded now so that they
-  // arrive while warp 0 runs the Thomas solve
+  // arrive while the solver finishes
   float ppo[KPT], acs[KPT];
-  if (active) {
+  if (w < NW && active) {
 #pragma unroll
     for (int m = 0; m < KPT; m++) {
       const int k = 1 + w + m * NW;
       ppo[m] = 0.0f; acs[m] = 0.0f;
       if (k <= nk) {
-        const long o = iS(g, i, j, k);
-        ppo[m] = io.pp_in[o];
-        acs[m] = p.first ? LDG(&io.wa[o]) * beta : io.rrw[o];
+        const uint32_t o = oc + (uint32_t)k * planeS;
+        ppo[m] = *F(io.pp_in, o);
+        acs[m] = p.first ? LDG(F(io.wa, o)) * beta : *F(io.rrw, o);
       }
     }
   }
 
-  // ---------------- phase 2: Thomas solve for w, k = 2..nk ----------------
-  // The first and last levels are peeled off so that the loop body has no
-  // branches and its shared-memory reads (independent of the recurrence)
-  // can be issued ahead of the dependent chain; nk >= 6 (cm1g_init).
-  if (w == 0 && active) {
-    float d1p, d2p;
-    {
-      const int k = 2;
-      const float mm = S(MM, k);
-      const float bb = 1.0f - asq * (+mm * (-S(P1, k) + S(P2, k - 1)));
-      const float dd = S(DD, k) + alph * (-mm * (S(PF, k) - S(PF, k - 1)));
-      const float cc = -asq * (-mm * S(P2, k));
-      // __frcp_rn is the correctly rounded 1/x, the same value as 1.0f/x
-      const float rr = __frcp_rn(bb);
-      d1p = -cc * rr;
-      d2p = dd * rr;
-      S(MM, k) = d1p; S(DD, k) = d2p;
-    }
+  // ---------------- phase 2: Thomas solve for w, k = 2..nk (the solver warp) ----------------
+  if (w == NW) {
+    float p1m = 0.0f, p2m = 0.0f, pfm = 0.0f, d1p = 0.0f, d2p = 0.0f;
+#pragma unroll 1
+    for (int m0 = 0; m0 * NW < nk; m0 += GS) {
+      bar_wait(1 + m0 / GS, NBT);
+      const int ke = min(nk, (m0 + GS) * NW);
+      int k = 1 + m0 * NW;
+      if (k == 1) { p1m = S(P1, 1); p2m = S(P2, 1); pfm = S(PF, 1); k = 2; }
+      // with d1p = d2p = 0 the general form gives level 2's values
 #pragma unroll 4
-    for (int k = 3; k < nk; k++) {
-      const float mm = S(MM, k);
-      const float bb = 1.0f - asq * (+mm * (-S(P1, k) + S(P2, k - 1)));
-      const float dd = S(DD, k) + alph * (-mm * (S(PF, k) - S(PF, k - 1)));
-      const float aa = -asq * (+mm * S(P1, k - 1));
-      const float cc = -asq * (-mm * S(P2, k));
-      const float rr = __frcp_rn(aa * d1p + bb);
-      d1p = -cc * rr;
-      d2p = (dd - aa * d2p) * rr;
-      S(MM, k) = d1p; S(DD, k) = d2p;
+      for (; k <= ke; k++) {
+        const float mm = S(MM, k), p1 = S(P1, k), p2 = S(P2, k), pf = S(PF, k);
+        const float bb = 1.0f - asq * (+mm * (-p1 + p2m));
+        const float dd = S(DD, k) + alph * (-mm * (pf - pfm));
+        const float aa = -asq * (+mm * p1m);
+        const float cc = -asq * (-mm * p2);
+        // __frcp_rn is the correctly rounded 1/x, the same value as 1.0f/x
+        const float rr = __frcp_rn(aa * d1p + bb);
+        d1p = -cc * rr;
+        d2p = (dd - aa * d2p) * rr;
+        S(MM, k) = d1p; S(DD, k) = d2p;
+        p1m = p1; p2m = p2; pfm = pf;
+      }
     }
-    {
-      const int k = nk;
-      const float mm = S(MM, k);
-      const float bb = 1.0f - asq * (+mm * (-S(P1, k) + S(P2, k - 1)));
-      const float dd = S(DD, k) + alph * (-mm * (S(PF, k) - S(PF, k - 1)));
-      const float aa = -asq * (+mm * S(P1, k - 1));
-      const float rr = __frcp_rn(aa * d1p + bb);
-      S(DD, k) = (dd - aa * d2p) * rr;   // w(nk)
-    }
-    float wup = S(DD, nk);
-#pragma unroll 4
+    float wup = d2p;   // w(nk)
+#pragma unroll 8
     for (int k = nk - 1; k >= 2; k--) {
       wup = S(MM, k) * wup + S(DD, k);
       S(DD, k) = wup;
@@ -405,23 +447,23 @@ __global__ void __launch_bounds__(TX * NW, CM1G_SND_MINB) k_sound_tile(DGrid g, 
   __syncthreads();
 
   // ---------------- phase 3 ----------------
-  if (active) {
+  if (w < NW && active) {
 #pragma unroll
     for (int m = 0; m < KPT; m++) {
       const int k = 1 + w + m * NW;
       if (k > nk) break;
-      const long o = iS(g, i, j, k);
+      const uint32_t o = oc + (uint32_t)k * planeS;
       const float wk = S(DD, k);
       const float wkp = (k < nk) ? S(DD, k + 1) : 0.0f;
       float pn = S(PF, k) + alph * (wk * S(P1, k) + wkp * S(P2, k));
       if (fabsf(pn) < g.smeps) pn = 0.0f;
       const float d1 = g.kdiv * (pn - ppo[m]);
       const float ac = acs[m];
-      io.pp_out[o] = pn;
-      io.ppd_out[o] = pn + d1;
-      if (p.write_ppx) io.ppx[o] = d1;
-      if (k >= 2) io.w_out[o] = wk;
-      io.rrw[o] = p.last ? (ac + wk * alph) * p.tavg : ac + wk;
+      *G(io.pp_out, o) = pn;
+      *G(io.ppd_out, o) = pn + d1;
+      if (p.write_ppx) *G(io.ppx, o) = d1;
+      if (k >= 2) *G(io.w_out, o) = wk;
+      *G(io.rrw, o) = p.last ? (ac + wk * alph) * p.tavg : ac + wk;
     }
   }
 #undef S
@@ -451,10 +493,6 @@ __global__ void __launch_bounds__(TX * NW, CM1G_SND_MINB) k_sound_tile(DGrid g, 
 // The arithmetic and its order are those of the tile form.
 // ---------------------------------------------------------------------
 static const int SNC_TX = 32;
-// grids with at least this many columns (ni*nj) use the column-sweep form
-#ifndef CM1G_SOUND_COL_MIN_COLUMNS
-#define CM1G_SOUND_COL_MIN_COLUMNS (1L << 20)
-#endif
 
 template <int TX, int TY>
 __global__ void __launch_bounds__(TX * TY, 5) k_sound_col(DGrid g, SoundIO io, SoundStep p) {
@@ -690,29 +728,36 @@ void sound_nloop(int nsound, int nrk, float dt, int *nloop_out, float *dts_out) 
   *dts_out = dts;
 }
 
-size_t sound_smem_bytes(const DGrid &g) { return (size_t)5 * (g.nk + 2) * SND_TX * sizeof(float); }
-int sound_max_nk() { return SND_NW * SND_KPT; }
-// grids with more levels run the column sweep
-static bool sound_tall(const DGrid &g) { return g.nk > SND_NW * SND_KPT; }
+static size_t sound_smem_bytes(const DGrid &g) {
+  return (size_t)SND_NARR * (g.nk + 2) * SND_TX * sizeof(float) + (size_t)(g.nk + 1) * sizeof(SndLev);
+}
+int sound_max_nk() { return SND_MAXNK; }
+// the tile forms hold sound_max_nk() levels and index with 32-bit byte
+// offsets; other grids run the column sweep
+static bool sound_tall(const DGrid &g) { return g.nk > SND_MAXNK || nU(g) >= (1L << 30) || nV(g) >= (1L << 30); }
 
-// The acoustic kernel's forms (kNumSoundCfgs): the tile form with 8 or 4
-// warps over the levels of 32 columns, and the column sweep with 32 x 4 or
-// 32 x 2 columns per block.  Both tile forms cover SND_NW * SND_KPT levels.
-static_assert(SND_NW * SND_KPT == (SND_NW / 2) * (SND_KPT * 2), "both tile forms cover the same levels");
+// The tile form by size: 7 explicit warps (three blocks an SM) hold 84 levels,
+// 10 (two blocks an SM, as the longer columns' shared memory allows) hold 130;
+// when the grid has no more than one tile for each of the 148 SMs, 16 explicit
+// warps shorten the one wave.  Times of the final stage's substeps (6), one
+// B200: 256x256x80 0.85 ms (7 warps) against 0.89 (10) and 1.29 (16);
+// 512x512x128 5.16 ms (10); 64x64x40 0.104 ms (16) against 0.121 (7).
+typedef void (*SoundTileFn)(DGrid, SoundIO, SoundStep);
+struct SoundTile { SoundTileFn fn; int nw, kpt; };
+static const SoundTile kSoundTiles[3] = {
+    {k_sound_tile<7, 12, 3>, 7, 12}, {k_sound_tile<10, 13, 2>, 10, 13}, {k_sound_tile<16, 8, 1>, 16, 8}};
+static int sound_tile_of(const DGrid &g, int cfg) {
+  const long tiles = (long)((g.ni + SND_TX - 1) / SND_TX) * g.nj;
+  if (cfg == 1 || tiles <= 148) return 2;
+  return g.nk <= kSoundTiles[0].nw * kSoundTiles[0].kpt ? 0 : 1;
+}
 
 static void sound_set_attributes() {
   static bool done = false;
   if (done) return;
-  cudaFuncSetAttribute(k_sound_tile<SND_TX, SND_NW, SND_KPT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       200 * 1024);
+  for (const SoundTile &t : kSoundTiles)
+    cudaFuncSetAttribute(t.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024);
   cudaFuncSetAttribute(k_openbc_restrict, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  cudaFuncSetAttribute(k_sound_tile<SND_TX, SND_NW / 2, SND_KPT * 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       200 * 1024);
-  // three blocks of 5 column arrays each; the rest of the unified L1 stays
-  // cache for the neighbour reads of phase 1
-  cudaFuncSetAttribute(k_sound_tile<SND_TX, SND_NW, SND_KPT>, cudaFuncAttributePreferredSharedMemoryCarveout, 70);
-  cudaFuncSetAttribute(k_sound_tile<SND_TX, SND_NW / 2, SND_KPT * 2>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                       70);
   done = true;
 }
 
@@ -733,13 +778,12 @@ void launch_sound(const DGrid &g, int nsound, int nrk, float dt,
   int nloop;
   float dts;
   sound_nloop(nsound, nrk, dt, &nloop, &dts);
-  // The column-sweep form keeps one thread per column, so it needs many
-  // columns to fill the GPU; smaller grids use the tile form, whose warps
-  // split the levels of a column.  g.sound_cfg (set by the autotuner or
-  // cm1g_set_tune) overrides the choice, and CM1G_SOUND_FORM=col|tile
-  // (read at each call) overrides both.
+  // The tile form unless the column does not fit it (1024x1024x128: 20.4 ms
+  // for 6 substeps against 26.5 of the column sweep).  g.sound_cfg (set by
+  // the autotuner or cm1g_set_tune) overrides the choice, and
+  // CM1G_SOUND_FORM=col|tile (read at each call) overrides both.
   int cfg = g.sound_cfg;
-  if (cfg < 0 || cfg >= kNumSoundCfgs) cfg = ((long)g.ni * g.nj >= (long)CM1G_SOUND_COL_MIN_COLUMNS) ? 2 : 0;
+  if (cfg < 0 || cfg >= kNumSoundCfgs) cfg = 0;
   if (const char *f = getenv("CM1G_SOUND_FORM")) {
     if (!strcmp(f, "col")) cfg = 2;
     else if (!strcmp(f, "tile")) cfg = 0;
@@ -749,7 +793,9 @@ void launch_sound(const DGrid &g, int nsound, int nrk, float dt,
   if (tall && cfg < 2) cfg = 2;
   const bool restrict_open = g.roflux && ((g.wbc == 2 && g.ibw) || (g.ebc == 2 && g.ibe) ||
                                           (g.sbc == 2 && g.ibs) || (g.nbc == 2 && g.ibn));
-  const int cty = (cfg == 3) ? 2 : 4, nw = (cfg == 1) ? SND_NW / 2 : SND_NW;
+  const int cty = (cfg == 3) ? 2 : 4;
+  const SoundTile &T = kSoundTiles[sound_tile_of(g, cfg)];
+  const int nw = T.nw + 1;
   const bool col = cfg >= 2;
   dim3 blk = col ? dim3(SNC_TX, cty) : dim3(SND_TX, nw);
   dim3 grid = col ? dim3((g.ni + SNC_TX - 1) / SNC_TX, (g.nj + cty - 1) / cty)
@@ -787,10 +833,9 @@ void launch_sound(const DGrid &g, int nsound, int nrk, float dt,
     {
       ProfScope _ps("k_sound_step", st);
       switch (cfg) {
-        case 1: k_sound_tile<SND_TX, SND_NW / 2, SND_KPT * 2><<<grid, blk, smem, st>>>(g, io, sp); break;
         case 2: k_sound_col<SNC_TX, 4><<<grid, blk, 0, st>>>(g, io, sp); break;
         case 3: k_sound_col<SNC_TX, 2><<<grid, blk, 0, st>>>(g, io, sp); break;
-        default: k_sound_tile<SND_TX, SND_NW, SND_KPT><<<grid, blk, smem, st>>>(g, io, sp); break;
+        default: T.fn<<<grid, blk, smem, st>>>(g, io, sp); break;
       }
     }
     if (nl) *nl += 1;

@@ -528,9 +528,9 @@ int cm1g_pdefq_noalloc(const cm1g_config_t *cfg, float rmax, double *asq,
  * a tile, levels per block; the block has one more row of threads than the
  * tile has cell rows) and mom_shape those of the momentum pass
  * (cm1g_tile_shape: x and y threads of a block, levels per block);
- * sound_form selects the acoustic kernel: -1 automatic (by the number of
- * columns), 0 tile form with 8 warps over the levels of 32 columns, 1 the
- * same with 4 warps, 2 column sweep with 32 x 4 columns per block, 3 column
+ * sound_form selects the acoustic kernel: -1 automatic, 0 tile form of 32
+ * columns with the warps over the levels chosen by the grid's size, 1 the
+ * same with 16 of them, 2 column sweep with 32 x 4 columns per block, 3 column
  * sweep with 32 x 2.  step_ms is the measured large-step time of the
  * configuration (cm1g_autotune; 0 when not measured). */
 typedef struct cm1g_tune {
