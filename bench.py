@@ -67,8 +67,7 @@ def kernel_bytes_per_step(cfg):
     k_advs_tile_pdef1 + k_advs_pdef2: the final-stage positive-definite pass
     of one field, together the same 28 B (their six work arrays are scratch).
     k_sound_step: one acoustic small step, 23 floats (92 B) per cell.
-    k_advu/k_advv/k_advw: read u, v, w and the fixed tendency, write the
-    tendency (20 B each)."""
+    k_mom: read u, v, w and their fixed tendencies, write the tendencies (36 B)."""
     moist = cfg.imoist == 1
     nq = cfg.numq if moist else 0
     npt = cfg.npt if cfg.iptra else 0
@@ -81,7 +80,7 @@ def kernel_bytes_per_step(cfg):
             "k_advs_tile": 3 * (28 * nsc + tht) - 28 * pdef3,
             "k_advs_tile_pdef1": 20 * pdef3, "k_advs_pdef2": 8 * pdef3,
             "k_sound_step": 4 * ACOUSTIC_FLOATS_PER_CELL * S,
-            "k_advu": 3 * 20, "k_advv": 3 * 20, "k_advw": 3 * 20}
+            "k_mom": 3 * 36}
 
 
 def kernel_roofline(name, prof, bpc, cells, hbm, peak_kind, traffic_per_launch=None):

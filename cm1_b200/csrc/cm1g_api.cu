@@ -136,6 +136,30 @@ static int set_err(int code, const char *fmt, ...) {
   return code;
 }
 
+int cm1g::tile_levels(long tiles, int nk, int slots, int over, int kcmax) {
+  int best = 0;
+  long best_end = 0;
+  for (int kc = 4; kc <= kcmax; kc += kc < 16 ? 1 : kc < 32 ? 2 : 4) {
+    const int nch = (nk + kc - 1) / kc;
+    std::map<long, long> free_at{{0, slots}};   // end of the slots' last block -> slots
+    long end = 0;
+    for (int part = 0; part < 2; part++) {      // the full chunks, then the last one of every tile
+      const long len = over + (part ? nk - (nch - 1) * kc : kc);
+      for (long n = part ? tiles : tiles * (nch - 1); n > 0;) {
+        const auto it = free_at.begin();
+        const long t = it->first, m = std::min(n, it->second);
+        if ((it->second -= m) == 0) free_at.erase(it);
+        free_at[t + len] += m;
+        end = std::max(end, t + len);
+        n -= m;
+      }
+    }
+    if (!best || end < best_end) { best = kc; best_end = end; }
+    if (kc >= nk) break;
+  }
+  return best;
+}
+
 int cm1g::report_error(int code, const char *msg) { return set_err(code, "%s", msg); }
 
 #define CUCHK(x)                                                                                   \

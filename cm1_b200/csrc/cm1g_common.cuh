@@ -236,14 +236,10 @@ struct EnerIn {
   float lv1, ls1;
 };
 
-// Levels that a block of a marching tile kernel owns, given the tiles of a
-// level: as many as still leave two blocks for each of the 148 SMs twice over
-// (a block loads the level below its first one again), at least 8.
-inline int tile_levels(long tiles, int nk) {
-  int kc = nk;
-  while (kc > 8 && tiles * ((nk + kc - 1) / kc) < 4L * 148) kc = (kc + 1) / 2;
-  return kc < 8 ? 8 : kc;
-}
+// Levels that a block of a marching tile kernel owns, at most kcmax: the
+// choice whose blocks, handed to `slots` resident blocks in launch order,
+// finish first (a block costs its levels plus `over` for its first ones).
+int tile_levels(long tiles, int nk, int slots, int over, int kcmax);
 
 // Records a message for cm1g_last_error() and returns code (C++ linkage,
 // not part of the C-ABI).

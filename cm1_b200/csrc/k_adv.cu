@@ -1,11 +1,11 @@
 // k_adv.cu -- flux-form advection tendencies (adv.F, adv_routines.F).
 //
-// The production passes are k-marching tiles (k_mom_tile for u, v, w;
-// k_advs_tile for the scalars): each face flux is evaluated once, from a
-// level staged in shared memory with its 3-point halo, instead of being
-// stored in dumx/dumy/dumz; the rho0-weighted fluxes rru/rrv/rrw and their
-// divergence are formed on the fly, so a momentum pass reads u, v, w (and
-// theta/qv for buoyancy) and writes only the tendency.  The per-point
+// The production passes are k-marching tiles (k_mom for u, v, w, or
+// k_mom_tile with the 6th-order diffusion; k_advs_tile for the scalars): each
+// face flux is evaluated once, from a level staged in shared memory with its
+// 3-point halo, instead of being stored in dumx/dumy/dumz; the rho0-weighted
+// fluxes rru/rrv/rrw and their divergence are formed on the fly, so a momentum
+// pass reads u, v, w (and theta/qv for buoyancy) and writes only the tendency.  The per-point
 // scalar kernels (k_advs, k_advs_pdef1/2) serve the per-routine entry
 // cm1g_advs.  Every expression keeps the reference's operand order.
 #include "cm1g_common.cuh"
@@ -51,7 +51,8 @@ __device__ __forceinline__ float buoy_v(const DGrid &g, float th3, float qvv, bo
 
 
 // ---------------------------------------------------------------------
-// Tiled momentum advection (the production path of advu/advv/advw).
+// Tiled momentum advection with the 6th-order diffusion (one component a
+// launch; without it all three advance in k_mom below).
 //
 // divx of the momentum pass (solve2.F:590-596) is formed once per stage at
 // the s-points i = 0..ni+1, j = 0..nj+1 by k_mom_divx.  k_mom_tile then
@@ -127,7 +128,7 @@ __device__ __forceinline__ float hflux_mom(float r, const float *p, int stride) 
   return r * flx5(up ? a0 : a5, up ? a1 : a4, up ? a2 : a3, up ? a3 : a2, up ? a4 : a1);
 }
 
-template <int TX, int TY, int KC, int STAG, int DIFF>
+template <int TX, int TY, int KC, int STAG>
 __global__ void __launch_bounds__(TX * TY, 3) k_mom_tile(DGrid g, Vel q, const float *__restrict__ divx,
                                                       const float *ten1, float *ten,
                                                       const float *__restrict__ th3d, const float *__restrict__ qv,
@@ -305,7 +306,7 @@ __global__ void __launch_bounds__(TX * TY, 3) k_mom_tile(DGrid g, Vel q, const f
         if (STAG == 2) r = 0.5f * (r0k * p[2] + r0k * p[3]);
         fx[f] = hflux_mom(r, p, 1);
         fxv[f] = r;
-        if (DIFF) {
+        {
           // the face between p[2] and p[3]: s-point fxi (u: adv.F:1190-1193),
           // u-point fxi (v: adv.F:2128-2132; w: adv.F:3124-3130)
           const int ii = fxi[s], jj = fxj[s];
@@ -331,7 +332,7 @@ __global__ void __launch_bounds__(TX * TY, 3) k_mom_tile(DGrid g, Vel q, const f
         if (STAG == 3) r = 0.5f * (r0k * p[2 * SP] + r0k * p[3 * SP]);
         fy[fy_] = hflux_mom(r, p, SP);
         fyv[fy_] = r;
-        if (DIFF) {
+        {
           // the face between p[2 SP] and p[3 SP]: v-point fyj (u: adv.F:1210-1215;
           // w: adv.F:3146-3152), s-point fyj (v: adv.F:2151-2153)
           const int ii = fyi[s], jj = fyj[s];
@@ -421,7 +422,7 @@ __global__ void __launch_bounds__(TX * TY, 3) k_mom_tile(DGrid g, Vel q, const f
           advy = advy - ww * (c1k * (RRVk(nj + 1, k - 1) - RRVk(nj, k - 1)) + c2k * (RRVk(nj + 1, k) - RRVk(nj, k))) *
                             g.rdy * LDG(&g.vh[nj - g.jb]);
       }
-      if (DIFF) {   // adv.F:1199-1201, 1220-1222; 2139-2141, 2160-2162; 3135-3137, 3160-3162
+      {   // adv.F:1199-1201, 1220-1222; 2139-2141, 2160-2162; 3135-3137, 3160-3162
         const float ddx = df.coef * (dfx[xi + 1] - dfx[xi]), ddy = df.coef * (dfy[yi + TX] - dfy[yi]);
         if (STAG == 2) {
           const float rs = LDG(&df.rho[iS(g, i - 1, j, k)]) + LDG(&df.rho[iS(g, i, j, k)]);
@@ -465,6 +466,347 @@ __global__ void __launch_bounds__(TX * TY, 3) k_mom_tile(DGrid g, Vel q, const f
   }
 }
 
+// ---------------------------------------------------------------------
+// Momentum advection of all three components in one pass (advu, advv, advw).
+//
+// A block owns 31 x (TY-1) points and KC levels and marches upward.  u, v and
+// w of a level are staged once, with their 3-point halo, by asynchronous
+// copies into a ring of six levels (k-1, k, k+1 in use, three in flight) and
+// serve as the advected field of their own component and as the face
+// velocities and divergence of all three.  Thread (lane, row) evaluates, for
+// every component, the x face west of its point, the y face south of it and
+// the z face above it (hadv_flx5/vadv_flx5, stag=2/3/4): the east face comes
+// from the next lane by a shuffle, the north face from the next row through
+// shared memory, the lower face from the level below in registers; the last
+// lane and row only supply faces.  The face velocities are formed exactly as
+// the reference forms them (ubar/vbar/wbar of adv_routines.F:1388-1460,
+// 3299-3384), divx as solve2.F:590-596 does, and the open-boundary fixes of
+// adv.F are applied in the blocks that touch an open edge.
+//
+// Bound by instruction issue and latency: 890 warp instructions per 32 points
+// at 60 % issue, 36 % of the DRAM rate.  256x256x80: 0.230 ms against 0.370
+// for a divergence pass and one marching tile per component, which staged u, v
+// and w separately and read them again as face velocities; 64x64x40: 27 us
+// against 62.  Three blocks an SM at 72 registers spill and measured 4 to 14 %
+// slower than two at 96; 16 rows of threads 5 to 15 % slower than 9.
+// ---------------------------------------------------------------------
+// vertical profiles of one level
+struct MomLev { float rho0, c1, c2, rf0, mh, rr0, rrf0, mf; };
+constexpr int MOM_TY = 9;          // rows of threads
+constexpr int MOM_KC = 64;         // levels of a block at most
+
+struct MomIO {
+  const float *uten1, *vten1, *wten1;
+  float *uten, *vten, *wten;
+  const float *th3d, *qv, *b8;     // buoyancy of w: theta and qv, or the array of the stage set-up, or none
+};
+
+__device__ __forceinline__ void cp_async4(void *dst, const float *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+
+template <int WHICH>
+__global__ void __launch_bounds__(32 * MOM_TY, 2) k_mom(DGrid g, Vel q, MomIO io, int kc) {
+  constexpr int TY = MOM_TY;
+  constexpr int NT = 32 * TY;
+  constexpr int SW = 38, SH = TY + 6, SP = 40;             // staged columns, rows and pitch
+  constexpr int NST = (SW * SH + NT - 1) / NT;
+  constexpr int PLANE = SH * SP;
+  constexpr bool DU = (WHICH & 1) != 0, DV = (WHICH & 2) != 0, DW = (WHICH & 4) != 0;
+  constexpr int RD = 6;
+  __shared__ float ring[RD][3][PLANE];
+  __shared__ float fyu[TY][32], fyv[TY][32], fyw[TY][32];
+  extern __shared__ float4 mom_lev[];    // levels kc0-1 .. kc1+1
+  const int lane = threadIdx.x, row = threadIdx.y, tid = lane + 32 * row;
+  const int i0 = 1 + (int)blockIdx.x * 31, j0 = 1 + (int)blockIdx.y * (TY - 1);
+  const int i = i0 + lane, j = j0 + row;
+  const int ni = g.ni, nj = g.nj, nk = g.nk, NI = g.NI;
+  const int plS = NI * g.NJ, plU = (NI + 1) * g.NJ, plV = NI * (g.NJ + 1);   // < 2^31 points (cm1g_init)
+  const bool in = i <= ni + 2 && j <= nj + 2;              // the last u and v points need the face beyond them
+  const bool own = i <= ni + 1 && j <= nj + 1 && lane < 31 && row < TY - 1;
+  const bool own_u = DU && own && i >= (g.ibw ? 2 : 1) && i <= (g.ibe ? ni : ni + 1) && j <= nj;
+  const bool own_v = DV && own && j >= (g.ibs ? 2 : 1) && j <= (g.ibn ? nj : nj + 1) && i <= ni;
+  const bool own_w = DW && own && i <= ni && j <= nj;
+  const bool doitw = g.wbc == 2 && g.ibw, doite = g.ebc == 2 && g.ibe;
+  const bool doits = g.sbc == 2 && g.ibs, doitn = g.nbc == 2 && g.ibn;
+  const bool edge = (doitw && i0 == 1) || (doite && i0 + 31 >= ni) || (doits && j0 == 1) || (doitn && j0 + TY - 1 >= nj);
+  const int oc = in ? (i - g.ib) + NI * (j - g.jb) : 0, ocu = in ? (i - g.ib) + (NI + 1) * (j - g.jb) : 0;
+  const int kc0 = 1 + (int)blockIdx.z * kc, kc1 = min(nk, kc0 + kc - 1);
+  const float rdx = g.rdx, rdy = g.rdy, rdz = g.rdz, smeps = g.smeps;
+  float uh = 0, uhw = 0, vh = 0, vhs = 0, uf = 0, vf = 0;
+  if (in) {
+    uh = LDG(&g.uh[i - g.ib]); uhw = LDG(&g.uh[i - 1 - g.ib]); uf = LDG(&g.uf[i - g.ib]);
+    vh = LDG(&g.vh[j - g.jb]); vhs = LDG(&g.vh[j - 1 - g.jb]); vf = LDG(&g.vf[j - g.jb]);
+  }
+
+  MomLev *LV = reinterpret_cast<MomLev *>(mom_lev) - (kc0 - 1);
+  for (int k = kc0 - 1 + tid; k <= kc1 + 1; k += NT) {
+    LV[k] = MomLev{LDG(&g.rho0[k]), LDG(&g.c1[k]), LDG(&g.c2[k]), LDG(&g.rf0[k]), LDG(&g.mh[k]), LDG(&g.rr0[k]),
+                   LDG(&g.rrf0[k]), LDG(&g.mf[k])};
+  }
+
+  // ---- staging
+  int so[NST], sd[NST];            // in-plane source offset of an s-shaped plane (-1: none), slot
+  unsigned sm = 0;                 // bit s: row exists in u and w; bit 8+s: in v; the u offset is so + (jj - jb)
+  int sr[NST];
+#pragma unroll
+  for (int s = 0; s < NST; s++) {
+    const int t = tid + s * NT;
+    so[s] = 0; sd[s] = 0; sr[s] = 0;
+    if (t < SW * SH) {
+      const int yy = t / SW, xx = t - yy * SW;
+      const int ii = i0 - 3 + xx, jj = j0 - 3 + yy;
+      sd[s] = yy * SP + xx;
+      so[s] = (ii - g.ib) + NI * (jj - g.jb);
+      sr[s] = jj - g.jb;
+      if (ii <= ni + g.ngxy + 1 && jj <= nj + g.ngxy) sm |= 1u << s;                   // u
+      if (ii <= ni + g.ngxy && jj <= nj + g.ngxy + 1) sm |= 0x100u << s;               // v
+      if (ii <= ni + g.ngxy && jj <= nj + g.ngxy) sm |= 0x10000u << s;                 // w
+    }
+  }
+  int slot = 0, lev = kc0 - 1;     // next slot and level to stage
+  auto issue = [&]() {
+    float *d = &ring[slot][0][0];
+    const int k = lev++;
+    slot = slot + 1 == RD ? 0 : slot + 1;
+#pragma unroll
+    for (int s = 0; s < NST && k <= kc1 + 1; s++) {
+      if (sm & (1u << s)) cp_async4(d + sd[s], q.u + (k * plU + so[s] + sr[s]));
+      if (sm & (0x100u << s)) cp_async4(d + PLANE + sd[s], q.v + (k * plV + so[s]));
+      if (sm & (0x10000u << s)) cp_async4(d + 2 * PLANE + sd[s], q.w + (k * plS + so[s]));
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int d = 0; d < RD - 1; d++) issue();
+
+  // ---- column windows: a(k-2 .. k+3) of each component
+  auto AU = [&](int kk) -> float { return (kk >= 0 && kk <= nk + 1) ? LDG(&q.u[kk * plU + ocu]) : 0.0f; };
+  auto AV = [&](int kk) -> float { return (kk >= 0 && kk <= nk + 1) ? LDG(&q.v[kk * plV + oc]) : 0.0f; };
+  auto AW = [&](int kk) -> float { return (kk >= 0 && kk <= nk + 2) ? LDG(&q.w[kk * plS + oc]) : 0.0f; };
+  // rf0-weighted w of a neighbour column (offset d) at w-level kk (solve2.F:509-516)
+  auto RWg = [&](int kk, float rf, float w) -> float { return (kk <= 1 || kk >= nk + 1) ? 0.0f : rf * w; };
+  auto RW = [&](int kk, float w) -> float { return RWg(kk, LDG(&g.rf0[kk]), w); };
+  float uw[6], vw[6], ww[6];
+  float fzu = 0.0f, fzv = 0.0f, fzw = 0.0f, divm = 0.0f;
+#pragma unroll
+  for (int d = 0; d < 6; d++) { uw[d] = vw[d] = ww[d] = 0.0f; }
+  if (own) {
+#pragma unroll
+    for (int d = 0; d < 6; d++) {
+      if (DU) uw[d] = AU(kc0 - 2 + d);
+      if (DV) vw[d] = AV(kc0 - 2 + d);
+      if (DW) ww[d] = AW(kc0 - 2 + d);
+    }
+    if (kc0 >= 2) {                 // the faces below level kc0
+      const float rc = RW(kc0, LDG(&q.w[kc0 * plS + oc]));
+      float z[6];
+      if (DU) {
+        z[0] = AU(kc0 - 3);
+#pragma unroll
+        for (int d = 0; d < 5; d++) z[d + 1] = uw[d];
+        fzu = zflux_uv(g, z, 0.5f * (rc + RW(kc0, LDG(&q.w[kc0 * plS + oc - 1]))), kc0);
+      }
+      if (DV) {
+        z[0] = AV(kc0 - 3);
+#pragma unroll
+        for (int d = 0; d < 5; d++) z[d + 1] = vw[d];
+        fzv = zflux_uv(g, z, 0.5f * (rc + RW(kc0, LDG(&q.w[kc0 * plS + oc - NI]))), kc0);
+      }
+      if (DW) {
+        z[0] = AW(kc0 - 3);
+#pragma unroll
+        for (int d = 0; d < 5; d++) z[d + 1] = ww[d];
+        fzw = zflux_w(g, z, 0.5f * (RW(kc0 - 1, LDG(&q.w[(kc0 - 1) * plS + oc])) + rc), kc0 - 1);
+      }
+    }
+  }
+  // buoyancy of a level: from its theta and qv, or as the stage set-up left it
+  auto buoy = [&](float t, float q, int k) -> float {
+    return io.b8 ? t : io.th3d ? buoy_v(g, t, q, io.qv != nullptr, k) : 0.0f;
+  };
+  float bu0 = 0.0f;                // of level k-1
+  if (own_w && kc0 >= 2) {
+    const int o = (kc0 - 1) * plS + oc;
+    float t = 0.0f, qq = 0.0f;
+    if (io.b8) t = LDG(&io.b8[o]);
+    else if (io.th3d) { t = LDG(&io.th3d[o]); if (io.qv) qq = LDG(&io.qv[o]); }
+    bu0 = buoy(t, qq, kc0 - 1);
+  }
+  const int pc = (row + 3) * SP + lane + 3;                // the point in a staged plane
+  // rho0-weighted velocities of a staged level (solve2.F:499-516) and divx (solve2.F:590-596)
+  auto DIV = [&](const float *P, const float *Pup, int k, const MomLev &lv, float rfu, int d, float uhd, float vhd) -> float {
+    const float r0 = lv.rho0;
+    const float *u = P + pc + d, *v = P + PLANE + pc + d;
+    float x = ((r0 * u[1] - r0 * u[0]) * rdx * uhd + (r0 * v[SP] - r0 * v[0]) * rdy * vhd) +
+              (RWg(k + 1, rfu, Pup[2 * PLANE + pc + d]) - RWg(k, lv.rf0, P[2 * PLANE + pc + d])) * rdz * lv.mh;
+    if (fabsf(x) < smeps) x = 0.0f;
+    return x;
+  };
+
+  int sl = 0;                      // slot of level k-1
+  for (int k = kc0; k <= kc1; k++) {
+    // this level's own inputs and the next tops of the column windows
+    float t1u = 0, t1v = 0, t1w = 0, nu = 0, nv = 0, nw = 0, tb1 = 0, tq1 = 0;
+    const int ou = k * plU + ocu, ov = k * plV + oc, ow = k * plS + oc;
+    if (own_u) t1u = io.uten1[ou];
+    if (own_v) t1v = io.vten1[ov];
+    if (own_w) {
+      t1w = k >= 2 ? io.wten1[ow] : 0.0f;
+      if (io.b8) tb1 = LDG(&io.b8[ow]);
+      else if (io.th3d) { tb1 = LDG(&io.th3d[ow]); if (io.qv) tq1 = LDG(&io.qv[ow]); }
+    }
+    if (own) {
+      if (DU) nu = AU(k + 4);
+      if (DV) nv = AV(k + 4);
+      if (DW) nw = AW(k + 4);
+    }
+    if (own && k + 3 <= kc1) {      // levels ahead towards L2
+      if (own_u) prefetch_l2(&io.uten1[ou + 3 * plU]);
+      if (own_v) prefetch_l2(&io.vten1[ov + 3 * plV]);
+      if (own_w) {
+        prefetch_l2(&io.wten1[ow + 3 * plS]);
+        if (io.b8) prefetch_l2(&io.b8[ow + 3 * plS]);
+        else if (io.th3d) { prefetch_l2(&io.th3d[ow + 3 * plS]); if (io.qv) prefetch_l2(&io.qv[ow + 3 * plS]); }
+      }
+    }
+    // groups are committed one a level, up to k+3 here: level k+1 has landed
+    asm volatile("cp.async.wait_group %0;" ::"n"(RD - 4) : "memory");
+    __syncthreads();
+    issue();                       // level k+4 into the slot of level k-2
+    const int s0 = sl + 1 >= RD ? sl + 1 - RD : sl + 1, s1 = s0 + 1 == RD ? 0 : s0 + 1;
+    const float *Pm = &ring[sl][0][0], *P = &ring[s0][0][0], *Pp = &ring[s1][0][0];
+    sl = s0;
+    const MomLev lv = LV[k];
+    const float r0k = lv.rho0, r0m = LV[k - 1].rho0, rfu = LV[k + 1].rf0, c1k = lv.c1, c2k = lv.c2;
+    const float cc2 = 0.5f * (c2k + c2k), cc1 = 1.0f - cc2;
+    float fxu = 0, fxv = 0, fxw = 0, fyu0 = 0, fyv0 = 0, fyw0 = 0, rxw = 0, ryw = 0;
+    const float *pu = P + pc, *pv = P + PLANE + pc, *pw = P + 2 * PLANE + pc;
+    if (in) {
+      if (DU) {
+        fxu = hflux_mom(0.5f * (r0k * pu[-1] + r0k * pu[0]), pu - 3, 1);
+        fyu0 = hflux_mom(0.5f * (r0k * pv[0] + r0k * pv[-1]), pu - 3 * SP, SP);
+      }
+      if (DV) {
+        fxv = hflux_mom(0.5f * (r0k * pu[0] + r0k * pu[-SP]), pv - 3, 1);
+        fyv0 = hflux_mom(0.5f * (r0k * pv[-SP] + r0k * pv[0]), pv - 3 * SP, SP);
+      }
+      if (DW && k >= 2) {
+        rxw = cc2 * (r0k * pu[0]) + cc1 * (r0m * Pm[pc]);
+        ryw = cc2 * (r0k * pv[0]) + cc1 * (r0m * Pm[PLANE + pc]);
+        fxw = hflux_mom(rxw, pw - 3, 1);
+        fyw0 = hflux_mom(ryw, pw - 3 * SP, SP);
+      }
+    }
+    if (DU) fyu[row][lane] = fyu0;
+    if (DV) fyv[row][lane] = fyv0;
+    if (DW) fyw[row][lane] = fyw0;
+    float fxu1 = 0, fxv1 = 0, fxw1 = 0;
+    if (DU) fxu1 = __shfl_down_sync(0xffffffffu, fxu, 1);
+    if (DV) fxv1 = __shfl_down_sync(0xffffffffu, fxv, 1);
+    if (DW) fxw1 = __shfl_down_sync(0xffffffffu, fxw, 1);
+    float hzu = 0, hzv = 0, hzw = 0, div0 = 0, divx = 0, divy = 0;
+    if (own) {
+      // the faces above: w-level k+1 for u and v, s-level k for w
+      const float *wu = Pp + 2 * PLANE + pc;
+      const float rc = RWg(k + 1, rfu, wu[0]);
+      if (k + 1 <= nk) {
+        if (DU) hzu = zflux_uv(g, uw, 0.5f * (rc + RWg(k + 1, rfu, wu[-1])), k + 1);
+        if (DV) hzv = zflux_uv(g, vw, 0.5f * (rc + RWg(k + 1, rfu, wu[-SP])), k + 1);
+      }
+      if (DW) hzw = zflux_w(g, ww, 0.5f * (RWg(k, lv.rf0, pw[0]) + rc), k);
+      if (DW && k == kc0 && k >= 2) divm = DIV(Pm, P, k - 1, LV[k - 1], lv.rf0, 0, uh, vh);
+      div0 = DIV(P, Pp, k, lv, rfu, 0, uh, vh);
+      if (DU) divx = DIV(P, Pp, k, lv, rfu, -1, uhw, vh);
+      if (DV) divy = DIV(P, Pp, k, lv, rfu, -SP, uh, vhs);
+    }
+    __syncthreads();
+    if (own_u) {
+      const float ac = pu[0];
+      float fy0 = fyu0, fyp = fyu[row + 1][lane];
+      float advx = -(fxu1 - fxu) * rdx * uf, advy;
+      if (!edge) {
+        advy = -(fyp - fy0) * rdy * vh;
+      } else {
+        const bool fs = doits && j == 1 && (r0k * pv[0] + r0k * pv[-1]) >= 0.0f;
+        const bool fn = doitn && j == nj && (r0k * pv[SP] + r0k * pv[SP - 1]) <= 0.0f;
+        if (fs) fy0 = fyp;
+        if (fn) fyp = fy0;
+        advy = -(fyp - fy0) * rdy * vh;
+        const float dd = ((r0k * pv[SP - 1] - r0k * pv[-1]) + (r0k * pv[SP] - r0k * pv[0]));
+        if (fs) advy = advy - ac * 0.5f * dd * rdy * vh;
+        if (fn) advy = advy - ac * 0.5f * dd * rdy * vh;
+      }
+      const float mhk = lv.mh;
+      float advz;
+      if (k == 1) advz = -hzu * rdz * mhk;
+      else if (k == nk) advz = +fzu * rdz * mhk;
+      else advz = -(hzu - fzu) * rdz * mhk;
+      io.uten[ou] = t1u + (((advx + advy) + advz) + ac * 0.5f * (div0 + divx)) * lv.rr0;
+    }
+    if (own_v) {
+      const float ac = pv[0];
+      float fx0 = fxv, fxp = fxv1;
+      float advx;
+      const float advy = -(fyv[row + 1][lane] - fyv0) * rdy * vf;
+      if (!edge) {
+        advx = -(fxp - fx0) * rdx * uh;
+      } else {
+        const bool fw = doitw && i == 1 && (r0k * pu[0] + r0k * pu[-SP]) >= 0.0f;
+        const bool fe = doite && i == ni && (r0k * pu[1] + r0k * pu[1 - SP]) <= 0.0f;
+        if (fw) fx0 = fxp;
+        if (fe) fxp = fx0;
+        advx = -(fxp - fx0) * rdx * uh;
+        const float dd = ((r0k * pu[1 - SP] - r0k * pu[-SP]) + (r0k * pu[1] - r0k * pu[0]));
+        if (fw) advx = advx - ac * 0.5f * dd * rdx * uh;
+        if (fe) advx = advx - ac * 0.5f * dd * rdx * uh;
+      }
+      const float mhk = lv.mh;
+      float advz;
+      if (k == 1) advz = -hzv * rdz * mhk;
+      else if (k == nk) advz = +fzv * rdz * mhk;
+      else advz = -(hzv - fzv) * rdz * mhk;
+      io.vten[ov] = t1v + (((advx + advy) + advz) + ac * 0.5f * (div0 + divy)) * lv.rr0;
+    }
+    const float bu1 = own_w ? buoy(tb1, tq1, k) : 0.0f;
+    if (own_w && k >= 2) {
+      const float ac = pw[0];
+      float fx0 = fxw, fxp = fxw1, fy0 = fyw0, fyp = fyw[row + 1][lane];
+      float advx, advy;
+      if (!edge) {
+        advx = -(fxp - fx0) * rdx * uh;
+        advy = -(fyp - fy0) * rdy * vh;
+      } else {
+        const float *mu = Pm + pc, *mv = Pm + PLANE + pc;
+        const float rxe = cc2 * (r0k * pu[1]) + cc1 * (r0m * mu[1]), ryn = cc2 * (r0k * pv[SP]) + cc1 * (r0m * mv[SP]);
+        const bool fw = doitw && i == 1 && rxw >= 0.0f, fe = doite && i == ni && rxe <= 0.0f;
+        const bool fs = doits && j == 1 && ryw >= 0.0f, fn = doitn && j == nj && ryn <= 0.0f;
+        if (fw) fx0 = fxp;
+        if (fe) fxp = fx0;
+        if (fs) fy0 = fyp;
+        if (fn) fyp = fy0;
+        advx = -(fxp - fx0) * rdx * uh;
+        advy = -(fyp - fy0) * rdy * vh;
+        const float dx = c1k * (r0m * mu[1] - r0m * mu[0]) + c2k * (r0k * pu[1] - r0k * pu[0]);
+        const float dy = c1k * (r0m * mv[SP] - r0m * mv[0]) + c2k * (r0k * pv[SP] - r0k * pv[0]);
+        if (fw) advx = advx - ac * dx * rdx * uh;
+        if (fe) advx = advx - ac * dx * rdx * uh;
+        if (fs) advy = advy - ac * dy * rdy * vh;
+        if (fn) advy = advy - ac * dy * rdy * vh;
+      }
+      const float advz = -(hzw - fzw) * rdz * lv.mf;
+      float t = t1w + (((advx + advy) + advz) + ac * (c2k * div0 + c1k * divm)) * lv.rrf0;
+      if (io.b8 || io.th3d) t = t + (c1k * bu0 + c2k * bu1);
+      io.wten[ow] = t;
+    }
+#pragma unroll
+    for (int d = 0; d < 5; d++) { uw[d] = uw[d + 1]; vw[d] = vw[d + 1]; ww[d] = ww[d + 1]; }
+    uw[5] = nu; vw[5] = nv; ww[5] = nw;
+    fzu = hzu; fzv = hzv; fzw = hzw;
+    divm = div0; bu0 = bu1;
+  }
+}
+
 template <int TX, int TY, int KC>
 static void mom_tiles_shape(const DGrid &g, const Vel &q, const float *uten1, const float *vten1,
                             const float *wten1, float *uten, float *vten, float *wten, const float *th3d,
@@ -475,20 +817,17 @@ static void mom_tiles_shape(const DGrid &g, const Vel &q, const float *uten1, co
   if (which & 1) {
     dim3 grid((g.ni + 1 + TX - 1) / TX, (g.nj + TY - 1) / TY, kch);
     ProfScope _ps("k_advu", st);
-    if (df.rho) k_mom_tile<TX, TY, KC, 2, 1><<<grid, blk, 0, st>>>(g, q, divx, uten1, uten, nullptr, nullptr, nullptr, df);
-    else k_mom_tile<TX, TY, KC, 2, 0><<<grid, blk, 0, st>>>(g, q, divx, uten1, uten, nullptr, nullptr, nullptr, df);
+    k_mom_tile<TX, TY, KC, 2><<<grid, blk, 0, st>>>(g, q, divx, uten1, uten, nullptr, nullptr, nullptr, df);
   }
   if (which & 2) {
     dim3 grid((g.ni + TX - 1) / TX, (g.nj + 1 + TY - 1) / TY, kch);
     ProfScope _ps("k_advv", st);
-    if (df.rho) k_mom_tile<TX, TY, KC, 3, 1><<<grid, blk, 0, st>>>(g, q, divx, vten1, vten, nullptr, nullptr, nullptr, df);
-    else k_mom_tile<TX, TY, KC, 3, 0><<<grid, blk, 0, st>>>(g, q, divx, vten1, vten, nullptr, nullptr, nullptr, df);
+    k_mom_tile<TX, TY, KC, 3><<<grid, blk, 0, st>>>(g, q, divx, vten1, vten, nullptr, nullptr, nullptr, df);
   }
   if (which & 4) {
     dim3 grid((g.ni + TX - 1) / TX, (g.nj + TY - 1) / TY, kchw);
     ProfScope _ps("k_advw", st);
-    if (df.rho) k_mom_tile<TX, TY, KC, 4, 1><<<grid, blk, 0, st>>>(g, q, divx, wten1, wten, th3d, qv, b8, df);
-    else k_mom_tile<TX, TY, KC, 4, 0><<<grid, blk, 0, st>>>(g, q, divx, wten1, wten, th3d, qv, b8, df);
+    k_mom_tile<TX, TY, KC, 4><<<grid, blk, 0, st>>>(g, q, divx, wten1, wten, th3d, qv, b8, df);
   }
 }
 
@@ -499,7 +838,25 @@ void launch_adv_momentum(const DGrid &g, const float *u, const float *v, const f
                          int which) {
   // which: bit 0 u (advu), bit 1 v (advv), bit 2 w (advw)
   Vel q{u, v, w};
-  const Diff6 df = diff ? *diff : Diff6{};
+  if (!diff) {
+    const MomIO io{uten1, vten1, wten1, uten, vten, wten, th3d, qv, b8};
+    ProfScope _ps("k_mom", st);
+    // launch shape 0: the levels that end first; the other shapes: their table's levels
+    const long tiles = (long)((g.ni + 31) / 31) * ((g.nj + MOM_TY - 1) / (MOM_TY - 1));
+    int kc = g.tile_mom > 0 ? kTileShapes[g.tile_mom][2] : tile_levels(tiles, g.nk, 2 * 148, 3, MOM_KC);
+    if (kc > MOM_KC) kc = MOM_KC;
+    const size_t sm = (size_t)(kc + 2) * sizeof(MomLev);
+    dim3 blk(32, MOM_TY), grid((g.ni + 31) / 31, (g.nj + MOM_TY - 1) / (MOM_TY - 1), (g.nk + kc - 1) / kc);
+    switch (which) {
+      case 1: k_mom<1><<<grid, blk, sm, st>>>(g, q, io, kc); break;
+      case 2: k_mom<2><<<grid, blk, sm, st>>>(g, q, io, kc); break;
+      case 4: k_mom<4><<<grid, blk, sm, st>>>(g, q, io, kc); break;
+      default: k_mom<7><<<grid, blk, sm, st>>>(g, q, io, kc); break;
+    }
+    if (nl) *nl += 1;
+    return;
+  }
+  const Diff6 df = *diff;
   {
     dim3 grid((g.ni + 2 + 127) / 128, g.nj + 2, g.nk);
     ProfScope _ps("k_mom_divx", st);
