@@ -234,7 +234,7 @@ struct cm1g_ctx {
   double *mp_qbud = nullptr;                  // qbudget(1..7) and asq(1..3), accumulated on the device
   int *mp_err = nullptr;
   float *d2s = nullptr;                       // scratch of the 2nd-order diffusion (cm1g_diff2)
-  float *les = nullptr;                       // scratch of the Smagorinsky LES tendencies (cm1g_turbsmag)
+  float *les = nullptr;                       // eddy viscosities of cm1g_turbsmag when the caller gives no arrays
 };
 
 // Makes the context's profile (if any) the active one for the calling thread.
@@ -2337,7 +2337,7 @@ extern "C" int cm1g_turbsmag(cm1g_ctx_t *c, float csm, int32_t tconfig, int32_t 
   if (thten1 && npt && (!pta || !ptten)) return set_err(CM1G_ERR_ARG, "turbsmag with tracers needs pta/ptten");
   const size_t ns = nS(g), nw = nW(g);
   if (!c->les) {
-    c->les = (float *)dalloc(c, (6 * ns + 6 * nw) * sizeof(float));
+    c->les = (float *)dalloc(c, 2 * nw * sizeof(float));
     if (!c->les) return set_err(CM1G_ERR_NOMEM, "turbsmag scratch");
   }
   ProfActive pa(c);
@@ -2352,16 +2352,13 @@ extern "C" int cm1g_turbsmag(cm1g_ctx_t *c, float csm, int32_t tconfig, int32_t 
   a.rho = S.in(rho, ns, false); a.tha = S.in(tha, ns, false);
   a.uten = S.in(uten1, nU(g), true); a.vten = S.in(vten1, nV(g), true); a.wten = S.in(wten1, nW(g), true);
   if (thten1) {
-    a.thten = S.in(thten1, ns, true);
-    a.numq = 0;
-    a.npt = npt;
-    a.pta = npt ? S.in(pta, npt * ns, false) : nullptr;
-    a.ptten = npt ? S.in(ptten, npt * ns, true) : nullptr;
+    a.s[0] = a.tha; a.sten[0] = S.in(thten1, ns, true);
+    a.nsc = 1;
+    const float *dp = npt ? S.in(pta, npt * ns, false) : nullptr;
+    float *dpt = npt ? S.in(ptten, npt * ns, true) : nullptr;
+    for (int n = 0; n < npt; n++) { a.s[a.nsc] = dp + n * ns; a.sten[a.nsc++] = dpt + n * ns; }
   }
   float *p = c->les;
-  a.t11 = p; p += ns; a.t22 = p; p += ns; a.t33 = p; p += ns; a.t12 = p; p += ns;
-  a.cx = p; p += ns; a.cy = p; p += ns;
-  a.s13 = p; p += nw; a.s23 = p; p += nw; a.t13 = p; p += nw; a.t23 = p; p += nw;
   a.kmh = kmh ? S.in(kmh, nw, true) : p; p += nw;
   a.kmv = kmv ? S.in(kmv, nw, true) : p;
   if (S.err) return set_err(CM1G_ERR_NOMEM, "staging alloc");

@@ -11,11 +11,23 @@
 //             uten1, vten1, wten1, thten1, qten, ptten (turbtend.F:18-692,
 //             1052-1424, 1816-2180, 2473-2885; solve1.F:1113-1240)
 //
-// Four launches: k_les_strain (rho*S_ij at every point), k_les_km (N^2, the
-// deformations and kmh/kmv, the halo ring evaluated at its periodic image),
-// k_les_stress (t_ij in place; t13/t23 with the bottom and top rows; the
-// scalar fluxes' face coefficients, shared by every scalar) and
-// k_les_tend (momentum and all scalars, blockIdx.z over levels and fields).
+// Two launches, both tiles of columns that march upward with the values of
+// the level below in registers:
+//   k_les_km    the strains, N^2 and the deformations of a w-level, and from
+//               them kmh and kmv (the halo ring is written from its periodic
+//               image, which equals bcw's copy)
+//   k_les_tend  the strains again, the stresses t_ij, the scalar fluxes' face
+//               coefficients, and every tendency
+// The strains and stresses live in registers, warp shuffles (x neighbours)
+// and a few shared rows (y neighbours) only: forming the strain twice costs
+// about 60 binary32 operations a point, storing and re-reading the twelve
+// strain, stress and coefficient arrays cost 48 to 100 bytes a point.
+// Bound by instruction issue (62 to 73 % of the cycles; 558 and 890 warp
+// instructions per 32 points), at 42 to 50 % of the DRAM rate.  256x256x128
+// with theta and two tracers: 0.583 ms a call against 1.33 for the four
+// point-parallel passes before.  With every neighbour loaded instead of
+// shuffled the two passes took 0.81 ms, and without reading a level's
+// tendencies ahead of its stores (which may alias for the compiler) 1.03 ms.
 // Binary32 in the Fortran's evaluation order (--fmad=false); the logarithm
 // of calcnm and the cube root of tconfig=1 are evaluated in binary64 and
 // rounded once.
@@ -24,263 +36,340 @@
 
 namespace cm1g {
 
-// w-level density rf (solve3.F:660-678)
-__device__ __forceinline__ float les_rf(const DGrid &g, const TurbArgs &a, int i, int j, int k) {
-  const long pl = (long)g.NI * g.NJ;
-  const long o = iS(g, i, j, k);
-  if (k == 1) return a.cgs1 * a.rho[o] + a.cgs2 * a.rho[o + pl] + a.cgs3 * a.rho[o + 2 * pl];
-  if (k == g.nk + 1) return a.cgt1 * a.rho[o - pl] + a.cgt2 * a.rho[o - 2 * pl] + a.cgt3 * a.rho[o - 3 * pl];
-  return LDG(&g.c1[k]) * a.rho[o - pl] + LDG(&g.c2[k]) * a.rho[o];
-}
-
-// calcdef, Cartesian without terrain (turb.F:4772-4790, 4880-4893)
-__global__ void k_les_strain(DGrid g, TurbArgs a) {
-  const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);   // 0 .. ni+1
-  const int j = (int)blockIdx.y;                                // 0 .. nj+1
-  const int k = 1 + (int)blockIdx.z;                            // 1 .. nk
-  if (i > g.ni + 1) return;
-  const float rdx = g.rdx, rdy = g.rdy, rdz = g.rdz;
-  const float *rho = a.rho, *ua = a.ua, *va = a.va, *wa = a.wa;
-  const long o = iS(g, i, j, k);
-  const float uh = LDG(&g.uh[i - g.ib]), vh = LDG(&g.vh[j - g.jb]);
-  const float uf = LDG(&g.uf[i - g.ib]), vf = LDG(&g.vf[j - g.jb]);
-  const float temz = rdz * LDG(&g.mh[k]);
-  a.t11[o] = rho[o] * (ua[iU(g, i + 1, j, k)] - ua[iU(g, i, j, k)]) * rdx * uh;
-  a.t22[o] = rho[o] * (va[iV(g, i, j + 1, k)] - va[iV(g, i, j, k)]) * rdy * vh;
-  a.t33[o] = rho[o] * (wa[iW(g, i, j, k + 1)] - wa[iW(g, i, j, k)]) * temz;
-  a.t12[o] = 0.5f * ((ua[iU(g, i, j, k)] - ua[iU(g, i, j - 1, k)]) * rdy * vf +
-                     (va[iV(g, i, j, k)] - va[iV(g, i - 1, j, k)]) * rdx * uf) * 0.25f *
-             ((rho[iS(g, i - 1, j - 1, k)] + rho[o]) + (rho[iS(g, i - 1, j, k)] + rho[iS(g, i, j - 1, k)]));
-  if (k >= 2 && i >= 1 && j >= 1) {
-    const float mfk = LDG(&g.mf[k]);
-    a.s13[o] = 0.5f * ((wa[iW(g, i, j, k)] - wa[iW(g, i - 1, j, k)]) * rdx * uf +
-                       (ua[iU(g, i, j, k)] - ua[iU(g, i, j, k - 1)]) * rdz * 0.5f * (mfk + mfk)) *
-               0.5f * (les_rf(g, a, i - 1, j, k) + les_rf(g, a, i, j, k));
-    a.s23[o] = 0.5f * ((wa[iW(g, i, j, k)] - wa[iW(g, i, j - 1, k)]) * rdy * vf +
-                       (va[iV(g, i, j, k)] - va[iV(g, i, j, k - 1)]) * rdz * 0.5f * (mfk + mfk)) *
-               0.5f * (les_rf(g, a, i, j - 1, k) + les_rf(g, a, i, j, k));
-  }
-}
-
 __device__ __forceinline__ float sq(float x) { return x * x; }
 
-// calcnm (dry), the deformations of calcdef (turb.F:5366-5390) and kmh/kmv
-// of turbsmag; (i, j) on the halo ring takes the value of its periodic image
-// (bcw), and the bottom and top rows are zero (bcw flag 1, bc.F:1126-1137).
-__global__ void k_les_km(DGrid g, TurbArgs a) {
-  const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);   // 0 .. ni+1
-  const int j = (int)blockIdx.y;                                // 0 .. nj+1
-  const int k = 1 + (int)blockIdx.z;                            // 1 .. nk+1
-  if (i > g.ni + 1) return;
-  const long od = iS(g, i, j, k);
-  if (k == 1 || k == g.nk + 1) { a.kmh[od] = 0.0f; a.kmv[od] = 0.0f; return; }
-  const int ii = i < 1 ? i + g.ni : (i > g.ni ? i - g.ni : i);
-  const int jj = j < 1 ? j + g.nj : (j > g.nj ? j - g.nj : j);
-  const long pl = (long)g.NI * g.NJ;
-  const long o = iS(g, ii, jj, k), om = o - pl;
-  const float c1 = LDG(&g.c1[k]), c2 = LDG(&g.c2[k]);
-  const float tmp11 = c1 * sq(a.t11[om]) + c2 * sq(a.t11[o]);
-  const float tmp22 = c1 * sq(a.t22[om]) + c2 * sq(a.t22[o]);
-  const float tmp33 = c1 * sq(a.t33[om]) + c2 * sq(a.t33[o]);
-  const long o11 = iS(g, ii + 1, jj + 1, k), o01 = iS(g, ii, jj + 1, k), o10 = iS(g, ii + 1, jj, k);
-  const float tmp12 = 0.25f * (c1 * ((sq(a.t12[om]) + sq(a.t12[o11 - pl])) + (sq(a.t12[o01 - pl]) + sq(a.t12[o10 - pl]))) +
-                               c2 * ((sq(a.t12[o]) + sq(a.t12[o11])) + (sq(a.t12[o01]) + sq(a.t12[o10]))));
-  const float tmp13 = 0.5f * (sq(a.s13[o]) + sq(a.s13[o10]));
-  const float tmp23 = 0.5f * (sq(a.s23[o]) + sq(a.s23[o01]));
-  const float rf = les_rf(g, a, ii, jj, k);
-  const float rrf = 1.0f / sq(rf);
-  const float defv = 4.0f * (tmp13 + tmp23) * rrf;
-  const float defh = (2.0f * ((tmp11 + tmp22) + tmp33) + 4.0f * tmp12) * rrf;
-  // calcnm, imoist=0 (turb.F:5458-5468)
-  const float th0k = LDG(&g.th0[k]), th0m = LDG(&g.th0[k - 1]);
-  const float q = (th0k + a.tha[o]) / (th0m + a.tha[om]);
-  const float nm = (float)log((double)q) * g.c.g * g.rdz * LDG(&g.mf[k]);
-  const float dmin = 1.0e-10f;
-  const float rmf = 1.0f / LDG(&g.mf[k]);
-  const float dxr = g.dx * LDG(&g.ruh[ii - g.ib]), dyr = g.dy * LDG(&g.rvh[jj - g.jb]);
-  float kmh, kmv;
-  if (a.tconfig == 1) {
-    const float grd = (float)pow((double)((dxr * dyr) * (g.dz * rmf)), (double)0.33333333f);
-    kmh = sq(a.csm * grd) * sqrtf(fmaxf(defv + defh - nm * a.prinv, dmin));
-    kmv = kmh;
-  } else {
-    const float lenh = sqrtf(dxr * dyr);
-    const float grd = g.dz * rmf;
-    kmh = sq(a.csm * lenh) * sqrtf(fmaxf(defh, dmin));
-    kmv = sq(a.csm * grd) * sqrtf(fmaxf(defv - nm * a.prinv, dmin));
-  }
-  a.kmh[od] = kmh;
-  a.kmv[od] = kmv;
-}
+__device__ __forceinline__ float from_west(float v) { return __shfl_up_sync(0xffffffffu, v, 1); }
+__device__ __forceinline__ float from_east(float v) { return __shfl_down_sync(0xffffffffu, v, 1); }
 
-// gettau (Cartesian) with sfcstress's bottom row and the top row
-__global__ void k_les_stress(DGrid g, TurbArgs a) {
-  const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);   // 0 .. ni+1
-  const int j = (int)blockIdx.y;                                // 0 .. nj+1
-  const int k = 1 + (int)blockIdx.z;                            // 1 .. nk+1
-  if (i > g.ni + 1) return;
-  const int nk = g.nk;
-  const long pl = (long)g.NI * g.NJ;
-  const long o = iS(g, i, j, k);
-  const float *kmh = a.kmh, *kmv = a.kmv;
-  if (k <= nk) {
-    const float tem = kmh[o] + kmh[o + pl];
-    a.t11[o] = a.t11[o] * tem;
-    a.t22[o] = a.t22[o] * tem;
-    a.t33[o] = a.t33[o] * tem;
-    if (i >= 1 && j >= 1) {
-      const long omm = iS(g, i - 1, j - 1, k), om0 = iS(g, i - 1, j, k), o0m = iS(g, i, j - 1, k);
-      a.t12[o] = a.t12[o] * 0.25f *
-                 (((kmh[omm] + kmh[o]) + (kmh[om0] + kmh[o0m])) +
-                  ((kmh[omm + pl] + kmh[o + pl]) + (kmh[om0 + pl] + kmh[o0m + pl])));
-    }
-  }
-  if (i < 1 || j < 1) return;
-  const long ox = iS(g, i - 1, j, k), oy = iS(g, i, j - 1, k);
-  if (k <= nk) {
-    // turbs' face coefficients (turbtend.F:68-77): khh = kmh * prinv at the
-    // four points, summed as the Fortran does, times -0.125 (rho + rho); the
-    // Fortran's left-to-right product forms this factor first
-    const float pr = a.prinv;
-    a.cx[o] = -0.125f * (a.rho[o] + a.rho[ox]) * ((kmh[o] * pr + kmh[ox] * pr) + (kmh[o + pl] * pr + kmh[ox + pl] * pr));
-    a.cy[o] = -0.125f * (a.rho[o] + a.rho[oy]) * ((kmh[o] * pr + kmh[oy] * pr) + (kmh[o + pl] * pr + kmh[oy + pl] * pr));
-  }
-  if (k >= 2 && k <= nk) {
-    a.t13[o] = a.s13[o] * (kmv[ox] + kmv[o]);
-    a.t23[o] = a.s23[o] * (kmv[oy] + kmv[o]);
-  } else if (k == 1) {
-    if (a.bbc == 1) {            // free slip: t13(1) = t13(2)
-      a.t13[o] = a.s13[o + pl] * (kmv[ox + pl] + kmv[o + pl]);
-      a.t23[o] = a.s23[o + pl] * (kmv[oy + pl] + kmv[o + pl]);
-    } else {                     // no slip (turb.F:4550-4562), ugr = ua, vgr = va
-      const float rdz = g.rdz, mf = LDG(&g.mf[1]);
-      a.t13[o] = 2.0f * a.ua[iU(g, i, j, 1)] * rdz * 0.5f * (mf + mf) * 0.5f *
-                 (les_rf(g, a, i - 1, j, 1) + les_rf(g, a, i, j, 1)) * 0.5f * (kmv[ox + pl] + kmv[o + pl]);
-      a.t23[o] = 2.0f * a.va[iV(g, i, j, 1)] * rdz * 0.5f * (mf + mf) * 0.5f *
-                 (les_rf(g, a, i, j - 1, 1) + les_rf(g, a, i, j, 1)) * 0.5f * (kmv[oy + pl] + kmv[o + pl]);
-    }
-  } else {
-    if (a.tbc == 1) {            // free slip: t13(nk+1) = t13(nk)
-      a.t13[o] = a.s13[o - pl] * (kmv[ox - pl] + kmv[o - pl]);
-      a.t23[o] = a.s23[o - pl] * (kmv[oy - pl] + kmv[o - pl]);
-    } else {                     // no slip (turb.F:4407-4419)
-      const float rdz = g.rdz, mf = LDG(&g.mf[nk + 1]);
-      a.t13[o] = -(2.0f * a.ua[iU(g, i, j, nk)] * rdz * 0.5f * (mf + mf) * 0.5f *
-                   (les_rf(g, a, i - 1, j, nk + 1) + les_rf(g, a, i, j, nk + 1)) * 0.5f * (kmv[ox - pl] + kmv[o - pl]));
-      a.t23[o] = -(2.0f * a.va[iV(g, i, j, nk)] * rdz * 0.5f * (mf + mf) * 0.5f *
-                   (les_rf(g, a, i, j - 1, nk + 1) + les_rf(g, a, i, j, nk + 1)) * 0.5f * (kmv[oy - pl] + kmv[o - pl]));
-    }
-  }
-}
+// Rows of threads of a tile (x: 32 lanes, of which 30 own points).
+constexpr int LK_TY = 16, LT_TY = 12;
 
-// scalar value as turbs sees it: theta minus th0r plus th0 (solve1.F:1184-1195)
-__device__ __forceinline__ float les_s(const DGrid &g, const float *s, bool th, int i, int j, int k) {
-  const float v = s[iS(g, i, j, k)];
-  return th ? (LDG(&g.th0[k]) - 300.0f) + v : v;
-}
-
-// x/y flux dumx, dumy of turbs (turbtend.F:66-78): the face coefficient
-// times the difference, rdx and the metric, in the Fortran's order
-__device__ __forceinline__ float les_sfx(const DGrid &g, const TurbArgs &a, const float *s, bool th, int i, int j, int k,
-                                         bool ydir) {
-  const int im = ydir ? i : i - 1, jm = ydir ? j - 1 : j;
-  const long o = iS(g, i, j, k);
-  const float met = ydir ? LDG(&g.vf[j - g.jb]) : LDG(&g.uf[i - g.ib]);
-  return (ydir ? a.cy[o] : a.cx[o]) * (les_s(g, s, th, i, j, k) - les_s(g, s, th, im, jm, k)) * (ydir ? g.rdy : g.rdx) *
-         met;
-}
-
-// vertical flux dumz of turbsz, explicit (turbtend.F:480-510)
-__device__ __forceinline__ float les_sfz(const DGrid &g, const TurbArgs &a, const float *s, bool th, int i, int j, int k) {
-  const int nk = g.nk;
-  if (k == 1 || k == nk + 1) {
-    if (a.bcturbs == 1) return 0.0f;
-    k = (k == 1) ? 2 : nk;
-  }
-  const float khv = a.kmv[iS(g, i, j, k)] * a.prinv;
-  return -khv * (les_s(g, s, th, i, j, k) - les_s(g, s, th, i, j, k - 1)) * g.rdz * LDG(&g.mf[k]) *
-         les_rf(g, a, i, j, k);
-}
-
-// tendencies: blockIdx.z < nk for momentum level k; then one z per (scalar, k)
-__global__ void k_les_tend(DGrid g, TurbArgs a) {
-  const int i = 1 + (int)(blockIdx.x * blockDim.x + threadIdx.x);   // 1 .. ni+1
-  const int j = 1 + (int)blockIdx.y;                                // 1 .. nj+1
-  const int nk = g.nk;
-  const int z = (int)blockIdx.z;
-  const int k = 1 + z % nk, f = z / nk;
-  if (i > g.ni + 1) return;
+// calcdef (turb.F:4772-4790, 4880-4893, 5366-5390), calcnm (dry) and kmh/kmv
+// of turbsmag.  A block owns 30 x (LK_TY-1) columns: thread (lane, row) is the
+// point (30 bx + lane, (LK_TY-1) by + 1 + row); the outer lanes and the last
+// row only supply neighbours.  It marches through the w-levels kc0 ..
+// kc0+kc-1, the level above loading while a level computes.  The bottom and
+// top rows are zero (bcw flag 1, bc.F:1126-1137).
+__global__ void __launch_bounds__(32 * LK_TY, 2) k_les_km(DGrid g, TurbArgs a, int kc) {
+  __shared__ float s12[2][LK_TY][32], s23s[2][LK_TY][32];
+  const int lane = threadIdx.x, row = threadIdx.y;
+  const int i = (int)blockIdx.x * 30 + lane, j = 1 + (int)blockIdx.y * (LK_TY - 1) + row;
+  const int ni = g.ni, nj = g.nj, nk = g.nk, NI = g.NI;
+  const int pl = NI * g.NJ, plU = (NI + 1) * g.NJ, plV = NI * (g.NJ + 1);   // < 2^31 points (cm1g_init)
+  const bool valid = i <= ni + 1 && j <= nj + 1;
+  const bool owner = lane >= 1 && lane < 31 && row < LK_TY - 1 && i <= ni && j <= nj;
+  const int kc0 = 2 + (int)blockIdx.z * kc, kc1 = min(nk, kc0 + kc - 1);
   const float rdx = g.rdx, rdy = g.rdy, rdz = g.rdz;
-  const long pl = (long)g.NI * g.NJ;
-  const long o = iS(g, i, j, k);
-  if (f == 0) {
-    const float tem = rdz * 0.5f;
-    if (j <= g.nj) {   // turbu (turbtend.F:1101-1104, 1290-1296; turbuz 1408-1416)
-      const float tx = (a.t11[o] - a.t11[iS(g, i - 1, j, k)]) * rdx * LDG(&g.uf[i - g.ib]);
-      const float ty = (a.t12[iS(g, i, j + 1, k)] - a.t12[o]) * rdy * LDG(&g.vh[j - g.jb]);
-      const float tz = (a.t13[o + pl] - a.t13[o]) * tem * (LDG(&g.mh[k]) + LDG(&g.mh[k]));
-      const float rru0 = 1.0f / (0.5f * (a.rho[iS(g, i - 1, j, k)] + a.rho[o]));
-      const long ou = iU(g, i, j, k);
-      a.uten[ou] = a.uten[ou] + ((tx + ty) + tz) * rru0;
+  // threads outside the arrays' ring follow the column (ib, jb+1) and supply nothing that is used
+  const int ic = valid ? i - g.ib : 0, jc = valid ? j - g.jb : 1;
+  const float uh = LDG(&g.uh[ic]), vh = LDG(&g.vh[jc]), uf = LDG(&g.uf[ic]), vf = LDG(&g.vf[jc]);
+  const int oc = ic + NI * jc, ocu = ic + (NI + 1) * jc;
+  const float dxr = g.dx * LDG(&g.ruh[ic]), dyr = g.dy * LDG(&g.rvh[jc]);
+
+  // a value of an owned column and its periodic images on the halo ring
+  auto put = [&](float *q, int k, float v) {
+    float *r = q + k * pl + oc;
+    const int dx = (i == 1) ? ni : (i == ni ? -ni : 0), dy = (j == 1) ? nj * NI : (j == nj ? -nj * NI : 0);
+    r[0] = v;
+    if (dx) r[dx] = v;
+    if (dy) r[dy] = v;
+    if (dx && dy) r[dx + dy] = v;
+    if (ni == 1 && dx) { r[-dx] = v; if (dy) r[dy - dx] = v; }
+    if (nj == 1 && dy) { r[-dy] = v; if (dx) { r[dx - dy] = v; if (ni == 1) r[-dx - dy] = v; } }
+  };
+  if (owner && kc0 == 2) { put(a.kmh, 1, 0.0f); put(a.kmv, 1, 0.0f); }
+  if (owner && kc1 == nk) { put(a.kmh, nk + 1, 0.0f); put(a.kmv, nk + 1, 0.0f); }
+
+  // a level of the column and of its y neighbours (x neighbours come by shuffles)
+  struct Lev { float u, us, v, vn, w, ws, r, rs, th; };
+  auto load = [&](int k) -> Lev {
+    const int o = k * pl + oc, ou = k * plU + ocu, ov = k * plV + oc;
+    return Lev{LDG(&a.ua[ou]), LDG(&a.ua[ou - (NI + 1)]), LDG(&a.va[ov]), LDG(&a.va[ov + NI]), LDG(&a.wa[o]),
+               LDG(&a.wa[o - NI]), LDG(&a.rho[o]), LDG(&a.rho[o - NI]), LDG(&a.tha[o])};
+  };
+  // of the level below: u, v, rho, theta, the squared strains, the sum of t12^2 over the four corners
+  float u0 = 0, v0 = 0, r0 = 0, rs0 = 0, th_0 = 0, q11 = 0, q22 = 0, q33 = 0, g12 = 0;
+  float lastarg = -1.0f, grd1 = 0.0f;   // tconfig 1: the grid scale changes only with the metrics
+  Lev c = load(kc0 - 1);
+  int b = 0;
+  for (int k = kc0 - 1; k <= kc1; k++, b ^= 1) {
+    const bool wl = k >= kc0;        // a w-level of this block
+    const Lev n = load(k + 1);
+    if (k + 3 <= kc1) {              // levels ahead towards L2
+      const int o = (k + 3) * pl + oc;
+      prefetch_l2(&a.ua[(k + 3) * plU + ocu]); prefetch_l2(&a.va[(k + 3) * plV + oc]);
+      prefetch_l2(&a.wa[o]); prefetch_l2(&a.rho[o]); prefetch_l2(&a.tha[o]);
     }
-    if (i <= g.ni) {   // turbv
-      const float tx = (a.t12[iS(g, i + 1, j, k)] - a.t12[o]) * rdx * LDG(&g.uh[i - g.ib]);
-      const float ty = (a.t22[o] - a.t22[iS(g, i, j - 1, k)]) * rdy * LDG(&g.vf[j - g.jb]);
-      const float tz = (a.t23[o + pl] - a.t23[o]) * tem * (LDG(&g.mh[k]) + LDG(&g.mh[k]));
-      const float rrv0 = 1.0f / (0.5f * (a.rho[iS(g, i, j - 1, k)] + a.rho[o]));
-      const long ov = iV(g, i, j, k);
-      a.vten[ov] = a.vten[ov] + ((tx + ty) + tz) * rrv0;
+    const float t11 = c.r * (from_east(c.u) - c.u) * rdx * uh;
+    const float t22 = c.r * (c.vn - c.v) * rdy * vh;
+    const float t33 = c.r * (n.w - c.w) * (rdz * LDG(&g.mh[k]));
+    const float t12 = 0.5f * ((c.u - c.us) * rdy * vf + (c.v - from_west(c.v)) * rdx * uf) * 0.25f *
+                      ((from_west(c.rs) + c.r) + (from_west(c.r) + c.rs));
+    float t13 = 0.0f, t23 = 0.0f, rfc = 1.0f;
+    const float c1 = LDG(&g.c1[k]), c2 = LDG(&g.c2[k]), mf = LDG(&g.mf[k]);
+    if (wl) {
+      rfc = c1 * r0 + c2 * c.r;
+      const float rfy = c1 * rs0 + c2 * c.rs;
+      t13 = 0.5f * ((c.w - from_west(c.w)) * rdx * uf + (c.u - u0) * rdz * 0.5f * (mf + mf)) * 0.5f * (from_west(rfc) + rfc);
+      t23 = 0.5f * ((c.w - c.ws) * rdy * vf + (c.v - v0) * rdz * 0.5f * (mf + mf)) * 0.5f * (rfy + rfc);
     }
-    if (i <= g.ni && j <= g.nj && k >= 2) {   // turbw
-      const float tx = (a.t13[iS(g, i + 1, j, k)] - a.t13[o]) * rdx * LDG(&g.uh[i - g.ib]);
-      const float ty = (a.t23[iS(g, i, j + 1, k)] - a.t23[o]) * rdy * LDG(&g.vh[j - g.jb]);
-      const float tz = (a.t33[o] - a.t33[o - pl]) * rdz * LDG(&g.mf[k]);
-      const long ow = iW(g, i, j, k);
-      a.wten[ow] = a.wten[ow] + ((tx + ty) + tz) / les_rf(g, a, i, j, k);
+    s12[b][row][lane] = t12;
+    s23s[b][row][lane] = t23;
+    const float t12e = from_east(t12), t13e = from_east(t13);
+    __syncthreads();
+    if (owner) {
+      const float n11 = sq(t11), n22 = sq(t22), n33 = sq(t33);
+      const float n12 = (sq(t12) + sq(s12[b][row + 1][lane + 1])) + (sq(s12[b][row + 1][lane]) + sq(t12e));
+      if (wl) {
+        const float tmp11 = c1 * q11 + c2 * n11, tmp22 = c1 * q22 + c2 * n22, tmp33 = c1 * q33 + c2 * n33;
+        const float tmp12 = 0.25f * (c1 * g12 + c2 * n12);
+        const float tmp13 = 0.5f * (sq(t13) + sq(t13e));
+        const float tmp23 = 0.5f * (sq(t23) + sq(s23s[b][row + 1][lane]));
+        const float rrf = 1.0f / sq(rfc);
+        const float defv = 4.0f * (tmp13 + tmp23) * rrf;
+        const float defh = (2.0f * ((tmp11 + tmp22) + tmp33) + 4.0f * tmp12) * rrf;
+        // calcnm, imoist=0 (turb.F:5458-5468)
+        const float q = (LDG(&g.th0[k]) + c.th) / (LDG(&g.th0[k - 1]) + th_0);
+        const float nm = (float)log((double)q) * g.c.g * rdz * mf;
+        const float dmin = 1.0e-10f;
+        const float rmf = 1.0f / mf;
+        float kmh, kmv;
+        if (a.tconfig == 1) {
+          const float arg = (dxr * dyr) * (g.dz * rmf);
+          if (arg != lastarg) { grd1 = (float)pow((double)arg, (double)0.33333333f); lastarg = arg; }
+          kmh = sq(a.csm * grd1) * sqrtf(fmaxf(defv + defh - nm * a.prinv, dmin));
+          kmv = kmh;
+        } else {
+          const float lenh = sqrtf(dxr * dyr);
+          const float grd = g.dz * rmf;
+          kmh = sq(a.csm * lenh) * sqrtf(fmaxf(defh, dmin));
+          kmv = sq(a.csm * grd) * sqrtf(fmaxf(defv - nm * a.prinv, dmin));
+        }
+        put(a.kmh, k, kmh);
+        put(a.kmv, k, kmv);
+      }
+      q11 = n11; q22 = n22; q33 = n33; g12 = n12;
     }
-    return;
+    u0 = c.u; v0 = c.v; r0 = c.r; rs0 = c.rs; th_0 = c.th;
+    c = n;
   }
-  if (i > g.ni || j > g.nj) return;
-  // turbs: field f-1 (theta, then q, then tracers)
-  const int n = f - 1;
-  const long ns = (long)pl * g.NK;
-  const bool th = n == 0;
-  const float *s = th ? a.tha : (n <= a.numq ? a.qa + (n - 1) * ns : a.pta + (n - 1 - a.numq) * ns);
-  float *sten = th ? a.thten : (n <= a.numq ? a.qten + (n - 1) * ns : a.ptten + (n - 1 - a.numq) * ns);
-  const float tx = -(les_sfx(g, a, s, th, i + 1, j, k, false) - les_sfx(g, a, s, th, i, j, k, false)) * rdx *
-                   LDG(&g.uh[i - g.ib]);
-  const float ty = -(les_sfx(g, a, s, th, i, j + 1, k, true) - les_sfx(g, a, s, th, i, j, k, true)) * rdy *
-                   LDG(&g.vh[j - g.jb]);
-  const float tz = -(les_sfz(g, a, s, th, i, j, k + 1) - les_sfz(g, a, s, th, i, j, k)) * rdz * LDG(&g.mh[k]);
-  const float rr = 1.0f / a.rho[o];
-  sten[o] = sten[o] + ((tx + ty) + tz) * rr;
+}
+
+// gettau (Cartesian) with sfcstress's bottom row and the top row (turb.F:
+// 4059-4582), then turbu, turbv, turbw (turbtend.F:1101-1104, 1290-1296,
+// 1408-1416, 1816-2180, 2473-2885) and turbs/turbsz of the scalars n0 ..
+// n0+NS-1 (turbtend.F:66-78, 480-510).  A block owns 30 x (LT_TY-2) points:
+// thread (lane, row) is the point (30 bx + lane, (LT_TY-2) by + row); the
+// outer lanes and rows only supply neighbours.  It marches through the
+// s-levels kc0 .. kc0+kc-1, the level above loading while a level computes.
+// MOM: add the momentum tendencies too.
+template <int NS, bool MOM>
+__global__ void __launch_bounds__(32 * LT_TY, 2) k_les_tend(DGrid g, TurbArgs a, int kc, int n0) {
+  __shared__ float s12[2][LT_TY][32], s22[2][LT_TY][32], s23[2][LT_TY][32], scy[2][LT_TY][32];
+  const int lane = threadIdx.x, row = threadIdx.y;
+  const int i = (int)blockIdx.x * 30 + lane, j = (int)blockIdx.y * (LT_TY - 2) + row;
+  const int ni = g.ni, nj = g.nj, nk = g.nk, NI = g.NI;
+  const int pl = NI * g.NJ, plU = (NI + 1) * g.NJ, plV = NI * (g.NJ + 1);   // < 2^31 points (cm1g_init)
+  const bool valid = i <= ni + 2 && j <= nj + 1;           // the last u point needs the column east of it
+  const bool owner = lane >= 1 && lane < 31 && row >= 1 && row < LT_TY - 1 && i <= ni + 1 && j <= nj + 1;
+  const bool own_u = owner && j <= nj, own_v = owner && i <= ni, own_s = own_u && own_v;
+  const int kc0 = 1 + (int)blockIdx.z * kc, kc1 = min(nk, kc0 + kc - 1);
+  const float rdx = g.rdx, rdy = g.rdy, rdz = g.rdz, tem = rdz * 0.5f, pr = a.prinv;
+  // threads outside the arrays' ring follow the column (ib, jb+1) and supply nothing that is used
+  const int ic = valid ? i - g.ib : 0, jc = valid ? j - g.jb : 1;
+  const float uh = LDG(&g.uh[ic]), vh = LDG(&g.vh[jc]), uf = LDG(&g.uf[ic]), vf = LDG(&g.vf[jc]), vfn = LDG(&g.vf[jc + 1]);
+  const int oc = ic + NI * jc, ocu = ic + (NI + 1) * jc;
+
+  // a level of the column and of its y neighbours (x neighbours come by shuffles)
+  struct Lev { float u, us, v, vn, w, ws, r, rs, kh, khs, kv, kvs; };
+  auto load = [&](int k) -> Lev {
+    const int o = k * pl + oc, ou = k * plU + ocu, ov = k * plV + oc;
+    return Lev{LDG(&a.ua[ou]), LDG(&a.ua[ou - (NI + 1)]), LDG(&a.va[ov]), LDG(&a.va[ov + NI]), LDG(&a.wa[o]),
+               LDG(&a.wa[o - NI]), LDG(&a.rho[o]), LDG(&a.rho[o - NI]), LDG(&a.kmh[o]), LDG(&a.kmh[o - NI]),
+               LDG(&a.kmv[o]), LDG(&a.kmv[o - NI])};
+  };
+  // w-level density at the bottom (kk = 1) and top (nk+1) rows, offset d from the column
+  auto rf_end = [&](int d, int kk) -> float {
+    const float *q = a.rho + kk * pl + oc + d;
+    if (kk == 1) return a.cgs1 * q[0] + a.cgs2 * q[pl] + a.cgs3 * q[2 * pl];
+    return a.cgt1 * q[-pl] + a.cgt2 * q[-2 * pl] + a.cgt3 * q[-3 * pl];
+  };
+  struct WLev { float t13, t23, rf; };
+  // an inner w-level kk = 2..nk from the s-levels below and above it
+  auto inner = [&](const Lev &lo, const Lev &hi, int kk) -> WLev {
+    const float c1 = LDG(&g.c1[kk]), c2 = LDG(&g.c2[kk]), mf = LDG(&g.mf[kk]);
+    const float rfc = c1 * lo.r + c2 * hi.r, rfy = c1 * lo.rs + c2 * hi.rs;
+    const float x13 = 0.5f * ((hi.w - from_west(hi.w)) * rdx * uf + (hi.u - lo.u) * rdz * 0.5f * (mf + mf)) * 0.5f * (from_west(rfc) + rfc);
+    const float x23 = 0.5f * ((hi.w - hi.ws) * rdy * vf + (hi.v - lo.v) * rdz * 0.5f * (mf + mf)) * 0.5f * (rfy + rfc);
+    return WLev{x13 * (from_west(hi.kv) + hi.kv), x23 * (hi.kvs + hi.kv), rfc};
+  };
+  // no slip at the bottom or top row kk (turb.F:4407-4419, 4550-4562), ugr = ua,
+  // vgr = va: l the s-level beside the row, kv the viscosities of the nearest inner w-level
+  auto noslip = [&](const Lev &l, const Lev &kv, int kk) -> WLev {
+    const float mf = LDG(&g.mf[kk]), rfc = rf_end(0, kk);
+    return WLev{2.0f * l.u * rdz * 0.5f * (mf + mf) * 0.5f * (from_west(rfc) + rfc) * 0.5f * (from_west(kv.kv) + kv.kv),
+                2.0f * l.v * rdz * 0.5f * (mf + mf) * 0.5f * (rf_end(-NI, kk) + rfc) * 0.5f * (kv.kvs + kv.kv), rfc};
+  };
+
+  Lev c = load(kc0);
+  WLev wlo{0.0f, 0.0f, 1.0f};
+  float t33m = 0.0f, sc[NS > 0 ? NS : 1], fzl[NS > 0 ? NS : 1];
+  const bool theta = NS > 0 && n0 == 0;
+  auto SV = [&](int n, int k, int d) -> float {   // the scalar as turbs sees it (solve1.F:1184-1195)
+    const float v = LDG(&a.s[n0 + n][k * pl + oc + d]);
+    return (n == 0 && theta) ? (LDG(&g.th0[k]) - 300.0f) + v : v;
+  };
+#pragma unroll
+  for (int n = 0; n < NS; n++) { sc[n] = SV(n, kc0, 0); fzl[n] = 0.0f; }
+  if (kc0 > 1) {
+    const Lev m = load(kc0 - 1);
+    wlo = inner(m, c, kc0);
+    t33m = m.r * (c.w - m.w) * (rdz * LDG(&g.mh[kc0 - 1])) * (m.kh + c.kh);
+#pragma unroll
+    for (int n = 0; n < NS; n++) fzl[n] = -(c.kv * pr) * (sc[n] - SV(n, kc0 - 1, 0)) * rdz * LDG(&g.mf[kc0]) * wlo.rf;
+  }
+  float k40 = (from_west(c.khs) + c.kh) + (from_west(c.kh) + c.khs);
+  float hx0 = c.kh * pr + from_west(c.kh) * pr, hy0 = c.kh * pr + c.khs * pr;
+  int b = 0;
+  for (int k = kc0; k <= kc1; k++, b ^= 1) {
+    const int o = k * pl + oc, ou = k * plU + ocu, ov = k * plV + oc;
+    // every global read of the level, before anything is stored
+    const Lev n = load(k + 1);
+    float tu = 0, tv = 0, tw = 0, ts[NS > 0 ? NS : 1], sn[NS > 0 ? NS : 1], ss[NS > 0 ? NS : 1], sno[NS > 0 ? NS : 1];
+    if (MOM) {
+      if (own_u) tu = a.uten[ou];
+      if (own_v) tv = a.vten[ov];
+      if (own_s && k >= 2) tw = a.wten[o];
+    }
+#pragma unroll
+    for (int m = 0; m < NS; m++) {
+      ts[m] = own_s ? a.sten[n0 + m][o] : 0.0f;
+      sn[m] = SV(m, k + 1, 0);
+      ss[m] = SV(m, k, -NI);
+      sno[m] = SV(m, k, NI);
+    }
+    if (k + 3 <= kc1) {              // levels ahead towards L2
+      const int o3 = o + 3 * pl, o2 = o + 2 * pl;
+      prefetch_l2(&a.ua[ou + 3 * plU]); prefetch_l2(&a.va[ov + 3 * plV]);
+      prefetch_l2(&a.wa[o3]); prefetch_l2(&a.rho[o3]); prefetch_l2(&a.kmh[o3]); prefetch_l2(&a.kmv[o3]);
+      if (MOM) { prefetch_l2(&a.uten[ou + 2 * plU]); prefetch_l2(&a.vten[ov + 2 * plV]); prefetch_l2(&a.wten[o2]); }
+#pragma unroll
+      for (int m = 0; m < NS; m++) { prefetch_l2(&a.s[n0 + m][o3]); prefetch_l2(&a.sten[n0 + m][o2]); }
+    }
+    const float mhk = LDG(&g.mh[k]), rx = from_west(c.r), temk = c.kh + n.kh;
+    // the w-levels of this s-level's bottom and top
+    WLev whi;
+    if (k < nk) {
+      whi = inner(c, n, k + 1);
+      if (k == 1) {
+        if (a.bbc == 1) { wlo.t13 = whi.t13; wlo.t23 = whi.t23; }     // free slip: t13(1) = t13(2)
+        else wlo = noslip(c, n, 1);
+      }
+    } else if (a.tbc == 1) {
+      whi = wlo;                                                      // t13(nk+1) = t13(nk)
+    } else {
+      whi = noslip(c, c, nk + 1);
+      whi.t13 = -whi.t13;
+      whi.t23 = -whi.t23;
+    }
+    const float hx1 = n.kh * pr + from_west(n.kh) * pr, hy1 = n.kh * pr + n.khs * pr;
+    // turbs' face coefficients (turbtend.F:68-77): khh = kmh * prinv at the
+    // four points, summed as the Fortran does, times -0.125 (rho + rho)
+    const float cx = -0.125f * (c.r + rx) * (hx0 + hx1), cy = -0.125f * (c.r + c.rs) * (hy0 + hy1);
+    float t11 = 0, t22 = 0, t33 = 0, t12 = 0, t11w = 0, t12e = 0, t13e = 0;
+    const float k41 = (from_west(n.khs) + n.kh) + (from_west(n.kh) + n.khs);
+    if (MOM) {
+      t11 = c.r * (from_east(c.u) - c.u) * rdx * uh * temk;
+      t22 = c.r * (c.vn - c.v) * rdy * vh * temk;
+      t33 = c.r * (n.w - c.w) * (rdz * mhk) * temk;
+      t12 = 0.5f * ((c.u - c.us) * rdy * vf + (c.v - from_west(c.v)) * rdx * uf) * 0.25f *
+            ((from_west(c.rs) + c.r) + (rx + c.rs)) * 0.25f * (k40 + k41);
+      s12[b][row][lane] = t12;
+      s22[b][row][lane] = t22;
+      s23[b][row][lane] = wlo.t23;
+      t11w = from_west(t11);
+      t12e = from_east(t12);
+      t13e = from_east(wlo.t13);
+    }
+    if (NS > 0) scy[b][row][lane] = cy;
+    __syncthreads();
+    if (MOM) {
+      if (own_u) {   // turbu
+        const float tx = (t11 - t11w) * rdx * uf;
+        const float ty = (s12[b][row + 1][lane] - t12) * rdy * vh;
+        const float tz = (whi.t13 - wlo.t13) * tem * (mhk + mhk);
+        const float rru0 = 1.0f / (0.5f * (rx + c.r));
+        a.uten[ou] = tu + ((tx + ty) + tz) * rru0;
+      }
+      if (own_v) {   // turbv
+        const float tx = (t12e - t12) * rdx * uh;
+        const float ty = (t22 - s22[b][row - 1][lane]) * rdy * vf;
+        const float tz = (whi.t23 - wlo.t23) * tem * (mhk + mhk);
+        const float rrv0 = 1.0f / (0.5f * (c.rs + c.r));
+        a.vten[ov] = tv + ((tx + ty) + tz) * rrv0;
+      }
+      if (own_s && k >= 2) {   // turbw
+        const float tx = (t13e - wlo.t13) * rdx * uh;
+        const float ty = (s23[b][row + 1][lane] - wlo.t23) * rdy * vh;
+        const float tz = (t33 - t33m) * rdz * LDG(&g.mf[k]);
+        a.wten[o] = tw + ((tx + ty) + tz) / wlo.rf;
+      }
+    }
+    if (NS > 0) {
+      const float cyn = row < LT_TY - 1 ? scy[b][row + 1][lane] : 0.0f, rr = 1.0f / c.r;
+      const float khh = n.kv * pr, mfh = k < nk ? LDG(&g.mf[k + 1]) : 0.0f;
+#pragma unroll
+      for (int m = 0; m < NS; m++) {
+        const float fx0 = cx * (sc[m] - from_west(sc[m])) * rdx * uf, fx1 = from_east(fx0);
+        const float fy0 = cy * (sc[m] - ss[m]) * rdy * vf, fy1 = cyn * (sno[m] - sc[m]) * rdy * vfn;
+        // vertical fluxes: at the bottom and top boundaries zero (bcturbs 1)
+        // or the nearest inner level's flux
+        float fz1;
+        if (k < nk) fz1 = -khh * (sn[m] - sc[m]) * rdz * mfh * whi.rf;
+        else fz1 = a.bcturbs == 1 ? 0.0f : fzl[m];
+        const float fz0 = k > 1 ? fzl[m] : (a.bcturbs == 1 ? 0.0f : fz1);
+        const float tx = -(fx1 - fx0) * rdx * uh;
+        const float ty = -(fy1 - fy0) * rdy * vh;
+        const float tz = -(fz1 - fz0) * rdz * mhk;
+        if (own_s) a.sten[n0 + m][o] = ts[m] + ((tx + ty) + tz) * rr;
+        fzl[m] = fz1;
+        sc[m] = sn[m];
+      }
+    }
+    wlo = whi; t33m = t33; k40 = k41; hx0 = hx1; hy0 = hy1;
+    c = n;
+  }
+}
+
+template <bool MOM>
+static void les_tend(const DGrid &g, const TurbArgs &a, int ns, int n0, cudaStream_t st) {
+  dim3 blk(32, LT_TY), grid((g.ni + 1 + 29) / 30, (g.nj + 1 + LT_TY - 3) / (LT_TY - 2));
+  const int kc = tile_levels((long)grid.x * grid.y, g.nk, 2 * 148, 3, 128);
+  grid.z = (g.nk + kc - 1) / kc;
+  ProfScope _ps("k_les_tend", st);
+  switch (ns) {
+    case 0: k_les_tend<0, MOM><<<grid, blk, 0, st>>>(g, a, kc, n0); break;
+    case 1: k_les_tend<1, MOM><<<grid, blk, 0, st>>>(g, a, kc, n0); break;
+    case 2: k_les_tend<2, MOM><<<grid, blk, 0, st>>>(g, a, kc, n0); break;
+    default: k_les_tend<3, MOM><<<grid, blk, 0, st>>>(g, a, kc, n0); break;
+  }
 }
 
 void launch_turbsmag(const DGrid &g, const TurbArgs &a, cudaStream_t st, int64_t *nl) {
-  // one row of 128 points per block (32 x 8 blocks measured no faster)
-  const int bx = 128;
   {
-    dim3 grid((g.ni + 2 + bx - 1) / bx, g.nj + 2, g.nk);
-    ProfScope _ps("k_les_strain", st);
-    k_les_strain<<<grid, bx, 0, st>>>(g, a);
-  }
-  {
-    dim3 grid((g.ni + 2 + bx - 1) / bx, g.nj + 2, g.nk + 1);
+    dim3 grid((g.ni + 29) / 30, (g.nj + LK_TY - 2) / (LK_TY - 1));
+    const int kc = tile_levels((long)grid.x * grid.y, g.nk - 1, 2 * 148, 3, 128);
+    grid.z = (g.nk - 1 + kc - 1) / kc;
     ProfScope _ps("k_les_km", st);
-    k_les_km<<<grid, bx, 0, st>>>(g, a);
+    k_les_km<<<grid, dim3(32, LK_TY), 0, st>>>(g, a, kc);
   }
-  {
-    dim3 grid((g.ni + 2 + bx - 1) / bx, g.nj + 2, g.nk + 1);
-    ProfScope _ps("k_les_stress", st);
-    k_les_stress<<<grid, bx, 0, st>>>(g, a);
+  // momentum with up to three scalars, then three scalars a launch
+  les_tend<true>(g, a, a.nsc < 3 ? a.nsc : 3, 0, st);
+  if (nl) *nl += 2;
+  for (int n0 = 3; n0 < a.nsc; n0 += 3) {
+    les_tend<false>(g, a, a.nsc - n0 < 3 ? a.nsc - n0 : 3, n0, st);
+    if (nl) *nl += 1;
   }
-  {
-    const int nf = 1 + (a.thten ? 1 + a.numq + a.npt : 0);
-    dim3 grid((g.ni + 1 + bx - 1) / bx, g.nj + 1, g.nk * nf);
-    ProfScope _ps("k_les_tend", st);
-    k_les_tend<<<grid, bx, 0, st>>>(g, a);
-  }
-  if (nl) *nl += 4;
 }
 
 }  // namespace cm1g

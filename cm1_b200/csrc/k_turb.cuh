@@ -4,6 +4,8 @@
 
 namespace cm1g {
 
+constexpr int kTurbMaxScalars = 1 + 2 * 8;   // theta, up to 8 q arrays and 8 tracers
+
 struct TurbArgs {
   float csm;                                  // Smagorinsky constant (uniform csm of turbsmag)
   float prinv;                                // 1/Prandtl number (turb.F:3421-3422)
@@ -11,16 +13,12 @@ struct TurbArgs {
   int tconfig, bcturbs, bbc, tbc;
   const float *ua, *va, *wa, *rho, *tha;
   float *uten, *vten, *wten;
-  // scalars: theta (s = th0 - th0r + tha), then numq q arrays and npt tracers
-  const float *qa, *pta;
-  float *thten, *qten, *ptten;
-  int numq, npt;
-  // scratch: rho*S_ij, then the stresses (s-shaped t11, t22, t33, t12 in
-  // place; w-shaped t13, t23 formed from s13, s23); kmh, kmv (w-shaped)
-  float *t11, *t22, *t33, *t12, *s13, *s23, *t13, *t23, *kmh, *kmv;
-  // face coefficients of turbs' x/y fluxes, -0.125*(rho+rho)*(sum of khh)
-  // (s-shaped, faces i or j = 1 .. n+1), shared by every scalar
-  float *cx, *cy;
+  // scalars of the tendencies: theta first (s = th0 - th0r + tha), then the
+  // tracers; none when nsc is 0
+  int nsc;
+  const float *s[kTurbMaxScalars];
+  float *sten[kTurbMaxScalars];
+  float *kmh, *kmv;                           // eddy viscosities (w-shaped; the halo ring is written)
 };
 
 void launch_turbsmag(const DGrid &g, const TurbArgs &a, cudaStream_t st, int64_t *nl);
