@@ -2279,7 +2279,7 @@ extern "C" int cm1g_diff2(cm1g_ctx_t *c, float kdiff2, int32_t idiff, int32_t bb
   const bool scal = idiff == 1;
   if (scal && (!tha || !thten1 || (numq && (!qa || !qten)) || (npt && (!pta || !ptten))))
     return set_err(CM1G_ERR_ARG, "diff2 with idiff=1 needs tha/thten1, qa/qten, pta/ptten");
-  if (!c->d2s) {
+  if (!c->d2s && diff2_walls(g)) {
     const size_t bS = nS(g) * sizeof(float), bW = nW(g) * sizeof(float);
     c->d2s = (float *)dalloc(c, 6 * bS + 3 * bW);
     if (!c->d2s) return set_err(CM1G_ERR_NOMEM, "diff2 scratch");
@@ -2288,14 +2288,16 @@ extern "C" int cm1g_diff2(cm1g_ctx_t *c, float kdiff2, int32_t idiff, int32_t bb
   Stager S(c);
   const size_t ns = nS(g);
   Diff2Args a{};
-  a.kdiff2 = kdiff2; a.bbc = bbc; a.tbc = tbc; a.momentum = 1;
+  a.kdiff2 = kdiff2; a.bbc = bbc; a.tbc = tbc;
   a.cgs1 = cgs[0]; a.cgs2 = cgs[1]; a.cgs3 = cgs[2]; a.cgt1 = cgt[0]; a.cgt2 = cgt[1]; a.cgt3 = cgt[2];
   a.ua = S.in(ua, nU(g), false); a.va = S.in(va, nV(g), false); a.wa = S.in(wa, nW(g), false);
   a.rho = S.in(rho, ns, false);
   a.uten = S.in(uten1, nU(g), true); a.vten = S.in(vten1, nV(g), true); a.wten = S.in(wten1, nW(g), true);
-  float *p = c->d2s;
-  a.rr = p; p += ns; a.divx = p; p += ns; a.t11 = p; p += ns; a.t22 = p; p += ns; a.t33 = p; p += ns;
-  a.t12 = p; p += ns; a.rf = p; p += nW(g); a.t13 = p; p += nW(g); a.t23 = p;
+  if (c->d2s) {
+    float *p = c->d2s;
+    a.rr = p; p += ns; a.divx = p; p += ns; a.t11 = p; p += ns; a.t22 = p; p += ns; a.t33 = p; p += ns;
+    a.t12 = p; p += ns; a.rf = p; p += nW(g); a.t13 = p; p += nW(g); a.t23 = p;
+  }
   a.nsc = 0;
   if (scal) {   // solve1.F:706-733: theta, every q, every tracer
     a.s[a.nsc] = S.in(tha, ns, false); a.sten[a.nsc++] = S.in(thten1, ns, true);

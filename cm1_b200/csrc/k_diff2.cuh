@@ -8,7 +8,7 @@ constexpr int kDiff2MaxScalars = 1 + 2 * 8;   // theta, up to 8 q arrays and 8 t
 
 struct Diff2Args {
   float kdiff2;
-  int bbc, tbc, momentum;
+  int bbc, tbc;
   float cgs1, cgs2, cgs3, cgt1, cgt2, cgt3;   // rf extrapolation to the bottom and top w-levels
   const float *ua, *va, *wa, *rho;
   float *uten, *vten, *wten;
@@ -19,6 +19,8 @@ struct Diff2Args {
   float *sten[kDiff2MaxScalars];
 };
 
+// true where a lateral boundary is a wall: launch_diff2 then needs the scratch arrays
+bool diff2_walls(const DGrid &g);
 void launch_diff2(const DGrid &g, const Diff2Args &a, cudaStream_t st, int64_t *nl);
 
 }  // namespace cm1g
