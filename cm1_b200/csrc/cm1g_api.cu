@@ -1849,12 +1849,12 @@ extern "C" int cm1g_stat_setup(cm1g_ctx_t *c, const cm1g_stat_opts_t *o, int32_t
   const int maxlev = nk + 1;
   int npl = 1;
   for (const StatJob &j : jobs) npl = std::max(npl, (j.ie - j.i0 + 1) * (j.je - j.j0 + 1));
-  const int nch = stat_chunks(npl);
+  const int nch = stat_chunks(npl, nk);
   if ((int)jobs.size() > c->st_cap_jobs) {
     if (c->d_st_jobs) { cudaFree(c->d_st_jobs); cudaFree(c->d_st_lev); c->d_st_jobs = nullptr; c->d_st_lev = nullptr; }
     c->st_cap_jobs = (int)jobs.size() + 16;
     CUCHK(cudaMalloc(&c->d_st_jobs, c->st_cap_jobs * sizeof(StatJob)));
-    CUCHK(cudaMalloc(&c->d_st_lev, (size_t)c->st_cap_jobs * maxlev * stat_chunks((g.ni + 1) * (g.nj + 1)) *
+    CUCHK(cudaMalloc(&c->d_st_lev, (size_t)c->st_cap_jobs * maxlev * stat_chunks((g.ni + 1) * (g.nj + 1), nk) *
                                        sizeof(StatLev)));
   }
   if ((int)ops.size() > c->st_cap_ops) {
@@ -1966,7 +1966,7 @@ extern "C" int cm1g_statpack(cm1g_ctx_t *c, double mtime, float dt, const float 
   for (int n = 0; n < numq && n < CM1G_MAXQ; n++) if (o.cloudvar[n]) k.cloudmask |= 1u << n;
   k.zh = c->d_st_zh; k.zf = c->d_st_zf;
   const int nops = (int)c->st_ops.size();
-  launch_stat(g, f, k, c->d_st_jobs, (int)c->st_jobs.size(), c->d_st_lev, g.nk + 1, c->st_nch, c->d_st_ops, nops,
+  launch_stat(g, f, k, c->st_jobs.data(), c->d_st_jobs, (int)c->st_jobs.size(), c->d_st_lev, g.nk + 1, c->st_nch, c->d_st_ops, nops,
               c->d_rstat, c->stream, &c->nlaunch);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return set_err(CM1G_ERR_CUDA, "%s", cudaGetErrorString(e));

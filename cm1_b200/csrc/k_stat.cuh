@@ -39,9 +39,9 @@ struct StatJob {
   float r1, r2;       // interpolation weights of SK_WLEV
 };
 
+// one chunk of one level of a job: its extrema, or the sums of a budget
 struct StatLev {
   float vmax, vmin;
-  int imax, imin;     // first location in the level (linear index over the i-j range)
   double s[4];
 };
 // records: [job][level][chunk]
@@ -75,10 +75,16 @@ struct StatConsts {
   const float *zh, *zf;                               // level heights (device, index k)
 };
 
-// chunks of one level of npl points (the first grid dimension of k_stat_levels)
-int stat_chunks(int npl);
-void launch_stat(const DGrid &g, const StatFields &f, const StatConsts &s, const StatJob *jobs, int njobs,
-                 StatLev *lev, int maxlev, int nch, const StatOp *ops, int nops, float *rstat, cudaStream_t st,
+// the jobs of one k_stat_levels launch
+constexpr int ST_MAXREST = 64;
+struct StatRest { int n; int job[ST_MAXREST], first[ST_MAXREST]; };
+
+// chunks of one level of npl points on a grid of nlev levels (the first grid
+// dimension of k_stat_flow and k_stat_levels)
+int stat_chunks(int npl, int nlev);
+// hjobs and jobs: the job list on the host and on the device
+void launch_stat(const DGrid &g, const StatFields &f, const StatConsts &s, const StatJob *hjobs, const StatJob *jobs,
+                 int njobs, StatLev *lev, int maxlev, int nch, const StatOp *ops, int nops, float *rstat, cudaStream_t st,
                  int64_t *nl);
 
 }  // namespace cm1g
