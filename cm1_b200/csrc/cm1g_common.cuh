@@ -104,11 +104,20 @@ __device__ __forceinline__ float flx5(float s1, float s2, float s3, float s4, fl
 // The fast path folds the three divisions into one over the common
 // denominator d1^2 d2^2 d3^2.  Both binary64 results lie within 17 units of
 // the last binary64 place, times max|q_i|, of the exact weighted average, so
-// they differ by less than 2^-46 max|q_i|; when the folded value is farther
-// than that from both ends of the rounding interval of its binary32 result,
-// the reference's value rounds to the same binary32 number.  Otherwise (about
-// one face in a million) the face is evaluated exactly as the reference
-// does, so the result is always the reference's binary32 value.
+// they differ by less than 2^-46 max|q_i|.  Where the folded value v, in
+// [2^E, 2^(E+1)), is within a factor 1024 of max|q_i|, that is less than 2^17
+// units of its last place 2^(E-52); binary32 rounding discards v's last 29
+// bits and changes where they are 2^28, so when they are farther than 2^17
+// from that, the reference's value rounds to the same binary32 number.
+// Otherwise (about one face in two thousand, and values a thousand times
+// smaller than their stencil, as at the edge of a tracer) the distance is
+// formed in binary64, and where that does not decide either the face is
+// evaluated exactly as the reference does, so the result is always the
+// reference's binary32 value.
+//
+// Products by 2, 4 and 0.25 are exact, so fusing them with the addition that
+// follows gives the binary32 value of the separate operations; the folded
+// binary64 path fuses freely.
 static __device__ __noinline__ float weno5_ref(double b1, double b2, double b3, float q1, float q2, float q3,
                                                double weps) {
   const double tau = fabs(b1 - b3);
@@ -123,38 +132,40 @@ static __device__ __noinline__ float weno5_ref(double b1, double b2, double b3, 
 __device__ __forceinline__ float weno5(float s1, float s2, float s3, float s4, float s5, double weps) {
   const float c1312 = 13.0f / 12.0f;
   float t, u;
-  t = (s1 - 2.0f * s2) + s3; u = (s1 - 4.0f * s2) + 3.0f * s3;
-  double b1 = (double)(c1312 * (t * t) + 0.25f * (u * u));
-  t = (s2 - 2.0f * s3) + s4; u = s2 - s4;
-  double b2 = (double)(c1312 * (t * t) + 0.25f * (u * u));
-  t = (s3 - 2.0f * s4) + s5; u = (3.0f * s3 - 4.0f * s4) + s5;
-  double b3 = (double)(c1312 * (t * t) + 0.25f * (u * u));
-  float q1 = ((2.0f / 6.0f) * s1 + (-7.0f / 6.0f) * s2) + (11.0f / 6.0f) * s3;
-  float q2 = ((-1.0f / 6.0f) * s2 + (5.0f / 6.0f) * s3) + (2.0f / 6.0f) * s4;
-  float q3 = ((2.0f / 6.0f) * s3 + (5.0f / 6.0f) * s4) + (-1.0f / 6.0f) * s5;
-  double tau = fabs(b1 - b3);
-  double d1 = b1 + weps, d2 = b2 + weps, d3 = b3 + weps;
-  double tt = tau * tau;
-  if (tau < 1.0e30 * d1 && tau < 1.0e30 * d2 && tau < 1.0e30 * d3) {
-    double e1 = d1 * d1, e2 = d2 * d2, e3 = d3 * d3;
-    double a1 = (double)0.1f * (e1 + tt) * (e2 * e3);
-    double a2 = (double)0.6f * (e2 + tt) * (e1 * e3);
-    double a3 = (double)0.3f * (e3 + tt) * (e1 * e2);
-    double num = (a1 * (double)q1 + a2 * (double)q2) + a3 * (double)q3;
-    double den = (a1 + a2) + a3;
-    const double v = num / den;
+  t = __fmaf_rn(-2.0f, s2, s1) + s3; u = __fmaf_rn(-4.0f, s2, s1) + 3.0f * s3;
+  const float f1 = __fmaf_rn(0.25f, u * u, c1312 * (t * t));
+  t = __fmaf_rn(-2.0f, s3, s2) + s4; u = s2 - s4;
+  const float f2 = __fmaf_rn(0.25f, u * u, c1312 * (t * t));
+  t = __fmaf_rn(-2.0f, s4, s3) + s5; u = __fmaf_rn(-4.0f, s4, 3.0f * s3) + s5;
+  const float f3 = __fmaf_rn(0.25f, u * u, c1312 * (t * t));
+  const float q1 = ((2.0f / 6.0f) * s1 + (-7.0f / 6.0f) * s2) + (11.0f / 6.0f) * s3;
+  const float q2 = ((-1.0f / 6.0f) * s2 + (5.0f / 6.0f) * s3) + (2.0f / 6.0f) * s4;
+  const float q3 = ((2.0f / 6.0f) * s3 + (5.0f / 6.0f) * s4) + (-1.0f / 6.0f) * s5;
+  const double b1 = (double)f1, b2 = (double)f2, b3 = (double)f3;
+  const double tau = fabs(b1 - b3);
+  const double d1 = b1 + weps, d2 = b2 + weps, d3 = b3 + weps;
+  // no weight reaches its bound 1e30 where tau < 2^98 weps (compared by exponent)
+  if (__double2hiint(tau) < __double2hiint(weps) + (98 << 20) ||
+      (tau < 1.0e30 * d1 && tau < 1.0e30 * d2 && tau < 1.0e30 * d3)) {
+    const double tt = tau * tau, e1 = d1 * d1, e2 = d2 * d2, e3 = d3 * d3;
+    const double a1 = (double)0.1f * (e1 + tt) * (e2 * e3);
+    const double a2 = (double)0.6f * (e2 + tt) * (e1 * e3);
+    const double a3 = (double)0.3f * (e3 + tt) * (e1 * e2);
+    const double num = __fma_rn(a3, (double)q3, __fma_rn(a2, (double)q2, a1 * (double)q1));
+    const double v = num / ((a1 + a2) + a3);
     const float f = (float)v;
     const float qm = fmaxf(fmaxf(fabsf(q1), fabsf(q2)), fabsf(q3));
+    const int off = abs((__double2loint(v) & 0x1fffffff) - 0x10000000);
+    // the floor 1.2e-35 keeps f a normal binary32 number
+    if (off > (1 << 17) && fabsf(f) * 1024.0f >= fmaxf(qm, 1.2e-35f)) return f;
     if (qm == 0.0f) return 0.0f;   // q1 = q2 = q3 = 0: both forms give exactly 0
-    // e = v - f is exact (Sterbenz); f's rounding interval reaches h = 2^(E-24)
-    // on each side (E = the binary exponent of f), h/2 toward zero when f is a
-    // power of two; v's binary32 rounding is safe when |e| + delta < h.
-    const double fd = (double)f;
-    const double e = v - fd;
+    // the same test for any |v|: e = v - f is exact (Sterbenz); f's rounding
+    // interval reaches h = 2^(E-24) on each side (E = the binary exponent of
+    // f), h/2 toward zero when f is a power of two
+    const double fd = (double)f, e = v - fd;
     double h = __hiloint2double(__double2hiint(fd) & 0x7ff00000, 0) * 5.9604644775390625e-08;   // 2^-24
     if ((__float_as_int(f) & 0x7fffff) == 0) h = 0.5 * h;
-    const double delta = (double)qm * 1.4210854715202004e-14;   // 2^-46
-    if (fabs(e) + delta < h) return f;
+    if (fabs(e) + (double)qm * 1.4210854715202004e-14 < h) return f;                            // 2^-46
   }
   return weno5_ref(b1, b2, b3, q1, q2, q3, weps);
 }
