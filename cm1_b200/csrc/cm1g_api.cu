@@ -645,7 +645,6 @@ static void run_solve2(cm1g_ctx *c, const cm1g_state_t *d, float dt, double mass
     }
     launch_stage_prep(g, th_in, d->pp3d, qv_in, liq, cf.imoist, cf.eqtset, c->t11, c->t22, c->thterm, c->piadv, st,
                       nl);
-    launch_bc(g, c->t11, 2, 0, st, nl);
     if (diffit) df.coef = cf.kdiff6 / 64.0f / dttmp;   // adv.F:80-82, 962-964
     launch_adv_momentum(g, d->u3d, d->v3d, d->w3d, d->uten1, d->vten1, d->wten1, c->uten, c->vten, c->wten,
                         th_in, qv_in, c->mdivx, st, nl, diffit ? &df : nullptr, liq.b8);
@@ -768,7 +767,6 @@ static void run_solve3(cm1g_ctx *c, const cm1g_state_t *d) {
     launch_bc_batch(g, arr.data(), which.data(), nullptr, (int)arr.size(), st, nl);
   }
   launch_ppx_update(g, d->pp3d, d->ppx, st, nl);
-  launch_bc(g, d->ppx, 2, 0, st, nl);
   // solve3.F:546-640 rollover
   {
     std::vector<const float *> src;

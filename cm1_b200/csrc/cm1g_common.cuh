@@ -79,6 +79,16 @@ __host__ __device__ __forceinline__ long nW(const DGrid &g) { return (long)g.NI 
 
 #define LDG(p) __ldg(p)
 
+// The physical point that the fills of a scalar copy to the halo point at n
+// of 1..N along one direction (bc.F:180-518: periodic, open, or a wall's
+// mirror image; a single row beyond the edge copies the edge in every
+// non-periodic case).
+__device__ __forceinline__ int bc_source(int n, int N, int lo, int hi) {
+  if (n < 1) return lo == 1 ? n + N : lo == 2 ? 1 : 1 - n;
+  if (n > N) return hi == 1 ? n - N : hi == 2 ? N : 2 * N + 1 - n;
+  return n;
+}
+
 // brings the line of p into L2; the marching kernels call it for the levels ahead
 __device__ __forceinline__ void prefetch_l2(const float *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 

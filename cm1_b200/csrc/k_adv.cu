@@ -1161,8 +1161,9 @@ __global__ void k_advs_pdef2(DGrid g, SAdv a, const float *__restrict__ advx, co
 
 // Tiled form of pass 2: a block owns TX x TY columns and marches upward;
 // each level's dumx (with its +-2 halo in x) and dumy (+-2 in y) are staged
-// in shared memory (double-buffered, one barrier per level), dumz comes
-// from a per-column register window, and every read of a level is issued
+// in shared memory (double-buffered, one barrier per level; beyond the domain's
+// edges from the points that the lateral bc copies there, pdef.F:102, 338),
+// dumz comes from a per-column register window, and every read of a level is issued
 // one level ahead.  Same arithmetic as k_advs_pdef2.
 template <int TX, int TY, int KC>
 __global__ void __launch_bounds__(TX * TY) k_advs_pdef2_tile(DGrid g, SAdv a, const float *__restrict__ advx,
@@ -1192,7 +1193,7 @@ __global__ void __launch_bounds__(TX * TY) k_advs_pdef2_tile(DGrid g, SAdv a, co
     xo[q] = -1; xs[q] = 0;
     if (t < XW * TY) {
       const int yy = t / XW, xx = t - yy * XW, ii = i0 - 2 + xx, jj = j0 + yy;
-      if (ii <= ni + 2 && jj <= nj) { xo[q] = (ii - g.ib) + NI * (jj - g.jb); xs[q] = t; }
+      if (ii <= ni + 2 && jj <= nj) { xo[q] = (bc_source(ii, ni, g.wbc, g.ebc) - g.ib) + NI * (jj - g.jb); xs[q] = t; }
     }
   }
 #pragma unroll
@@ -1201,7 +1202,7 @@ __global__ void __launch_bounds__(TX * TY) k_advs_pdef2_tile(DGrid g, SAdv a, co
     yo[q] = -1; ys[q] = 0;
     if (t < TX * YH) {
       const int yy = t / TX, xx = t - yy * TX, ii = i0 + xx, jj = j0 - 2 + yy;
-      if (ii <= ni && jj <= nj + 2) { yo[q] = (ii - g.ib) + NI * (jj - g.jb); ys[q] = t; }
+      if (ii <= ni && jj <= nj + 2) { yo[q] = (ii - g.ib) + NI * (bc_source(jj, nj, g.sbc, g.nbc) - g.jb); ys[q] = t; }
     }
   }
   const int kc0 = 1 + (int)blockIdx.z * KC, kc1 = min(nk, kc0 + KC - 1);
@@ -1563,8 +1564,6 @@ __global__ void __launch_bounds__(TX * (TY + 1), 3) k_advs_tile(DGrid g, SAdv a,
 }
 
 void launch_bc(const DGrid &g, float *a, int which, int wflag, cudaStream_t st, int64_t *nlaunch);
-void launch_bc_batch(const DGrid &g, float *const *arrays, const int *which, const int *wflag, int n,
-                     cudaStream_t st, int64_t *nlaunch);
 
 // One k_advs_tile launch: WENO and the 6th-order diffusion (a.df.rho set)
 // select compile-time variants, so the plain pass carries no diffusion code.
@@ -1601,11 +1600,6 @@ static void advs_tiled_shape(const DGrid &g, const SAdv &a, STileOut o, int weno
   {
     ProfScope _ps("k_advs_tile_pdef1", st);
     advs_tile_launch<TX, TY, KC, MODE_PDEF1>(grid, blk, st, weno, g, a, o, 1, pdefweno, weps, dt, flush);
-  }
-  {
-    float *arr[2] = {o.dumx, o.dumy};
-    const int which[2] = {1, 1};
-    launch_bc_batch(g, arr, which, nullptr, 2, st, nl);
   }
   {
     ProfScope _ps("k_advs_pdef2", st);

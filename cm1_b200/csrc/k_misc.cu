@@ -8,59 +8,81 @@ namespace cm1g {
 
 // ---------------------------------------------------------------------
 // stage set-up: theta_rho (t11), ppterm (t22), thterm (solve2.F:313-446)
-// on the interior and piadv = pi0+pp' on 0..ni+1 x 0..nj+1 (solve2.F:1027-1038)
+// on the interior and piadv = pi0+pp' on 0..ni+1 x 0..nj+1 (solve2.F:1027-1038).
+// On the ring around the interior t11 is formed from the point that bcp would
+// copy it from.  A thread takes SP_K levels, whose loads are issued together
+// (256x256x80, moist: one level a thread 62 us, four 45 us, 3.3 TB/s).
 // ---------------------------------------------------------------------
-__global__ void k_stage_prep(DGrid g, const float *__restrict__ th3d, const float *__restrict__ pp3d,
-                             const float *__restrict__ qv, LiquidIn liq, int imoist, int eqtset,
-                             float *__restrict__ t11, float *__restrict__ t22, float *__restrict__ thterm,
-                             float *__restrict__ piadv) {
-  const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);       // 0..ni+1
-  const int j = (int)blockIdx.y;                                     // 0..nj+1
-  const int k = 1 + (int)blockIdx.z;
-  if (i > g.ni + 1) return;
-  const long o = iS(g, i, j, k);
-  const float pp = LDG(&pp3d[o]);
-  piadv[o] = LDG(&g.pi0[k]) + pp;
-  if (i < 1 || i > g.ni || j < 1 || j > g.nj) return;
+static const int SP_K = 4;
+__global__ void __launch_bounds__(256) k_stage_prep(DGrid g, const float *__restrict__ th3d,
+                                                    const float *__restrict__ pp3d, const float *__restrict__ qv,
+                                                    LiquidIn liq, int imoist, int eqtset, float *__restrict__ t11,
+                                                    float *__restrict__ t22, float *__restrict__ thterm,
+                                                    float *__restrict__ piadv) {
+  const int i = (int)(blockIdx.x * 32 + threadIdx.x);               // 0..ni+1
+  const int j = (int)(blockIdx.y * 8 + threadIdx.y);                // 0..nj+1
+  const int k0 = 1 + (int)blockIdx.z * SP_K;
+  if (i > g.ni + 1 || j > g.nj + 1) return;
+  const int plane = g.NI * g.NJ;                                    // < 2^31 points (cm1g_init)
+  const int oc = (i - g.ib) + g.NI * (j - g.jb);
+  const int is = bc_source(i, g.ni, g.wbc, g.ebc), js = bc_source(j, g.nj, g.sbc, g.nbc);
+  const int sc = (is - g.ib) + g.NI * (js - g.jb);
+  const bool inside = sc == oc;
+  float pp[SP_K], th[SP_K], qq[SP_K], l0[SP_K], l1[SP_K];
+#pragma unroll
+  for (int m = 0; m < SP_K; m++) {
+    const int k = min(k0 + m, g.nk), o = k * plane + oc, s = k * plane + sc;
+    pp[m] = LDG(&pp3d[o]);
+    th[m] = LDG(&th3d[s]);
+    qq[m] = imoist ? LDG(&qv[s]) : 0.0f;
+    l0[m] = liq.n > 0 ? LDG(&liq.q[0][s]) : 0.0f;
+    l1[m] = liq.n > 1 ? LDG(&liq.q[1][s]) : 0.0f;
+  }
   const Consts &c = g.c;
-  const float th3 = LDG(&th3d[o]), th0 = LDG(&g.th0[k]), pi0 = LDG(&g.pi0[k]);
-  if (imoist) {
-    const float q = fmaxf(LDG(&qv[o]), 0.0f);
-    // dum2: the liquid species in index order (solve2.F:315-345); no ice
-    float d2 = 0.0f;
-    if (liq.n > 0) {
-      d2 = LDG(&liq.q[0][o]);
-      for (int n = 1; n < liq.n; n++) d2 = d2 + LDG(&liq.q[n][o]);
-    }
-    const float d3 = 0.0f;
-    const float qli = fmaxf(0.0f, d2 + d3);
-    // buoyancy dum8 at s-points (solve2.F:395-396) when liquid is present;
-    // without it k_mom_tile forms the same expression from theta and qv
-    if (liq.b8)
-      liq.b8[o] = c.g * ((th3 * LDG(&g.rth0[k]) + c.repsm1 * (q - LDG(&g.qv0[k]))) -
-                         ((qli - LDG(&g.qc0[k])) - LDG(&g.qi0[k])));
-    t11[o] = (th0 + th3) * (1.0f + c.reps * q) / ((1.0f + q) + qli);
-    if (eqtset == 2) {
-      const float cpli = c.cpl * fmaxf(0.0f, d2) + c.cpi * fmaxf(0.0f, d3);
-      const float cpm = (c.cp + c.cpv * q) + cpli;
-      const float cvm = 1.0f / ((c.cv + c.cvv * q) + cpli);
-      thterm[o] = (th0 + th3) * ((c.rd + c.rv * q) - c.rovcp * cpm) * cvm;
-      t22[o] = (pi0 + pp) * c.rovcp * cpm * cvm;
+#pragma unroll
+  for (int m = 0; m < SP_K; m++) {
+    const int k = k0 + m;
+    if (k > g.nk) break;
+    const int o = k * plane + oc;
+    const float th3 = th[m], th0 = LDG(&g.th0[k]), pi0 = LDG(&g.pi0[k]);
+    piadv[o] = pi0 + pp[m];
+    if (imoist) {
+      const float q = fmaxf(qq[m], 0.0f);
+      // dum2: the liquid species in index order (solve2.F:315-345); no ice
+      float d2 = 0.0f;
+      if (liq.n > 0) d2 = l0[m];
+      if (liq.n > 1) d2 = d2 + l1[m];
+      const float d3 = 0.0f;
+      const float qli = fmaxf(0.0f, d2 + d3);
+      t11[o] = (th0 + th3) * (1.0f + c.reps * q) / ((1.0f + q) + qli);
+      if (!inside) continue;
+      // buoyancy dum8 at s-points (solve2.F:395-396) when liquid is present;
+      // without it k_mom forms the same expression from theta and qv
+      if (liq.b8)
+        liq.b8[o] = c.g * ((th3 * LDG(&g.rth0[k]) + c.repsm1 * (q - LDG(&g.qv0[k]))) -
+                           ((qli - LDG(&g.qc0[k])) - LDG(&g.qi0[k])));
+      if (eqtset == 2) {
+        const float cpli = c.cpl * fmaxf(0.0f, d2) + c.cpi * fmaxf(0.0f, d3);
+        const float cpm = (c.cp + c.cpv * q) + cpli;
+        const float cvm = 1.0f / ((c.cv + c.cvv * q) + cpli);
+        thterm[o] = (th0 + th3) * ((c.rd + c.rv * q) - c.rovcp * cpm) * cvm;
+        t22[o] = (pi0 + pp[m]) * c.rovcp * cpm * cvm;
+      } else {
+        t22[o] = (pi0 + pp[m]) * c.rddcv;
+      }
     } else {
-      t22[o] = (pi0 + pp) * c.rddcv;
+      t11[o] = th0 + th3;
+      if (inside) t22[o] = (pi0 + pp[m]) * c.rddcv;
     }
-  } else {
-    t11[o] = th0 + th3;
-    t22[o] = (pi0 + pp) * c.rddcv;
   }
 }
 
 void launch_stage_prep(const DGrid &g, const float *th3d, const float *pp3d, const float *qv, const LiquidIn &liq,
                        int imoist, int eqtset, float *t11, float *t22, float *thterm, float *piadv, cudaStream_t st,
                        int64_t *nl) {
-  dim3 grid((g.ni + 2 + 127) / 128, g.nj + 2, g.nk);
-  // j index offset: blockIdx.y = j directly (0..nj+1)
-  { ProfScope _ps("k_stage_prep", st); k_stage_prep<<<grid, 128, 0, st>>>(g, th3d, pp3d, qv, liq, imoist, eqtset, t11, t22, thterm, piadv); }
+  dim3 grid((g.ni + 2 + 31) / 32, (g.nj + 2 + 7) / 8, (g.nk + SP_K - 1) / SP_K);
+  ProfScope _ps("k_stage_prep", st);
+  k_stage_prep<<<grid, dim3(32, 8), 0, st>>>(g, th3d, pp3d, qv, liq, imoist, eqtset, t11, t22, thterm, piadv);
   if (nl) *nl += 1;
 }
 
@@ -410,15 +432,37 @@ void launch_pdefq(const DGrid &g, float rmax, const float *rho, float *q, double
 }
 
 // ---------------------------------------------------------------------
-// solve3 pieces: ppx = pp3d + ppx (solve3.F:276-283) and the rollover
-// copies over the reference's ranges (solve3.F:546-640).
+// solve3 pieces: ppx = pp3d + ppx (solve3.F:276-283) with bcp's ring, whose
+// points are written by the thread that owns the point they copy; and the
+// rollover copies over the reference's ranges (solve3.F:546-640).
 // ---------------------------------------------------------------------
-__global__ void k_ppx_update(DGrid g, const float *__restrict__ pp3d, float *ppx) {
-  const int i = 1 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  const int j = 1 + (int)blockIdx.y, k = 1 + (int)blockIdx.z;
-  if (i > g.ni) return;
-  const long o = iS(g, i, j, k);
-  ppx[o] = LDG(&pp3d[o]) + ppx[o];
+static const int PX_K = 4;      // levels of a thread, loaded together
+__global__ void __launch_bounds__(256) k_ppx_update(DGrid g, const float *__restrict__ pp3d, float *__restrict__ ppx) {
+  const int i = 1 + (int)(blockIdx.x * 32 + threadIdx.x), j = 1 + (int)(blockIdx.y * 8 + threadIdx.y);
+  const int k0 = 1 + (int)blockIdx.z * PX_K;
+  const int ni = g.ni, nj = g.nj, NI = g.NI;
+  if (i > ni || j > nj) return;
+  const int plane = NI * g.NJ, oc = (i - g.ib) + NI * (j - g.jb);
+  float v[PX_K];
+#pragma unroll
+  for (int m = 0; m < PX_K; m++) {
+    const int o = min(k0 + m, g.nk) * plane + oc;
+    v[m] = LDG(&pp3d[o]) + ppx[o];
+  }
+  // ring columns and rows that bcp copies from this point (offsets from it; 0: none)
+  const int xw = (g.wbc == 1 ? i == ni : i == 1) ? -i : 0, xe = (g.ebc == 1 ? i == 1 : i == ni) ? ni + 1 - i : 0;
+  const int ys = (g.sbc == 1 ? j == nj : j == 1) ? -j * NI : 0, yn = (g.nbc == 1 ? j == 1 : j == nj) ? (nj + 1 - j) * NI : 0;
+#pragma unroll
+  for (int m = 0; m < PX_K; m++) {
+    if (k0 + m > g.nk) break;
+    float *r = ppx + (k0 + m) * plane + oc;
+    const float x = v[m];
+    r[0] = x;
+    if (xw) r[xw] = x;
+    if (xe) r[xe] = x;
+    if (ys) { r[ys] = x; if (xw) r[ys + xw] = x; if (xe) r[ys + xe] = x; }
+    if (yn) { r[yn] = x; if (xw) r[yn + xw] = x; if (xe) r[yn + xe] = x; }
+  }
 }
 
 // Rollover copies dst = src over i = ilo..ihi, j = jlo..jhi, k = 1..nk
@@ -447,8 +491,8 @@ __global__ void k_copy_batch(CopyBatch b) {
 }
 
 void launch_ppx_update(const DGrid &g, const float *pp3d, float *ppx, cudaStream_t st, int64_t *nl) {
-  dim3 grid((g.ni + 127) / 128, g.nj, g.nk);
-  { ProfScope _ps("k_ppx_update", st); k_ppx_update<<<grid, 128, 0, st>>>(g, pp3d, ppx); }
+  dim3 grid((g.ni + 31) / 32, (g.nj + 7) / 8, (g.nk + PX_K - 1) / PX_K);
+  { ProfScope _ps("k_ppx_update", st); k_ppx_update<<<grid, dim3(32, 8), 0, st>>>(g, pp3d, ppx); }
   if (nl) *nl += 1;
 }
 
