@@ -110,74 +110,110 @@ __device__ __forceinline__ float flx5(float s1, float s2, float s3, float s4, fl
 //
 // The reference (adv_routines.F:6166-6205) forms each weight with its own
 // binary64 division, w_i = c_i (1 + min(1e30, tau/(b_i+weps))^2), and the
-// face value as (w1 q1 + w2 q2 + w3 q3)/(w1 + w2 + w3) rounded to binary32.
-// The fast path folds the three divisions into one over the common
-// denominator d1^2 d2^2 d3^2.  Both binary64 results lie within 17 units of
-// the last binary64 place, times max|q_i|, of the exact weighted average, so
-// they differ by less than 2^-46 max|q_i|.  Where the folded value v, in
-// [2^E, 2^(E+1)), is within a factor 1024 of max|q_i|, that is less than 2^17
-// units of its last place 2^(E-52); binary32 rounding discards v's last 29
-// bits and changes where they are 2^28, so when they are farther than 2^17
-// from that, the reference's value rounds to the same binary32 number.
-// Otherwise (about one face in two thousand, and values a thousand times
-// smaller than their stencil, as at the edge of a tracer) the distance is
-// formed in binary64, and where that does not decide either the face is
-// evaluated exactly as the reference does, so the result is always the
-// reference's binary32 value.
+// face value as (w1 q1 + w2 q2 + w3 q3)/(w1 + w2 + w3) rounded to binary32
+// (weno5_exact).  weno5_fast folds the three divisions into one over the common
+// denominator d1^2 d2^2 d3^2.  The weights are positive and each has a
+// relative error of a few units of the last binary64 place, so both binary64
+// results lie within 17 such units, times A = (w1 |q1| + w2 |q2| + w3 |q3|) /
+// (w1 + w2 + w3), of the exact weighted average: they differ by less than
+// 2^-46 A.  Where the folded value v, in [2^E, 2^(E+1)), is within a factor
+// 1024 of A, that is less than 2^17 units of its last place 2^(E-52); binary32
+// rounding discards v's last 29 bits and changes where they are 2^28, so when
+// they are farther than 2^17 from that, the reference's value rounds to the
+// same binary32 number.  Otherwise (one face in two thousand, and values a
+// thousand times smaller than their terms) v - 2^-46 A and v + 2^-46 A are both
+// rounded: where they agree, the reference's value between them does too.  Where
+// not (a tie to 14 digits, which the nominal weights make of neighbouring
+// candidate values; a weight at its bound), weno5_fast returns NaN and its caller
+// evaluates the face with weno5_exact, from the stencil where it lies, so that a
+// kernel's main loop holds nothing for it.
 //
 // Products by 2, 4 and 0.25 are exact, so fusing them with the addition that
 // follows gives the binary32 value of the separate operations; the folded
 // binary64 path fuses freely.
-static __device__ __noinline__ float weno5_ref(double b1, double b2, double b3, float q1, float q2, float q3,
-                                               double weps) {
-  const double tau = fabs(b1 - b3);
-  double r;
-  r = fmin(1.0e30, tau / (b1 + weps)); double w1 = (double)0.1f * (1.0 + r * r);
-  r = fmin(1.0e30, tau / (b2 + weps)); double w2 = (double)0.6f * (1.0 + r * r);
-  r = fmin(1.0e30, tau / (b3 + weps)); double w3 = (double)0.3f * (1.0 + r * r);
-  double num = (w1 * (double)q1 + w2 * (double)q2) + w3 * (double)q3;
-  double den = (w1 + w2) + w3;
-  return (float)(num / den);
-}
-__device__ __forceinline__ float weno5(float s1, float s2, float s3, float s4, float s5, double weps) {
+// smoothness indicators and the three candidate values of a stencil
+struct Weno5Terms { float f1, f2, f3, q1, q2, q3; };
+__device__ __forceinline__ Weno5Terms weno5_terms(float s1, float s2, float s3, float s4, float s5) {
   const float c1312 = 13.0f / 12.0f;
+  Weno5Terms w;
   float t, u;
   t = __fmaf_rn(-2.0f, s2, s1) + s3; u = __fmaf_rn(-4.0f, s2, s1) + 3.0f * s3;
-  const float f1 = __fmaf_rn(0.25f, u * u, c1312 * (t * t));
+  w.f1 = __fmaf_rn(0.25f, u * u, c1312 * (t * t));
   t = __fmaf_rn(-2.0f, s3, s2) + s4; u = s2 - s4;
-  const float f2 = __fmaf_rn(0.25f, u * u, c1312 * (t * t));
+  w.f2 = __fmaf_rn(0.25f, u * u, c1312 * (t * t));
   t = __fmaf_rn(-2.0f, s4, s3) + s5; u = __fmaf_rn(-4.0f, s4, 3.0f * s3) + s5;
-  const float f3 = __fmaf_rn(0.25f, u * u, c1312 * (t * t));
-  const float q1 = ((2.0f / 6.0f) * s1 + (-7.0f / 6.0f) * s2) + (11.0f / 6.0f) * s3;
-  const float q2 = ((-1.0f / 6.0f) * s2 + (5.0f / 6.0f) * s3) + (2.0f / 6.0f) * s4;
-  const float q3 = ((2.0f / 6.0f) * s3 + (5.0f / 6.0f) * s4) + (-1.0f / 6.0f) * s5;
-  const double b1 = (double)f1, b2 = (double)f2, b3 = (double)f3;
+  w.f3 = __fmaf_rn(0.25f, u * u, c1312 * (t * t));
+  w.q1 = ((2.0f / 6.0f) * s1 + (-7.0f / 6.0f) * s2) + (11.0f / 6.0f) * s3;
+  w.q2 = ((-1.0f / 6.0f) * s2 + (5.0f / 6.0f) * s3) + (2.0f / 6.0f) * s4;
+  w.q3 = ((2.0f / 6.0f) * s3 + (5.0f / 6.0f) * s4) + (-1.0f / 6.0f) * s5;
+  return w;
+}
+// n/d rounded to nearest by Markstein's method (IBM J. Res. Dev. 34, 1990):
+// Newton's iteration gives 1/d to the last place, and one correction of n/d by
+// its exact residual rounds correctly.  For d > 1e-60 and quotients and operands
+// below 1e200, or not finite.  Unlike the operator it has no subroutine for
+// the extremes of the range, whose call would cost the main loop registers.
+__device__ __forceinline__ double div_rn(double n, double d) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+  y = __fma_rn(y, __fma_rn(-d, y, 1.0), y);
+  y = __fma_rn(y, __fma_rn(-d, y, 1.0), y);
+  y = __fma_rn(y, __fma_rn(-d, y, 1.0), y);
+  const double q = n * y;
+  return d < 1.0e300 ? __fma_rn(__fma_rn(-d, q, n), y, q) : n * 0.0;
+}
+__device__ __forceinline__ float weno5_exact(float s1, float s2, float s3, float s4, float s5, double weps) {
+  const Weno5Terms w = weno5_terms(s1, s2, s3, s4, s5);
+  if (w.q1 == 0.0f && w.q2 == 0.0f && w.q3 == 0.0f) return 0.0f;
+  const double b1 = (double)w.f1, b2 = (double)w.f2, b3 = (double)w.f3;
+  const double tau = fabs(b1 - b3);
+  double r;
+  r = fmin(1.0e30, div_rn(tau, b1 + weps)); const double w1 = (double)0.1f * (1.0 + r * r);
+  r = fmin(1.0e30, div_rn(tau, b2 + weps)); const double w2 = (double)0.6f * (1.0 + r * r);
+  r = fmin(1.0e30, div_rn(tau, b3 + weps)); const double w3 = (double)0.3f * (1.0 + r * r);
+  const double num = (w1 * (double)w.q1 + w2 * (double)w.q2) + w3 * (double)w.q3;
+  return (float)div_rn(num, (w1 + w2) + w3);
+}
+__device__ __forceinline__ float weno5_fast(float s1, float s2, float s3, float s4, float s5, double weps) {
+  // a stencil of zeros, which fills most of a tracer's or a hydrometeor's field
+  const int any = __float_as_int(s1) | __float_as_int(s2) | __float_as_int(s3) | __float_as_int(s4) | __float_as_int(s5);
+  if ((any << 1) == 0) return 0.0f;
+  const Weno5Terms w = weno5_terms(s1, s2, s3, s4, s5);
+  const double b1 = (double)w.f1, b2 = (double)w.f2, b3 = (double)w.f3;
   const double tau = fabs(b1 - b3);
   const double d1 = b1 + weps, d2 = b2 + weps, d3 = b3 + weps;
-  // no weight reaches its bound 1e30 where tau < 2^98 weps (compared by exponent)
-  if (__double2hiint(tau) < __double2hiint(weps) + (98 << 20) ||
-      (tau < 1.0e30 * d1 && tau < 1.0e30 * d2 && tau < 1.0e30 * d3)) {
-    const double tt = tau * tau, e1 = d1 * d1, e2 = d2 * d2, e3 = d3 * d3;
-    const double a1 = (double)0.1f * (e1 + tt) * (e2 * e3);
-    const double a2 = (double)0.6f * (e2 + tt) * (e1 * e3);
-    const double a3 = (double)0.3f * (e3 + tt) * (e1 * e2);
-    const double num = __fma_rn(a3, (double)q3, __fma_rn(a2, (double)q2, a1 * (double)q1));
-    const double v = num / ((a1 + a2) + a3);
-    const float f = (float)v;
-    const float qm = fmaxf(fmaxf(fabsf(q1), fabsf(q2)), fabsf(q3));
-    const int off = abs((__double2loint(v) & 0x1fffffff) - 0x10000000);
-    // the floor 1.2e-35 keeps f a normal binary32 number
-    if (off > (1 << 17) && fabsf(f) * 1024.0f >= fmaxf(qm, 1.2e-35f)) return f;
-    if (qm == 0.0f) return 0.0f;   // q1 = q2 = q3 = 0: both forms give exactly 0
-    // the same test for any |v|: e = v - f is exact (Sterbenz); f's rounding
-    // interval reaches h = 2^(E-24) on each side (E = the binary exponent of
-    // f), h/2 toward zero when f is a power of two
-    const double fd = (double)f, e = v - fd;
-    double h = __hiloint2double(__double2hiint(fd) & 0x7ff00000, 0) * 5.9604644775390625e-08;   // 2^-24
-    if ((__float_as_int(f) & 0x7fffff) == 0) h = 0.5 * h;
-    if (fabs(e) + (double)qm * 1.4210854715202004e-14 < h) return f;                            // 2^-46
-  }
-  return weno5_ref(b1, b2, b3, q1, q2, q3, weps);
+  const double tt = tau * tau, e1 = d1 * d1, e2 = d2 * d2, e3 = d3 * d3;
+  const double a1 = (double)0.1f * (e1 + tt) * (e2 * e3);
+  const double a2 = (double)0.6f * (e2 + tt) * (e1 * e3);
+  const double a3 = (double)0.3f * (e3 + tt) * (e1 * e2);
+  const double p1 = (double)w.q1, p2 = (double)w.q2, p3 = (double)w.q3;
+  const double num = __fma_rn(a3, p3, __fma_rn(a2, p2, a1 * p1));
+  const double A = __fma_rn(a3, fabs(p3), __fma_rn(a2, fabs(p2), a1 * fabs(p1)));   // times the denominator
+  const double den = (a1 + a2) + a3;
+  // num/den to a few units of the last place: Newton's iteration for 1/den from
+  // the 20 bits of rcp.approx.ftz.f64 (once: 40 bits), then one correction of
+  // the quotient by its residual; not a number where den has no normal reciprocal
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(den));
+  y = __fma_rn(y, __fma_rn(-den, y, 1.0), y);
+  const double v0 = num * y, v = __fma_rn(__fma_rn(-den, v0, num), y, v0);
+  const float f = (float)v;
+  // v's last 29 bits against 2^28 -+ 2^17, without the bits above them
+  const unsigned off = 8u * (unsigned)__double2loint(v) - 8u * ((1u << 28) - (1u << 17));
+  // no weight reaches its bound 1e30 where tau < 2^98 (b_i + weps), by exponent;
+  // the floor 1.2e-35 keeps f a normal binary32 number
+  const int ht = __double2hiint(tau) - (98 << 20);
+  if (ht < __double2hiint(weps) && off > 8u << 18 && fabs(num) * 1024.0 >= A && fabsf(f) >= 1.2e-35f) return f;
+  const double e = A * y * 0x1p-46;
+  const float lo = (float)(v - e), hi = (float)(v + e);
+  if (ht < __double2hiint((double)fminf(fminf(w.f1, w.f2), w.f3) + weps) && lo == hi &&
+      __float_as_int(lo) == __float_as_int(hi))
+    return f;
+  return __int_as_float(0x7fffffff);
+}
+__device__ __forceinline__ float weno5(float s1, float s2, float s3, float s4, float s5, double weps) {
+  const float f = weno5_fast(s1, s2, s3, s4, s5, weps);
+  return f != f ? weno5_exact(s1, s2, s3, s4, s5, weps) : f;
 }
 
 __device__ __forceinline__ float upstrpd(float s1, float s2, float s3, double weps) {

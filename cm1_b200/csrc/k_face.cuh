@@ -87,27 +87,49 @@ __device__ __forceinline__ float zflux_win(const DGrid &g, const float *wv, floa
                                            double weps) {
   return zflux_core(wv, r, kk, g.nk, LDG(&g.c1[kk]), LDG(&g.c2[kk]), weno, pdefweno, weps);
 }
-// The same face where 4 <= kk <= nk-2 (full 5-point stencils on both sides),
-// the case of every level but the two lowest and two highest faces.
-__device__ __forceinline__ float zflux_inner(const float *wv, float r, int weno, int pdefweno, double weps) {
-  auto A = [&](int d) { return wv[d + 3]; };
+// A face value in the reference's upwind order with the full 5-point stencil on
+// both sides; NaN where weno5_fast leaves it undecided.  sm3..sp2 are the values
+// around the face between sm1 and s0.  pdef: stencils below weps give 0
+// (adv_routines.F:2386-2421).
+__device__ __forceinline__ float face5(float r, float sm3, float sm2, float sm1, float s0, float sp1, float sp2, int weno,
+                                       int pdef, double weps) {
   const bool up = (r >= 0.0f);
-  const float s1 = up ? A(-3) : A(2), s2 = up ? A(-2) : A(1), s3 = up ? A(-1) : A(0), s4 = up ? A(0) : A(-1),
-              s5 = up ? A(1) : A(-2);
+  const float s1 = up ? sm3 : sp2, s2 = up ? sm2 : sp1, s3 = up ? sm1 : s0, s4 = up ? s0 : sm1, s5 = up ? sp1 : sm2;
   if (!weno) return r * flx5(s1, s2, s3, s4, s5);
-  if (pdefweno == 1) return (absmax5(s1, s2, s3, s4, s5) > (float)weps) ? r * weno5(s1, s2, s3, s4, s5, weps) : 0.0f;
-  return r * weno5(s1, s2, s3, s4, s5, weps);
+  if (pdef == 1 && !(absmax5(s1, s2, s3, s4, s5) > (float)weps)) return 0.0f;
+  return r * weno5_fast(s1, s2, s3, s4, s5, weps);
 }
-
-// horizontal face flux from five upwind-ordered values
-__device__ __forceinline__ float hflux5(float r, float sm3, float sm2, float sm1, float s0, float sp1, float sp2,
-                                        int weno, int pdef, double weps) {
-  float s1, s2, s3, s4, s5;
-  if (r >= 0.0f) { s1 = sm3; s2 = sm2; s3 = sm1; s4 = s0; s5 = sp1; }
-  else { s1 = sp2; s2 = sp1; s3 = s0; s4 = sm1; s5 = sm2; }
+// horizontal face flux, every value decided (weno5)
+__device__ __forceinline__ float hflux5(float r, float sm3, float sm2, float sm1, float s0, float sp1, float sp2, int weno,
+                                        int pdef, double weps) {
+  const bool up = (r >= 0.0f);
+  const float s1 = up ? sm3 : sp2, s2 = up ? sm2 : sp1, s3 = up ? sm1 : s0, s4 = up ? s0 : sm1, s5 = up ? sp1 : sm2;
   if (!weno) return r * flx5(s1, s2, s3, s4, s5);
   if (pdef == 1 && !(absmax5(s1, s2, s3, s4, s5) > (float)weps)) return 0.0f;
   return r * weno5(s1, s2, s3, s4, s5, weps);
+}
+// the same face with weno5_exact
+__device__ __forceinline__ float face5_exact(float r, float sm3, float sm2, float sm1, float s0, float sp1, float sp2,
+                                             double weps) {
+  const bool up = (r >= 0.0f);
+  return r * weno5_exact(up ? sm3 : sp2, up ? sm2 : sp1, up ? sm1 : s0, up ? s0 : sm1, up ? sp1 : sm2, weps);
+}
+// The vertical face at level kk (2..nk) of a column, wv[d+3] = s(kk+d): fz is
+// face5's value, which the two lowest and the two highest faces replace where
+// the 5-point stencil does not fit (zflux_core's cases).
+__device__ __forceinline__ float zface_edge(float fz, const float *wv, float r, int kk, int nk, const float *c1,
+                                            const float *c2, int weno, int pdefweno, double weps) {
+  if (kk == 2 || kk == nk) {
+    const bool lin = kk == 2 ? r >= 0.0f : weno ? !(r > 0.0f) : !(r >= 0.0f);
+    if (lin) return r * (LDG(&c1[kk]) * wv[2] + LDG(&c2[kk]) * wv[3]);
+  } else if (kk == 3) {
+    if (!(weno && pdefweno == 1 ? r > 0.0f : r >= 0.0f)) return fz;
+  } else {
+    if (r >= 0.0f || (weno && pdefweno == 1 && !(r < 0.0f))) return fz;
+  }
+  const bool hi = kk == nk || kk == 3;   // upwind from below
+  const float s1 = hi ? wv[1] : wv[4], s2 = hi ? wv[2] : wv[3], s3 = hi ? wv[3] : wv[2];
+  return r * (weno ? upstrpd(s1, s2, s3, weps) : flx3(s1, s2, s3));
 }
 
 }  // namespace cm1g

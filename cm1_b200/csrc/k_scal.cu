@@ -17,12 +17,21 @@
 //    the plane's row pitch SP is chosen congruent to NI modulo 4, so that
 //    every row lands with element x at plane[c + r*SP + x] for a c that is
 //    the same for all rows of the plane;
-//  * each x- and y-face flux is evaluated once (hflux5, the WENO5 or
+//  * each x- and y-face flux is evaluated once (face5, the WENO5 or
 //    5th-order value), the vertical face of the level above comes from a
-//    per-thread register window of the column (zflux_win) and is carried to
-//    the next level;
+//    per-thread register window of the column and is carried to the next level;
 //  * one barrier per item: the face fluxes and face velocities are double
 //    buffered by item parity.
+//
+// Bound by instruction issue: three faces are some 400 of an item's 730
+// instructions, at 24 warps a SM (80 registers).  So the faces that the fast
+// WENO5 leaves open are evaluated beside it from shared memory without a call,
+// the item's global reads are issued after its faces and not before (their
+// registers are then free while a face is evaluated), and a flux lies beside
+// its velocity in one 8-byte word.  256x256x80, seven fields: 1.33 ms a stage
+// where the faces at a tracer's edge and in uniform layers took the reference's
+// divisions one by one, now 1.14 ms; 512x512x128, three fields: 4.1 to 2.95 ms.
+// (Two blocks a SM without the limit of 80 registers: 10 % slower.)
 //
 // Every face value and the update use the operations of k_advs_tile in the
 // same order, so the result is bit-identical to advancing the fields one
@@ -86,18 +95,80 @@ __host__ __device__ __forceinline__ int scal_pitch(int NI) {
   return p0 + (((NI - p0) % 4) + 4) % 4;
 }
 
+// Profiles of one level k of a block, read as two 16-byte words.
+struct __align__(16) ScLev {
+  float r0, rf, rf1, mh;     // rho0(k), rf0(k), rf0(k+1), mh(k)
+  float rr, th, th3, pad;    // rr0(k), th0(k)-300, th0(k+3)-300
+};
+
+// The stage's new value of one cell from its faces, (flux, averaged velocity)
+// each, with the open-boundary fix-ups of adv.F where the tile touches an open
+// edge; fz* and w* are the vertical fluxes and averaged velocities.
+__device__ __forceinline__ float scal_update(const DGrid &g, const ScalPass &P, const ScalField &F, float2 xw, float2 xe,
+                                             float2 ys, float2 yn, float fzlo, float fzhi, float wlo, float whi, float4 la,
+                                             float4 lb, int i, int j, int k, bool edge, float uh_i, float vh_j, float sc,
+                                             float ten, float base, float tht) {
+  const float r0k = la.x, mhk = la.w;
+  float fx0 = xw.x, fxp = xe.x, fy0 = ys.x, fyp = yn.x;
+  const float fu0 = xw.y * r0k, fu1 = xe.y * r0k, fv0 = ys.y * r0k, fv1 = yn.y * r0k;
+  const float rdx = g.rdx, rdy = g.rdy, rdz = g.rdz, smeps = g.smeps;
+  float advx, advy;
+  if (!edge) {
+    advx = -(fxp - fx0) * rdx * uh_i;
+    advy = -(fyp - fy0) * rdy * vh_j;
+  } else {
+    const bool w = g.wbc == 2 && g.ibw && i == 1 && fu0 >= 0.0f, e = g.ebc == 2 && g.ibe && i == g.ni && fu1 <= 0.0f;
+    const bool s = g.sbc == 2 && g.ibs && j == 1 && fv0 >= 0.0f, n = g.nbc == 2 && g.ibn && j == g.nj && fv1 <= 0.0f;
+    // adv.F:212-268
+    if (w) fx0 = fxp;
+    if (e) fxp = fx0;
+    if (s) fy0 = fyp;
+    if (n) fyp = fy0;
+    advx = -(fxp - fx0) * rdx * uh_i;
+    advy = -(fyp - fy0) * rdy * vh_j;
+    // adv.F:286-335
+    if (w) advx = advx - sc * (fu1 - fu0) * rdx * uh_i;
+    if (e) advx = advx - sc * (fu1 - fu0) * rdx * uh_i;
+    if (s) advy = advy - sc * (fv1 - fv0) * rdy * vh_j;
+    if (n) advy = advy - sc * (fv1 - fv0) * rdy * vh_j;
+  }
+  float advz;
+  if (k == 1) advz = -fzhi * rdz * mhk;
+  else if (k == g.nk) advz = +fzlo * rdz * mhk;
+  else advz = -(fzhi - fzlo) * rdz * mhk;
+  float div = ((fu1 - fu0) * rdx * uh_i + (fv1 - fv0) * rdy * vh_j) + (whi * la.z - wlo * la.y) * rdz * mhk;
+  if (fabsf(div) < smeps) div = 0.0f;
+  if (F.sadd && P.thterm) {   // getdiv of the averaged velocities (misclibs.F:127-136)
+    float rd = ((xe.y - xw.y) * rdx * uh_i + (yn.y - ys.y) * rdy * vh_j) + (whi - wlo) * rdz * mhk;
+    if (fabsf(rd) < smeps) rd = 0.0f;
+    ten = ten - rd * tht;
+  }
+  ten = ten + (((advx + advy) + advz) + sc * div) * lb.x;
+  float v = base + P.dt * ten;
+  if (F.flush && fabsf(v) < smeps) v = 0.0f;
+  return v;
+}
+
+__device__ __forceinline__ ScLev scal_level(const DGrid &g, int k) {
+  ScLev l;
+  l.r0 = LDG(&g.rho0[k]); l.rf = LDG(&g.rf0[k]); l.rf1 = LDG(&g.rf0[k + 1]); l.mh = LDG(&g.mh[k]);
+  l.rr = LDG(&g.rr0[k]); l.th = LDG(&g.th0[k]) - 300.0f;
+  l.th3 = k + 3 <= g.nk + 1 ? LDG(&g.th0[k + 3]) - 300.0f : 0.0f;
+  l.pad = 0.0f;
+  return l;
+}
+
 template <int TX, int TY, int KC, int WENO>
-__global__ void __launch_bounds__(TX * (TY + 1), 3) k_scal_tile(DGrid g, ScalPass P) {
-  constexpr int NT = TX * (TY + 1);
+__global__ void __launch_bounds__(TX * (TY + 1), 3) k_scal_tile(const __grid_constant__ DGrid g,
+                                                                 const __grid_constant__ ScalPass P) {
   constexpr int SW = TX + 6, SH = TY + 6;                  // staged columns and rows
   constexpr int RD = 4;                                     // ring of staged planes
   constexpr int PL = ((8 + (SH - 1) * (TX + 19) + TX + 12) + 3) / 4 * 4;   // floats per plane
   constexpr int NFX = (TX + 1) * TY, NFY = TX * (TY + 1);
-  constexpr int NL = KC + 8;                                // cached profile levels kc0-3 .. kc0+KC+4
   static_assert(SH <= 32, "one lane per staged row");
   __shared__ __align__(128) float ring[RD][PL];
-  __shared__ float fx[2][NFX], ux[2][NFX], fy[2][NFY], vy[2][NFY];
-  __shared__ float prof[7][NL];   // rho0, rf0, mh, rr0, th0-300, c1, c2 by level
+  __shared__ float2 fx[2][NFX], fy[2][NFY];                // flux and averaged velocity of each face
+  __shared__ ScLev lev[KC];
   __shared__ __align__(8) uint64_t bars[RD];
 
   const int tx = threadIdx.x, ty = threadIdx.y, tid = tx + TX * ty, lane = tid & 31;
@@ -107,62 +178,43 @@ __global__ void __launch_bounds__(TX * (TY + 1), 3) k_scal_tile(DGrid g, ScalPas
   const int i = i0 + tx, j = j0 + ty;
   const int ni = g.ni, nj = g.nj, nk = g.nk, NI = g.NI, NJ = g.NJ;
   const bool active = (ty < TY && i <= ni && j <= nj);
-  const bool doitw = (g.wbc == 2 && g.ibw), doite = (g.ebc == 2 && g.ibe);
-  const bool doits = (g.sbc == 2 && g.ibs), doitn = (g.nbc == 2 && g.ibn);
-  // the open-boundary fix-ups of adv.F touch only the cells next to an open edge
-  const bool edge = (doitw && i0 == 1) || (doite && i0 + TX - 1 >= ni) || (doits && j0 == 1) ||
-                    (doitn && j0 + TY - 1 >= nj);
-  const int je = nj + g.ngxy;
-  // 32-bit offsets: cm1g_init refuses arrays of 2^31 points or more
   const int planeS = NI * NJ, planeU = (NI + 1) * NJ, planeV = NI * (NJ + 1);
   const int SP = scal_pitch<TX>(NI);
   const float uh_i = active ? LDG(&g.uh[i - g.ib]) : 0.0f, vh_j = active ? LDG(&g.vh[j - g.jb]) : 0.0f;
-  const int oc = active ? (i - g.ib) + NI * (j - g.jb) : 0;   // the column's in-plane offset
   const int orow0 = (i0 - 3 - g.ib) + NI * (j0 - 3 - g.jb);    // first staged element of a plane
   const int kc0 = 1 + (int)blockIdx.z * KC, kc1 = min(nk, kc0 + KC - 1);
   const int nlev = kc1 - kc0 + 1, nitem = P.n * nlev;
-  const int kb0 = kc0 - 3;                                     // level of prof[.][0]
-  const float rdx = g.rdx, rdy = g.rdy, rdz = g.rdz, smeps = g.smeps, dt = P.dt;
 
   // faces of this thread: a cell row's thread owns the x face on the west of
   // its cell and the y face on its south; the extra row's threads own the y
   // faces north of the tile and (the first TY of them) the x faces east of it,
-  // so that every cell thread evaluates three faces and no thread more
-  int fxo = -1, fxs = 0, fyo = -1, fys = 0, fxd = NFX, fyd;
+  // so that every cell thread evaluates three faces and no thread more.
+  // oc: the thread's column in an s or v plane; xo: its x face in a u plane
+  // (bytes); xs, ys: the stencils' first values in a staged plane
+  const bool yface_on = (i <= ni && j <= nj + 1);
+  const int oc = yface_on ? (i - g.ib) + NI * (j - g.jb) : 0;
+  const int ys = ty * SP + tx + 3;
+  bool xface_on = false;
+  int xo = 0, xs = 0, xd = 0;
   {
-    int xrow = ty, xcol = tx;
-    if (ty == TY) { xrow = tx; xcol = TX; }
-    if (xrow < TY) {
-      fxd = xrow * (TX + 1) + xcol;
-      const int ii = i0 + xcol, jj = j0 + xrow;
-      if (ii <= ni + 1 && jj <= nj) { fxo = (ii - g.ib) + (NI + 1) * (jj - g.jb); fxs = (xrow + 3) * SP + xcol; }
+    const int xrow = ty < TY ? ty : tx, xcol = ty < TY ? tx : TX;
+    const int ii = i0 + xcol, jj = j0 + xrow;
+    if (xrow < TY && ii <= ni + 1 && jj <= nj) {
+      xface_on = true;
+      xo = (ii - g.ib) + (NI + 1) * (jj - g.jb);
+      xs = (xrow + 3) * SP + xcol;
+      xd = xrow * (TX + 1) + xcol;
     }
-    fyd = ty * TX + tx;
-    const int ii = i0 + tx, jj = j0 + ty;
-    if (ii <= ni && jj <= nj + 1) { fyo = (ii - g.ib) + NI * (jj - g.jb); fys = ty * SP + tx + 3; }
   }
-  const int csel = (ty + 3) * SP + tx + 3;   // the cell in a staged plane
-  const int xi = ty * (TX + 1) + tx, yi = ty * TX + tx;
 
-  // vertical profiles of the block's levels (0 outside 0..nk+1)
-  for (int e = tid; e < 7 * NL; e += NT) {
-    const int a = e / NL, k = kb0 + e - a * NL;
-    float v = 0.0f;
-    if (k >= 0 && k <= nk + 1) {
-      switch (a) {
-        case 0: v = LDG(&g.rho0[k]); break;
-        case 1: v = LDG(&g.rf0[k]); break;
-        case 2: v = LDG(&g.mh[k]); break;
-        case 3: v = LDG(&g.rr0[k]); break;
-        case 4: v = LDG(&g.th0[k]) - 300.0f; break;
-        case 5: v = LDG(&g.c1[k]); break;
-        default: v = LDG(&g.c2[k]); break;
-      }
-    }
-    prof[a][e - a * NL] = v;
+  // profiles of the block's levels (0 above nk+1, not used there)
+  if (tid < nlev) {
+    lev[tid] = scal_level(g, kc0 + tid);
   }
-  const float *PR0 = prof[0] - kb0, *PRF = prof[1] - kb0, *PMH = prof[2] - kb0, *PRR = prof[3] - kb0,
-              *PTH = prof[4] - kb0, *PC1 = prof[5] - kb0, *PC2 = prof[6] - kb0;
+
+  // the open-boundary fix-ups of adv.F touch only the cells next to an open edge
+  const bool edge = (g.wbc == 2 && g.ibw && i0 == 1) || (g.ebc == 2 && g.ibe && i0 + TX - 1 >= ni) ||
+                    (g.sbc == 2 && g.ibs && j0 == 1) || (g.nbc == 2 && g.ibn && j0 + TY - 1 >= nj);
 
   // ---- staging: items in order (field, level) -> ring slot item % RD
   const uint32_t bar0 = smem_u32(&bars[0]);
@@ -171,14 +223,14 @@ __global__ void __launch_bounds__(TX * (TY + 1), 3) k_scal_tile(DGrid g, ScalPas
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
-  // warp 0: the row copies of the item (field nf, level kf) into slot `slot`
-  // (rows beyond je are never read)
+  // the row copies of the item (field nf, level kf) into slot `slot` (rows
+  // beyond the last halo row are never read)
   auto issue = [&](int nf, int kf, int slot) {
     const float *p0 = P.f[nf].s + (kf * planeS + orow0);
     const int l0 = (int)(((uintptr_t)p0 >> 2) & 3);
     uint32_t bytes = 0, dst = 0;
     const float *src = nullptr;
-    if (lane < SH && j0 - 3 + lane <= je) {
+    if (lane < SH && j0 - 3 + lane <= nj + g.ngxy) {
       const uintptr_t a0 = (uintptr_t)(p0 + lane * NI);
       const uintptr_t as = a0 & ~(uintptr_t)15, ae = (a0 + 4 * SW + 15) & ~(uintptr_t)15;
       const int lr = (int)((a0 >> 2) & 3);
@@ -200,148 +252,116 @@ __global__ void __launch_bounds__(TX * (TY + 1), 3) k_scal_tile(DGrid g, ScalPas
   if (stager)
     while (it_ < RD && it_ < nitem) issue_next();
 
-  // ---- per-item global reads, issued one item ahead
-  float pru = 0.0f, prv = 0.0f, pwhi = 0.0f, pe0 = 0.0f, pe1 = 0.0f, pe2 = 0.0f, pwtop = 0.0f;
+  // ---- per-item global reads: issued once the previous item's faces are done,
+  // so that they are in flight during its update and take no register while a
+  // face is evaluated (the faces need nearly all 80 of them)
+  float ru = 0.0f, rv = 0.0f, whi = 0.0f, e0 = 0.0f, e1 = 0.0f, e2 = 0.0f, stop = 0.0f;
   auto fetch = [&](int nf, int kf) {
     const ScalField &F = P.f[nf];
-    const float *uk = P.rru + kf * planeU, *vk = P.rrv + kf * planeV;
-    pru = (fxo >= 0) ? LDG(&uk[fxo]) : 0.0f;
-    prv = (fyo >= 0) ? LDG(&vk[fyo]) : 0.0f;
+    if (xface_on) ru = LDG(&P.rru[kf * planeU + xo]);
+    if (yface_on) rv = LDG(&P.rrv[kf * planeV + oc]);
     if (active) {
       const int o = kf * planeS + oc;
-      pwhi = (kf + 1 >= nk + 1) ? 0.0f : LDG(&P.rrw[o + planeS]);
-      pe0 = F.ten1[o];
-      pe1 = LDG(&F.sbase[o]);
-      if (F.sadd && P.thterm) pe2 = LDG(&P.thterm[o]);
-      float v = 0.0f;
-      if (kf + 3 <= nk + 1) {
-        v = LDG(&F.s[o + 3 * planeS]);
-        if (F.sadd) v = PTH[kf + 3] + v;
-      }
-      pwtop = v;
+      whi = (kf == nk) ? 0.0f : LDG(&P.rrw[o + planeS]);
+      e0 = F.ten1[o];
+      e1 = LDG(&F.sbase[o]);
+      if (F.sadd && P.thterm) e2 = LDG(&P.thterm[o]);
+      // s(kf+3), the last value under the upper face of level kf
+      stop = (kf + 3 <= nk + 1) ? LDG(&F.s[o + 3 * planeS]) : 0.0f;
     }
   };
 
-  float wv[6] = {0, 0, 0, 0, 0, 0};   // s(k-2 .. k+3) of the column, for the top face of level k
   int tfail = -1, t = 0;
   fetch(0, kc0);
   for (int n = 0; n < P.n && tfail < 0; n++) {
     const ScalField &F = P.f[n];
-    const int sadd = F.sadd, pdw = F.pdefweno, flush = F.flush;
+    const int sadd = F.sadd, pdw = F.pdefweno;
     const double weps = F.weps;
-    const bool tht = sadd && P.thterm;
-    float *snew = F.snew;
-    // the column window and the face below the first level
-    float fzlo = 0.0f, fwlo = 0.0f, wlo = 0.0f;
+    // the column window, wv[d] = s(k-2+d) for the upper face of level k, and
+    // the face below the first level; the window's last value is fetched
+    float wv[6] = {0, 0, 0, 0, 0, 0}, fzlo = 0.0f, wlo = 0.0f;
     if (active) {
-      const float *sc = F.s + oc;
-      auto SV = [&](int kk) -> float {
-        float v = LDG(&sc[kk * planeS]);
-        if (sadd) v = PTH[kk] + v;
-        return v;
-      };
+      float w0 = 0.0f;
 #pragma unroll
-      for (int d = 0; d < 6; d++) {
+      for (int d = -1; d < 5; d++) {
         const int kk = kc0 - 2 + d;
-        wv[d] = (kk >= 0 && kk <= nk + 1) ? SV(kk) : 0.0f;
-      }
-      wlo = (kc0 <= 1) ? 0.0f : LDG(&P.rrw[kc0 * planeS + oc]);
-      fwlo = wlo * PRF[kc0];
-      if (kc0 >= 2) {
-        float w0[6];
-#pragma unroll
-        for (int d = 0; d < 6; d++) {
-          const int kk = kc0 - 3 + d;
-          w0[d] = (kk >= 0 && kk <= nk + 1) ? SV(kk) : 0.0f;
+        float v = 0.0f;
+        if (kk >= 0 && kk <= nk + 1) {
+          v = LDG(&F.s[kk * planeS + oc]);
+          if (sadd) v = (LDG(&g.th0[kk]) - 300.0f) + v;
         }
-        fzlo = zflux_core(w0, fwlo, kc0, nk, PC1[kc0], PC2[kc0], WENO, pdw, weps);
+        if (d < 0) w0 = v;
+        else wv[d] = v;
+      }
+      if (kc0 >= 2) {
+        wlo = LDG(&P.rrw[kc0 * planeS + oc]);
+        const float r = wlo * lev[0].rf;
+        const float w[6] = {w0, wv[0], wv[1], wv[2], wv[3], wv[4]};
+        fzlo = face5(r, w0, wv[0], wv[1], wv[2], wv[3], wv[4], WENO, pdw, weps);
+        if (WENO && fzlo != fzlo) fzlo = face5_exact(r, w0, wv[0], wv[1], wv[2], wv[3], wv[4], weps);
+        if (kc0 <= 3 || kc0 >= nk - 1) fzlo = zface_edge(fzlo, w, r, kc0, nk, g.c1, g.c2, WENO, pdw, weps);
       }
     }
+    int cal = (int)(((uintptr_t)(F.s + (kc0 * planeS + orow0)) >> 2) & 3);   // alignment of the staged plane
     for (int k = kc0; k <= kc1; k++, t++) {
-      const float r0k = PR0[k], th0m = sadd ? PTH[k] : 0.0f;
-      const float ru0 = pru, rv0 = prv;
-      const float whi = pwhi, e0 = pe0, e1 = pe1, e2 = pe2;
-      if (k < kc1) fetch(n, k + 1);                 // pwtop becomes s(k+4): the next level's window top
-      else if (n + 1 < P.n) fetch(n + 1, kc0);
+      const float4 la = *(const float4 *)&lev[k - kc0].r0, lb = *(const float4 *)&lev[k - kc0].rr;
+      const float r0k = la.x, th0m = lb.y;
       const int b = t & 1, slot = t % RD;
       // ---- the staged plane of this item
       const bool ok = mbar_wait(bar0 + 8 * slot, (uint32_t)((t / RD) & 1));
-      const float *pl = &ring[slot][(int)((((uintptr_t)(F.s + (k * planeS + orow0))) >> 2) & 3) + 4];
+      const float *pl = &ring[slot][cal + 4];
+      cal = (cal + planeS) & 3;
       // ---- face values: each x/y face once, the upper z face once per column
-      auto xface = [&](float ru) {
-        const float *p = pl + fxs;
-        float s0 = p[0], s1 = p[1], s2 = p[2], s3 = p[3], s4 = p[4], s5 = p[5];
-        if (sadd) { s0 = th0m + s0; s1 = th0m + s1; s2 = th0m + s2; s3 = th0m + s3; s4 = th0m + s4; s5 = th0m + s5; }
-        fx[b][fxd] = hflux5(ru * r0k, s0, s1, s2, s3, s4, s5, WENO, 0, weps);
-        ux[b][fxd] = ru;
+      auto staged = [&](float *s, int o, int st) {
+#pragma unroll
+        for (int d = 0; d < 6; d++) { s[d] = pl[o + d * st]; if (sadd) s[d] = th0m + s[d]; }
       };
-      auto yface = [&](float rv) {
-        const float *p = pl + fys;
-        float s0 = p[0], s1 = p[SP], s2 = p[2 * SP], s3 = p[3 * SP], s4 = p[4 * SP], s5 = p[5 * SP];
-        if (sadd) { s0 = th0m + s0; s1 = th0m + s1; s2 = th0m + s2; s3 = th0m + s3; s4 = th0m + s4; s5 = th0m + s5; }
-        fy[b][fyd] = hflux5(rv * r0k, s0, s1, s2, s3, s4, s5, WENO, 0, weps);
-        vy[b][fyd] = rv;
-      };
-      if (fxo >= 0) xface(ru0);
-      if (fyo >= 0) yface(rv0);
-      const float fwhi = whi * PRF[k + 1];
-      float fzhi = 0.0f, sc = 0.0f;
+      if (xface_on) {
+        float s[6];
+        staged(s, xs, 1);
+        float f = face5(ru * r0k, s[0], s[1], s[2], s[3], s[4], s[5], WENO, 0, weps);
+        if (WENO && f != f) { staged(s, xs, 1); f = face5_exact(ru * r0k, s[0], s[1], s[2], s[3], s[4], s[5], weps); }
+        fx[b][xd] = make_float2(f, ru);
+      }
+      if (yface_on) {
+        float s[6];
+        staged(s, ys, SP);
+        float f = face5(rv * r0k, s[0], s[1], s[2], s[3], s[4], s[5], WENO, 0, weps);
+        if (WENO && f != f) { staged(s, ys, SP); f = face5_exact(rv * r0k, s[0], s[1], s[2], s[3], s[4], s[5], weps); }
+        fy[b][tid] = make_float2(f, rv);
+      }
+      float fzhi = 0.0f;
       if (active) {
-        sc = pl[csel];
-        if (sadd) sc = th0m + sc;
+        wv[5] = (sadd && k + 3 <= nk + 1) ? lb.z + stop : stop;
         const int kk = k + 1;
-        if (kk >= 4 && kk <= nk - 2) fzhi = zflux_inner(wv, fwhi, WENO, pdw, weps);
-        else if (kk <= nk) fzhi = zflux_core(wv, fwhi, kk, nk, PC1[kk], PC2[kk], WENO, pdw, weps);
+        const float r = whi * la.z;
+        if (kk <= nk) {
+          fzhi = face5(r, wv[0], wv[1], wv[2], wv[3], wv[4], wv[5], WENO, pdw, weps);
+          if (WENO && fzhi != fzhi) fzhi = face5_exact(r, wv[0], wv[1], wv[2], wv[3], wv[4], wv[5], weps);
+          if (kk <= 3 || kk >= nk - 1) fzhi = zface_edge(fzhi, wv, r, kk, nk, g.c1, g.c2, WENO, pdw, weps);
+        }
+      }
+      float sc = 0.0f;
+      if (active) {
+        sc = pl[ys + 3 * SP];
+        if (sadd) sc = th0m + sc;
       }
       if (__syncthreads_or(!ok)) { tfail = t; break; }
       // the plane of this item has been read: its slot takes the item RD later
       if (stager && it_ < nitem) issue_next();
+      const float whik = whi, ten1 = e0, base = e1, tht = e2;
+      if (k < kc1) fetch(n, k + 1);
+      else if (n + 1 < P.n) fetch(n + 1, kc0);
       if (active) {
-        float fx0 = fx[b][xi], fxp = fx[b][xi + 1], fy0 = fy[b][yi], fyp = fy[b][yi + TX];
-        const float u0r = ux[b][xi], u1r = ux[b][xi + 1], v0r = vy[b][yi], v1r = vy[b][yi + TX];
-        const float fu0 = u0r * r0k, fu1 = u1r * r0k, fv0 = v0r * r0k, fv1 = v1r * r0k;
-        float advx, advy;
-        if (!edge) {
-          advx = -(fxp - fx0) * rdx * uh_i;
-          advy = -(fyp - fy0) * rdy * vh_j;
-        } else {
-          // adv.F:212-268
-          if (doitw && i == 1 && fu0 >= 0.0f) fx0 = fxp;
-          if (doite && i == ni && fu1 <= 0.0f) fxp = fx0;
-          if (doits && j == 1 && fv0 >= 0.0f) fy0 = fyp;
-          if (doitn && j == nj && fv1 <= 0.0f) fyp = fy0;
-          advx = -(fxp - fx0) * rdx * uh_i;
-          advy = -(fyp - fy0) * rdy * vh_j;
-          // adv.F:286-335
-          if (doitw && i == 1 && fu0 >= 0.0f) advx = advx - sc * (fu1 - fu0) * rdx * uh_i;
-          if (doite && i == ni && fu1 <= 0.0f) advx = advx - sc * (fu1 - fu0) * rdx * uh_i;
-          if (doits && j == 1 && fv0 >= 0.0f) advy = advy - sc * (fv1 - fv0) * rdy * vh_j;
-          if (doitn && j == nj && fv1 <= 0.0f) advy = advy - sc * (fv1 - fv0) * rdy * vh_j;
-        }
-        const float mhk = PMH[k];
-        float advz;
-        if (k == 1) advz = -fzhi * rdz * mhk;
-        else if (k == nk) advz = +fzlo * rdz * mhk;
-        else advz = -(fzhi - fzlo) * rdz * mhk;
-        float div = ((fu1 - fu0) * rdx * uh_i + (fv1 - fv0) * rdy * vh_j) + (fwhi - fwlo) * rdz * mhk;
-        if (fabsf(div) < smeps) div = 0.0f;
-        float ten = e0;
-        if (tht) {   // getdiv of the averaged velocities (misclibs.F:127-136)
-          float rd = ((u1r - u0r) * rdx * uh_i + (v1r - v0r) * rdy * vh_j) + (whi - wlo) * rdz * mhk;
-          if (fabsf(rd) < smeps) rd = 0.0f;
-          ten = ten - rd * e2;
-        }
-        ten = ten + (((advx + advy) + advz) + sc * div) * PRR[k];
-        float v = e1 + dt * ten;
-        if (flush && fabsf(v) < smeps) v = 0.0f;
-        snew[k * planeS + oc] = v;
+        const float2 xw = fx[b][xd], xe = fx[b][xd + 1], ysw = fy[b][tid], yn = fy[b][tid + TX];
+        const float v = scal_update(g, P, F, xw, xe, ysw, yn, fzlo, fzhi, wlo, whik, la, lb, i, j, k, edge, uh_i, vh_j, sc,
+                                    ten1, base, tht);
+        F.snew[k * planeS + oc] = v;
         // slide the column window and carry the upper face to the next level
 #pragma unroll
         for (int d = 0; d < 5; d++) wv[d] = wv[d + 1];
-        wv[5] = pwtop;
         fzlo = fzhi;
-        fwlo = fwhi;
-        wlo = whi;
+        wlo = whik;
       }
     }
   }
