@@ -64,8 +64,8 @@ def kernel_bytes_per_step(cfg):
     and every tracer; at stage 3 the fields without the positive-definite
     pass (theta, and tracers when pdtra=0).
     k_advs_tile: one field per launch (28 B, + 4 B thterm for moist theta).
-    k_advs_tile_pdef1 + k_advs_pdef2: the final-stage positive-definite pass
-    of one field, together the same 28 B (their six work arrays are scratch).
+    k_scal_pdef + k_pdef_fix: the final-stage positive-definite pass of one
+    field, together the same 28 B (their six work arrays are scratch).
     k_sound_step: one acoustic small step, 23 floats (92 B) per cell.
     k_mom: read u, v, w and their fixed tendencies, write the tendencies (36 B)."""
     moist = cfg.imoist == 1
@@ -78,7 +78,7 @@ def kernel_bytes_per_step(cfg):
     S = nloop_total(cfg.nsound)
     return {"k_scal_tile": 16 * fused_fields + 3 * (12 + tht),
             "k_advs_tile": 3 * (28 * nsc + tht) - 28 * pdef3,
-            "k_advs_tile_pdef1": 20 * pdef3, "k_advs_pdef2": 8 * pdef3,
+            "k_scal_pdef": 20 * pdef3, "k_pdef_fix": 8 * pdef3,
             "k_sound_step": 4 * ACOUSTIC_FLOATS_PER_CELL * S,
             "k_mom": 3 * 36}
 

@@ -40,10 +40,12 @@ void launch_adv_momentum(const DGrid &g, const float *u, const float *v, const f
                          const float *vten1, const float *wten1, float *uten, float *vten, float *wten,
                          const float *th3d, const float *qv, float *divx, cudaStream_t st, int64_t *nl,
                          const Diff6 *diff = nullptr, const float *b8 = nullptr, int which = 7);
-void launch_advs(const DGrid &g, const float *rru, const float *rrv, const float *rrw, int weighted,
-                 const float *divx, const float *s, const float *s0, int sadd, const float *ten1,
-                 const float *thterm, float *sten_out, float *snew, int weno, int pdef, int pdefweno,
-                 double weps, float dt, int flush, float *scratch, cudaStream_t st, int64_t *nl);
+void launch_advs(const DGrid &g, const float *rru, const float *rrv, const float *rrw, const float *divx, const float *s,
+                 const float *s0, float *sten, int weno, int pdef, int pdefweno, double weps, float dt, float *scratch,
+                 unsigned *neg, float *tsave, int *err, cudaStream_t st, int64_t *nl);
+void launch_scal_pdef(const DGrid &g, const ScalField &f, const float *rru, const float *rrv, const float *rrw, int weno,
+                      float dt, float *scratch, unsigned *neg, int *err, cudaStream_t st, int64_t *nl);
+size_t scal_neg_words(const DGrid &g);
 void launch_advs_tiled(const DGrid &g, const float *rru, const float *rrv, const float *rrw, const float *s,
                        const float *s0, int sadd, const float *ten1, const float *thterm, float *snew, int weno,
                        int pdef, int pdefweno, double weps, float dt, int flush, float *scratch, cudaStream_t st,
@@ -185,6 +187,7 @@ struct cm1g_ctx {
   float *rbnd = nullptr; // roflux = 1: restricted open-boundary u/v of an acoustic step
   float *sx[2 * (1 + 2 * CM1G_MAXQ)] = {};   // per-scalar stage buffers
   float *pdefscr = nullptr;                   // 6 s-arrays
+  unsigned *pdefneg = nullptr;                // signs of its provisional masses (scal_neg_words)
   float *mdivx = nullptr;                     // divx of the momentum pass
   float *rr = nullptr;                        // 1/rho as solve2 keeps it (6th-order diffusion)
   // learned closure of theta's horizontal faces (cm1g_closure_set)
@@ -202,6 +205,7 @@ struct cm1g_ctx {
   double *ener = nullptr;                     // calcener chunk sums (4 x nk x chunks) and results
   float *fscal = nullptr;
   int *cflbits = nullptr;
+  int *advs_err = nullptr;                    // cm1g_advs: a staging wait gave up (pinned, read after its synchronize)
   unsigned long long *mm = nullptr;
   // host staging (for host-pointer calls)
   cm1g_state_t dst{};
@@ -427,8 +431,8 @@ extern "C" int cm1g_init(const cm1g_config_t *cfg, const cm1g_grid_t *gr, cm1g_c
     c->rbnd = (float *)dalloc(c, (size_t)2 * (g.NJ + g.NI) * g.NK * sizeof(float));
   int nsc = 1 + (cfg->imoist ? cfg->numq : 0) + (cfg->iptra ? cfg->npt : 0);
   for (int s = 0; s < 2 * nsc; s++) c->sx[s] = (float *)dalloc(c, bS);
-  bool pdef_needed = cfg->imoist || (cfg->iptra && cfg->pdtra);
-  c->pdefscr = (float *)dalloc(c, (pdef_needed ? 6 : 6) * bS);
+  c->pdefscr = (float *)dalloc(c, 6 * bS);
+  c->pdefneg = (unsigned *)dalloc(c, scal_neg_words(g) * sizeof(unsigned));
   c->mdivx = (float *)dalloc(c, bS);
   if (cfg->idiff == 1) c->rr = (float *)dalloc(c, bS);
   c->ener = (double *)dalloc(c, ((size_t)4 * g.nk * ener_chunks(g) + 8) * sizeof(double));
@@ -464,6 +468,12 @@ extern "C" int cm1g_init(const cm1g_config_t *cfg, const cm1g_grid_t *gr, cm1g_c
   }
   for (void *p : c->allocs)
     if (!p) { cm1g_finalize(c); return set_err(CM1G_ERR_NOMEM, "scratch alloc"); }
+  if (cudaHostAlloc((void **)&c->advs_err, sizeof(int), cudaHostAllocDefault) != cudaSuccess) {
+    (void)cudaGetLastError();
+    cm1g_finalize(c);
+    return set_err(CM1G_ERR_NOMEM, "scratch alloc");
+  }
+  *c->advs_err = 0;
   if (!c->mm) { cm1g_finalize(c); return set_err(CM1G_ERR_NOMEM, "scratch alloc"); }
   if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) {
     cm1g_finalize(c);
@@ -491,6 +501,7 @@ extern "C" int cm1g_finalize(cm1g_ctx_t *c) {
   for (void *p : {(void *)c->d_st_jobs, (void *)c->d_st_ops, (void *)c->d_st_lev, (void *)c->d_rstat,
                   (void *)c->d_st_zh, (void *)c->d_st_zf})
     if (p) cudaFree(p);
+  if (c->advs_err) cudaFreeHost(c->advs_err);
   for (auto &b : c->stage_pool) cudaFree(b.first);
   if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
   delete c;
@@ -645,6 +656,7 @@ static void run_solve2(cm1g_ctx *c, const cm1g_state_t *d, float dt, double mass
     }
     launch_stage_prep(g, th_in, d->pp3d, qv_in, liq, cf.imoist, cf.eqtset, c->t11, c->t22, c->thterm, c->piadv, st,
                       nl);
+    launch_bc(g, c->t11, 2, 0, st, nl);
     if (diffit) df.coef = cf.kdiff6 / 64.0f / dttmp;   // adv.F:80-82, 962-964
     launch_adv_momentum(g, d->u3d, d->v3d, d->w3d, d->uten1, d->vten1, d->wten1, c->uten, c->vten, c->wten,
                         th_in, qv_in, c->mdivx, st, nl, diffit ? &df : nullptr, liq.b8);
@@ -661,13 +673,16 @@ static void run_solve2(cm1g_ctx *c, const cm1g_state_t *d, float dt, double mass
     // learned closure and the flux capture use the per-field tiles below.
     const bool fused = c->scal_fused && !diffit && !c->cl_on && !(nrk == 3 && c->cap_fx);
     std::vector<char> done(nsc, 0);
+    auto field = [&](int s, int sadd, double weps, int flush, int pdefweno) {
+      ScalField f{};
+      f.s = buf_in(s, nrk); f.sbase = base[s]; f.ten1 = ten1[s]; f.snew = buf_out(s, nrk);
+      f.weps = weps; f.sadd = sadd; f.flush = flush; f.pdefweno = pdefweno;
+      return f;
+    };
     if (fused) {
       std::vector<ScalField> fl;
       auto add = [&](int s, int sadd, double weps, int flush, int pdefweno) {
-        ScalField f{};
-        f.s = buf_in(s, nrk); f.sbase = base[s]; f.ten1 = ten1[s]; f.snew = buf_out(s, nrk);
-        f.weps = weps; f.sadd = sadd; f.flush = flush; f.pdefweno = pdefweno;
-        fl.push_back(f);
+        fl.push_back(field(s, sadd, weps, flush, pdefweno));
         done[s] = 1;
       };
       add(0, 1, (double)(10.0f * 1.0e-18f), 1, 0);
@@ -696,6 +711,11 @@ static void run_solve2(cm1g_ctx *c, const cm1g_state_t *d, float dt, double mass
     for (int n = 0; n < numq; n++) {
       const int s = 1 + n;
       if (done[s]) continue;
+      if (nrk == 3 && c->scal_fused && !diffit) {
+        launch_scal_pdef(g, field(s, 0, (double)(cf.qmag[n] * 1.0e-18f), 1, (n + 1 == cf.nqv) ? 0 : 1), c->rru, c->rrv,
+                         c->rrw, weno, dttmp, c->pdefscr, c->pdefneg, c->cflbits + 1, st, nl);
+        continue;
+      }
       launch_advs_tiled(g, c->rru, c->rrv, c->rrw, buf_in(s, nrk), base[s], 0, ten1[s], nullptr, buf_out(s, nrk),
                         weno, nrk == 3 ? 1 : 0, (n + 1 == cf.nqv) ? 0 : 1, (double)(cf.qmag[n] * 1.0e-18f), dttmp, 1,
                         c->pdefscr, st, nl, nullptr, diffit ? &df : nullptr);
@@ -713,6 +733,11 @@ static void run_solve2(cm1g_ctx *c, const cm1g_state_t *d, float dt, double mass
       const int s = 1 + numq + n;
       if (done[s]) continue;
       const int pdef = (nrk == 3 && cf.pdtra == 1) ? 1 : 0;
+      if (pdef && c->scal_fused && !diffit) {
+        launch_scal_pdef(g, field(s, 0, (double)(1.0f * 1.0e-18f), 0, 1), c->rru, c->rrv, c->rrw, weno, dttmp, c->pdefscr,
+                         c->pdefneg, c->cflbits + 1, st, nl);
+        continue;
+      }
       launch_advs_tiled(g, c->rru, c->rrv, c->rrw, buf_in(s, nrk), base[s], 0, ten1[s], nullptr, buf_out(s, nrk),
                         weno, pdef, 1, (double)(1.0f * 1.0e-18f), dttmp, 0, c->pdefscr, st, nl, nullptr,
                         diffit ? &df : nullptr);
@@ -767,6 +792,7 @@ static void run_solve3(cm1g_ctx *c, const cm1g_state_t *d) {
     launch_bc_batch(g, arr.data(), which.data(), nullptr, (int)arr.size(), st, nl);
   }
   launch_ppx_update(g, d->pp3d, d->ppx, st, nl);
+  launch_bc(g, d->ppx, 2, 0, st, nl);
   // solve3.F:546-640 rollover
   {
     std::vector<const float *> src;
@@ -1423,16 +1449,17 @@ extern "C" int cm1g_advs(cm1g_ctx_t *c, int32_t nrk, int32_t wflag, const float 
   const float *ds0 = s0 ? S.in(s0, nS(g), false) : nullptr;
   float *dten = S.in(sten, nS(g), true);
   const int weno = (wflag == 1) && (c->cfg.advwenos == 1 || (c->cfg.advwenos == 2 && nrk == 3));
-  if (!pdef) {
-    launch_advs(g, dru, drv, drw, 0, ddx, ds, ds0 ? ds0 : ds, 0, dten, nullptr, dten, nullptr, weno, 0, pdefweno,
-                weps, dt, 0, c->pdefscr, c->stream, &c->nlaunch);
-  } else {
-    launch_advs(g, dru, drv, drw, 0, ddx, ds, ds0, 0, dten, nullptr, dten, nullptr, weno, 1, pdefweno, weps, dt,
-                0, c->pdefscr, c->stream, &c->nlaunch);
-  }
+  // t11 is scratch of the large step, set anew by each of its stages
+  launch_advs(g, dru, drv, drw, ddx, ds, ds0, dten, weno, pdef != 0, pdefweno, weps, dt, c->pdefscr, c->pdefneg, c->t11,
+              c->advs_err, c->stream, &c->nlaunch);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return set_err(CM1G_ERR_CUDA, "%s", cudaGetErrorString(e));
-  return S.finish();
+  const int rc = S.finish();
+  if (rc == CM1G_OK && *c->advs_err) {
+    *c->advs_err = 0;
+    return set_err(CM1G_ERR_CUDA, "advs: staged data did not arrive (bulk-copy wait gave up)");
+  }
+  return rc;
 }
 
 // Momentum advection of the components selected by `which` (bit 0 u, 1 v,

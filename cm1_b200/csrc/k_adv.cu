@@ -5,9 +5,11 @@
 // face flux is evaluated once, from a level staged in shared memory with its
 // 3-point halo, instead of being stored in dumx/dumy/dumz; the rho0-weighted
 // fluxes rru/rrv/rrw and their divergence are formed on the fly, so a momentum
-// pass reads u, v, w (and theta/qv for buoyancy) and writes only the tendency.  The per-point
-// scalar kernels (k_advs, k_advs_pdef1/2) serve the per-routine entry
-// cm1g_advs.  Every expression keeps the reference's operand order.
+// pass reads u, v, w (and theta/qv for buoyancy) and writes only the tendency.
+// The scalars of a plain step and the per-routine entry cm1g_advs take
+// k_scal_tile; k_advs_tile here serves the learned closure, the flux capture and
+// the 6th-order diffusion, one field a launch.  Every expression keeps the
+// reference's operand order.
 #include "cm1g_common.cuh"
 #include "k_face.cuh"
 
@@ -898,193 +900,6 @@ struct SAdv {
   Diff6 df{};                       // 6th-order diffusion (df.rho null: none)
 };
 
-__device__ __forceinline__ float sval(const DGrid &g, const SAdv &a, int i, int j, int k) {
-  float v = LDG(&a.s[iS(g, i, j, k)]);
-  if (a.sadd) v = (LDG(&g.th0[k]) - 300.0f) + v;
-  return v;
-}
-__device__ __forceinline__ float FU(const DGrid &g, const SAdv &a, int i, int j, int k) {
-  float v = LDG(&a.rru[iU(g, i, j, k)]);
-  return a.weighted ? v * LDG(&g.rho0[k]) : v;
-}
-__device__ __forceinline__ float FV(const DGrid &g, const SAdv &a, int i, int j, int k) {
-  float v = LDG(&a.rrv[iV(g, i, j, k)]);
-  return a.weighted ? v * LDG(&g.rho0[k]) : v;
-}
-__device__ __forceinline__ float FW(const DGrid &g, const SAdv &a, int i, int j, int k) {
-  if (a.weighted && (k <= 1 || k >= g.nk + 1)) return 0.0f;
-  float v = LDG(&a.rrw[iW(g, i, j, k)]);
-  return a.weighted ? v * LDG(&g.rf0[k]) : v;
-}
-// getdiv of the averaged velocities (misclibs.F:127-136), for the moist theta term
-__device__ __forceinline__ float RAWDIV(const DGrid &g, const SAdv &a, int i, int j, int k) {
-  auto W = [&](int kk) { return (kk <= 1 || kk >= g.nk + 1) ? 0.0f : LDG(&a.rrw[iW(g, i, j, kk)]); };
-  float d = ((LDG(&a.rru[iU(g, i + 1, j, k)]) - LDG(&a.rru[iU(g, i, j, k)])) * g.rdx * LDG(&g.uh[i - g.ib]) +
-             (LDG(&a.rrv[iV(g, i, j + 1, k)]) - LDG(&a.rrv[iV(g, i, j, k)])) * g.rdy * LDG(&g.vh[j - g.jb])) +
-            (W(k + 1) - W(k)) * g.rdz * LDG(&g.mh[k]);
-  if (fabsf(d) < g.smeps) d = 0.0f;
-  return d;
-}
-__device__ __forceinline__ float SDIV(const DGrid &g, const SAdv &a, int i, int j, int k) {
-  if (a.divx) return LDG(&a.divx[iS(g, i, j, k)]);
-  float d = ((FU(g, a, i + 1, j, k) - FU(g, a, i, j, k)) * g.rdx * LDG(&g.uh[i - g.ib]) +
-             (FV(g, a, i, j + 1, k) - FV(g, a, i, j, k)) * g.rdy * LDG(&g.vh[j - g.jb])) +
-            (FW(g, a, i, j, k + 1) - FW(g, a, i, j, k)) * g.rdz * LDG(&g.mh[k]);
-  if (fabsf(d) < g.smeps) d = 0.0f;
-  return d;
-}
-
-// x-face flux dumx(i,j,k) (hadv_flx5/hadv_weno5 stag=1)
-__device__ __forceinline__ float sflux_x(const DGrid &g, const SAdv &a, int i, int j, int k, int weno, int pdef, double weps) {
-  float r = FU(g, a, i, j, k), s1, s2, s3, s4, s5;
-  if (r >= 0.0f) { s1 = sval(g, a, i - 3, j, k); s2 = sval(g, a, i - 2, j, k); s3 = sval(g, a, i - 1, j, k); s4 = sval(g, a, i, j, k); s5 = sval(g, a, i + 1, j, k); }
-  else { s1 = sval(g, a, i + 2, j, k); s2 = sval(g, a, i + 1, j, k); s3 = sval(g, a, i, j, k); s4 = sval(g, a, i - 1, j, k); s5 = sval(g, a, i - 2, j, k); }
-  if (!weno) return r * flx5(s1, s2, s3, s4, s5);
-  if (pdef == 1 && !(absmax5(s1, s2, s3, s4, s5) > (float)weps)) return 0.0f;
-  return r * weno5(s1, s2, s3, s4, s5, weps);
-}
-__device__ __forceinline__ float sflux_y(const DGrid &g, const SAdv &a, int i, int j, int k, int weno, int pdef, double weps) {
-  float r = FV(g, a, i, j, k), s1, s2, s3, s4, s5;
-  if (r >= 0.0f) { s1 = sval(g, a, i, j - 3, k); s2 = sval(g, a, i, j - 2, k); s3 = sval(g, a, i, j - 1, k); s4 = sval(g, a, i, j, k); s5 = sval(g, a, i, j + 1, k); }
-  else { s1 = sval(g, a, i, j + 2, k); s2 = sval(g, a, i, j + 1, k); s3 = sval(g, a, i, j, k); s4 = sval(g, a, i, j - 1, k); s5 = sval(g, a, i, j - 2, k); }
-  if (!weno) return r * flx5(s1, s2, s3, s4, s5);
-  if (pdef == 1 && !(absmax5(s1, s2, s3, s4, s5) > (float)weps)) return 0.0f;
-  return r * weno5(s1, s2, s3, s4, s5, weps);
-}
-// vertical flux dumz(i,j,kk), kk=2..nk (vadv_flx5 / vadv_weno5 stag=1)
-__device__ __forceinline__ float sflux_z(const DGrid &g, const SAdv &a, int i, int j, int kk, int weno, int pdefweno, double weps) {
-  const int nk = g.nk;
-  auto A = [&](int k) { return sval(g, a, i, j, k); };
-  float r = FW(g, a, i, j, kk);
-  const float c1k = LDG(&g.c1[kk]), c2k = LDG(&g.c2[kk]);
-  if (!weno) {
-    if (kk >= 4 && kk <= nk - 2) {
-      if (r >= 0.0f) return r * flx5(A(kk - 3), A(kk - 2), A(kk - 1), A(kk), A(kk + 1));
-      return r * flx5(A(kk + 2), A(kk + 1), A(kk), A(kk - 1), A(kk - 2));
-    }
-    if (kk == 2) {
-      if (r >= 0.0f) return r * (c1k * A(kk - 1) + c2k * A(kk));
-      return r * flx3(A(kk + 1), A(kk), A(kk - 1));
-    }
-    if (kk == nk) {
-      if (r >= 0.0f) return r * flx3(A(kk - 2), A(kk - 1), A(kk));
-      return r * (c1k * A(kk - 1) + c2k * A(kk));
-    }
-    if (kk == 3) {
-      if (r >= 0.0f) return r * flx3(A(kk - 2), A(kk - 1), A(kk));
-      return r * flx5(A(kk + 2), A(kk + 1), A(kk), A(kk - 1), A(kk - 2));
-    }
-    if (r >= 0.0f) return r * flx5(A(kk - 3), A(kk - 2), A(kk - 1), A(kk), A(kk + 1));
-    return r * flx3(A(kk + 1), A(kk), A(kk - 1));
-  }
-  // WENO: lower-order pieces at 2 and nk are common to both forms
-  if (kk == 2) {
-    if (r >= 0.0f) return r * (c1k * A(kk - 1) + c2k * A(kk));
-    return r * upstrpd(A(kk + 1), A(kk), A(kk - 1), weps);
-  }
-  if (kk == nk) {
-    if (r > 0.0f) return r * upstrpd(A(kk - 2), A(kk - 1), A(kk), weps);
-    return r * (c1k * A(kk - 1) + c2k * A(kk));
-  }
-  if (pdefweno == 1) {
-    // vadv_weno5 pdef form (adv_routines.F:2386-2421) then vadv_lwr_weno_35_b
-    if (kk == 3 && r > 0.0f) return r * upstrpd(A(kk - 2), A(kk - 1), A(kk), weps);
-    if (kk == nk - 1 && r < 0.0f) return r * upstrpd(A(kk + 1), A(kk), A(kk - 1), weps);
-    float s1, s2, s3, s4, s5;
-    if (r >= 0.0f) { s1 = A(kk - 3); s2 = A(kk - 2); s3 = A(kk - 1); s4 = A(kk); s5 = A(kk + 1); }
-    else { s1 = A(kk + 2); s2 = A(kk + 1); s3 = A(kk); s4 = A(kk - 1); s5 = A(kk - 2); }
-    bool doit = absmax5(s1, s2, s3, s4, s5) > (float)weps;
-    return doit ? r * weno5(s1, s2, s3, s4, s5, weps) : 0.0f;
-  }
-  if (kk >= 4 && kk <= nk - 2) {
-    if (r >= 0.0f) return r * weno5(A(kk - 3), A(kk - 2), A(kk - 1), A(kk), A(kk + 1), weps);
-    return r * weno5(A(kk + 2), A(kk + 1), A(kk), A(kk - 1), A(kk - 2), weps);
-  }
-  if (kk == 3) {
-    if (r >= 0.0f) return r * upstrpd(A(kk - 2), A(kk - 1), A(kk), weps);
-    return r * weno5(A(kk + 2), A(kk + 1), A(kk), A(kk - 1), A(kk - 2), weps);
-  }
-  if (r >= 0.0f) return r * weno5(A(kk - 3), A(kk - 2), A(kk - 1), A(kk), A(kk + 1), weps);
-  return r * upstrpd(A(kk + 1), A(kk), A(kk - 1), weps);
-}
-
-struct AdvParts { float advx, advy, advz; };
-
-// advx/advy/advz of one cell with the open-bc inflow fix-ups (adv.F:129-335, 451-577)
-__device__ __forceinline__ AdvParts advs_parts(const DGrid &g, const SAdv &a, int i, int j, int k,
-                                               int weno, int pdef, int pdefweno, double weps) {
-  const int ni = g.ni, nj = g.nj, nk = g.nk;
-  const bool doitw = (g.wbc == 2 && g.ibw), doite = (g.ebc == 2 && g.ibe);
-  const bool doits = (g.sbc == 2 && g.ibs), doitn = (g.nbc == 2 && g.ibn);
-  float fx0 = sflux_x(g, a, i, j, k, weno, pdef, weps), fxp = sflux_x(g, a, i + 1, j, k, weno, pdef, weps);
-  if (doitw && i == 1 && FU(g, a, 1, j, k) >= 0.0f) fx0 = fxp;
-  if (doite && i == ni && FU(g, a, ni + 1, j, k) <= 0.0f) fxp = fx0;
-  float fy0 = sflux_y(g, a, i, j, k, weno, pdef, weps), fyp = sflux_y(g, a, i, j + 1, k, weno, pdef, weps);
-  if (doits && j == 1 && FV(g, a, i, 1, k) >= 0.0f) fy0 = fyp;
-  if (doitn && j == nj && FV(g, a, i, nj + 1, k) <= 0.0f) fyp = fy0;
-  AdvParts p;
-  p.advx = -(fxp - fx0) * g.rdx * LDG(&g.uh[i - g.ib]);
-  p.advy = -(fyp - fy0) * g.rdy * LDG(&g.vh[j - g.jb]);
-  float sc = sval(g, a, i, j, k);
-  if (doitw && i == 1 && FU(g, a, 1, j, k) >= 0.0f)
-    p.advx = p.advx - sc * (FU(g, a, 2, j, k) - FU(g, a, 1, j, k)) * g.rdx * LDG(&g.uh[1 - g.ib]);
-  if (doite && i == ni && FU(g, a, ni + 1, j, k) <= 0.0f)
-    p.advx = p.advx - sc * (FU(g, a, ni + 1, j, k) - FU(g, a, ni, j, k)) * g.rdx * LDG(&g.uh[ni - g.ib]);
-  if (doits && j == 1 && FV(g, a, i, 1, k) >= 0.0f)
-    p.advy = p.advy - sc * (FV(g, a, i, 2, k) - FV(g, a, i, 1, k)) * g.rdy * LDG(&g.vh[1 - g.jb]);
-  if (doitn && j == nj && FV(g, a, i, nj + 1, k) <= 0.0f)
-    p.advy = p.advy - sc * (FV(g, a, i, nj + 1, k) - FV(g, a, i, nj, k)) * g.rdy * LDG(&g.vh[nj - g.jb]);
-  const float mhk = LDG(&g.mh[k]);
-  if (k == 1) p.advz = -sflux_z(g, a, i, j, 2, weno, pdefweno, weps) * g.rdz * mhk;
-  else if (k == nk) p.advz = +sflux_z(g, a, i, j, nk, weno, pdefweno, weps) * g.rdz * mhk;
-  else p.advz = -(sflux_z(g, a, i, j, k + 1, weno, pdefweno, weps) - sflux_z(g, a, i, j, k, weno, pdefweno, weps)) * g.rdz * mhk;
-  return p;
-}
-
-// Non-pdef scalar pass: sten_out = sten_in + (adv + s*divx)*rr0, and when
-// snew is given, snew = s0 + dt*sten_out with the smeps flush (solve2.F:1419-1425).
-__global__ void k_advs(DGrid g, SAdv a, const float *sten_in,
-                       float *sten_out, float *__restrict__ snew, const float *__restrict__ sbase,
-                       int weno, int pdefweno, double weps, float dt, int flush) {
-  const int i = 1 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  const int j = 1 + (int)blockIdx.y, k = 1 + (int)blockIdx.z;
-  if (i > g.ni) return;
-  AdvParts p = advs_parts(g, a, i, j, k, weno, 0, pdefweno, weps);
-  long o = iS(g, i, j, k);
-  float ten = sten_in[o];
-  if (a.thterm) ten = ten - RAWDIV(g, a, i, j, k) * LDG(&a.thterm[o]);
-  ten = ten + (((p.advx + p.advy) + p.advz) + sval(g, a, i, j, k) * SDIV(g, a, i, j, k)) * LDG(&g.rr0[k]);
-  if (sten_out) sten_out[o] = ten;
-  if (snew) {
-    float v = LDG(&sbase[o]) + dt * ten;
-    if (flush && fabsf(v) < g.smeps) v = 0.0f;
-    snew[o] = v;
-  }
-}
-
-// pdef pass 1: advx/advy/advz and the provisional masses of pdefx1/y1/z
-// (pdef.F:35-102, 289-340, 478-496).
-__global__ void k_advs_pdef1(DGrid g, SAdv a, float *__restrict__ advx, float *__restrict__ advy, float *__restrict__ advz,
-                             float *__restrict__ dumx, float *__restrict__ dumy, float *__restrict__ dumz,
-                             int weno, int pdefweno, double weps, float dt) {
-  const int i = 1 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  const int j = 1 + (int)blockIdx.y, k = 1 + (int)blockIdx.z;
-  if (i > g.ni) return;
-  const int ni = g.ni, nj = g.nj;
-  AdvParts p = advs_parts(g, a, i, j, k, weno, 1, pdefweno, weps);
-  long o = iS(g, i, j, k);
-  advx[o] = p.advx; advy[o] = p.advy; advz[o] = p.advz;
-  const float s = sval(g, a, i, j, k), s0 = LDG(&a.s0[o]), r0k = LDG(&g.rho0[k]);
-  float dx = r0k * s0 + dt * (p.advx + s * (FU(g, a, i + 1, j, k) - FU(g, a, i, j, k)) * g.rdx * LDG(&g.uh[i - g.ib]));
-  if (g.wbc == 2 && g.ibw && i == 1 && FU(g, a, 1, j, k) >= 0.0f) dx = r0k * s0;
-  if (g.ebc == 2 && g.ibe && i == ni && FU(g, a, ni + 1, j, k) <= 0.0f) dx = r0k * s0;
-  float dy = r0k * s0 + dt * (p.advy + s * (FV(g, a, i, j + 1, k) - FV(g, a, i, j, k)) * g.rdy * LDG(&g.vh[j - g.jb]));
-  if (g.sbc == 2 && g.ibs && j == 1 && FV(g, a, i, 1, k) >= 0.0f) dy = r0k * s0;
-  if (g.nbc == 2 && g.ibn && j == nj && FV(g, a, i, nj + 1, k) <= 0.0f) dy = r0k * s0;
-  float dz = r0k * s0 + dt * (p.advz + s * (FW(g, a, i, j, k + 1) - FW(g, a, i, j, k)) * g.rdz * LDG(&g.mh[k]));
-  dumx[o] = dx; dumy[o] = dy; dumz[o] = dz;
-}
-
 // Mass moved into point c by the pdef scatter of pdefx2/pdefy2/pdefz
 // (pdef.F:158-174), gathered in the scatter's loop order: contribution from
 // the lower neighbour, then the point itself, then the upper neighbour.
@@ -1119,52 +934,12 @@ __device__ __forceinline__ void pdef_gather(float dm2, float dm1, float d0, floa
   *mass = m; *flag = f;
 }
 
-// pdef pass 2: pdefz, pdefx2, pdefy2 fixes (pdef.F:117-264, 358-454,
-// 459-581) and the tendency/update of adv.F:650-659 + solve2.F:1513-1520.
-// dumx/dumy carry halo values filled by the lateral bc (pdef.F:102, 338).
-__global__ void k_advs_pdef2(DGrid g, SAdv a, const float *__restrict__ advx, const float *__restrict__ advy,
-                             const float *__restrict__ advz, const float *__restrict__ dumx,
-                             const float *__restrict__ dumy, const float *__restrict__ dumz,
-                             const float *sten_in, float *sten_out, float *__restrict__ snew,
-                             const float *__restrict__ sbase, float dt, int flush) {
-  const int i = 1 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  const int j = 1 + (int)blockIdx.y, k = 1 + (int)blockIdx.z;
-  if (i > g.ni) return;
-  const int nk = g.nk;
-  const float smeps = g.smeps, rdt = 1.0f / dt;
-  long o = iS(g, i, j, k);
-  const float s = sval(g, a, i, j, k), s0 = LDG(&a.s0[o]), r0k = LDG(&g.rho0[k]);
-  float m; bool f;
-  // z (pdefz): dum(0)=dum(nk+1)=0
-  auto DZ = [&](int kk) { return (kk < 1 || kk > nk) ? 0.0f : LDG(&dumz[iS(g, i, j, kk)]); };
-  float az = LDG(&advz[o]);
-  pdef_gather(DZ(k - 2), DZ(k - 1), DZ(k), DZ(k + 1), DZ(k + 2), smeps, &m, &f);
-  if (f) az = (DZ(k) + m - r0k * s0) * rdt - s * (FW(g, a, i, j, k + 1) - FW(g, a, i, j, k)) * g.rdz * LDG(&g.mh[k]);
-  // x (pdefx2)
-  auto DX = [&](int ii) { return LDG(&dumx[iS(g, ii, j, k)]); };
-  float ax = LDG(&advx[o]);
-  pdef_gather(DX(i - 2), DX(i - 1), DX(i), DX(i + 1), DX(i + 2), smeps, &m, &f);
-  if (f) ax = (DX(i) + m - r0k * s0) * rdt - s * (FU(g, a, i + 1, j, k) - FU(g, a, i, j, k)) * g.rdx * LDG(&g.uh[i - g.ib]);
-  // y (pdefy2)
-  auto DY = [&](int jj) { return LDG(&dumy[iS(g, i, jj, k)]); };
-  float ay = LDG(&advy[o]);
-  pdef_gather(DY(j - 2), DY(j - 1), DY(j), DY(j + 1), DY(j + 2), smeps, &m, &f);
-  if (f) ay = (DY(j) + m - r0k * s0) * rdt - s * (FV(g, a, i, j + 1, k) - FV(g, a, i, j, k)) * g.rdy * LDG(&g.vh[j - g.jb]);
-  float ten = sten_in[o] + (((ax + ay) + az) + s * SDIV(g, a, i, j, k)) * LDG(&g.rr0[k]);
-  if (sten_out) sten_out[o] = ten;
-  if (snew) {
-    float v = LDG(&sbase[o]) + dt * ten;
-    if (flush && fabsf(v) < g.smeps) v = 0.0f;
-    snew[o] = v;
-  }
-}
-
 // Tiled form of pass 2: a block owns TX x TY columns and marches upward;
 // each level's dumx (with its +-2 halo in x) and dumy (+-2 in y) are staged
 // in shared memory (double-buffered, one barrier per level; beyond the domain's
 // edges from the points that the lateral bc copies there, pdef.F:102, 338),
 // dumz comes from a per-column register window, and every read of a level is issued
-// one level ahead.  Same arithmetic as k_advs_pdef2.
+// one level ahead.
 template <int TX, int TY, int KC>
 __global__ void __launch_bounds__(TX * TY) k_advs_pdef2_tile(DGrid g, SAdv a, const float *__restrict__ advx,
                                                              const float *__restrict__ advy, const float *__restrict__ advz,
@@ -1632,31 +1407,6 @@ void launch_advs_tiled(const DGrid &g, const float *rru, const float *rrv, const
     default: CM1G_ADVS_SHAPE(0)
   }
 #undef CM1G_ADVS_SHAPE
-}
-
-// One advs call + RK update.  s = field (full halo), s0 = RK base,
-// ten1 = fixed tendency.  pdef selects the two-pass positive-definite form.
-// scratch must hold 6 s-arrays when pdef is set.
-void launch_advs(const DGrid &g, const float *rru, const float *rrv, const float *rrw, int weighted,
-                 const float *divx, const float *s, const float *s0, int sadd, const float *ten1,
-                 const float *thterm, float *sten_out, float *snew, int weno, int pdef, int pdefweno,
-                 double weps, float dt, int flush, float *scratch, cudaStream_t st, int64_t *nl) {
-  SAdv a{rru, rrv, rrw, s, s0, divx, thterm, weighted, sadd};
-  const int bx = 128;
-  dim3 grid((g.ni + bx - 1) / bx, g.nj, g.nk);
-  if (!pdef) {
-    { ProfScope _ps("k_advs", st); k_advs<<<grid, bx, 0, st>>>(g, a, ten1, sten_out, snew, s0, weno, pdefweno, weps, dt, flush); }
-    if (nl) *nl += 1;
-    return;
-  }
-  long n = nS(g);
-  float *advx = scratch, *advy = scratch + n, *advz = scratch + 2 * n;
-  float *dumx = scratch + 3 * n, *dumy = scratch + 4 * n, *dumz = scratch + 5 * n;
-  { ProfScope _ps("k_advs_pdef1", st); k_advs_pdef1<<<grid, bx, 0, st>>>(g, a, advx, advy, advz, dumx, dumy, dumz, weno, pdefweno, weps, dt); }
-  launch_bc(g, dumx, 1, 0, st, nl);
-  launch_bc(g, dumy, 1, 0, st, nl);
-  { ProfScope _ps("k_advs_pdef2", st); k_advs_pdef2<<<grid, bx, 0, st>>>(g, a, advx, advy, advz, dumx, dumy, dumz, ten1, sten_out, snew, s0, dt, flush); }
-  if (nl) *nl += 2;
 }
 
 }  // namespace cm1g

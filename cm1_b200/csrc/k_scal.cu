@@ -52,6 +52,15 @@ struct ScalPass {
   const float *thterm;          // moist theta: thten -= div(u_avg) * thterm (solve2.F:1320-1329); null: none
   float dt;
   int *err;                     // set to 1 when a block gives up waiting for its staged data
+  // positive-definite pass (one field): advx, advy, advz and the provisional
+  // masses dumx, dumy, dumz; a word for each level chunk, row and 32 columns,
+  // bit m set where a provisional mass at level m of the chunk is negative
+  float *adv[3], *dum[3];
+  unsigned *neg;
+  // the caller's own mass fluxes (adv.F's arguments) in place of velocities to
+  // weight: its divx, and where the positive-definite pass keeps its tendency
+  const float *divx;
+  float *tsave;
 };
 
 namespace {
@@ -101,52 +110,54 @@ struct __align__(16) ScLev {
   float rr, th, th3, pad;    // rr0(k), th0(k)-300, th0(k+3)-300
 };
 
-// The stage's new value of one cell from its faces, (flux, averaged velocity)
-// each, with the open-boundary fix-ups of adv.F where the tile touches an open
-// edge; fz* and w* are the vertical fluxes and averaged velocities.
-__device__ __forceinline__ float scal_update(const DGrid &g, const ScalPass &P, const ScalField &F, float2 xw, float2 xe,
-                                             float2 ys, float2 yn, float fzlo, float fzhi, float wlo, float whi, float4 la,
-                                             float4 lb, int i, int j, int k, bool edge, float uh_i, float vh_j, float sc,
-                                             float ten, float base, float tht) {
+// One cell's advection from its faces, (flux, averaged velocity) each, with the
+// open-boundary fix-ups of adv.F where the tile touches an open edge; fz* and w*
+// are the vertical fluxes and averaged velocities; in la the density is 1 where
+// the velocities are the caller's mass fluxes.
+struct ScAdv {
+  float x, y, z, sum;          // advx, advy, advz and (advx + advy + advz + s div)/rho0
+  bool w, e, s, n;             // inflow through an open edge
+};
+__device__ __forceinline__ ScAdv scal_advection(const DGrid &g, float2 xw, float2 xe, float2 ys, float2 yn, float fzlo,
+                                                float fzhi, float wlo, float whi, float4 la, float rr0, int i, int j, int k,
+                                                bool edge, float uh_i, float vh_j, float sc, const float *divx) {
   const float r0k = la.x, mhk = la.w;
   float fx0 = xw.x, fxp = xe.x, fy0 = ys.x, fyp = yn.x;
   const float fu0 = xw.y * r0k, fu1 = xe.y * r0k, fv0 = ys.y * r0k, fv1 = yn.y * r0k;
-  const float rdx = g.rdx, rdy = g.rdy, rdz = g.rdz, smeps = g.smeps;
-  float advx, advy;
+  const float rdx = g.rdx, rdy = g.rdy, rdz = g.rdz;
+  ScAdv a;
+  a.w = a.e = a.s = a.n = false;
   if (!edge) {
-    advx = -(fxp - fx0) * rdx * uh_i;
-    advy = -(fyp - fy0) * rdy * vh_j;
+    a.x = -(fxp - fx0) * rdx * uh_i;
+    a.y = -(fyp - fy0) * rdy * vh_j;
   } else {
-    const bool w = g.wbc == 2 && g.ibw && i == 1 && fu0 >= 0.0f, e = g.ebc == 2 && g.ibe && i == g.ni && fu1 <= 0.0f;
-    const bool s = g.sbc == 2 && g.ibs && j == 1 && fv0 >= 0.0f, n = g.nbc == 2 && g.ibn && j == g.nj && fv1 <= 0.0f;
+    a.w = g.wbc == 2 && g.ibw && i == 1 && fu0 >= 0.0f; a.e = g.ebc == 2 && g.ibe && i == g.ni && fu1 <= 0.0f;
+    a.s = g.sbc == 2 && g.ibs && j == 1 && fv0 >= 0.0f; a.n = g.nbc == 2 && g.ibn && j == g.nj && fv1 <= 0.0f;
     // adv.F:212-268
-    if (w) fx0 = fxp;
-    if (e) fxp = fx0;
-    if (s) fy0 = fyp;
-    if (n) fyp = fy0;
-    advx = -(fxp - fx0) * rdx * uh_i;
-    advy = -(fyp - fy0) * rdy * vh_j;
+    if (a.w) fx0 = fxp;
+    if (a.e) fxp = fx0;
+    if (a.s) fy0 = fyp;
+    if (a.n) fyp = fy0;
+    a.x = -(fxp - fx0) * rdx * uh_i;
+    a.y = -(fyp - fy0) * rdy * vh_j;
     // adv.F:286-335
-    if (w) advx = advx - sc * (fu1 - fu0) * rdx * uh_i;
-    if (e) advx = advx - sc * (fu1 - fu0) * rdx * uh_i;
-    if (s) advy = advy - sc * (fv1 - fv0) * rdy * vh_j;
-    if (n) advy = advy - sc * (fv1 - fv0) * rdy * vh_j;
+    if (a.w) a.x = a.x - sc * (fu1 - fu0) * rdx * uh_i;
+    if (a.e) a.x = a.x - sc * (fu1 - fu0) * rdx * uh_i;
+    if (a.s) a.y = a.y - sc * (fv1 - fv0) * rdy * vh_j;
+    if (a.n) a.y = a.y - sc * (fv1 - fv0) * rdy * vh_j;
   }
-  float advz;
-  if (k == 1) advz = -fzhi * rdz * mhk;
-  else if (k == g.nk) advz = +fzlo * rdz * mhk;
-  else advz = -(fzhi - fzlo) * rdz * mhk;
-  float div = ((fu1 - fu0) * rdx * uh_i + (fv1 - fv0) * rdy * vh_j) + (whi * la.z - wlo * la.y) * rdz * mhk;
-  if (fabsf(div) < smeps) div = 0.0f;
-  if (F.sadd && P.thterm) {   // getdiv of the averaged velocities (misclibs.F:127-136)
-    float rd = ((xe.y - xw.y) * rdx * uh_i + (yn.y - ys.y) * rdy * vh_j) + (whi - wlo) * rdz * mhk;
-    if (fabsf(rd) < smeps) rd = 0.0f;
-    ten = ten - rd * tht;
+  if (k == 1) a.z = -fzhi * rdz * mhk;
+  else if (k == g.nk) a.z = +fzlo * rdz * mhk;
+  else a.z = -(fzhi - fzlo) * rdz * mhk;
+  float div;
+  if (divx) {
+    div = *divx;
+  } else {
+    div = ((fu1 - fu0) * rdx * uh_i + (fv1 - fv0) * rdy * vh_j) + (whi * la.z - wlo * la.y) * rdz * mhk;
+    if (fabsf(div) < g.smeps) div = 0.0f;
   }
-  ten = ten + (((advx + advy) + advz) + sc * div) * lb.x;
-  float v = base + P.dt * ten;
-  if (F.flush && fabsf(v) < smeps) v = 0.0f;
-  return v;
+  a.sum = (((a.x + a.y) + a.z) + sc * div) * rr0;
+  return a;
 }
 
 __device__ __forceinline__ ScLev scal_level(const DGrid &g, int k) {
@@ -158,7 +169,11 @@ __device__ __forceinline__ ScLev scal_level(const DGrid &g, int k) {
   return l;
 }
 
-template <int TX, int TY, int KC, int WENO>
+// PDEF: the first pass of the positive-definite scheme (pdef.F:35-102, 289-340,
+// 478-496) of one field: advx..dumz and neg beside the value that holds where no
+// neighbouring provisional mass is negative (k_pdef_fix does the other cells).
+// RAW: the caller's mass fluxes and divx; the value is the tendency.
+template <int TX, int TY, int KC, int WENO, int PDEF, int RAW>
 __global__ void __launch_bounds__(TX * (TY + 1), 3) k_scal_tile(const __grid_constant__ DGrid g,
                                                                  const __grid_constant__ ScalPass P) {
   constexpr int SW = TX + 6, SH = TY + 6;                  // staged columns and rows
@@ -262,16 +277,18 @@ __global__ void __launch_bounds__(TX * (TY + 1), 3) k_scal_tile(const __grid_con
     if (yface_on) rv = LDG(&P.rrv[kf * planeV + oc]);
     if (active) {
       const int o = kf * planeS + oc;
-      whi = (kf == nk) ? 0.0f : LDG(&P.rrw[o + planeS]);
+      whi = (!RAW && kf == nk) ? 0.0f : LDG(&P.rrw[o + planeS]);
       e0 = F.ten1[o];
-      e1 = LDG(&F.sbase[o]);
-      if (F.sadd && P.thterm) e2 = LDG(&P.thterm[o]);
+      if (PDEF || !RAW) e1 = LDG(&F.sbase[o]);
+      if (RAW) e2 = LDG(&P.divx[o]);
+      else if (!PDEF && F.sadd && P.thterm) e2 = LDG(&P.thterm[o]);
       // s(kf+3), the last value under the upper face of level kf
       stop = (kf + 3 <= nk + 1) ? LDG(&F.s[o + 3 * planeS]) : 0.0f;
     }
   };
 
   int tfail = -1, t = 0;
+  unsigned neg = 0;
   fetch(0, kc0);
   for (int n = 0; n < P.n && tfail < 0; n++) {
     const ScalField &F = P.f[n];
@@ -293,9 +310,9 @@ __global__ void __launch_bounds__(TX * (TY + 1), 3) k_scal_tile(const __grid_con
         if (d < 0) w0 = v;
         else wv[d] = v;
       }
+      if (RAW || kc0 >= 2) wlo = LDG(&P.rrw[kc0 * planeS + oc]);
       if (kc0 >= 2) {
-        wlo = LDG(&P.rrw[kc0 * planeS + oc]);
-        const float r = wlo * lev[0].rf;
+        const float r = RAW ? wlo : wlo * lev[0].rf;
         const float w[6] = {w0, wv[0], wv[1], wv[2], wv[3], wv[4]};
         fzlo = face5(r, w0, wv[0], wv[1], wv[2], wv[3], wv[4], WENO, pdw, weps);
         if (WENO && fzlo != fzlo) fzlo = face5_exact(r, w0, wv[0], wv[1], wv[2], wv[3], wv[4], weps);
@@ -305,7 +322,7 @@ __global__ void __launch_bounds__(TX * (TY + 1), 3) k_scal_tile(const __grid_con
     int cal = (int)(((uintptr_t)(F.s + (kc0 * planeS + orow0)) >> 2) & 3);   // alignment of the staged plane
     for (int k = kc0; k <= kc1; k++, t++) {
       const float4 la = *(const float4 *)&lev[k - kc0].r0, lb = *(const float4 *)&lev[k - kc0].rr;
-      const float r0k = la.x, th0m = lb.y;
+      const float r0k = RAW ? 1.0f : la.x, th0m = lb.y;
       const int b = t & 1, slot = t % RD;
       // ---- the staged plane of this item
       const bool ok = mbar_wait(bar0 + 8 * slot, (uint32_t)((t / RD) & 1));
@@ -319,14 +336,14 @@ __global__ void __launch_bounds__(TX * (TY + 1), 3) k_scal_tile(const __grid_con
       if (xface_on) {
         float s[6];
         staged(s, xs, 1);
-        float f = face5(ru * r0k, s[0], s[1], s[2], s[3], s[4], s[5], WENO, 0, weps);
+        float f = face5(ru * r0k, s[0], s[1], s[2], s[3], s[4], s[5], WENO, PDEF, weps);
         if (WENO && f != f) { staged(s, xs, 1); f = face5_exact(ru * r0k, s[0], s[1], s[2], s[3], s[4], s[5], weps); }
         fx[b][xd] = make_float2(f, ru);
       }
       if (yface_on) {
         float s[6];
         staged(s, ys, SP);
-        float f = face5(rv * r0k, s[0], s[1], s[2], s[3], s[4], s[5], WENO, 0, weps);
+        float f = face5(rv * r0k, s[0], s[1], s[2], s[3], s[4], s[5], WENO, PDEF, weps);
         if (WENO && f != f) { staged(s, ys, SP); f = face5_exact(rv * r0k, s[0], s[1], s[2], s[3], s[4], s[5], weps); }
         fy[b][tid] = make_float2(f, rv);
       }
@@ -334,7 +351,7 @@ __global__ void __launch_bounds__(TX * (TY + 1), 3) k_scal_tile(const __grid_con
       if (active) {
         wv[5] = (sadd && k + 3 <= nk + 1) ? lb.z + stop : stop;
         const int kk = k + 1;
-        const float r = whi * la.z;
+        const float r = RAW ? whi : whi * la.z;
         if (kk <= nk) {
           fzhi = face5(r, wv[0], wv[1], wv[2], wv[3], wv[4], wv[5], WENO, pdw, weps);
           if (WENO && fzhi != fzhi) fzhi = face5_exact(r, wv[0], wv[1], wv[2], wv[3], wv[4], wv[5], weps);
@@ -349,21 +366,51 @@ __global__ void __launch_bounds__(TX * (TY + 1), 3) k_scal_tile(const __grid_con
       if (__syncthreads_or(!ok)) { tfail = t; break; }
       // the plane of this item has been read: its slot takes the item RD later
       if (stager && it_ < nitem) issue_next();
-      const float whik = whi, ten1 = e0, base = e1, tht = e2;
+      const float whik = whi, ten1 = e0, base = e1, e2k = e2;
+      bool negative = false;
       if (k < kc1) fetch(n, k + 1);
       else if (n + 1 < P.n) fetch(n + 1, kc0);
       if (active) {
         const float2 xw = fx[b][xd], xe = fx[b][xd + 1], ysw = fy[b][tid], yn = fy[b][tid + TX];
-        const float v = scal_update(g, P, F, xw, xe, ysw, yn, fzlo, fzhi, wlo, whik, la, lb, i, j, k, edge, uh_i, vh_j, sc,
-                                    ten1, base, tht);
-        F.snew[k * planeS + oc] = v;
+        const ScAdv a = scal_advection(g, xw, xe, ysw, yn, fzlo, fzhi, wlo, whik,
+                                       RAW ? make_float4(1.0f, 1.0f, 1.0f, la.w) : la, lb.x, i, j, k, edge, uh_i, vh_j, sc,
+                                       RAW ? &e2k : nullptr);
+        const int o = k * planeS + oc;
+        float ten = ten1;
+        if (!RAW && !PDEF && sadd && P.thterm) {   // getdiv of the averaged velocities (misclibs.F:127-136)
+          float rd = ((xe.y - xw.y) * g.rdx * uh_i + (yn.y - ysw.y) * g.rdy * vh_j) + (whik - wlo) * g.rdz * la.w;
+          if (fabsf(rd) < g.smeps) rd = 0.0f;
+          ten = ten - rd * e2k;
+        }
+        ten = ten + a.sum;
+        float v = RAW ? ten : base + P.dt * ten;
+        if (!RAW && F.flush && fabsf(v) < g.smeps) v = 0.0f;
+        if (PDEF) {   // provisional masses
+          const float dt = P.dt, m0 = la.x * base;
+          const float fu0 = xw.y * r0k, fu1 = xe.y * r0k, fv0 = ysw.y * r0k, fv1 = yn.y * r0k;
+          float dx = m0 + dt * (a.x + sc * (fu1 - fu0) * g.rdx * uh_i), dy = m0 + dt * (a.y + sc * (fv1 - fv0) * g.rdy * vh_j);
+          if (a.w || a.e) dx = m0;
+          if (a.s || a.n) dy = m0;
+          const float fwhi = RAW ? whik : whik * la.z, fwlo = RAW ? wlo : wlo * la.y;
+          const float dz = m0 + dt * (a.z + sc * (fwhi - fwlo) * g.rdz * la.w);
+          P.adv[0][o] = a.x; P.adv[1][o] = a.y; P.adv[2][o] = a.z;
+          P.dum[0][o] = dx; P.dum[1][o] = dy; P.dum[2][o] = dz;
+          if (RAW) P.tsave[o] = ten1;
+          negative = dx < 0.0f || dy < 0.0f || dz < 0.0f;
+        }
+        F.snew[o] = v;
         // slide the column window and carry the upper face to the next level
 #pragma unroll
         for (int d = 0; d < 5; d++) wv[d] = wv[d + 1];
         fzlo = fzhi;
         wlo = whik;
       }
+      if (PDEF && __any_sync(0xffffffffu, negative)) neg |= 1u << (k - kc0);
     }
+  }
+  if (PDEF && ty < TY && j <= nj && i - lane <= ni && lane == 0) {
+    const int nch = (ni + 31) / 32;
+    P.neg[((int)blockIdx.z * nj + j - 1) * nch + (i - 1) / 32] = neg;
   }
   if (tfail >= 0) {
     // leave no bulk copy in flight into this block's shared memory: wait (each
@@ -373,11 +420,154 @@ __global__ void __launch_bounds__(TX * (TY + 1), 3) k_scal_tile(const __grid_con
   }
 }
 
-template <int TX, int TY, int KC>
-static void scal_shape(const DGrid &g, const ScalPass &P, int weno, cudaStream_t st) {
+// Mass moved into point c by the pdef scatter of pdefx2/pdefy2/pdefz
+// (pdef.F:158-174), gathered in the scatter's loop order: contribution from
+// the lower neighbour, then the point itself, then the upper neighbour.
+__device__ __forceinline__ void pdef_gather(float dm2, float dm1, float d0, float dp1, float dp2, float smeps, float *mass,
+                                            bool *flag) {
+  float m = 0.0f;
+  bool f = false;
+  if (dm1 < 0.0f) {  // the point below scatters: we are its upper neighbour
+    float foo1 = fmaxf(0.0f, dm2), foo2 = fmaxf(0.0f, d0);
+    if (foo1 + foo2 > smeps) {
+      float foo3 = fmaxf(dm1, -(foo1 + foo2)) / (foo1 + foo2);
+      m = m + foo2 * foo3;
+      if (d0 > smeps) f = true;
+    }
+  }
+  if (d0 < 0.0f) {
+    float foo1 = fmaxf(0.0f, dm1), foo2 = fmaxf(0.0f, dp1);
+    if (foo1 + foo2 > smeps) {
+      float foo3 = fmaxf(d0, -(foo1 + foo2)) / (foo1 + foo2);
+      m = m - (foo1 + foo2) * foo3;
+      f = true;
+    }
+  }
+  if (dp1 < 0.0f) {
+    float foo1 = fmaxf(0.0f, d0), foo2 = fmaxf(0.0f, dp2);
+    if (foo1 + foo2 > smeps) {
+      float foo3 = fmaxf(dp1, -(foo1 + foo2)) / (foo1 + foo2);
+      m = m + foo1 * foo3;
+      if (d0 > smeps) f = true;
+    }
+  }
+  *mass = m; *flag = f;
+}
+
+// Second pass of the positive-definite scheme: pdefz, pdefx2, pdefy2
+// (pdef.F:117-264, 358-454, 459-581) and the update of adv.F:650-659 and
+// solve2.F:1513-1520, for the cells whose value they change.  A warp owns 32
+// columns of a row over a chunk of KC levels; it reads the chunk's word of
+// negative provisional masses and its neighbours' (a cell changes only if its
+// own, or one beside it in x, y or z, is negative) and visits the levels named
+// there.  A field without such masses costs the launch (256x256x80: 10 us against
+// 135 us when every cell read the six arrays back), a tracer of a few blobs after
+// two stages 135 us as before (waiting on its 15 masses a cell), and the host
+// entry at 251x187x79 100 us with every level named.  Beyond the domain the masses are those of the points that the lateral
+// bc copies there (pdef.F:102, 338).
+template <int RAW>
+__global__ void __launch_bounds__(256) k_pdef_fix(const __grid_constant__ DGrid g, const __grid_constant__ ScalPass P, int KC) {
+  const int lane = (int)(threadIdx.x & 31), wid = (int)(blockIdx.x * 8 + (threadIdx.x >> 5));
+  const int ni = g.ni, nj = g.nj, nk = g.nk, NI = g.NI, nch = (ni + 31) / 32, nkb = (nk + KC - 1) / KC;
+  if (wid >= nch * nj * nkb) return;
+  const int ch = wid % nch, j = 1 + (wid / nch) % nj, kb = wid / (nch * nj);
+  const int i0 = 1 + 32 * ch, i = i0 + lane, kc0 = 1 + kb * KC;
+  auto bcx = [&](int ii) { return bc_source(ii, ni, g.wbc, g.ebc); };
+  auto bcy = [&](int jj) { return bc_source(jj, nj, g.sbc, g.nbc); };
+  unsigned w = 0;
+  {   // lane 0 own, 1-2 x neighbours, 3-4 y neighbours, 5-6 the chunks below and above
+    int c = ch, r = j, b = kb;
+    if (lane == 1) c = (bcx(i0 - 1) - 1) / 32;
+    if (lane == 2) c = (bcx(min(i0 + 31, ni) + 1) - 1) / 32;
+    if (lane == 3) r = bcy(j - 1);
+    if (lane == 4) r = bcy(j + 1);
+    if (lane == 5) b = kb - 1;
+    if (lane == 6) b = kb + 1;
+    if (lane < 7 && b >= 0 && b < nkb) w = P.neg[(b * nj + r - 1) * nch + c];
+    if (lane == 0) w |= (w << 1) | (w >> 1);
+    if (lane == 5) w >>= KC - 1;
+    if (lane == 6) w = (w & 1) << (KC - 1);
+  }
+  unsigned todo = __reduce_or_sync(0xffffffffu, w);
+  const int left = nk - kc0 + 1;
+  if (left < 32) todo &= (1u << left) - 1;
+  if (KC < 32) todo &= (1u << KC) - 1;
+  if (i > ni) return;
+  const ScalField &F = P.f[0];
+  const int plane = NI * g.NJ, oc = (i - g.ib) + NI * (j - g.jb);
+  const int xr = NI * (j - g.jb) - g.ib, yc = i - g.ib;
+  const int xm2 = xr + bcx(i - 2), xm1 = xr + bcx(i - 1), xp1 = xr + bcx(i + 1), xp2 = xr + bcx(i + 2);
+  const int ym2 = yc + NI * (bcy(j - 2) - g.jb), ym1 = yc + NI * (bcy(j - 1) - g.jb);
+  const int yp1 = yc + NI * (bcy(j + 1) - g.jb), yp2 = yc + NI * (bcy(j + 2) - g.jb);
+  const float smeps = g.smeps, rdt = 1.0f / P.dt;
+  for (; todo; todo &= todo - 1) {
+    const int k = kc0 + __ffs(todo) - 1, ok = k * plane, o = ok + oc;
+    const float *X = P.dum[0] + ok, *Y = P.dum[1] + ok, *Z = P.dum[2] + o;
+    const float x0 = LDG(&X[oc]), y0 = LDG(&Y[oc]), z0 = LDG(&Z[0]);
+    float mx, my, mz;
+    bool fx, fy, fz;
+    pdef_gather(LDG(&X[xm2]), LDG(&X[xm1]), x0, LDG(&X[xp1]), LDG(&X[xp2]), smeps, &mx, &fx);
+    pdef_gather(LDG(&Y[ym2]), LDG(&Y[ym1]), y0, LDG(&Y[yp1]), LDG(&Y[yp2]), smeps, &my, &fy);
+    pdef_gather(k > 2 ? LDG(&Z[-2 * plane]) : 0.0f, k > 1 ? LDG(&Z[-plane]) : 0.0f, z0, k < nk ? LDG(&Z[plane]) : 0.0f,
+                k < nk - 1 ? LDG(&Z[2 * plane]) : 0.0f, smeps, &mz, &fz);
+    if (!(fx || fy || fz)) continue;   // the first pass's value stands
+    const float r0 = LDG(&g.rho0[k]), r0k = RAW ? 1.0f : r0, mhk = LDG(&g.mh[k]);
+    const float uh_i = LDG(&g.uh[i - g.ib]), vh_j = LDG(&g.vh[j - g.jb]);
+    float s = LDG(&F.s[o]);
+    if (F.sadd) s = (LDG(&g.th0[k]) - 300.0f) + s;
+    const float s0 = LDG(&F.sbase[o]);
+    const float *u = P.rru + k * ((NI + 1) * g.NJ) + (i - g.ib) + (NI + 1) * (j - g.jb);
+    const float *v = P.rrv + k * (NI * (g.NJ + 1)) + oc;
+    const float fu0 = LDG(&u[0]) * r0k, fu1 = LDG(&u[1]) * r0k, fv0 = LDG(&v[0]) * r0k, fv1 = LDG(&v[NI]) * r0k;
+    const float fwlo = RAW ? LDG(&P.rrw[o]) : k == 1 ? 0.0f : LDG(&P.rrw[o]) * LDG(&g.rf0[k]);
+    const float fwhi = RAW ? LDG(&P.rrw[o + plane]) : k == nk ? 0.0f : LDG(&P.rrw[o + plane]) * LDG(&g.rf0[k + 1]);
+    float ax = LDG(&P.adv[0][o]), ay = LDG(&P.adv[1][o]), az = LDG(&P.adv[2][o]);
+    if (fx) ax = (x0 + mx - r0 * s0) * rdt - s * (fu1 - fu0) * g.rdx * uh_i;
+    if (fy) ay = (y0 + my - r0 * s0) * rdt - s * (fv1 - fv0) * g.rdy * vh_j;
+    if (fz) az = (z0 + mz - r0 * s0) * rdt - s * (fwhi - fwlo) * g.rdz * mhk;
+    float div;
+    if (RAW) {
+      div = LDG(&P.divx[o]);
+    } else {
+      div = ((fu1 - fu0) * g.rdx * uh_i + (fv1 - fv0) * g.rdy * vh_j) + (fwhi - fwlo) * g.rdz * mhk;
+      if (fabsf(div) < smeps) div = 0.0f;
+    }
+    const float ten = (RAW ? P.tsave[o] : F.ten1[o]) + (((ax + ay) + az) + s * div) * LDG(&g.rr0[k]);
+    float x = RAW ? ten : s0 + P.dt * ten;
+    if (!RAW && F.flush && fabsf(x) < smeps) x = 0.0f;
+    F.snew[o] = x;
+  }
+}
+
+template <int TX, int TY, int KC, int PDEF, int RAW>
+static void scal_shape(const DGrid &g, const ScalPass &P, int weno, cudaStream_t st, int64_t *nl) {
   dim3 blk(TX, TY + 1), grid((g.ni + TX - 1) / TX, (g.nj + TY - 1) / TY, (g.nk + KC - 1) / KC);
-  if (weno) k_scal_tile<TX, TY, KC, 1><<<grid, blk, 0, st>>>(g, P);
-  else k_scal_tile<TX, TY, KC, 0><<<grid, blk, 0, st>>>(g, P);
+  {
+    ProfScope _ps(PDEF ? "k_scal_pdef" : "k_scal_tile", st);
+    if (weno) k_scal_tile<TX, TY, KC, 1, PDEF, RAW><<<grid, blk, 0, st>>>(g, P);
+    else k_scal_tile<TX, TY, KC, 0, PDEF, RAW><<<grid, blk, 0, st>>>(g, P);
+  }
+  if (PDEF) {
+    const int warps = (g.ni + 31) / 32 * g.nj * (int)grid.z;
+    ProfScope _ps("k_pdef_fix", st);
+    k_pdef_fix<RAW><<<(warps + 7) / 8, 256, 0, st>>>(g, P, KC);
+  }
+  if (nl) *nl += PDEF ? 2 : 1;
+}
+
+template <int PDEF>
+static void scal_launch(const DGrid &g, const ScalPass &P, int weno, cudaStream_t st, int64_t *nl) {
+  static_assert(kNumTileShapes == 5, "one case per tile shape");
+#define CM1G_SCAL_SHAPE(m) \
+  case m: scal_shape<kScalShapes[m][0], kScalShapes[m][1], kScalShapes[m][2], PDEF, 0>(g, P, weno, st, nl); break;
+  switch (g.tile_adv) {
+    CM1G_SCAL_SHAPE(1)
+    CM1G_SCAL_SHAPE(2)
+    CM1G_SCAL_SHAPE(3)
+    CM1G_SCAL_SHAPE(4)
+    default: scal_shape<kScalShapes[0][0], kScalShapes[0][1], kScalShapes[0][2], PDEF, 0>(g, P, weno, st, nl);
+  }
+#undef CM1G_SCAL_SHAPE
 }
 
 // One launch for `n` fields (at most SC_MAX) advanced by the same averaged
@@ -390,19 +580,42 @@ void launch_scal_pass(const DGrid &g, const ScalField *f, int n, const float *rr
     P.n = (n - a < SC_MAX) ? n - a : SC_MAX;
     for (int m = 0; m < P.n; m++) P.f[m] = f[a + m];
     P.rru = rru; P.rrv = rrv; P.rrw = rrw; P.thterm = thterm; P.dt = dt; P.err = err;
-    ProfScope _ps("k_scal_tile", st);
-    static_assert(kNumTileShapes == 5, "one case per tile shape");
-#define CM1G_SCAL_SHAPE(m) \
-  case m: scal_shape<kScalShapes[m][0], kScalShapes[m][1], kScalShapes[m][2]>(g, P, weno, st); break;
-    switch (g.tile_adv) {
-      CM1G_SCAL_SHAPE(1)
-      CM1G_SCAL_SHAPE(2)
-      CM1G_SCAL_SHAPE(3)
-      CM1G_SCAL_SHAPE(4)
-      default: CM1G_SCAL_SHAPE(0)
-    }
-#undef CM1G_SCAL_SHAPE
-    if (nl) *nl += 1;
+    scal_launch<0>(g, P, weno, st, nl);
+  }
+}
+
+static void pdef_scratch(const DGrid &g, ScalPass &P, float *scratch, unsigned *neg) {
+  const long n = nS(g);
+  for (int d = 0; d < 3; d++) { P.adv[d] = scratch + d * n; P.dum[d] = scratch + (3 + d) * n; }
+  P.neg = neg;
+}
+
+// The positive-definite pass of one field (f.pdefweno as its vertical form);
+// scratch holds 6 s-arrays, neg scal_neg_words(g) words.
+void launch_scal_pdef(const DGrid &g, const ScalField &f, const float *rru, const float *rrv, const float *rrw, int weno,
+                      float dt, float *scratch, unsigned *neg, int *err, cudaStream_t st, int64_t *nl) {
+  ScalPass P{};
+  P.n = 1; P.f[0] = f; P.rru = rru; P.rrv = rrv; P.rrw = rrw; P.dt = dt; P.err = err;
+  pdef_scratch(g, P, scratch, neg);
+  scal_launch<1>(g, P, weno, st, nl);
+}
+
+size_t scal_neg_words(const DGrid &g) { return (size_t)((g.nk + 7) / 8) * g.nj * ((g.ni + 31) / 32); }
+
+// adv.F's advs: sten += the advection of s by the caller's mass fluxes, with its
+// divx; pdef with the RK base s0 (tsave: an s-array that keeps sten).
+void launch_advs(const DGrid &g, const float *rru, const float *rrv, const float *rrw, const float *divx, const float *s,
+                 const float *s0, float *sten, int weno, int pdef, int pdefweno, double weps, float dt, float *scratch,
+                 unsigned *neg, float *tsave, int *err, cudaStream_t st, int64_t *nl) {
+  ScalPass P{};
+  P.n = 1; P.rru = rru; P.rrv = rrv; P.rrw = rrw; P.divx = divx; P.dt = dt; P.err = err; P.tsave = tsave;
+  P.f[0].s = s; P.f[0].sbase = s0; P.f[0].ten1 = sten; P.f[0].snew = sten; P.f[0].weps = weps; P.f[0].pdefweno = pdefweno;
+  constexpr int TX = kScalShapes[1][0], TY = kScalShapes[1][1], KC = kScalShapes[1][2];
+  if (pdef) {
+    pdef_scratch(g, P, scratch, neg);
+    scal_shape<TX, TY, KC, 1, 1>(g, P, weno, st, nl);
+  } else {
+    scal_shape<TX, TY, KC, 0, 1>(g, P, weno, st, nl);
   }
 }
 

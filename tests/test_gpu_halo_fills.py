@@ -1,9 +1,9 @@
-"""The one-launch halo fills (all sides periodic or all open) and the two-phase
-fills of mixed sides, on the smallest grid, at odd sizes and one point past a
-block of 128 rows or columns: every halo point, the corners that keep or copy
-an older value included, is the reference's bit for bit.  And a large step with
-walls and mixed sides, whose ring points and positive-definite masses are read
-from the points that the fills copy there."""
+"""The halo fills on the smallest grid, at odd sizes and one point past a block
+of 128 rows or columns, with periodic, open, wall and mixed sides: every halo
+point, the corners that keep or copy an older value included, is the reference's
+bit for bit.  And a large step with walls and mixed sides, whose
+positive-definite masses beyond the domain are read from the points that the
+fills copy there."""
 import ctypes as C
 
 import numpy as np
