@@ -23,9 +23,9 @@
 #include "../../include/cm1g.h"
 
 namespace cm1g {
-void launch_bc(const DGrid &g, float *a, int which, int wflag, cudaStream_t st, int64_t *nlaunch);
+void launch_bc(const DGrid &g, float *a, int which, int wflag, cudaStream_t st, int64_t *nlaunch, bool merge = true);
 void launch_bc_batch(const DGrid &g, float *const *arrays, const int *which, const int *wflag, int n,
-                     cudaStream_t st, int64_t *nlaunch);
+                     cudaStream_t st, int64_t *nlaunch, bool merge = true);
 void launch_tend_init(const DGrid &g, const TendIn &t, cudaStream_t st, int64_t *nl);
 void launch_closure_faces(int ni, int nj, int nk, int ngxy, int dir, const float *s, const float *th0, int sadd,
                           const float *vel, float dtdx, const float *params, float widen, float *phi, cudaStream_t st);
@@ -61,7 +61,7 @@ void launch_sound(const DGrid &g, int nsound, int nrk, float dt, const float *ua
                   float *sv2, float *d1, float *d2, float *lu, float *rbnd, cudaStream_t st, int64_t *nl);
 int sound_max_nk();
 void launch_stage_prep(const DGrid &g, const float *th3d, const float *pp3d, const float *qv, const LiquidIn &liq,
-                       int imoist, int eqtset, float *t11, float *t22, float *thterm, float *piadv, cudaStream_t st,
+                       int imoist, int eqtset, float *t11, float *t22, float *thterm, float *piadv, int ring, cudaStream_t st,
                        int64_t *nl);
 void launch_radbc4(const DGrid &g, const float *ua, const float *u3d, const float *va, const float *v3d,
                    float *rw, float *re, float *rs, float *rn, float dt, cudaStream_t st, int64_t *nl);
@@ -77,7 +77,7 @@ void launch_cfl(const DGrid &g, const float *u, const float *v, const float *w, 
                 cudaStream_t st, int64_t *nl);
 void launch_pdefq(const DGrid &g, float rmax, const float *rho, float *q, double *bud, double *asq,
                   cudaStream_t st, int64_t *nl);
-void launch_ppx_update(const DGrid &g, const float *pp3d, float *ppx, cudaStream_t st, int64_t *nl);
+void launch_ppx_update(const DGrid &g, const float *pp3d, float *ppx, int ring, cudaStream_t st, int64_t *nl);
 void launch_copy_batch(const DGrid &g, const float *const *src, float *const *dst, const int *stag, const int *ilo,
                        const int *ihi, const int *jlo, const int *jhi, int n, cudaStream_t st, int64_t *nl);
 void launch_level_mass(const DGrid &g, const float *rho, double *lev, cudaStream_t st, int64_t *nl);
@@ -613,7 +613,9 @@ static void closure_phi(cm1g_ctx *c, const float *th, float dt, cudaStream_t st,
   }
 }
 
-static void run_solve2(cm1g_ctx *c, const cm1g_state_t *d, float dt, double mass1) {
+// merge: fill halos in one launch, and rings where their array is formed (the
+// members of an ensemble fill them as launches of their own, k_bc.cu)
+static void run_solve2(cm1g_ctx *c, const cm1g_state_t *d, float dt, double mass1, bool merge = true) {
   const DGrid &g = c->g;
   const cm1g_config_t &cf = c->cfg;
   cudaStream_t st = c->stream;
@@ -654,9 +656,9 @@ static void run_solve2(cm1g_ctx *c, const cm1g_state_t *d, float dt, double mass
       for (int n = cf.nql1; n <= cf.nql2 && liq.n < 2; n++) liq.q[liq.n++] = buf_in(n, nrk);
       liq.b8 = c->b8;
     }
-    launch_stage_prep(g, th_in, d->pp3d, qv_in, liq, cf.imoist, cf.eqtset, c->t11, c->t22, c->thterm, c->piadv, st,
-                      nl);
-    launch_bc(g, c->t11, 2, 0, st, nl);
+    launch_stage_prep(g, th_in, d->pp3d, qv_in, liq, cf.imoist, cf.eqtset, c->t11, c->t22, c->thterm, c->piadv, merge,
+                      st, nl);
+    if (!merge) launch_bc(g, c->t11, 2, 0, st, nl, merge);
     if (diffit) df.coef = cf.kdiff6 / 64.0f / dttmp;   // adv.F:80-82, 962-964
     launch_adv_momentum(g, d->u3d, d->v3d, d->w3d, d->uten1, d->vten1, d->wten1, c->uten, c->vten, c->wten,
                         th_in, qv_in, c->mdivx, st, nl, diffit ? &df : nullptr, liq.b8);
@@ -727,7 +729,7 @@ static void run_solve2(cm1g_ctx *c, const cm1g_state_t *d, float dt, double mass
                      c->part3, c->part4, nrk == 3 && cf.apmasscon == 1, st, nl);
     // the tracers below read rho's halo through the diffusion: fill it where
     // the reference does, before them (solve2.F:1681-1684)
-    if (diffit && nrk < 3) launch_bc(g, d->rho, 2, 0, st, nl);
+    if (diffit && nrk < 3) launch_bc(g, d->rho, 2, 0, st, nl, merge);
     // passive tracers (solve2.F:1880-1970)
     for (int n = 0; n < npt; n++) {
       const int s = 1 + numq + n;
@@ -755,7 +757,7 @@ static void run_solve2(cm1g_ctx *c, const cm1g_state_t *d, float dt, double mass
         arr.push_back(d->pp3d); which.push_back(2); flag.push_back(0);
         for (int s = 0; s < nsc; s++) { arr.push_back(buf_out(s, nrk)); which.push_back(1); flag.push_back(0); }
       }
-      launch_bc_batch(g, arr.data(), which.data(), flag.data(), (int)arr.size(), st, nl);
+      launch_bc_batch(g, arr.data(), which.data(), flag.data(), (int)arr.size(), st, nl, merge);
     }
     // dry-air mass fix (solve2.F:1976-2033)
     if (nrk == 3 && cf.apmasscon == 1)
@@ -771,12 +773,12 @@ static void run_solve2(cm1g_ctx *c, const cm1g_state_t *d, float dt, double mass
   }
   if (npt) {
     std::vector<int> which(npt, 1);
-    launch_bc_batch(g, tr.data(), which.data(), nullptr, npt, st, nl);
+    launch_bc_batch(g, tr.data(), which.data(), nullptr, npt, st, nl, merge);
   }
   (void)open;
 }
 
-static void run_solve3(cm1g_ctx *c, const cm1g_state_t *d) {
+static void run_solve3(cm1g_ctx *c, const cm1g_state_t *d, bool merge = true) {
   const DGrid &g = c->g;
   const cm1g_config_t &cf = c->cfg;
   cudaStream_t st = c->stream;
@@ -789,10 +791,10 @@ static void run_solve3(cm1g_ctx *c, const cm1g_state_t *d) {
     std::vector<float *> arr{d->pp3d, d->th3d, d->rho};
     std::vector<int> which{2, 1, 2};
     for (int n = 0; n < numq; n++) { arr.push_back(d->q3d + n * ns); which.push_back(1); }
-    launch_bc_batch(g, arr.data(), which.data(), nullptr, (int)arr.size(), st, nl);
+    launch_bc_batch(g, arr.data(), which.data(), nullptr, (int)arr.size(), st, nl, merge);
   }
-  launch_ppx_update(g, d->pp3d, d->ppx, st, nl);
-  launch_bc(g, d->ppx, 2, 0, st, nl);
+  launch_ppx_update(g, d->pp3d, d->ppx, merge, st, nl);
+  if (!merge) launch_bc(g, d->ppx, 2, 0, st, nl, merge);
   // solve3.F:546-640 rollover
   {
     std::vector<const float *> src;
@@ -843,14 +845,14 @@ static void run_kessler(cm1g_ctx *c, const cm1g_state_t *d, float dt) {
   launch_kessler(g, a, c->mp_part, c->mp_colbud, c->mp_qbud, c->stream, &c->nlaunch);
 }
 
-static void run_step(cm1g_ctx *c, const cm1g_state_t *d, float dt, double mass1) {
-  run_solve2(c, d, dt, mass1);
+static void run_step(cm1g_ctx *c, const cm1g_state_t *d, float dt, double mass1, bool merge = true) {
+  run_solve2(c, d, dt, mass1, merge);
   if (c->cfg.imoist && c->cfg.ptype == 1)   // cm1.F:3421-3431 (mp_driver)
     run_kessler(c, d, dt);
   else if (c->cfg.imoist)                   // cm1.F:3410-3415 (ptype=0)
     launch_pdefq(c->g, 0.0f, d->rho, d->q3d + (long)(c->cfg.nqv - 1) * nS(c->g), nullptr, nullptr, c->stream,
                  &c->nlaunch);
-  run_solve3(c, d);
+  run_solve3(c, d, merge);
 }
 
 static int fetch_scalars(cm1g_ctx *c, double *mass2, float *cflmax) {
@@ -1275,7 +1277,7 @@ static void ens_enqueue(cm1g_ens *e, const cm1g_state_t *st, const float *dt, co
   for (size_t q = 0; q < e->m.size(); q++) {
     cm1g_ctx *c = e->m[q];
     cudaStreamWaitEvent(c->stream, e->fork, 0);
-    run_step(c, &st[q], dt[q], mass1[q]);
+    run_step(c, &st[q], dt[q], mass1[q], false);
     cudaEventRecord(e->join[q], c->stream);
     cudaStreamWaitEvent(e->stream, e->join[q], 0);
   }

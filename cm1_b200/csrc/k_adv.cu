@@ -1338,8 +1338,6 @@ __global__ void __launch_bounds__(TX * (TY + 1), 3) k_advs_tile(DGrid g, SAdv a,
   }
 }
 
-void launch_bc(const DGrid &g, float *a, int which, int wflag, cudaStream_t st, int64_t *nlaunch);
-
 // One k_advs_tile launch: WENO and the 6th-order diffusion (a.df.rho set)
 // select compile-time variants, so the plain pass carries no diffusion code.
 template <int TX, int TY, int KC, int MODE>

@@ -2,10 +2,17 @@
 //
 // The reference fills west/east halos first and then copies whole
 // south/north rows (bcs, bcp, bcu, bcw; bc.F:180-523, 528-717, 942-1146),
-// except bcv which does south/north first (bc.F:722-937).  Each direction is
-// one kernel phase here so the corner values come out exactly as the serial
-// loop order leaves them.  Every phase reads only points the same phase does
-// not write, so its threads need no ordering among themselves.
+// except bcv which does south/north first (bc.F:722-937).  Where all four
+// sides are periodic or all four are open, one launch fills every halo point
+// from the physical point that the two fills in sequence copy there
+// (k_bc_fill); a launch's own time is most of either (64x64x40, a large step's
+// 16 launches as phases 124 us of 390, 4 in this form 34 us of 347).  Walls and
+// mixed sides, and the members of an ensemble, take each direction as one launch
+// (k_bc_phase): so the corner values come out exactly as the serial loop order
+// leaves them; every phase reads only points the same phase does not write, so
+// its threads need no ordering among themselves.  (In an ensemble other members
+// fill the gaps between launches: 5.42 against 5.47 ms for twelve, and there the
+// count of launches a member that callers see stays what it was.)
 #include "cm1g_common.cuh"
 
 namespace cm1g {
@@ -167,11 +174,89 @@ __global__ void k_bc_phase(DGrid g, BcBatch b, int phase) {
   }
 }
 
+// All four sides periodic (PER) or all four open, every array of the batch in
+// one launch.  Blocks below nbr take one thread per physical row (its west and
+// east halos), the others one thread per column (its south and north halos);
+// with all sides open the reference's sequence also leaves a few corner points
+// beyond the first halo ring with the value a neighbouring halo point had
+// before the fill: the thread that overwrites that point copies it first.
+// blockIdx.y = level; for w with the flag set, the planes past its levels each
+// zero BC_ZROWS rows of the bottom and top boundaries (bc.F:1127-1137).
+static const int BC_NT = 128, BC_ZROWS = 16;
+
+template <bool PER>
+__global__ void __launch_bounds__(BC_NT) k_bc_fill(DGrid g, BcBatch b, int nbr) {
+  const int n = (int)blockIdx.z, stag = b.stag[n], kp = (int)blockIdx.y;
+  float *__restrict__ a = b.a[n];
+  const int ni = g.ni, nj = g.nj, ng = g.ngxy;
+  const int lev = (stag == STAG_W) ? g.nk - 1 : g.nk;
+  const int ie = ni + (stag == STAG_U), je = nj + (stag == STAG_V);   // last physical point
+  const long pitch = (stag == STAG_U) ? g.NI + 1 : g.NI, plane = pitch * ((stag == STAG_V) ? g.NJ + 1 : g.NJ);
+  if (kp >= lev) {
+    const int j0 = (kp - lev) * BC_ZROWS, i = (int)((blockIdx.x - nbr) * BC_NT + threadIdx.x);
+    if (stag != STAG_W || !b.wflag[n] || (int)blockIdx.x < nbr || i > ni + 1) return;
+    for (int j = j0; j < j0 + BC_ZROWS && j <= nj + 1; j++) {
+      a[iW(g, i, j, 1)] = 0.0f;
+      a[iW(g, i, j, g.nk + 1)] = 0.0f;
+    }
+    return;
+  }
+  float *__restrict__ p = a + plane * (kp + (stag == STAG_W ? 2 : 1)) - pitch * g.jb - g.ib;   // p[i + pitch j]
+  const int w = b.pmode[n] ? 1 : ng;                                   // halo width
+  if ((int)blockIdx.x < nbr) {
+    const int j = 1 + (int)(blockIdx.x * BC_NT + threadIdx.x);
+    if (j > je) return;
+    float *r = p + pitch * j;
+    if (PER) {
+      for (int h = 1; h <= w; h++) { const float x = r[ni + 1 - h], y = r[ie - ni + h]; r[1 - h] = x; r[ie + h] = y; }
+    } else {
+      const float x = r[1], y = r[ie];
+      if (stag == STAG_V && (j == 1 || j == je)) {   // bcv fills its outer rows from the columns' old halos
+        const float ow = r[0], oe = r[ie + 1];
+        for (int h = 2; h <= ng; h++) {
+          const long jj = (j == 1) ? 1 - h : je + h;
+          p[pitch * jj] = ow;
+          p[ie + 1 + pitch * jj] = oe;
+        }
+      }
+      for (int h = 1; h <= w; h++) { r[1 - h] = x; r[ie + h] = y; }
+    }
+    return;
+  }
+  const int i = 1 - w + (int)((blockIdx.x - nbr) * BC_NT + threadIdx.x);
+  if (i > ie + w) return;
+  if (PER) {
+    const int si = i < 1 ? i + ni : (i > ie ? i - ni : i);
+    const float *q = p + si;
+    float *r = p + i;
+    for (int h = 1; h <= w; h++) { const float x = q[pitch * (nj + 1 - h)], y = q[pitch * (je - nj + h)]; r[pitch * (1 - h)] = x; r[pitch * (je + h)] = y; }
+    return;
+  }
+  const int si = min(max(i, 1), ie);
+  const float x = p[si + pitch], y = p[si + pitch * je];
+  float *r = p + i;
+  if (stag == STAG_V) {                              // columns past the physical ones: the first halo rows only
+    const int hh = (i >= 1 && i <= ie) ? w : 1;
+    for (int h = 1; h <= hh; h++) { r[pitch * (1 - h)] = x; r[pitch * (je + h)] = y; }
+    return;
+  }
+  if (i < 0 || i > ie + 1) return;                   // columns beyond the first halo ring keep their values
+  if (!b.pmode[n] && (i == 1 || i == ie)) {          // the x fill of the first halo rows ran before their y fill
+    const float os = r[0], on = r[pitch * (nj + 1)];
+    for (int h = 2; h <= ng; h++) {
+      const int d = (i == 1) ? -h : h;
+      r[d] = os;
+      r[d + pitch * (nj + 1)] = on;
+    }
+  }
+  for (int h = 1; h <= w; h++) { r[pitch * (1 - h)] = x; r[pitch * (je + h)] = y; }
+}
+
 static int bc_stag(int which) { return which == 3 ? STAG_U : which == 4 ? STAG_V : which == 5 ? STAG_W : STAG_S; }
 
 // which = 1 bcs, 2 bcp, 3 bcu, 4 bcv, 5 bcw, for each array of the list.
 void launch_bc_batch(const DGrid &g, float *const *arrays, const int *which, const int *wflag, int n,
-                     cudaStream_t st, int64_t *nlaunch) {
+                     cudaStream_t st, int64_t *nlaunch, bool merge) {
   for (int base = 0; base < n; base += BC_MAXB) {
     BcBatch b{};
     b.n = (n - base < BC_MAXB) ? n - base : BC_MAXB;
@@ -180,6 +265,20 @@ void launch_bc_batch(const DGrid &g, float *const *arrays, const int *which, con
       b.stag[q] = bc_stag(which[base + q]);
       b.pmode[q] = (which[base + q] == 2);
       b.wflag[q] = wflag ? wflag[base + q] : 0;
+    }
+    const bool per = g.wbc == 1 && g.ebc == 1 && g.sbc == 1 && g.nbc == 1;
+    const bool open = g.wbc == 2 && g.ebc == 2 && g.sbc == 2 && g.nbc == 2;
+    if (merge && (per || open)) {
+      int nz = 0;
+      for (int q = 0; q < b.n; q++)
+        if (b.stag[q] == STAG_W && b.wflag[q]) nz = (g.nj + 2 + BC_ZROWS - 1) / BC_ZROWS - 1;
+      const int nbr = (g.nj + 1 + BC_NT - 1) / BC_NT, nbc = (g.NI + 1 + BC_NT - 1) / BC_NT;
+      dim3 grid(nbr + nbc, g.nk + nz, b.n);
+      ProfScope _ps("k_bc_fill", st);
+      if (per) k_bc_fill<true><<<grid, BC_NT, 0, st>>>(g, b, nbr);
+      else k_bc_fill<false><<<grid, BC_NT, 0, st>>>(g, b, nbr);
+      if (nlaunch) *nlaunch += 1;
+      continue;
     }
     dim3 blk(128);
     const int span = (g.NI > g.NJ ? g.NI : g.NJ) + 1;
@@ -190,8 +289,8 @@ void launch_bc_batch(const DGrid &g, float *const *arrays, const int *which, con
   }
 }
 
-void launch_bc(const DGrid &g, float *a, int which, int wflag, cudaStream_t st, int64_t *nlaunch) {
-  launch_bc_batch(g, &a, &which, &wflag, 1, st, nlaunch);
+void launch_bc(const DGrid &g, float *a, int which, int wflag, cudaStream_t st, int64_t *nlaunch, bool merge) {
+  launch_bc_batch(g, &a, &which, &wflag, 1, st, nlaunch, merge);
 }
 
 }  // namespace cm1g

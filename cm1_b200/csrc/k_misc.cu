@@ -9,31 +9,35 @@ namespace cm1g {
 // ---------------------------------------------------------------------
 // stage set-up: theta_rho (t11), ppterm (t22), thterm (solve2.F:313-446)
 // on the interior and piadv = pi0+pp' on 0..ni+1 x 0..nj+1 (solve2.F:1027-1038).
-// A thread takes SP_K levels, whose loads are issued together
-// (256x256x80, moist: one level a thread 62 us, four 45 us, 3.3 TB/s).
+// With ring set, t11 on the ring around the interior is formed from the point
+// that bcp would copy it from, and needs no fill.  A thread takes SP_K levels,
+// whose loads are issued together (256x256x80, moist: one level a thread 62 us,
+// four 45 us, 3.3 TB/s).
 // ---------------------------------------------------------------------
 static const int SP_K = 4;
 __global__ void __launch_bounds__(256) k_stage_prep(DGrid g, const float *__restrict__ th3d,
                                                     const float *__restrict__ pp3d, const float *__restrict__ qv,
                                                     LiquidIn liq, int imoist, int eqtset, float *__restrict__ t11,
                                                     float *__restrict__ t22, float *__restrict__ thterm,
-                                                    float *__restrict__ piadv) {
+                                                    float *__restrict__ piadv, int ring) {
   const int i = (int)(blockIdx.x * 32 + threadIdx.x);               // 0..ni+1
   const int j = (int)(blockIdx.y * 8 + threadIdx.y);                // 0..nj+1
   const int k0 = 1 + (int)blockIdx.z * SP_K;
   if (i > g.ni + 1 || j > g.nj + 1) return;
   const int plane = g.NI * g.NJ;                                    // < 2^31 points (cm1g_init)
   const int oc = (i - g.ib) + g.NI * (j - g.jb);
-  const bool inside = i >= 1 && i <= g.ni && j >= 1 && j <= g.nj;
+  const int is = bc_source(i, g.ni, g.wbc, g.ebc), js = bc_source(j, g.nj, g.sbc, g.nbc);
+  const int sc = (is - g.ib) + g.NI * (js - g.jb);
+  const bool inside = sc == oc;
   float pp[SP_K], th[SP_K], qq[SP_K], l0[SP_K], l1[SP_K];
 #pragma unroll
   for (int m = 0; m < SP_K; m++) {
-    const int o = min(k0 + m, g.nk) * plane + oc;
+    const int k = min(k0 + m, g.nk), o = k * plane + oc, s = k * plane + sc;
     pp[m] = LDG(&pp3d[o]);
-    th[m] = LDG(&th3d[o]);
-    qq[m] = imoist ? LDG(&qv[o]) : 0.0f;
-    l0[m] = liq.n > 0 ? LDG(&liq.q[0][o]) : 0.0f;
-    l1[m] = liq.n > 1 ? LDG(&liq.q[1][o]) : 0.0f;
+    th[m] = LDG(&th3d[s]);
+    qq[m] = imoist ? LDG(&qv[s]) : 0.0f;
+    l0[m] = liq.n > 0 ? LDG(&liq.q[0][s]) : 0.0f;
+    l1[m] = liq.n > 1 ? LDG(&liq.q[1][s]) : 0.0f;
   }
   const Consts &c = g.c;
 #pragma unroll
@@ -43,7 +47,7 @@ __global__ void __launch_bounds__(256) k_stage_prep(DGrid g, const float *__rest
     const int o = k * plane + oc;
     const float th3 = th[m], th0 = LDG(&g.th0[k]), pi0 = LDG(&g.pi0[k]);
     piadv[o] = pi0 + pp[m];
-    if (!inside) continue;
+    if (!inside && !ring) continue;
     if (imoist) {
       const float q = fmaxf(qq[m], 0.0f);
       // dum2: the liquid species in index order (solve2.F:315-345); no ice
@@ -53,6 +57,7 @@ __global__ void __launch_bounds__(256) k_stage_prep(DGrid g, const float *__rest
       const float d3 = 0.0f;
       const float qli = fmaxf(0.0f, d2 + d3);
       t11[o] = (th0 + th3) * (1.0f + c.reps * q) / ((1.0f + q) + qli);
+      if (!inside) continue;
       // buoyancy dum8 at s-points (solve2.F:395-396) when liquid is present;
       // without it k_mom forms the same expression from theta and qv
       if (liq.b8)
@@ -69,17 +74,17 @@ __global__ void __launch_bounds__(256) k_stage_prep(DGrid g, const float *__rest
       }
     } else {
       t11[o] = th0 + th3;
-      t22[o] = (pi0 + pp[m]) * c.rddcv;
+      if (inside) t22[o] = (pi0 + pp[m]) * c.rddcv;
     }
   }
 }
 
 void launch_stage_prep(const DGrid &g, const float *th3d, const float *pp3d, const float *qv, const LiquidIn &liq,
-                       int imoist, int eqtset, float *t11, float *t22, float *thterm, float *piadv, cudaStream_t st,
-                       int64_t *nl) {
+                       int imoist, int eqtset, float *t11, float *t22, float *thterm, float *piadv, int ring,
+                       cudaStream_t st, int64_t *nl) {
   dim3 grid((g.ni + 2 + 31) / 32, (g.nj + 2 + 7) / 8, (g.nk + SP_K - 1) / SP_K);
   ProfScope _ps("k_stage_prep", st);
-  k_stage_prep<<<grid, dim3(32, 8), 0, st>>>(g, th3d, pp3d, qv, liq, imoist, eqtset, t11, t22, thterm, piadv);
+  k_stage_prep<<<grid, dim3(32, 8), 0, st>>>(g, th3d, pp3d, qv, liq, imoist, eqtset, t11, t22, thterm, piadv, ring);
   if (nl) *nl += 1;
 }
 
@@ -429,11 +434,13 @@ void launch_pdefq(const DGrid &g, float rmax, const float *rho, float *q, double
 }
 
 // ---------------------------------------------------------------------
-// solve3 pieces: ppx = pp3d + ppx (solve3.F:276-283), and the rollover copies
-// over the reference's ranges (solve3.F:546-640).
+// solve3 pieces: ppx = pp3d + ppx (solve3.F:276-283) with (ring set) bcp's
+// ring, whose points are written by the thread that owns the point they copy; and
+// the rollover copies over the reference's ranges (solve3.F:546-640).
 // ---------------------------------------------------------------------
 static const int PX_K = 4;      // levels of a thread, loaded together
-__global__ void __launch_bounds__(256) k_ppx_update(DGrid g, const float *__restrict__ pp3d, float *__restrict__ ppx) {
+__global__ void __launch_bounds__(256) k_ppx_update(DGrid g, const float *__restrict__ pp3d, float *__restrict__ ppx,
+                                                    int ring) {
   const int i = 1 + (int)(blockIdx.x * 32 + threadIdx.x), j = 1 + (int)(blockIdx.y * 8 + threadIdx.y);
   const int k0 = 1 + (int)blockIdx.z * PX_K;
   const int ni = g.ni, nj = g.nj, NI = g.NI;
@@ -445,9 +452,21 @@ __global__ void __launch_bounds__(256) k_ppx_update(DGrid g, const float *__rest
     const int o = min(k0 + m, g.nk) * plane + oc;
     v[m] = LDG(&pp3d[o]) + ppx[o];
   }
+  // ring columns and rows that bcp copies from this point (offsets from it; 0: none)
+  const int xw = (g.wbc == 1 ? i == ni : i == 1) ? -i : 0, xe = (g.ebc == 1 ? i == 1 : i == ni) ? ni + 1 - i : 0;
+  const int ys = (g.sbc == 1 ? j == nj : j == 1) ? -j * NI : 0, yn = (g.nbc == 1 ? j == 1 : j == nj) ? (nj + 1 - j) * NI : 0;
 #pragma unroll
-  for (int m = 0; m < PX_K; m++)
-    if (k0 + m <= g.nk) ppx[(k0 + m) * plane + oc] = v[m];
+  for (int m = 0; m < PX_K; m++) {
+    if (k0 + m > g.nk) break;
+    float *r = ppx + (k0 + m) * plane + oc;
+    const float x = v[m];
+    r[0] = x;
+    if (!ring) continue;
+    if (xw) r[xw] = x;
+    if (xe) r[xe] = x;
+    if (ys) { r[ys] = x; if (xw) r[ys + xw] = x; if (xe) r[ys + xe] = x; }
+    if (yn) { r[yn] = x; if (xw) r[yn + xw] = x; if (xe) r[yn + xe] = x; }
+  }
 }
 
 // Rollover copies dst = src over i = ilo..ihi, j = jlo..jhi, k = 1..nk
@@ -475,9 +494,9 @@ __global__ void k_copy_batch(CopyBatch b) {
   for (int i = c.ilo + lane; i <= c.ihi; i += 32) c.dst[base + i] = LDG(&c.src[base + i]);
 }
 
-void launch_ppx_update(const DGrid &g, const float *pp3d, float *ppx, cudaStream_t st, int64_t *nl) {
+void launch_ppx_update(const DGrid &g, const float *pp3d, float *ppx, int ring, cudaStream_t st, int64_t *nl) {
   dim3 grid((g.ni + 31) / 32, (g.nj + 7) / 8, (g.nk + PX_K - 1) / PX_K);
-  { ProfScope _ps("k_ppx_update", st); k_ppx_update<<<grid, dim3(32, 8), 0, st>>>(g, pp3d, ppx); }
+  { ProfScope _ps("k_ppx_update", st); k_ppx_update<<<grid, dim3(32, 8), 0, st>>>(g, pp3d, ppx, ring); }
   if (nl) *nl += 1;
 }
 

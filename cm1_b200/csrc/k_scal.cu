@@ -460,17 +460,18 @@ __device__ __forceinline__ void pdef_gather(float dm2, float dm1, float d0, floa
 // columns of a row over a chunk of KC levels; it reads the chunk's word of
 // negative provisional masses and its neighbours' (a cell changes only if its
 // own, or one beside it in x, y or z, is negative) and visits the levels named
-// there.  A field without such masses costs the launch (256x256x80: 10 us against
-// 135 us when every cell read the six arrays back), a tracer of a few blobs after
-// two stages 135 us as before (waiting on its 15 masses a cell), and the host
-// entry at 251x187x79 100 us with every level named.  Beyond the domain the masses are those of the points that the lateral
-// bc copies there (pdef.F:102, 338).
+// there, all loads of a level in flight at once.  A field without such masses
+// costs the launch (256x256x80: 10 us against 135 us when every cell read the six
+// arrays back), a tracer of a few blobs after two stages 100 us; the host entry at
+// 251x187x79 with every level named 74 us, where a thread a cell took 97.  Beyond
+// the domain the masses are those of the points that the lateral bc copies there
+// (pdef.F:102, 338).
 template <int RAW>
 __global__ void __launch_bounds__(256) k_pdef_fix(const __grid_constant__ DGrid g, const __grid_constant__ ScalPass P, int KC) {
-  const int lane = (int)(threadIdx.x & 31), wid = (int)(blockIdx.x * 8 + (threadIdx.x >> 5));
+  const int lane = (int)(threadIdx.x & 31);
   const int ni = g.ni, nj = g.nj, nk = g.nk, NI = g.NI, nch = (ni + 31) / 32, nkb = (nk + KC - 1) / KC;
-  if (wid >= nch * nj * nkb) return;
-  const int ch = wid % nch, j = 1 + (wid / nch) % nj, kb = wid / (nch * nj);
+  const int ch = (int)blockIdx.x, j = 1 + (int)(blockIdx.y * 8 + (threadIdx.x >> 5)), kb = (int)blockIdx.z;   // 8 rows a block
+  if (j > nj) return;
   const int i0 = 1 + 32 * ch, i = i0 + lane, kc0 = 1 + kb * KC;
   auto bcx = [&](int ii) { return bc_source(ii, ni, g.wbc, g.ebc); };
   auto bcy = [&](int jj) { return bc_source(jj, nj, g.sbc, g.nbc); };
@@ -504,24 +505,30 @@ __global__ void __launch_bounds__(256) k_pdef_fix(const __grid_constant__ DGrid 
     const int k = kc0 + __ffs(todo) - 1, ok = k * plane, o = ok + oc;
     const float *X = P.dum[0] + ok, *Y = P.dum[1] + ok, *Z = P.dum[2] + o;
     const float x0 = LDG(&X[oc]), y0 = LDG(&Y[oc]), z0 = LDG(&Z[0]);
-    float mx, my, mz;
-    bool fx, fy, fz;
-    pdef_gather(LDG(&X[xm2]), LDG(&X[xm1]), x0, LDG(&X[xp1]), LDG(&X[xp2]), smeps, &mx, &fx);
-    pdef_gather(LDG(&Y[ym2]), LDG(&Y[ym1]), y0, LDG(&Y[yp1]), LDG(&Y[yp2]), smeps, &my, &fy);
-    pdef_gather(k > 2 ? LDG(&Z[-2 * plane]) : 0.0f, k > 1 ? LDG(&Z[-plane]) : 0.0f, z0, k < nk ? LDG(&Z[plane]) : 0.0f,
-                k < nk - 1 ? LDG(&Z[2 * plane]) : 0.0f, smeps, &mz, &fz);
-    if (!(fx || fy || fz)) continue;   // the first pass's value stands
-    const float r0 = LDG(&g.rho0[k]), r0k = RAW ? 1.0f : r0, mhk = LDG(&g.mh[k]);
-    const float uh_i = LDG(&g.uh[i - g.ib]), vh_j = LDG(&g.vh[j - g.jb]);
+    const float xa = LDG(&X[xm2]), xb = LDG(&X[xm1]), xc = LDG(&X[xp1]), xd = LDG(&X[xp2]);
+    const float ya = LDG(&Y[ym2]), yb = LDG(&Y[ym1]), yc_ = LDG(&Y[yp1]), yd = LDG(&Y[yp2]);
+    const float za = k > 2 ? LDG(&Z[-2 * plane]) : 0.0f, zb = k > 1 ? LDG(&Z[-plane]) : 0.0f;
+    const float zc = k < nk ? LDG(&Z[plane]) : 0.0f, zd = k < nk - 1 ? LDG(&Z[2 * plane]) : 0.0f;
     float s = LDG(&F.s[o]);
-    if (F.sadd) s = (LDG(&g.th0[k]) - 300.0f) + s;
     const float s0 = LDG(&F.sbase[o]);
     const float *u = P.rru + k * ((NI + 1) * g.NJ) + (i - g.ib) + (NI + 1) * (j - g.jb);
     const float *v = P.rrv + k * (NI * (g.NJ + 1)) + oc;
-    const float fu0 = LDG(&u[0]) * r0k, fu1 = LDG(&u[1]) * r0k, fv0 = LDG(&v[0]) * r0k, fv1 = LDG(&v[NI]) * r0k;
-    const float fwlo = RAW ? LDG(&P.rrw[o]) : k == 1 ? 0.0f : LDG(&P.rrw[o]) * LDG(&g.rf0[k]);
-    const float fwhi = RAW ? LDG(&P.rrw[o + plane]) : k == nk ? 0.0f : LDG(&P.rrw[o + plane]) * LDG(&g.rf0[k + 1]);
+    const float u0 = LDG(&u[0]), u1 = LDG(&u[1]), v0 = LDG(&v[0]), v1 = LDG(&v[NI]);
+    const float w0 = (RAW || k > 1) ? LDG(&P.rrw[o]) : 0.0f, w1 = (RAW || k < nk) ? LDG(&P.rrw[o + plane]) : 0.0f;
     float ax = LDG(&P.adv[0][o]), ay = LDG(&P.adv[1][o]), az = LDG(&P.adv[2][o]);
+    const float t1 = RAW ? P.tsave[o] : F.ten1[o];
+    float mx, my, mz;
+    bool fx, fy, fz;
+    pdef_gather(xa, xb, x0, xc, xd, smeps, &mx, &fx);
+    pdef_gather(ya, yb, y0, yc_, yd, smeps, &my, &fy);
+    pdef_gather(za, zb, z0, zc, zd, smeps, &mz, &fz);
+    if (!(fx || fy || fz)) continue;   // the first pass's value stands
+    const float r0 = LDG(&g.rho0[k]), r0k = RAW ? 1.0f : r0, mhk = LDG(&g.mh[k]);
+    const float uh_i = LDG(&g.uh[i - g.ib]), vh_j = LDG(&g.vh[j - g.jb]);
+    if (F.sadd) s = (LDG(&g.th0[k]) - 300.0f) + s;
+    const float fu0 = u0 * r0k, fu1 = u1 * r0k, fv0 = v0 * r0k, fv1 = v1 * r0k;
+    const float fwlo = RAW ? w0 : k == 1 ? 0.0f : w0 * LDG(&g.rf0[k]);
+    const float fwhi = RAW ? w1 : k == nk ? 0.0f : w1 * LDG(&g.rf0[k + 1]);
     if (fx) ax = (x0 + mx - r0 * s0) * rdt - s * (fu1 - fu0) * g.rdx * uh_i;
     if (fy) ay = (y0 + my - r0 * s0) * rdt - s * (fv1 - fv0) * g.rdy * vh_j;
     if (fz) az = (z0 + mz - r0 * s0) * rdt - s * (fwhi - fwlo) * g.rdz * mhk;
@@ -532,7 +539,7 @@ __global__ void __launch_bounds__(256) k_pdef_fix(const __grid_constant__ DGrid 
       div = ((fu1 - fu0) * g.rdx * uh_i + (fv1 - fv0) * g.rdy * vh_j) + (fwhi - fwlo) * g.rdz * mhk;
       if (fabsf(div) < smeps) div = 0.0f;
     }
-    const float ten = (RAW ? P.tsave[o] : F.ten1[o]) + (((ax + ay) + az) + s * div) * LDG(&g.rr0[k]);
+    const float ten = t1 + (((ax + ay) + az) + s * div) * LDG(&g.rr0[k]);
     float x = RAW ? ten : s0 + P.dt * ten;
     if (!RAW && F.flush && fabsf(x) < smeps) x = 0.0f;
     F.snew[o] = x;
@@ -548,9 +555,8 @@ static void scal_shape(const DGrid &g, const ScalPass &P, int weno, cudaStream_t
     else k_scal_tile<TX, TY, KC, 0, PDEF, RAW><<<grid, blk, 0, st>>>(g, P);
   }
   if (PDEF) {
-    const int warps = (g.ni + 31) / 32 * g.nj * (int)grid.z;
     ProfScope _ps("k_pdef_fix", st);
-    k_pdef_fix<RAW><<<(warps + 7) / 8, 256, 0, st>>>(g, P, KC);
+    k_pdef_fix<RAW><<<dim3((g.ni + 31) / 32, (g.nj + 7) / 8, grid.z), 256, 0, st>>>(g, P, KC);
   }
   if (nl) *nl += PDEF ? 2 : 1;
 }

@@ -706,7 +706,6 @@ __global__ void __launch_bounds__(TX * TY, 5) k_sound_col(DGrid g, SoundIO io, S
 }
 
 
-void launch_bc(const DGrid &g, float *a, int which, int wflag, cudaStream_t st, int64_t *nlaunch);
 
 // Number of small steps and their length for RK stage nrk (sound.F:79-101).
 void sound_nloop(int nsound, int nrk, float dt, int *nloop_out, float *dts_out) {
