@@ -50,7 +50,8 @@ constexpr int kTileShapes[kNumTileShapes][3] = {{32, 8, 16}, {32, 8, 8}, {32, 4,
 // Tile shapes of the scalar passes (k_scal_tile, k_advs_tile), indexed like
 // kTileShapes: TX x TY cells and KC levels per block; the block has one more
 // row of TX threads than the tile has cell rows (the row that evaluates the
-// tile's north and east faces), so a block is TX x (TY + 1) threads.
+// tile's north and east faces), so a block is TX x (TY + 1) threads.  k_scal_tile
+// and k_mom choose the levels of the default by the grid's size.
 constexpr int kScalShapes[kNumTileShapes][3] = {{32, 7, 16}, {32, 7, 8}, {32, 3, 16}, {64, 3, 16}, {32, 7, 32}};
 // Forms of the acoustic kernel: 0 tile (32 columns, the warps over the levels
 // chosen by the grid's size), 1 tile with 16 explicit warps, 2 column sweep

@@ -5,7 +5,7 @@
 // 1951-1957).  All fields of a stage are advected by the same averaged
 // velocities rru/rrv/rrw, so one block advances every field over its tile:
 //
-//  * a block owns TX x TY columns and KC levels; it walks the items
+//  * a block owns TX x TY columns and kc levels; it walks the items
 //    (field n, level k) field by field, level by level upward;
 //  * the level of a field is staged in shared memory with its 3-point halo by
 //    one-dimensional bulk copies (cp.async.bulk), one per row, into a ring of
@@ -44,10 +44,11 @@
 namespace cm1g {
 
 constexpr int SC_MAX = 16;      // fields per launch
+constexpr int SC_KMAX = 32;     // levels per block at most (a word of signs holds a bit for each)
 
 struct ScalPass {
   ScalField f[SC_MAX];
-  int n;
+  int n, kc;                    // fields; levels per block
   const float *rru, *rrv, *rrw; // small-step-averaged velocities (sound.F:806-835)
   const float *thterm;          // moist theta: thten -= div(u_avg) * thterm (solve2.F:1320-1329); null: none
   float dt;
@@ -173,7 +174,7 @@ __device__ __forceinline__ ScLev scal_level(const DGrid &g, int k) {
 // 478-496) of one field: advx..dumz and neg beside the value that holds where no
 // neighbouring provisional mass is negative (k_pdef_fix does the other cells).
 // RAW: the caller's mass fluxes and divx; the value is the tendency.
-template <int TX, int TY, int KC, int WENO, int PDEF, int RAW>
+template <int TX, int TY, int WENO, int PDEF, int RAW>
 __global__ void __launch_bounds__(TX * (TY + 1), 3) k_scal_tile(const __grid_constant__ DGrid g,
                                                                  const __grid_constant__ ScalPass P) {
   constexpr int SW = TX + 6, SH = TY + 6;                  // staged columns and rows
@@ -183,7 +184,7 @@ __global__ void __launch_bounds__(TX * (TY + 1), 3) k_scal_tile(const __grid_con
   static_assert(SH <= 32, "one lane per staged row");
   __shared__ __align__(128) float ring[RD][PL];
   __shared__ float2 fx[2][NFX], fy[2][NFY];                // flux and averaged velocity of each face
-  __shared__ ScLev lev[KC];
+  __shared__ ScLev lev[SC_KMAX];
   __shared__ __align__(8) uint64_t bars[RD];
 
   const int tx = threadIdx.x, ty = threadIdx.y, tid = tx + TX * ty, lane = tid & 31;
@@ -197,7 +198,7 @@ __global__ void __launch_bounds__(TX * (TY + 1), 3) k_scal_tile(const __grid_con
   const int SP = scal_pitch<TX>(NI);
   const float uh_i = active ? LDG(&g.uh[i - g.ib]) : 0.0f, vh_j = active ? LDG(&g.vh[j - g.jb]) : 0.0f;
   const int orow0 = (i0 - 3 - g.ib) + NI * (j0 - 3 - g.jb);    // first staged element of a plane
-  const int kc0 = 1 + (int)blockIdx.z * KC, kc1 = min(nk, kc0 + KC - 1);
+  const int kc0 = 1 + (int)blockIdx.z * P.kc, kc1 = min(nk, kc0 + P.kc - 1);
   const int nlev = kc1 - kc0 + 1, nitem = P.n * nlev;
 
   // faces of this thread: a cell row's thread owns the x face on the west of
@@ -457,7 +458,7 @@ __device__ __forceinline__ void pdef_gather(float dm2, float dm1, float d0, floa
 // Second pass of the positive-definite scheme: pdefz, pdefx2, pdefy2
 // (pdef.F:117-264, 358-454, 459-581) and the update of adv.F:650-659 and
 // solve2.F:1513-1520, for the cells whose value they change.  A warp owns 32
-// columns of a row over a chunk of KC levels; it reads the chunk's word of
+// columns of a row over a chunk of the first pass's levels; it reads the chunk's word of
 // negative provisional masses and its neighbours' (a cell changes only if its
 // own, or one beside it in x, y or z, is negative) and visits the levels named
 // there, all loads of a level in flight at once.  A field without such masses
@@ -467,9 +468,9 @@ __device__ __forceinline__ void pdef_gather(float dm2, float dm1, float d0, floa
 // the domain the masses are those of the points that the lateral bc copies there
 // (pdef.F:102, 338).
 template <int RAW>
-__global__ void __launch_bounds__(256) k_pdef_fix(const __grid_constant__ DGrid g, const __grid_constant__ ScalPass P, int KC) {
+__global__ void __launch_bounds__(256) k_pdef_fix(const __grid_constant__ DGrid g, const __grid_constant__ ScalPass P) {
   const int lane = (int)(threadIdx.x & 31);
-  const int ni = g.ni, nj = g.nj, nk = g.nk, NI = g.NI, nch = (ni + 31) / 32, nkb = (nk + KC - 1) / KC;
+  const int ni = g.ni, nj = g.nj, nk = g.nk, NI = g.NI, KC = P.kc, nch = (ni + 31) / 32, nkb = (nk + KC - 1) / KC;
   const int ch = (int)blockIdx.x, j = 1 + (int)(blockIdx.y * 8 + (threadIdx.x >> 5)), kb = (int)blockIdx.z;   // 8 rows a block
   if (j > nj) return;
   const int i0 = 1 + 32 * ch, i = i0 + lane, kc0 = 1 + kb * KC;
@@ -546,34 +547,44 @@ __global__ void __launch_bounds__(256) k_pdef_fix(const __grid_constant__ DGrid 
   }
 }
 
-template <int TX, int TY, int KC, int PDEF, int RAW>
-static void scal_shape(const DGrid &g, const ScalPass &P, int weno, cudaStream_t st, int64_t *nl) {
-  dim3 blk(TX, TY + 1), grid((g.ni + TX - 1) / TX, (g.nj + TY - 1) / TY, (g.nk + KC - 1) / KC);
+// kc: levels per block; 0: those whose blocks finish first.  A block costs about
+// SC_OVER levels besides its own (its first plane's latency, the window and the
+// face below its first level).  Scalar passes of a step with 16, 8 and 32 levels
+// and with this rule: 64x64x40 82, 51, 137, 39 us; 203x150x61, four fields 713, 628,
+// 838, 665 us; 256x256x80 2.60, 2.53, 2.51, 2.47 ms; 512x512x128 6.78, 7.20, 6.74, 6.78 ms.
+// The host entry's single field takes at most 16: its second pass walks a chunk
+// level by level (251x187x79: 95 us with 20 levels, 76 with 12).
+constexpr int SC_OVER = 2;
+template <int TX, int TY, int PDEF, int RAW>
+static void scal_shape(const DGrid &g, ScalPass P, int kc, int weno, cudaStream_t st, int64_t *nl) {
+  dim3 blk(TX, TY + 1), grid((g.ni + TX - 1) / TX, (g.nj + TY - 1) / TY, 1);
+  if (!kc) kc = tile_levels((long)grid.x * grid.y, g.nk, 3 * 148, SC_OVER, RAW ? 16 : SC_KMAX);
+  P.kc = kc;
+  grid.z = (g.nk + kc - 1) / kc;
   {
     ProfScope _ps(PDEF ? "k_scal_pdef" : "k_scal_tile", st);
-    if (weno) k_scal_tile<TX, TY, KC, 1, PDEF, RAW><<<grid, blk, 0, st>>>(g, P);
-    else k_scal_tile<TX, TY, KC, 0, PDEF, RAW><<<grid, blk, 0, st>>>(g, P);
+    if (weno) k_scal_tile<TX, TY, 1, PDEF, RAW><<<grid, blk, 0, st>>>(g, P);
+    else k_scal_tile<TX, TY, 0, PDEF, RAW><<<grid, blk, 0, st>>>(g, P);
   }
   if (PDEF) {
     ProfScope _ps("k_pdef_fix", st);
-    k_pdef_fix<RAW><<<dim3((g.ni + 31) / 32, (g.nj + 7) / 8, grid.z), 256, 0, st>>>(g, P, KC);
+    k_pdef_fix<RAW><<<dim3((g.ni + 31) / 32, (g.nj + 7) / 8, grid.z), 256, 0, st>>>(g, P);
   }
   if (nl) *nl += PDEF ? 2 : 1;
 }
 
+// the tile of a shape, with the levels of its table but for the default's
 template <int PDEF>
 static void scal_launch(const DGrid &g, const ScalPass &P, int weno, cudaStream_t st, int64_t *nl) {
-  static_assert(kNumTileShapes == 5, "one case per tile shape");
-#define CM1G_SCAL_SHAPE(m) \
-  case m: scal_shape<kScalShapes[m][0], kScalShapes[m][1], kScalShapes[m][2], PDEF, 0>(g, P, weno, st, nl); break;
+  static_assert(kNumTileShapes == 5 && kScalShapes[0][0] == 32 && kScalShapes[0][1] == 7 && kScalShapes[1][1] == 7 &&
+                    kScalShapes[2][1] == 3 && kScalShapes[3][0] == 64 && kScalShapes[4][1] == 7,
+                "the tiles of the shapes");
+  const int kc = g.tile_adv > 0 ? kScalShapes[g.tile_adv][2] : 0;
   switch (g.tile_adv) {
-    CM1G_SCAL_SHAPE(1)
-    CM1G_SCAL_SHAPE(2)
-    CM1G_SCAL_SHAPE(3)
-    CM1G_SCAL_SHAPE(4)
-    default: scal_shape<kScalShapes[0][0], kScalShapes[0][1], kScalShapes[0][2], PDEF, 0>(g, P, weno, st, nl);
+    case 2: scal_shape<32, 3, PDEF, 0>(g, P, kc, weno, st, nl); break;
+    case 3: scal_shape<64, 3, PDEF, 0>(g, P, kc, weno, st, nl); break;
+    default: scal_shape<32, 7, PDEF, 0>(g, P, kc, weno, st, nl);
   }
-#undef CM1G_SCAL_SHAPE
 }
 
 // One launch for `n` fields (at most SC_MAX) advanced by the same averaged
@@ -606,7 +617,7 @@ void launch_scal_pdef(const DGrid &g, const ScalField &f, const float *rru, cons
   scal_launch<1>(g, P, weno, st, nl);
 }
 
-size_t scal_neg_words(const DGrid &g) { return (size_t)((g.nk + 7) / 8) * g.nj * ((g.ni + 31) / 32); }
+size_t scal_neg_words(const DGrid &g) { return (size_t)((g.nk + 3) / 4) * g.nj * ((g.ni + 31) / 32); }
 
 // adv.F's advs: sten += the advection of s by the caller's mass fluxes, with its
 // divx; pdef with the RK base s0 (tsave: an s-array that keeps sten).
@@ -616,12 +627,11 @@ void launch_advs(const DGrid &g, const float *rru, const float *rrv, const float
   ScalPass P{};
   P.n = 1; P.rru = rru; P.rrv = rrv; P.rrw = rrw; P.divx = divx; P.dt = dt; P.err = err; P.tsave = tsave;
   P.f[0].s = s; P.f[0].sbase = s0; P.f[0].ten1 = sten; P.f[0].snew = sten; P.f[0].weps = weps; P.f[0].pdefweno = pdefweno;
-  constexpr int TX = kScalShapes[1][0], TY = kScalShapes[1][1], KC = kScalShapes[1][2];
   if (pdef) {
     pdef_scratch(g, P, scratch, neg);
-    scal_shape<TX, TY, KC, 1, 1>(g, P, weno, st, nl);
+    scal_shape<32, 7, 1, 1>(g, P, 0, weno, st, nl);
   } else {
-    scal_shape<TX, TY, KC, 0, 1>(g, P, weno, st, nl);
+    scal_shape<32, 7, 0, 1>(g, P, 0, weno, st, nl);
   }
 }
 
