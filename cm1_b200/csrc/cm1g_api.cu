@@ -205,7 +205,7 @@ struct cm1g_ctx {
   double *ener = nullptr;                     // calcener chunk sums (4 x nk x chunks) and results
   float *fscal = nullptr;
   int *cflbits = nullptr;
-  int *advs_err = nullptr;                    // cm1g_advs: a staging wait gave up (pinned, read after its synchronize)
+  int *advs_err = nullptr;                    // cm1g_advs: a staging wait gave up (PinnedFlags slot; null: cflbits[2])
   unsigned long long *mm = nullptr;
   // host staging (for host-pointer calls)
   cm1g_state_t dst{};
@@ -240,6 +240,43 @@ struct cm1g_ctx {
   float *d2s = nullptr;                       // scratch of the 2nd-order diffusion (cm1g_diff2)
   float *les = nullptr;                       // eddy viscosities of cm1g_turbsmag when the caller gives no arrays
 };
+
+// Flags in pinned memory that a kernel can raise and the host read after a
+// synchronize, without a copy (12 us of cm1g_advs).  Pinning a page takes some
+// 5 ms, so one page serves the process: a context takes a slot at its creation and
+// gives it back; without one (more contexts than slots) it copies a device flag.
+struct PinnedFlags {
+  static constexpr int N = 1024;
+  std::mutex mu;
+  int *page = nullptr;
+  bool tried = false;
+  std::vector<int *> slots;
+  int *take() {
+    std::lock_guard<std::mutex> lk(mu);
+    if (!tried) {
+      tried = true;
+      if (cudaHostAlloc((void **)&page, N * sizeof(int), cudaHostAllocPortable) != cudaSuccess) {
+        (void)cudaGetLastError();
+        page = nullptr;
+      }
+      for (int q = 0; page && q < N; q++) slots.push_back(page + q);
+    }
+    if (slots.empty()) return nullptr;
+    int *p = slots.back();
+    slots.pop_back();
+    *p = 0;
+    return p;
+  }
+  void give(int *p) {
+    if (!p) return;
+    std::lock_guard<std::mutex> lk(mu);
+    slots.push_back(p);
+  }
+};
+static PinnedFlags &pinned_flags() {
+  static PinnedFlags *f = new PinnedFlags();   // never destroyed: contexts may be finalized at exit
+  return *f;
+}
 
 // Makes the context's profile (if any) the active one for the calling thread.
 struct ProfActive {
@@ -452,7 +489,8 @@ extern "C" int cm1g_init(const cm1g_config_t *cfg, const cm1g_grid_t *gr, cm1g_c
   c->bud = (double *)dalloc(c, (size_t)g.ni * g.nj * sizeof(double));
   c->lev = (double *)dalloc(c, (size_t)(g.nk + 2) * sizeof(double));
   c->fscal = (float *)dalloc(c, 16 * sizeof(float));
-  c->cflbits = (int *)dalloc(c, 16 * sizeof(int));   // [0] max CFL bits, [1] staging-wait error of k_scal_tile
+  c->advs_err = pinned_flags().take();
+  c->cflbits = (int *)dalloc(c, 16 * sizeof(int));   // [0] max CFL bits, [1], [2] staging-wait errors of a step and of cm1g_advs
   {
     const char *sp = getenv("CM1G_SCALAR_PASS");
     c->scal_fused = !(sp && strcmp(sp, "perfield") == 0);
@@ -468,12 +506,6 @@ extern "C" int cm1g_init(const cm1g_config_t *cfg, const cm1g_grid_t *gr, cm1g_c
   }
   for (void *p : c->allocs)
     if (!p) { cm1g_finalize(c); return set_err(CM1G_ERR_NOMEM, "scratch alloc"); }
-  if (cudaHostAlloc((void **)&c->advs_err, sizeof(int), cudaHostAllocDefault) != cudaSuccess) {
-    (void)cudaGetLastError();
-    cm1g_finalize(c);
-    return set_err(CM1G_ERR_NOMEM, "scratch alloc");
-  }
-  *c->advs_err = 0;
   if (!c->mm) { cm1g_finalize(c); return set_err(CM1G_ERR_NOMEM, "scratch alloc"); }
   if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) {
     cm1g_finalize(c);
@@ -497,11 +529,11 @@ extern "C" int cm1g_finalize(cm1g_ctx_t *c) {
   drop_graph(c);
   if (c->stream) cudaStreamSynchronize(c->stream);
   if (c->prof) { c->prof->drain(); delete c->prof; }
+  pinned_flags().give(c->advs_err);
   for (void *p : c->allocs) if (p) cudaFree(p);
   for (void *p : {(void *)c->d_st_jobs, (void *)c->d_st_ops, (void *)c->d_st_lev, (void *)c->d_rstat,
                   (void *)c->d_st_zh, (void *)c->d_st_zf})
     if (p) cudaFree(p);
-  if (c->advs_err) cudaFreeHost(c->advs_err);
   for (auto &b : c->stage_pool) cudaFree(b.first);
   if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
   delete c;
@@ -1453,12 +1485,15 @@ extern "C" int cm1g_advs(cm1g_ctx_t *c, int32_t nrk, int32_t wflag, const float 
   const int weno = (wflag == 1) && (c->cfg.advwenos == 1 || (c->cfg.advwenos == 2 && nrk == 3));
   // t11 is scratch of the large step, set anew by each of its stages
   launch_advs(g, dru, drv, drw, ddx, ds, ds0, dten, weno, pdef != 0, pdefweno, weps, dt, c->pdefscr, c->pdefneg, c->t11,
-              c->advs_err, c->stream, &c->nlaunch);
+              c->advs_err ? c->advs_err : c->cflbits + 2, c->stream, &c->nlaunch);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return set_err(CM1G_ERR_CUDA, "%s", cudaGetErrorString(e));
-  const int rc = S.finish();
-  if (rc == CM1G_OK && *c->advs_err) {
-    *c->advs_err = 0;
+  int copied = 0;
+  if (!c->advs_err) cudaMemcpyAsync(&copied, c->cflbits + 2, sizeof(int), cudaMemcpyDeviceToHost, c->stream);
+  const int rc = S.finish();   // synchronizes
+  if (rc == CM1G_OK && (c->advs_err ? *(volatile int *)c->advs_err : copied)) {
+    if (c->advs_err) *c->advs_err = 0;
+    else CUCHK(cudaMemsetAsync(c->cflbits + 2, 0, sizeof(int), c->stream));
     return set_err(CM1G_ERR_CUDA, "advs: staged data did not arrive (bulk-copy wait gave up)");
   }
   return rc;
