@@ -143,18 +143,19 @@ int cm1g::tile_levels(long tiles, int nk, int slots, int over, int kcmax) {
   long best_end = 0;
   for (int kc = 4; kc <= kcmax; kc += kc < 16 ? 1 : kc < 32 ? 2 : 4) {
     const int nch = (nk + kc - 1) / kc;
-    std::map<long, long> free_at{{0, slots}};   // end of the slots' last block -> slots
-    long end = 0;
-    for (int part = 0; part < 2; part++) {      // the full chunks, then the last one of every tile
-      const long len = over + (part ? nk - (nch - 1) * kc : kc);
-      for (long n = part ? tiles : tiles * (nch - 1); n > 0;) {
-        const auto it = free_at.begin();
-        const long t = it->first, m = std::min(n, it->second);
-        if ((it->second -= m) == 0) free_at.erase(it);
-        free_at[t + len] += m;
-        end = std::max(end, t + len);
-        n -= m;
-      }
+    // the full chunks in whole rounds of the slots, then the last chunk of every
+    // tile on the slots as they come free (end of a slot's last block -> slots)
+    const long len = over + kc, full = tiles * (nch - 1), rounds = full / slots, rest = full % slots;
+    std::map<long, long> free_at{{rounds * len, slots - rest}};
+    if (rest) free_at[(rounds + 1) * len] = rest;
+    long end = free_at.rbegin()->first;
+    for (long n = tiles; n > 0;) {
+      const auto it = free_at.begin();
+      const long t = it->first + over + nk - (nch - 1) * kc, m = std::min(n, it->second);
+      if ((it->second -= m) == 0) free_at.erase(it);
+      free_at[t] += m;
+      end = std::max(end, t);
+      n -= m;
     }
     if (!best || end < best_end) { best = kc; best_end = end; }
     if (kc >= nk) break;
@@ -243,8 +244,9 @@ struct cm1g_ctx {
 
 // Flags in pinned memory that a kernel can raise and the host read after a
 // synchronize, without a copy (12 us of cm1g_advs).  Pinning a page takes some
-// 5 ms, so one page serves the process: a context takes a slot at its creation and
-// gives it back; without one (more contexts than slots) it copies a device flag.
+// 5 ms, so one page serves the process: a context takes a slot with its first call
+// that needs one and gives it back; without one (more contexts than slots) it
+// copies a device flag.
 struct PinnedFlags {
   static constexpr int N = 1024;
   std::mutex mu;
@@ -489,7 +491,6 @@ extern "C" int cm1g_init(const cm1g_config_t *cfg, const cm1g_grid_t *gr, cm1g_c
   c->bud = (double *)dalloc(c, (size_t)g.ni * g.nj * sizeof(double));
   c->lev = (double *)dalloc(c, (size_t)(g.nk + 2) * sizeof(double));
   c->fscal = (float *)dalloc(c, 16 * sizeof(float));
-  c->advs_err = pinned_flags().take();
   c->cflbits = (int *)dalloc(c, 16 * sizeof(int));   // [0] max CFL bits, [1], [2] staging-wait errors of a step and of cm1g_advs
   {
     const char *sp = getenv("CM1G_SCALAR_PASS");
@@ -1483,6 +1484,7 @@ extern "C" int cm1g_advs(cm1g_ctx_t *c, int32_t nrk, int32_t wflag, const float 
   const float *ds0 = s0 ? S.in(s0, nS(g), false) : nullptr;
   float *dten = S.in(sten, nS(g), true);
   const int weno = (wflag == 1) && (c->cfg.advwenos == 1 || (c->cfg.advwenos == 2 && nrk == 3));
+  if (!c->advs_err) c->advs_err = pinned_flags().take();
   // t11 is scratch of the large step, set anew by each of its stages
   launch_advs(g, dru, drv, drw, ddx, ds, ds0, dten, weno, pdef != 0, pdefweno, weps, dt, c->pdefscr, c->pdefneg, c->t11,
               c->advs_err ? c->advs_err : c->cflbits + 2, c->stream, &c->nlaunch);

@@ -890,49 +890,13 @@ void launch_adv_momentum(const DGrid &g, const float *u, const float *v, const f
 // th0-300, solve2.F:1365-1372) is added to s when given.
 // ---------------------------------------------------------------------
 struct SAdv {
-  const float *__restrict__ rru, *__restrict__ rrv, *__restrict__ rrw;  // averaged velocities or fluxes
+  const float *__restrict__ rru, *__restrict__ rrv, *__restrict__ rrw;  // averaged velocities
   const float *__restrict__ s;      // advected field (full halo)
   const float *__restrict__ s0;     // RK base value (pdef only)
-  const float *__restrict__ divx;   // caller's divx (adv.F argument) or null: formed here
   const float *__restrict__ thterm; // moist theta: thten -= div(u_avg)*thterm (solve2.F:1320-1329)
-  int weighted;                     // 1: rru/rrv/rrw are velocities to be weighted here
   int sadd;                         // add th0(k)-th0r to s (theta)
   Diff6 df{};                       // 6th-order diffusion (df.rho null: none)
 };
-
-// Mass moved into point c by the pdef scatter of pdefx2/pdefy2/pdefz
-// (pdef.F:158-174), gathered in the scatter's loop order: contribution from
-// the lower neighbour, then the point itself, then the upper neighbour.
-__device__ __forceinline__ void pdef_gather(float dm2, float dm1, float d0, float dp1, float dp2, float smeps,
-                                            float *mass, bool *flag) {
-  float m = 0.0f;
-  bool f = false;
-  if (dm1 < 0.0f) {  // the point below scatters: we are its upper neighbour
-    float foo1 = fmaxf(0.0f, dm2), foo2 = fmaxf(0.0f, d0);
-    if (foo1 + foo2 > smeps) {
-      float foo3 = fmaxf(dm1, -(foo1 + foo2)) / (foo1 + foo2);
-      m = m + foo2 * foo3;
-      if (d0 > smeps) f = true;
-    }
-  }
-  if (d0 < 0.0f) {
-    float foo1 = fmaxf(0.0f, dm1), foo2 = fmaxf(0.0f, dp1);
-    if (foo1 + foo2 > smeps) {
-      float foo3 = fmaxf(d0, -(foo1 + foo2)) / (foo1 + foo2);
-      m = m - (foo1 + foo2) * foo3;
-      f = true;
-    }
-  }
-  if (dp1 < 0.0f) {
-    float foo1 = fmaxf(0.0f, d0), foo2 = fmaxf(0.0f, dp2);
-    if (foo1 + foo2 > smeps) {
-      float foo3 = fmaxf(dp1, -(foo1 + foo2)) / (foo1 + foo2);
-      m = m + foo1 * foo3;
-      if (d0 > smeps) f = true;
-    }
-  }
-  *mass = m; *flag = f;
-}
 
 // Tiled form of pass 2: a block owns TX x TY columns and marches upward;
 // each level's dumx (with its +-2 halo in x) and dumy (+-2 in y) are staged
@@ -1386,7 +1350,7 @@ void launch_advs_tiled(const DGrid &g, const float *rru, const float *rrv, const
                        const float *s0, int sadd, const float *ten1, const float *thterm, float *snew, int weno,
                        int pdef, int pdefweno, double weps, float dt, int flush, float *scratch, cudaStream_t st,
                        int64_t *nl, const TileExtras *ex, const Diff6 *diff) {
-  SAdv a{rru, rrv, rrw, s, s0, nullptr, thterm, 1, sadd};
+  SAdv a{rru, rrv, rrw, s, s0, thterm, sadd};
   if (diff) a.df = *diff;
   STileOut o{};
   o.sten_in = ten1; o.sbase = s0; o.snew = snew;

@@ -1,7 +1,7 @@
-// k_face.cuh -- face values of the scalar passes (hflux5, zflux_win) and the
-// spread of a tile's faces over its threads (FaceSlots), shared by the
-// per-scalar tile (k_adv.cu) and the fused multi-scalar pass (k_scal.cu) so
-// that both evaluate every face with the same binary32/binary64 operations.
+// k_face.cuh -- face values of the scalar passes, the spread of a tile's faces
+// over its threads (FaceSlots) and the exchange of the positive-definite scheme,
+// shared by the per-scalar tile (k_adv.cu) and the fused multi-scalar pass
+// (k_scal.cu) so that both use the same binary32/binary64 operations.
 #pragma once
 #include "cm1g_common.cuh"
 
@@ -130,6 +130,40 @@ __device__ __forceinline__ float zface_edge(float fz, const float *wv, float r, 
   const bool hi = kk == nk || kk == 3;   // upwind from below
   const float s1 = hi ? wv[1] : wv[4], s2 = hi ? wv[2] : wv[3], s3 = hi ? wv[3] : wv[2];
   return r * (weno ? upstrpd(s1, s2, s3, weps) : flx3(s1, s2, s3));
+}
+
+// Mass moved into point c by the pdef scatter of pdefx2/pdefy2/pdefz
+// (pdef.F:158-174), gathered in the scatter's loop order: contribution from
+// the lower neighbour, then the point itself, then the upper neighbour.
+__device__ __forceinline__ void pdef_gather(float dm2, float dm1, float d0, float dp1, float dp2, float smeps, float *mass,
+                                            bool *flag) {
+  float m = 0.0f;
+  bool f = false;
+  if (dm1 < 0.0f) {  // the point below scatters: we are its upper neighbour
+    float foo1 = fmaxf(0.0f, dm2), foo2 = fmaxf(0.0f, d0);
+    if (foo1 + foo2 > smeps) {
+      float foo3 = fmaxf(dm1, -(foo1 + foo2)) / (foo1 + foo2);
+      m = m + foo2 * foo3;
+      if (d0 > smeps) f = true;
+    }
+  }
+  if (d0 < 0.0f) {
+    float foo1 = fmaxf(0.0f, dm1), foo2 = fmaxf(0.0f, dp1);
+    if (foo1 + foo2 > smeps) {
+      float foo3 = fmaxf(d0, -(foo1 + foo2)) / (foo1 + foo2);
+      m = m - (foo1 + foo2) * foo3;
+      f = true;
+    }
+  }
+  if (dp1 < 0.0f) {
+    float foo1 = fmaxf(0.0f, d0), foo2 = fmaxf(0.0f, dp2);
+    if (foo1 + foo2 > smeps) {
+      float foo3 = fmaxf(dp1, -(foo1 + foo2)) / (foo1 + foo2);
+      m = m + foo1 * foo3;
+      if (d0 > smeps) f = true;
+    }
+  }
+  *mass = m; *flag = f;
 }
 
 }  // namespace cm1g

@@ -23,7 +23,7 @@
 //  * one barrier per item: the face fluxes and face velocities are double
 //    buffered by item parity.
 //
-// Bound by instruction issue: three faces are some 400 of an item's 730
+// Bound by instruction issue: three faces are some 400 of an item's 690
 // instructions, at 24 warps a SM (80 registers).  So the faces that the fast
 // WENO5 leaves open are evaluated beside it from shared memory without a call,
 // the item's global reads are issued after its faces and not before (their
@@ -419,40 +419,6 @@ __global__ void __launch_bounds__(TX * (TY + 1), 3) k_scal_tile(const __grid_con
     if (tid == 0) atomicExch(P.err, 1);
     for (int u = tfail; u < nitem && u < tfail + RD; u++) (void)mbar_wait(bar0 + 8 * (u % RD), (uint32_t)((u / RD) & 1));
   }
-}
-
-// Mass moved into point c by the pdef scatter of pdefx2/pdefy2/pdefz
-// (pdef.F:158-174), gathered in the scatter's loop order: contribution from
-// the lower neighbour, then the point itself, then the upper neighbour.
-__device__ __forceinline__ void pdef_gather(float dm2, float dm1, float d0, float dp1, float dp2, float smeps, float *mass,
-                                            bool *flag) {
-  float m = 0.0f;
-  bool f = false;
-  if (dm1 < 0.0f) {  // the point below scatters: we are its upper neighbour
-    float foo1 = fmaxf(0.0f, dm2), foo2 = fmaxf(0.0f, d0);
-    if (foo1 + foo2 > smeps) {
-      float foo3 = fmaxf(dm1, -(foo1 + foo2)) / (foo1 + foo2);
-      m = m + foo2 * foo3;
-      if (d0 > smeps) f = true;
-    }
-  }
-  if (d0 < 0.0f) {
-    float foo1 = fmaxf(0.0f, dm1), foo2 = fmaxf(0.0f, dp1);
-    if (foo1 + foo2 > smeps) {
-      float foo3 = fmaxf(d0, -(foo1 + foo2)) / (foo1 + foo2);
-      m = m - (foo1 + foo2) * foo3;
-      f = true;
-    }
-  }
-  if (dp1 < 0.0f) {
-    float foo1 = fmaxf(0.0f, d0), foo2 = fmaxf(0.0f, dp2);
-    if (foo1 + foo2 > smeps) {
-      float foo3 = fmaxf(dp1, -(foo1 + foo2)) / (foo1 + foo2);
-      m = m + foo1 * foo3;
-      if (d0 > smeps) f = true;
-    }
-  }
-  *mass = m; *flag = f;
 }
 
 // Second pass of the positive-definite scheme: pdefz, pdefx2, pdefy2
