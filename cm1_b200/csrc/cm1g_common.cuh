@@ -149,19 +149,22 @@ __device__ __forceinline__ Weno5Terms weno5_terms(float s1, float s2, float s3, 
   w.q3 = ((2.0f / 6.0f) * s3 + (5.0f / 6.0f) * s4) + (-1.0f / 6.0f) * s5;
   return w;
 }
-// n/d rounded to nearest by Markstein's method (IBM J. Res. Dev. 34, 1990):
-// Newton's iteration gives 1/d to the last place, and one correction of n/d by
-// its exact residual rounds correctly.  For d > 1e-60 and quotients and operands
-// below 1e200, or not finite.  Unlike the operator it has no subroutine for
-// the extremes of the range, whose call would cost the main loop registers.
+// n/d, d >= 0, rounded to nearest by Markstein's method (IBM J. Res. Dev. 34,
+// 1990): Newton's iteration gives 1/d to the last place, and one correction of n/d
+// by its exact residual rounds correctly, for d between 1e-60 and 1e200 and
+// quotients and operands below 1e200.  Where that gives no number (d zero or
+// infinite, n infinite, an operand not a number) the quotient is n times the
+// approximate reciprocal 0 or infinity of d, or n's infinity.  Unlike the operator
+// it has no subroutine for the extremes of the range, whose call would cost the
+// main loop registers.
 __device__ __forceinline__ double div_rn(double n, double d) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+  double y, y0;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(d));
+  y = __fma_rn(y0, __fma_rn(-d, y0, 1.0), y0);
   y = __fma_rn(y, __fma_rn(-d, y, 1.0), y);
   y = __fma_rn(y, __fma_rn(-d, y, 1.0), y);
-  y = __fma_rn(y, __fma_rn(-d, y, 1.0), y);
-  const double q = n * y;
-  return d < 1.0e300 ? __fma_rn(__fma_rn(-d, q, n), y, q) : n * 0.0;
+  const double q = n * y, r = __fma_rn(__fma_rn(-d, q, n), y, q);
+  return r == r ? r : n * y0;
 }
 __device__ __forceinline__ float weno5_exact(float s1, float s2, float s3, float s4, float s5, double weps) {
   const Weno5Terms w = weno5_terms(s1, s2, s3, s4, s5);

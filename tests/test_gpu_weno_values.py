@@ -78,3 +78,35 @@ def test_step_tracers_bitwise(bc, cm1g, oracle_lib):
     for n, kind in enumerate(KINDS):
         assert np.array_equal(dev["pt3d"][n].cpu().numpy()[sel], ref["pt3d"][n][sel], equal_nan=True), kind
     ctx.close()
+
+
+def _infinite(shape, rng):
+    """A smooth field with isolated infinities of both signs, points that are not
+    a number, and values near binary32's largest."""
+    a = _field("smooth", shape, rng)
+    p = rng.random(shape)
+    for q, x in enumerate((np.inf, -np.inf, np.nan, 3e38)):
+        a[(p >= 0.004 * q) & (p < 0.004 * (q + 1))] = x
+    return a
+
+
+@pytest.mark.parametrize("pdef", [0, 1])
+def test_advs_infinite(pdef, cm1g, oracle_lib):
+    """The divisions' infinities and not-a-numbers are those of the operator."""
+    _torch()
+    case = make_case("dry_bubble", ni=61, nj=23, nk=17, bc=1, advwenos=1)
+    rng = np.random.default_rng(7)
+    rru, rrv, rrw, divx, _, _, sten = _adv_inputs(case, rng, positive=True)
+    s = _infinite(case.lay.shape(1), rng)
+    s0, weps, dt, ref = s.copy(), 1e-18, f32(0.5), sten.copy()
+    g = case.grid_struct()
+    fp = lambda a: a.ctypes.data_as(C.POINTER(C.c_float))       # noqa: E731
+    assert oracle_lib.lib().oracle_advs(C.byref(case.cfg), C.byref(g), 1, 1, fp(rru), fp(rrv), fp(rrw), fp(divx), fp(s0),
+                                        fp(s), fp(ref), pdef, pdef, dt, weps) == 0
+    sel = case.lay.interior(1)
+    assert np.isinf(ref[sel]).sum() > 100 and np.isfinite(ref[sel]).sum() > 100
+    ctx = cm1g.Context(case.cfg, case.grid)
+    d = cm1g.to_device(dict(rru=rru, rrv=rrv, rrw=rrw, divx=divx, s0=s0, s=s, sten=sten))
+    ctx.advs(1, 1, d["divx"], d["rru"], d["rrv"], d["rrw"], d["s0"], d["s"], d["sten"], pdef, pdef, dt, weps)
+    assert np.array_equal(d["sten"].cpu().numpy()[sel], ref[sel], equal_nan=True)
+    ctx.close()
