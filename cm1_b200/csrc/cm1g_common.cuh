@@ -129,21 +129,28 @@ __device__ __forceinline__ float flx5(float s1, float s2, float s3, float s4, fl
 // evaluates the face with weno5_exact, from the stencil where it lies, so that a
 // kernel's main loop holds nothing for it.
 //
-// Products by 2, 4 and 0.25 are exact, so fusing them with the addition that
-// follows gives the binary32 value of the separate operations; the folded
-// binary64 path fuses freely.
+// Products by 2, 4 and 0.25 are exact while they stay in the normal range, so
+// fusing them with the addition that follows gives the binary32 value of the
+// separate operations but for a subnormal indicator's last bit (2^-149).
+// weno5_fast takes the fused form, and decides only where every denominator
+// b_i + weps is above 2^-90: that bit is then far below the denominators' own
+// rounding, and no product of theirs or of their squares leaves binary64's normal
+// range.  Smaller denominators (weps = 0 or below 2^-90, in a field of tiny or
+// equal values) go to weno5_exact, which rounds every operation.
 // smoothness indicators and the three candidate values of a stencil
 struct Weno5Terms { float f1, f2, f3, q1, q2, q3; };
+template <bool FUSED>
 __device__ __forceinline__ Weno5Terms weno5_terms(float s1, float s2, float s3, float s4, float s5) {
   const float c1312 = 13.0f / 12.0f;
   Weno5Terms w;
   float t, u;
-  t = __fmaf_rn(-2.0f, s2, s1) + s3; u = __fmaf_rn(-4.0f, s2, s1) + 3.0f * s3;
-  w.f1 = __fmaf_rn(0.25f, u * u, c1312 * (t * t));
-  t = __fmaf_rn(-2.0f, s3, s2) + s4; u = s2 - s4;
-  w.f2 = __fmaf_rn(0.25f, u * u, c1312 * (t * t));
-  t = __fmaf_rn(-2.0f, s4, s3) + s5; u = __fmaf_rn(-4.0f, s4, 3.0f * s3) + s5;
-  w.f3 = __fmaf_rn(0.25f, u * u, c1312 * (t * t));
+  auto add = [](float c, float x, float y) { return FUSED ? __fmaf_rn(c, x, y) : c * x + y; };
+  t = add(-2.0f, s2, s1) + s3; u = add(-4.0f, s2, s1) + 3.0f * s3;
+  w.f1 = add(0.25f, u * u, c1312 * (t * t));
+  t = add(-2.0f, s3, s2) + s4; u = s2 - s4;
+  w.f2 = add(0.25f, u * u, c1312 * (t * t));
+  t = add(-2.0f, s4, s3) + s5; u = add(-4.0f, s4, 3.0f * s3) + s5;
+  w.f3 = add(0.25f, u * u, c1312 * (t * t));
   w.q1 = ((2.0f / 6.0f) * s1 + (-7.0f / 6.0f) * s2) + (11.0f / 6.0f) * s3;
   w.q2 = ((-1.0f / 6.0f) * s2 + (5.0f / 6.0f) * s3) + (2.0f / 6.0f) * s4;
   w.q3 = ((2.0f / 6.0f) * s3 + (5.0f / 6.0f) * s4) + (-1.0f / 6.0f) * s5;
@@ -167,7 +174,7 @@ __device__ __forceinline__ double div_rn(double n, double d) {
   return r == r ? r : n * y0;
 }
 __device__ __forceinline__ float weno5_exact(float s1, float s2, float s3, float s4, float s5, double weps) {
-  const Weno5Terms w = weno5_terms(s1, s2, s3, s4, s5);
+  const Weno5Terms w = weno5_terms<false>(s1, s2, s3, s4, s5);
   if (w.q1 == 0.0f && w.q2 == 0.0f && w.q3 == 0.0f) return 0.0f;
   const double b1 = (double)w.f1, b2 = (double)w.f2, b3 = (double)w.f3;
   const double tau = fabs(b1 - b3);
@@ -182,7 +189,7 @@ __device__ __forceinline__ float weno5_fast(float s1, float s2, float s3, float 
   // a stencil of zeros, which fills most of a tracer's or a hydrometeor's field
   const int any = __float_as_int(s1) | __float_as_int(s2) | __float_as_int(s3) | __float_as_int(s4) | __float_as_int(s5);
   if ((any << 1) == 0) return 0.0f;
-  const Weno5Terms w = weno5_terms(s1, s2, s3, s4, s5);
+  const Weno5Terms w = weno5_terms<true>(s1, s2, s3, s4, s5);
   const double b1 = (double)w.f1, b2 = (double)w.f2, b3 = (double)w.f3;
   const double tau = fabs(b1 - b3);
   const double d1 = b1 + weps, d2 = b2 + weps, d3 = b3 + weps;
@@ -204,9 +211,9 @@ __device__ __forceinline__ float weno5_fast(float s1, float s2, float s3, float 
   const float f = (float)v;
   // v's last 29 bits against 2^28 -+ 2^17, without the bits above them
   const unsigned off = 8u * (unsigned)__double2loint(v) - 8u * ((1u << 28) - (1u << 17));
-  // no weight reaches its bound 1e30 where tau < 2^98 (b_i + weps), by exponent;
-  // the floor 1.2e-35 keeps f a normal binary32 number
-  const int ht = __double2hiint(tau) - (98 << 20);
+  // no weight reaches its bound 1e30 where tau < 2^98 (b_i + weps), by exponent,
+  // and b_i + weps is above 2^-90; the floor 1.2e-35 keeps f a normal binary32 number
+  const int ht = max(__double2hiint(tau) - (98 << 20), (1023 - 90) << 20);
   if (ht < __double2hiint(weps) && off > 8u << 18 && fabs(num) * 1024.0 >= A && fabsf(f) >= 1.2e-35f) return f;
   const double e = A * y * 0x1p-46;
   const float lo = (float)(v - e), hi = (float)(v + e);

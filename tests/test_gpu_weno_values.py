@@ -80,6 +80,30 @@ def test_step_tracers_bitwise(bc, cm1g, oracle_lib):
     ctx.close()
 
 
+@pytest.mark.parametrize("weps", [0.0, 5e-52, 1e-45, 1e-36, 1e-28])
+@pytest.mark.parametrize("kind,scale", [("tiny", 1e-12), ("ties", 1e-12), ("sparse", 1e-18), ("smooth", 1e-16)])
+def test_advs_small_weps(kind, scale, weps, cm1g, oracle_lib):
+    """Values and denominators so small that the squares and sixth powers of the
+    folded evaluation, or the smoothness indicators, leave the normal range."""
+    _torch()
+    case = make_case("dry_bubble", ni=61, nj=23, nk=17, bc=1, advwenos=1)
+    rng = np.random.default_rng(11)
+    rru, rrv, rrw, divx, _, _, sten = _adv_inputs(case, rng, positive=True)
+    s = (_field(kind, case.lay.shape(1), rng) * f32(scale)).astype(f32)
+    sten[...] = 0.0
+    s0, dt, ref = s.copy(), f32(0.5), sten.copy()
+    g = case.grid_struct()
+    fp = lambda a: a.ctypes.data_as(C.POINTER(C.c_float))       # noqa: E731
+    assert oracle_lib.lib().oracle_advs(C.byref(case.cfg), C.byref(g), 1, 1, fp(rru), fp(rrv), fp(rrw), fp(divx), fp(s0),
+                                        fp(s), fp(ref), 0, 0, dt, weps) == 0
+    ctx = cm1g.Context(case.cfg, case.grid)
+    d = cm1g.to_device(dict(rru=rru, rrv=rrv, rrw=rrw, divx=divx, s0=s0, s=s, sten=sten))
+    ctx.advs(1, 1, d["divx"], d["rru"], d["rrv"], d["rrw"], d["s0"], d["s"], d["sten"], 0, 0, dt, weps)
+    sel = case.lay.interior(1)
+    assert np.array_equal(d["sten"].cpu().numpy()[sel], ref[sel], equal_nan=True)
+    ctx.close()
+
+
 def _infinite(shape, rng):
     """A smooth field with isolated infinities of both signs, points that are not
     a number, and values near binary32's largest."""
