@@ -257,14 +257,18 @@ struct BwdSmem {
   __nv_bfloat16 x[BW_ROWS][8], dy[3][BW_ROWS][8];
 };
 
-// the three BF16 parts of two binary32 values
+// The three BF16 parts of two binary32 values, each the 8 leading significand
+// bits of what is left (cut off, not rounded: the largest values would round to
+// infinity).  An infinity is all in its first part, so that sums of products with
+// it are the infinities and not-a-numbers of the unsplit value's.
 __device__ __forceinline__ void split3(float a, float b, uint32_t q[3]) {
 #pragma unroll
   for (int s = 0; s < 3; s++) {
-    const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
-    q[s] = *reinterpret_cast<const uint32_t *>(&v);
-    a -= __low2float(v);
-    b -= __high2float(v);
+    const uint32_t ua = __float_as_uint(a), ub = __float_as_uint(b);
+    const float ha = __uint_as_float(ua & 0xffff0000u), hb = __uint_as_float(ub & 0xffff0000u);
+    q[s] = __byte_perm(ua, ub, 0x7632);
+    a = (s == 0 && a == ha) ? 0.0f : a - ha;
+    b = (s == 0 && b == hb) ? 0.0f : b - hb;
   }
 }
 // four / two transposed 8x8 tiles; every lane gives the address of one 16-byte row
@@ -443,6 +447,8 @@ __global__ void __launch_bounds__(32 * BW_WARPS, 2) k_mlp_backward(const float *
     atomicAdd(&grad[P_B1 + ib], gw1[3]);
     atomicAdd(&grad[P_B2 + ia], gb2[1]);
     atomicAdd(&grad[P_B2 + ib], gb2[3]);
+    atomicAdd(&grad[P_W1 + 7 * MLP_H + ia], 0.0f * gw1[1]);   // the padding's own: zero, if dz1 is finite
+    atomicAdd(&grad[P_W1 + 7 * MLP_H + ib], 0.0f * gw1[3]);
   }
 #pragma unroll
   for (int q = 0; q < 2; q++) {

@@ -129,3 +129,36 @@ def test_backward_matches_reference(n, shift, cm1g):
     R = mlp_ref
     for a, b in ((R.P_W1, R.P_B1), (R.P_B1, R.P_W2), (R.P_W2, R.P_B2), (R.P_B2, R.P_W3), (R.P_W3, R.P_B3), (R.P_B3, R.P_TOTAL)):
         assert np.abs(got[a:b] - exp[a:b]).max() <= 1e-5 * np.abs(exp[a:b]).max(), (a, b)
+
+
+@pytest.mark.parametrize("n", [1, 17, 200])
+def test_backward_of_infinite_gradients(n, cm1g):
+    """Infinite and not-a-number loss gradients of single rows, and one near
+    binary32's largest value: the same entries of the parameter gradient are
+    infinite, of either sign, and not a number as with unsplit operands, and the
+    others keep the bar above."""
+    torch = _torch()
+    rng = np.random.default_rng(n)
+    p = (mlp_ref.init_params(2) * 0.1).astype(np.float32)
+    x = rng.uniform(0.1, 1, (n, 8)).astype(np.float32)
+    x[:, 7] = 0
+    z1, z2 = (rng.uniform(-0.5, 1, (n, 64)).astype(np.float32) for _ in range(2))
+    for value in (np.inf, -np.inf, np.nan, 3.4e38):
+        dy = np.zeros((n, 8), np.float32)
+        dy[n // 2, 2] = value
+        dy[0, 0] += 1.0
+        D = {k: torch.from_numpy(a).cuda() for k, a in dict(p=p, x=x, z1=z1, z2=z2, dy=dy).items()}
+        G = torch.zeros(mlp_ref.P_TOTAL, device="cuda")
+        f = cm1g.ptr
+        cm1g.check(cm1g.lib().cm1g_mlp_backward(f(D["p"]), n, f(D["x"]), f(D["z1"]), f(D["z2"]), f(D["dy"]), f(G), None))
+        torch.cuda.synchronize()
+        with np.errstate(all="ignore"):
+            exp = mlp_ref.backward(p, x, z1, z2, dy)
+        got, fin = G.cpu().numpy(), np.isfinite(exp)
+        for pattern in (np.isnan, np.isposinf, np.isneginf):
+            assert np.array_equal(pattern(got), pattern(exp)), (value, pattern)
+        R = mlp_ref
+        for a, b in ((R.P_W1, R.P_B1), (R.P_B1, R.P_W2), (R.P_W2, R.P_B2), (R.P_B2, R.P_W3), (R.P_W3, R.P_B3), (R.P_B3, R.P_TOTAL)):
+            k = fin[a:b]
+            if k.any():
+                assert np.abs(got[a:b][k] - exp[a:b][k]).max() <= 1e-5 * np.abs(exp[a:b][k]).max(), (value, a, b)
