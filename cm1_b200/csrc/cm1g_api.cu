@@ -60,6 +60,7 @@ void launch_sound(const DGrid &g, int nsound, int nrk, float dt, const float *ua
                   float *radbce, float *radbcs, float *radbcn, float *su, float *sv, float *su2,
                   float *sv2, float *d1, float *d2, float *lu, float *rbnd, cudaStream_t st, int64_t *nl);
 int sound_max_nk();
+cudaError_t sound_init();
 void launch_stage_prep(const DGrid &g, const float *th3d, const float *pp3d, const float *qv, const LiquidIn &liq,
                        int imoist, int eqtset, float *t11, float *t22, float *thterm, float *piadv, int ring, cudaStream_t st,
                        int64_t *nl);
@@ -513,7 +514,8 @@ extern "C" int cm1g_init(const cm1g_config_t *cfg, const cm1g_grid_t *gr, cm1g_c
     return set_err(CM1G_ERR_CUDA, "stream create");
   }
   c->own_stream = true;
-  cudaError_t e = cudaDeviceSynchronize();
+  cudaError_t e = sound_init();
+  if (e == cudaSuccess) e = cudaDeviceSynchronize();
   if (e != cudaSuccess) { cm1g_finalize(c); return set_err(CM1G_ERR_CUDA, "init: %s", cudaGetErrorString(e)); }
   *out = c;
   return CM1G_OK;

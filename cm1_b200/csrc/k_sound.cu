@@ -751,13 +751,14 @@ static int sound_tile_of(const DGrid &g, int cfg) {
   return g.nk <= kSoundTiles[0].nw * kSoundTiles[0].kpt ? 0 : 1;
 }
 
-static void sound_set_attributes() {
-  static bool done = false;
-  if (done) return;
-  for (const SoundTile &t : kSoundTiles)
-    cudaFuncSetAttribute(t.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024);
-  cudaFuncSetAttribute(k_openbc_restrict, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  done = true;
+// The shared memory the kernels may take.  The limits belong to the current CUDA
+// context's copy of a kernel, so each cm1g context sets them when it is made.
+cudaError_t sound_init() {
+  for (const SoundTile &t : kSoundTiles) {
+    const cudaError_t e = cudaFuncSetAttribute(t.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaFuncSetAttribute(k_openbc_restrict, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
 }
 
 // One RK stage of acoustic steps.  At the first stage the reference starts
@@ -800,7 +801,6 @@ void launch_sound(const DGrid &g, int nsound, int nrk, float dt,
   dim3 grid = col ? dim3((g.ni + SNC_TX - 1) / SNC_TX, (g.nj + cty - 1) / cty)
                   : dim3((g.ni + SND_TX - 1) / SND_TX, g.nj);
   const size_t smem = col ? 0 : sound_smem_bytes(g);
-  sound_set_attributes();
   const float *uin = (nrk == 1) ? u3d : ua, *vin = (nrk == 1) ? v3d : va, *ppdin = ppx;
   for (int n = 1; n <= nloop; n++) {
     SoundIO io;

@@ -2,6 +2,10 @@
 16 explicit warps; the last level of each; blocks of 1, 31, 32 and 33 columns)
 against the column sweep.  Both evaluate every point with the same binary32
 operations in the same order, so the results must agree bit for bit."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -53,3 +57,40 @@ def test_tile_equals_column_sweep(ni, nj, nk, bc, nrk, cm1g, monkeypatch):
     for n in ("u3d", "v3d", "w3d", "pp3d", "ppx", "rru", "rrv", "rrw"):
         assert np.isfinite(got["col"][n][lay.interior({"u3d": 2, "rru": 2, "v3d": 3, "rrv": 3, "w3d": 4}.get(n, 1))]).all(), n
         assert np.array_equal(got["tile"][n], got["col"][n]), n
+
+
+TWO_CONTEXTS = """
+import ctypes as C
+import numpy as np
+from cm1_b200 import binding
+from cm1_b200.cases import make_case
+
+case = make_case("dry_bubble", ni=40, nj=8, nk=100)     # over 48 KB of shared memory a block
+cuda, ctx = C.CDLL("libcuda.so.1"), C.c_void_p()
+
+def step():
+    c = binding.Context(case.cfg, case.grid)
+    st = {k: v.copy() for k, v in case.state.items()}
+    c.step(st, case.dt, case.mass1)
+    c.close()
+    return st
+
+first = step()
+assert cuda.cuCtxCreate_v2(C.byref(ctx), 0, 0) == 0      # current from here on
+second = step()
+assert cuda.cuCtxDestroy_v2(ctx) == 0
+assert all(np.array_equal(first[k], second[k], equal_nan=True) for k in first)
+assert not np.array_equal(first["w3d"], case.state["w3d"])
+print("same step")
+"""
+
+
+def test_every_cuda_context_gets_the_kernels_limits(cm1g):
+    """A second CUDA context of a process (as a second device has one) launches
+    tiles that take more shared memory than the default limit."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", TWO_CONTEXTS], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "same step" in r.stdout, r.stdout + r.stderr
