@@ -1061,8 +1061,12 @@ extern "C" int cm1g_get_tune(cm1g_ctx_t *c, cm1g_tune_t *t) {
   return CM1G_OK;
 }
 
-// The cache key: device, grid shape and the options that change which
-// kernels run (no spaces, so that a cache file line splits on blanks).
+// Revision of the launch tables: counts up when an index comes to mean another
+// launch, so that a choice kept in a file is taken by the tables it was timed with.
+constexpr int kTuneRev = 2;
+
+// The cache key: device, grid shape, the options that change which kernels run
+// and the tables' revision (no spaces, so that a cache file line splits on blanks).
 static std::string tune_key(const cm1g_ctx *c) {
   cudaDeviceProp prop;
   char name[256] = "gpu";
@@ -1076,9 +1080,10 @@ static std::string tune_key(const cm1g_ctx *c) {
   for (char *p = name; *p; p++) if (*p == ' ' || *p == '\t') *p = '_';
   const cm1g_config_t &f = c->cfg;
   char key[512];
-  snprintf(key, sizeof key, "%s/sm%d/%dx%dx%d/h%d/q%d/t%d/w%d/pd%d/ns%d/bc%d%d%d%d", name,
+  snprintf(key, sizeof key, "%s/sm%d/%dx%dx%d/h%d/q%d/t%d/w%d/pd%d/ns%d/bc%d%d%d%d/df%d/rev%d", name,
            sms, f.ni, f.nj, f.nk, f.ngxy, f.imoist ? f.numq : 0,
-           f.iptra ? f.npt : 0, f.advwenos, f.pdtra, f.nsound, f.wbc, f.ebc, f.sbc, f.nbc);
+           f.iptra ? f.npt : 0, f.advwenos, f.pdtra, f.nsound, f.wbc, f.ebc, f.sbc, f.nbc, f.idiff,
+           kTuneRev);
   return key;
 }
 

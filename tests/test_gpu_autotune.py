@@ -116,3 +116,31 @@ def test_autotune_keeps_state_and_caches(cm1g, tmp_path):
         assert torch.equal(a[k], b[k]), k
     for c in (ctx, ctx2, ctx3):
         c.close()
+
+
+def test_cache_entries_of_other_launches_are_not_taken(cm1g, tmp_path):
+    """An entry written before an index came to mean another launch, or for the
+    same grid without the 6th-order diffusion (whose momentum pass is another
+    kernel), is not a timing of what would run now."""
+    _torch()
+
+    def tune(ni, cache, idiff=0):
+        case = make_case("dry_bubble", ni=ni, nj=24, nk=16)
+        if idiff:
+            case.cfg.idiff, case.cfg.difforder, case.cfg.kdiff6 = 1, 6, 0.04
+        ctx = cm1g.Context(case.cfg, case.grid)
+        t = ctx.autotune(cm1g.to_device(case.state), case.dt, case.mass1, reps=1, cache=cache)
+        ctx.close()
+        return t
+
+    seen, old = str(tmp_path / "seen.txt"), str(tmp_path / "old.txt")
+    tune(36, seen)
+    tune(36, seen, idiff=1)
+    keys = [line.split()[0] for line in open(seen)]
+    assert len(set(keys)) == 2, keys
+    # the key as it was without a revision of the tables and without the diffusion
+    key = keys[0].replace("36x24x16", "37x24x16")
+    key = key[:key.index("/bc") + 7]
+    with open(old, "w") as f:
+        f.write(key + " 4 1 1 123.0\n")
+    assert tune(37, old)["step_ms"] != 123.0
