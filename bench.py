@@ -217,15 +217,22 @@ def run_reference(args):
     return 0
 
 
-def _shapes(tune, binding):
-    """The launch shapes used (autotuner's choice, or the defaults)."""
+def _shapes(tune, binding, cfg):
+    """The launch shapes used (autotuner's choice, or the defaults).  Shape 0
+    of the scalar pass, and of the momentum pass without the 6th-order
+    diffusion, has its levels chosen by the grid's size; that momentum pass
+    owns 31 x 8 points a block in every shape."""
     if tune is None:
         return {"autotuned": False}
-    tab, stab = binding.tile_shapes(), binding.tile_shapes(scalar=True)
-    forms = {0: "tile 32 columns x 8 warps", 1: "tile 32 columns x 4 warps", 2: "column sweep 32x4",
-             3: "column sweep 32x2"}
-    return {"autotuned": True, "scalar_tile_cells_xyz": stab[tune["adv_shape"]],
-            "momentum_tile_xyz": tab[tune["mom_shape"]],
+    a, m = tune["adv_shape"], tune["mom_shape"]
+    scal, mom = list(binding.tile_shapes(scalar=True)[a]), list(binding.tile_shapes()[m])
+    if a == 0:
+        scal[2] = "by grid size"
+    if cfg.idiff == 0:
+        mom = [31, 8, mom[2] if m else "by grid size"]
+    forms = {0: "tile 32 columns, 7, 10 or 16 warps by grid size", 1: "tile 32 columns x 16 warps",
+             2: "column sweep 32x4", 3: "column sweep 32x2"}
+    return {"autotuned": True, "scalar_tile_cells_xyz": scal, "momentum_tile_xyz": mom,
             "acoustic": forms.get(tune["sound_form"], tune["sound_form"]), "tuned_step_ms": tune["step_ms"]}
 
 
@@ -510,7 +517,7 @@ def main():
                 "n_gpus": world, "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms_step,
                 "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f32",
                 "data": "synthetic (seeded, generated in-repo)",
-                "config": dict(workload_config(case, args), launch_shapes=_shapes(tune, binding)),
+                "config": dict(workload_config(case, args), launch_shapes=_shapes(tune, binding, cfg)),
                 "roofline": roof, "roofline_acoustic": roof_snd,
                 "step_roofline": {"algorithmic_bytes_per_cell": B, "achieved_gbs": step_gbs, "frac": step_gbs / hbm,
                                   "roofline_cell_updates_per_s": hbm * 1e9 / B},

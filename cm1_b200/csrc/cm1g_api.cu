@@ -1218,6 +1218,10 @@ extern "C" int cm1g_autotune(cm1g_ctx_t *c, float dt, double mass1, const cm1g_s
     bool have = false;
     for (int v = 0; v < ncand[knob] && rc == CM1G_OK; v++) {
       if (knob == 0 && v < 2 && c->g.nk > sound_max_nk()) continue;   // tile forms: too many levels
+      // k_mom takes only the levels of a shape: those of an earlier one are the same launch
+      bool same = false;
+      for (int e = 1; e < v && knob == 2 && c->cfg.idiff == 0; e++) same = same || kTileShapes[e][2] == kTileShapes[v][2];
+      if (same) continue;
       cm1g_tune_t t = cur;
       if (knob == 0) t.sound_form = v;
       else if (knob == 1) t.adv_shape = v;

@@ -42,16 +42,18 @@ struct DGrid {
   int tile_adv, tile_mom, sound_cfg;
 };
 
-// Tile shapes of the scalar and momentum passes: x and y extent of a block
-// (threads) and the levels one block marches through (z).  Entry 0 is the
-// default; the others are the autotuner's candidates.
+// Launch shapes of the momentum pass.  With the 6th-order diffusion (k_mom_tile):
+// x and y threads of a block and the levels it marches through.  Without it k_mom
+// owns 31 x 8 points a block whatever the entry, and takes the entry's levels only
+// (entry 0: levels chosen by the grid's size).  Entry 0 is the default; the others
+// are the autotuner's candidates.
 constexpr int kNumTileShapes = 5;
 constexpr int kTileShapes[kNumTileShapes][3] = {{32, 8, 16}, {32, 8, 8}, {32, 4, 16}, {64, 4, 16}, {32, 8, 32}};
 // Tile shapes of the scalar passes (k_scal_tile, k_advs_tile), indexed like
 // kTileShapes: TX x TY cells and KC levels per block; the block has one more
 // row of TX threads than the tile has cell rows (the row that evaluates the
 // tile's north and east faces), so a block is TX x (TY + 1) threads.  k_scal_tile
-// and k_mom choose the levels of the default by the grid's size.
+// chooses the levels of entry 0 by the grid's size; k_advs_tile takes all as listed.
 constexpr int kScalShapes[kNumTileShapes][3] = {{32, 7, 16}, {32, 7, 8}, {32, 3, 16}, {64, 3, 16}, {32, 7, 32}};
 // Forms of the acoustic kernel: 0 tile (32 columns, the warps over the levels
 // chosen by the grid's size), 1 tile with 16 explicit warps, 2 column sweep

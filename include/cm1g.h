@@ -526,13 +526,18 @@ int cm1g_pdefq_noalloc(const cm1g_config_t *cfg, float rmax, double *asq,
  * reference (its loops have no launch shapes).  adv_shape indexes the
  * tile shapes of the scalar passes (cm1g_scal_tile_shape: x and y cells of
  * a tile, levels per block; the block has one more row of threads than the
- * tile has cell rows) and mom_shape those of the momentum pass
- * (cm1g_tile_shape: x and y threads of a block, levels per block);
- * sound_form selects the acoustic kernel: -1 automatic, 0 tile form of 32
- * columns with the warps over the levels chosen by the grid's size, 1 the
- * same with 16 of them, 2 column sweep with 32 x 4 columns per block, 3 column
- * sweep with 32 x 2.  step_ms is the measured large-step time of the
- * configuration (cm1g_autotune; 0 when not measured). */
+ * tile has cell rows).  mom_shape indexes those of the momentum pass
+ * (cm1g_tile_shape): x and y threads and levels of a block with the
+ * 6th-order diffusion; without it a block owns 31 x 8 points and takes the
+ * shape's levels only.  Shape 0 is automatic: the fused scalar pass and the
+ * momentum pass without diffusion choose its levels by the grid's size, and
+ * the levels that the shape functions report for it are those of the passes
+ * that do not choose.  sound_form selects the acoustic kernel: -1 automatic,
+ * 0 tile form of 32 columns with the warps over the levels chosen by the
+ * grid's size (16 where there are at most 148 tiles, else 7 up to 84 levels
+ * and 10 above), 1 the same with 16 of them, 2 column sweep with 32 x 4
+ * columns per block, 3 column sweep with 32 x 2.  step_ms is the measured
+ * large-step time of the configuration (cm1g_autotune; 0 when not measured). */
 typedef struct cm1g_tune {
   int32_t adv_shape, mom_shape, sound_form;
   float step_ms;
@@ -551,8 +556,9 @@ int cm1g_get_tune(cm1g_ctx_t *ctx, cm1g_tune_t *tune);
  * copy of st (st itself is left unchanged; device or host pointers), each
  * as `reps` replays of the captured large step after one untimed replay,
  * one choice at a time (acoustic form, then scalar tile, then momentum
- * tile), and keeps the fastest on the context.  Results are cached per
- * device, grid shape and configuration: in the process, and, when
+ * tile; a candidate that is another's launch is not timed again), and keeps
+ * the fastest on the context.  Results are cached per device, grid shape,
+ * configuration and revision of the launch tables: in the process, and, when
  * cache_path is not NULL, in that text file (one line per entry); a cached
  * entry is applied without timing.  out (may be NULL) receives the choice. */
 int cm1g_autotune(cm1g_ctx_t *ctx, float dt, double mass1, const cm1g_state_t *st, int32_t reps,
