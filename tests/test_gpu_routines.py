@@ -219,3 +219,27 @@ def test_pdefq_calcmass_maxmin(cm1g, oracle_lib):
         gmx, gmn, gloc = ctx.maxmin(cm1g.to_device({"a": a})["a"], stag)
         assert (gmx, gmn) == (mx.value, mn.value)
         assert tuple(gloc) == tuple(loc)
+
+
+def test_advs_in_more_contexts_than_pinned_flags(cm1g):
+    """The entry's error flag is a slot of one pinned page for 1024 contexts; those
+    after them copy a flag from the device, and closed ones give theirs back."""
+    _torch()
+    case = make_case("dry_bubble", ni=4, nj=4, nk=6, advwenos=1)
+    arrays = _adv_inputs(case, np.random.default_rng(3), positive=False)
+
+    def advs(ctx):
+        rru, rrv, rrw, divx, s0, s, sten = arrays
+        out = sten.copy()
+        ctx.advs(1, 1, divx, rru, rrv, rrw, s0, s, out, 1, 0, f32(0.5), 1e-18)
+        return out
+
+    ctxs = [cm1g.Context(case.cfg, case.grid) for _ in range(1026)]
+    outs = [advs(c) for c in ctxs]
+    assert not np.array_equal(outs[0], arrays[-1]) and all(np.array_equal(o, outs[0]) for o in outs)
+    for c in ctxs[:600]:
+        c.close()
+    fresh = [cm1g.Context(case.cfg, case.grid) for _ in range(3)]
+    for c in fresh + ctxs[600:]:
+        assert np.array_equal(advs(c), outs[0])
+        c.close()
