@@ -268,10 +268,13 @@ void launch_bc_batch(const DGrid &g, float *const *arrays, const int *which, con
     }
     const bool per = g.wbc == 1 && g.ebc == 1 && g.sbc == 1 && g.nbc == 1;
     const bool open = g.wbc == 2 && g.ebc == 2 && g.sbc == 2 && g.nbc == 2;
-    if (merge && (per || open)) {
-      int nz = 0;
-      for (int q = 0; q < b.n; q++)
-        if (b.stag[q] == STAG_W && b.wflag[q]) nz = (g.nj + 2 + BC_ZROWS - 1) / BC_ZROWS - 1;
+    int nz = 0;
+    for (int q = 0; q < b.n; q++)
+      if (b.stag[q] == STAG_W && b.wflag[q]) nz = (g.nj + 2 + BC_ZROWS - 1) / BC_ZROWS - 1;
+    // a halo wider than the domain wraps around it more than once: its points copy
+    // halo points, which one launch would write and read at the same time
+    const bool once = open || (g.ngxy <= g.ni && g.ngxy <= g.nj);
+    if (merge && (per || open) && once) {
       const int nbr = (g.nj + 1 + BC_NT - 1) / BC_NT, nbc = (g.NI + 1 + BC_NT - 1) / BC_NT;
       dim3 grid(nbr + nbc, g.nk + nz, b.n);
       ProfScope _ps("k_bc_fill", st);

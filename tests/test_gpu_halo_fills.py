@@ -9,7 +9,7 @@ import ctypes as C
 import numpy as np
 import pytest
 
-from cm1_b200.cases import make_case
+from cm1_b200.cases import Layout, make_case
 from test_gpu_parity import TOL_RANGE, field_errors
 
 pytestmark = pytest.mark.gpu
@@ -47,6 +47,28 @@ def test_fills_bitwise(ni, nj, nk, sides, cm1g, oracle_lib):
             d = cm1g.to_device({"a": a})["a"]
             ctx.bc(which, d, flag)
             assert np.array_equal(d.cpu().numpy(), ref), (which, flag)
+    ctx.close()
+
+
+@pytest.mark.parametrize("sides", [(1, 1, 1, 1), (2, 2, 2, 2)])
+@pytest.mark.parametrize("ni,nj,ngxy", [(4, 9, 5), (9, 4, 5), (4, 4, 4), (4, 5, 7)])
+def test_wide_halos_bitwise(ni, nj, ngxy, sides, cm1g, oracle_lib):
+    """Halos as wide as the domain, and wider: periodic points then copy halo points."""
+    _torch()
+    case = _case(sides, ni=ni, nj=nj, nk=6)
+    case.cfg.ngxy, w = ngxy, ngxy - 3
+    grid = {k: np.ascontiguousarray(np.pad(a, [(0, 0)] * max(0, a.ndim - 2) + [(w, w)] * min(2, a.ndim), mode="edge"))
+            for k, a in case.grid.items()}
+    lay = Layout(ni, nj, 6, ngxy)
+    ctx = cm1g.Context(case.cfg, grid)
+    rng = np.random.default_rng(ni + nj)
+    for code, which in enumerate("spuvw", 1):
+        a = rng.normal(size=lay.shape(STAG[which])).astype(np.float32)
+        ref = a.copy()
+        assert oracle_lib.lib().oracle_bc(C.byref(case.cfg), code, ref.ctypes.data_as(C.POINTER(C.c_float)), 1) == 0
+        d = cm1g.to_device({"a": a})["a"]
+        ctx.bc(which, d, 1)
+        assert np.array_equal(d.cpu().numpy(), ref), which
     ctx.close()
 
 
