@@ -477,8 +477,8 @@ void launch_stat(const DGrid &g, const StatFields &f, const StatConsts &s, const
   StatRest R;
   R.n = 0;
   int flow = 0, nlev = 0;
-  auto rest = [&](bool end) {   // the jobs outside k_stat_flow, ST_MAXREST at a time
-    if (R.n == 0 || (!end && R.n < ST_MAXREST)) return;
+  auto rest = [&]() {   // the jobs outside k_stat_flow gathered so far
+    if (R.n == 0) return;
     dim3 grid((unsigned)nch, (unsigned)nlev);
     { ProfScope _ps("k_stat_levels", st); k_stat_levels<<<grid, ST_NT, 0, st>>>(g, f, s, jobs, R, lev, maxlev, nch); }
     if (nl) *nl += 1;
@@ -509,12 +509,12 @@ void launch_stat(const DGrid &g, const StatFields &f, const StatConsts &s, const
     else if (j.kind == SK_ENER) slot = &F.s[FS_ENER];
     if (j.nlev == 0) continue;
     if (slot) { *slot = q; flow = 1; continue; }
+    if (R.n == ST_MAXREST || nlev + j.nlev > 65535) rest();   // a launch grid's y extent
     R.first[R.n] = nlev;
     R.job[R.n++] = q;
     nlev += j.nlev;
-    rest(false);
   }
-  rest(true);
+  rest();
   if (flow) {
     dim3 grid((unsigned)nch, (unsigned)(F.m[FM_W] >= 0 ? g.nk + 1 : g.nk));
     { ProfScope _ps("k_stat_flow", st); k_stat_flow<<<grid, ST_NT, 0, st>>>(g, f, s, F, lev, maxlev, nch); }

@@ -95,6 +95,7 @@ def test_diff2_matches_oracle(name, over, bbc, tbc, idiff, cm1g, oracle_lib):
     ("dry_bubble", dict(ni=6, nj=4, nk=6), 1),                         # fewer points than a block has threads
     ("dry_bubble", dict(ni=300, nj=4, nk=7), 1),                       # rows longer than a block, fewer rows than warps
     ("supercell", dict(ni=32, nj=33, nk=44, npt=2), 1),
+    ("dry_bubble", dict(ni=4, nj=4, nk=8200, dz=1.0, npt=8), 0),       # more levels of tracers than a launch grid has rows
 ])
 def test_statpack_matches_oracle(name, over, steps, cm1g, oracle_lib):
     statpack.test_statpack_matches_oracle(name, over, steps, cm1g, oracle_lib)
