@@ -274,7 +274,7 @@ void launch_bc_batch(const DGrid &g, float *const *arrays, const int *which, con
     // a halo wider than the domain wraps around it more than once: its points copy
     // halo points, which one launch would write and read at the same time
     const bool once = open || (g.ngxy <= g.ni && g.ngxy <= g.nj);
-    if (merge && (per || open) && once) {
+    if (merge && (per || open) && once && g.nk + nz <= 65535) {   // a launch grid's y extent
       const int nbr = (g.nj + 1 + BC_NT - 1) / BC_NT, nbc = (g.NI + 1 + BC_NT - 1) / BC_NT;
       dim3 grid(nbr + nbc, g.nk + nz, b.n);
       ProfScope _ps("k_bc_fill", st);
