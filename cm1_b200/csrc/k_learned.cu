@@ -447,8 +447,9 @@ __global__ void __launch_bounds__(32 * BW_WARPS, 2) k_mlp_backward(const float *
     atomicAdd(&grad[P_B1 + ib], gw1[3]);
     atomicAdd(&grad[P_B2 + ia], gb2[1]);
     atomicAdd(&grad[P_B2 + ib], gb2[3]);
-    atomicAdd(&grad[P_W1 + 7 * MLP_H + ia], 0.0f * gw1[1]);   // the padding's own: zero, if dz1 is finite
-    atomicAdd(&grad[P_W1 + 7 * MLP_H + ib], 0.0f * gw1[3]);
+    const float pa = 0.0f * gw1[1], pb = 0.0f * gw1[3];       // the padding's own: not zero where dz1 is not finite
+    if (pa != 0.0f) atomicAdd(&grad[P_W1 + 7 * MLP_H + ia], pa);
+    if (pb != 0.0f) atomicAdd(&grad[P_W1 + 7 * MLP_H + ib], pb);
   }
 #pragma unroll
   for (int q = 0; q < 2; q++) {
