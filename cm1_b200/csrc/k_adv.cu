@@ -486,7 +486,8 @@ __global__ void __launch_bounds__(TX * TY, 3) k_mom_tile(DGrid g, Vel q, const f
 // adv.F are applied in the blocks that touch an open edge.
 //
 // Bound by instruction issue and latency: 890 warp instructions per 32 points
-// at 60 % issue, 36 % of the DRAM rate.  256x256x80: 0.230 ms against 0.370
+// at 60 % issue with 17 warps an SM; DRAM moves 159 MB (9 % of the peak), less than
+// the arrays because L2 keeps part of the tendencies.  256x256x80: 0.230 ms against 0.370
 // for a divergence pass and one marching tile per component, which staged u, v
 // and w separately and read them again as face velocities; 64x64x40: 27 us
 // against 62.  Three blocks an SM at 72 registers spill and measured 4 to 14 %

@@ -11,8 +11,9 @@
 // (k_bc_phase): so the corner values come out exactly as the serial loop order
 // leaves them; every phase reads only points the same phase does not write, so
 // its threads need no ordering among themselves.  (In an ensemble other members
-// fill the gaps between launches: 5.42 against 5.47 ms for twelve, and there the
-// count of launches a member that callers see stays what it was.)
+// fill the gaps between launches, so the form makes no difference there: 5.42 ms
+// against 5.47 for twelve.  Its members keep the two phases because callers read
+// the launches of a step, cm1g_ensemble_launch_count, and expect the phases in it.)
 #include "cm1g_common.cuh"
 
 namespace cm1g {

@@ -7,8 +7,9 @@
 // Without lateral walls one launch does it all (k_d2_flow): a tile of columns
 // marches upward, the tensor of a point is formed once and passed to the
 // neighbours that difference it by warp shuffles (x), shared rows (y) and
-// registers (z); 256x256x80 with theta and three tracers takes 0.274 ms (68 %
-// of the issue slots, 43 % of the DRAM rate) against 0.438 through memory.
+// registers (z); 256x256x80 with theta and three tracers takes 0.274 ms (67 %
+// of the issue slots, 26 % of the DRAM peak) against 0.438 through memory.  Up to
+// three scalars go with the momentum, further ones three a launch.
 // Lateral walls (free slip 3, no slip 4) rewrite the tensor
 // along the sides in the reference's order, corners included, so grids with
 // walls keep it in memory: k_d2_tensor forms rr, rf, divx and the raw

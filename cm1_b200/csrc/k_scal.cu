@@ -23,8 +23,8 @@
 //  * one barrier per item: the face fluxes and face velocities are double
 //    buffered by item parity.
 //
-// Bound by instruction issue: three faces are some 400 of an item's 690
-// instructions, at 24 warps a SM (80 registers).  So the faces that the fast
+// Bound by instruction issue (67 % of the cycles): three faces are some 400 of an
+// item's 650 to 760 instructions, at 24 warps a SM (80 registers).  So the faces that the fast
 // WENO5 leaves open are evaluated beside it from shared memory without a call,
 // the item's global reads are issued after its faces and not before (their
 // registers are then free while a face is evaluated), and a flux lies beside
@@ -205,8 +205,8 @@ __global__ void __launch_bounds__(TX * (TY + 1), 3) k_scal_tile(const __grid_con
   // its cell and the y face on its south; the extra row's threads own the y
   // faces north of the tile and (the first TY of them) the x faces east of it,
   // so that every cell thread evaluates three faces and no thread more.
-  // oc: the thread's column in an s or v plane; xo: its x face in a u plane
-  // (bytes); xs, ys: the stencils' first values in a staged plane
+  // oc: the thread's column in an s or v plane; xo: its x face in a u plane;
+  // xs, ys: the stencils' first values in a staged plane
   const bool yface_on = (i <= ni && j <= nj + 1);
   const int oc = yface_on ? (i - g.ib) + NI * (j - g.jb) : 0;
   const int ys = ty * SP + tx + 3;
@@ -519,7 +519,9 @@ __global__ void __launch_bounds__(256) k_pdef_fix(const __grid_constant__ DGrid 
 // and with this rule: 64x64x40 82, 51, 137, 39 us; 203x150x61, four fields 713, 628,
 // 838, 665 us; 256x256x80 2.60, 2.53, 2.51, 2.47 ms; 512x512x128 6.78, 7.20, 6.74, 6.78 ms.
 // The host entry's single field takes at most 16: its second pass walks a chunk
-// level by level (251x187x79: 95 us with 20 levels, 76 with 12).
+// level by level (251x187x79, the one grid measured: 95 us with 20 levels, 76 with
+// 12).  A step's passes keep the rule's choice: one launch's rule serves both, and
+// their words name few levels where tracers are sparse.
 constexpr int SC_OVER = 2;
 template <int TX, int TY, int PDEF, int RAW>
 static void scal_shape(const DGrid &g, ScalPass P, int kc, int weno, cudaStream_t st, int64_t *nl) {

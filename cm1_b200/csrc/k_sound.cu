@@ -18,8 +18,8 @@
 //
 // What bounds it: latency and instruction issue, not bytes.  At 256x256x80 a
 // launch takes 0.141 ms = 3.4 TB/s of its 92 B a cell (0.53 of the measured
-// HBM copy rate); it executes about 430 warp instructions per 32 cells and
-// issues in half of the cycles.  Before (8 warps, the solve on one of them
+// HBM copy rate); it executes about 490 warp instructions per 32 cells and
+// issues in 62 % of the cycles.  Before (8 warps, the solve on one of them
 // after a block barrier, 64-bit indices, profiles read per level): 0.184 ms,
 // 558 instructions; at 512x512x128 2.27 ms against 0.86 now.  What made the
 // difference: the solver warp hidden behind the loads, 32-bit byte offsets,

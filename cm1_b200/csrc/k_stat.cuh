@@ -19,8 +19,7 @@ enum StatKind {
   SK_CFL,        // Courant number
   SK_VORT,       // vertical vorticity at level k0
   SK_CLOUD,      // sum of the cloud species (level max decides the cloud levels)
-  SK_FIRST_SUM,
-  SK_MASS = SK_FIRST_SUM,  // dry-air mass
+  SK_MASS,       // dry-air mass; from here on sums
   SK_TMOIS,      // total moisture
   SK_QMAS,       // mass of one species (qn)
   SK_TMF,        // upward and downward mass flux

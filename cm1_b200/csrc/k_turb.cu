@@ -22,8 +22,8 @@
 // and a few shared rows (y neighbours) only: forming the strain twice costs
 // about 60 binary32 operations a point, storing and re-reading the twelve
 // strain, stress and coefficient arrays cost 48 to 100 bytes a point.
-// Bound by instruction issue (62 to 73 % of the cycles; 558 and 890 warp
-// instructions per 32 points), at 42 to 50 % of the DRAM rate.  256x256x128
+// Bound by instruction issue (71 and 61 % of the cycles; 558 and 884 warp
+// instructions per 32 points), at 14 and 25 % of the DRAM peak.  256x256x128
 // with theta and two tracers: 0.583 ms a call against 1.33 for the four
 // point-parallel passes before.  With every neighbour loaded instead of
 // shuffled the two passes took 0.81 ms, and without reading a level's
