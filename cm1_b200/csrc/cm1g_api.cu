@@ -571,7 +571,11 @@ struct Stager {
   float *dev_buffer(size_t n) {
     if (pool_i < c->stage_pool.size() && c->stage_pool[pool_i].second >= n) return c->stage_pool[pool_i++].first;
     float *p = nullptr;
-    if (cudaMalloc(&p, n * sizeof(float)) != cudaSuccess) { err = 1; return nullptr; }
+    if (cudaMalloc(&p, n * sizeof(float)) != cudaSuccess) {
+      (void)cudaGetLastError();   // reported through err, not by a later call
+      err = 1;
+      return nullptr;
+    }
     if (pool_i < c->stage_pool.size()) { cudaFree(c->stage_pool[pool_i].first); c->stage_pool[pool_i] = {p, n}; }
     else c->stage_pool.push_back({p, n});
     pool_i++;
@@ -1456,6 +1460,7 @@ extern "C" int cm1g_pdefq(cm1g_ctx_t *c, float rmax, double *asq, const float *r
   size_t ns = nS(c->g);
   const float *drho = S.in(rho, ns, false);
   float *dq = S.in(q3d, ns, true);
+  if (S.err) return set_err(CM1G_ERR_NOMEM, "staging alloc");
   CUCHK(cudaMemsetAsync(c->dscal + 8, 0, sizeof(double), c->stream));
   launch_pdefq(c->g, rmax, drho, dq, c->bud, c->dscal + 8, c->stream, &c->nlaunch);
   double a = 0.0;
@@ -1471,6 +1476,7 @@ static int bc_entry(cm1g_ctx_t *c, float *a, int which, int flag) {
   Stager S(c);
   size_t n = which == 3 ? nU(c->g) : which == 4 ? nV(c->g) : which == 5 ? nW(c->g) : nS(c->g);
   float *d = S.in(a, n, true);
+  if (S.err) return set_err(CM1G_ERR_NOMEM, "staging alloc");
   launch_bc(c->g, d, which, flag, c->stream, &c->nlaunch);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return set_err(CM1G_ERR_CUDA, "%s", cudaGetErrorString(e));
@@ -1494,6 +1500,7 @@ extern "C" int cm1g_advs(cm1g_ctx_t *c, int32_t nrk, int32_t wflag, const float 
   const float *ddx = S.in(divx, nS(g), false), *ds = S.in(s, nS(g), false);
   const float *ds0 = s0 ? S.in(s0, nS(g), false) : nullptr;
   float *dten = S.in(sten, nS(g), true);
+  if (S.err) return set_err(CM1G_ERR_NOMEM, "staging alloc");
   const int weno = (wflag == 1) && (c->cfg.advwenos == 1 || (c->cfg.advwenos == 2 && nrk == 3));
   if (!c->advs_err) c->advs_err = pinned_flags().take();
   // t11 is scratch of the large step, set anew by each of its stages
@@ -1599,6 +1606,7 @@ extern "C" int cm1g_calcmass(cm1g_ctx_t *c, const float *rho, double *tmass) {
   if (!c || !rho || !tmass) return set_err(CM1G_ERR_ARG, "null argument");
   Stager S(c);
   const float *dr = S.in(rho, nS(c->g), false);
+  if (S.err) return set_err(CM1G_ERR_NOMEM, "staging alloc");
   launch_level_mass(c->g, dr, c->lev, c->stream, &c->nlaunch);
   std::vector<double> lev(c->g.nk + 2);
   CUCHK(cudaMemcpyAsync(lev.data(), c->lev, lev.size() * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
@@ -1673,6 +1681,7 @@ extern "C" int cm1g_tendency_init(cm1g_ctx_t *c, int32_t irdamp, float rdalpha, 
   t.qten = numq ? S.in(qten, numq * ns, true) : nullptr;
   t.ptten = npt ? S.in(ptten, npt * ns, true) : nullptr;
   t.numq = numq; t.nq = numq + npt;
+  if (S.err) return set_err(CM1G_ERR_NOMEM, "staging alloc");
   launch_tend_init(g, t, c->stream, &c->nlaunch);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return set_err(CM1G_ERR_CUDA, "%s", cudaGetErrorString(e));
@@ -1693,6 +1702,7 @@ extern "C" int cm1g_calcener(cm1g_ctx_t *c, const float *zh, const float *rho, c
   e.tha = S.in(tha, ns, false);
   e.qv = qv ? S.in(qv, ns, false) : nullptr; e.ql = ql ? S.in(ql, ns, false) : nullptr;
   e.qi = qi ? S.in(qi, ns, false) : nullptr; e.vr = vr ? S.in(vr, ns, false) : nullptr;
+  if (S.err) return set_err(CM1G_ERR_NOMEM, "staging alloc");
   // constants.F:85-150: latent heats at the reference temperature to = 273.15
   const int tc = c->cfg.testcase;
   const float xlv = tc == 4 ? 2.47e6f : tc == 5 ? 2.50e6f : 2501000.0f, xls = 2834000.0f, to = 273.15f;
@@ -1716,6 +1726,7 @@ extern "C" int cm1g_maxmin(cm1g_ctx_t *c, const float *a, int32_t stag, float *a
   const DGrid &g = c->g;
   size_t n = stag == 2 ? nU(g) : stag == 3 ? nV(g) : stag == 4 ? nW(g) : nS(g);
   const float *d = S.in(a, n, false);
+  if (S.err) return set_err(CM1G_ERR_NOMEM, "staging alloc");
   launch_maxmin(g, d, stag, c->mm, c->stream, &c->nlaunch);
   unsigned long long h[2];
   CUCHK(cudaMemcpyAsync(h, c->mm, sizeof h, cudaMemcpyDeviceToHost, c->stream));
@@ -2021,6 +2032,7 @@ extern "C" int cm1g_statpack(cm1g_ctx_t *c, double mtime, float dt, const float 
   f.qa = (need_q && numq) ? S.in(qa, (size_t)numq * ns, false) : nullptr;
   f.pta = (need_pt && npt) ? S.in(pta, (size_t)npt * ns, false) : nullptr;
   f.prate = prate ? S.in(prate, (size_t)g.NI * g.NJ, false) : nullptr;
+  if (S.err) return set_err(CM1G_ERR_NOMEM, "staging alloc");
   f.qstride = (long)ns;
   const cm1g_stat_opts_t &o = c->st_opts;
   StatConsts k{};
