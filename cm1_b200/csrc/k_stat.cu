@@ -212,19 +212,22 @@ __global__ void __launch_bounds__(ST_NT, 3) k_stat_flow(DGrid g, StatFields f, S
       if (moe || ener) {
         const double qtot = (double)((qv + ql) + 0.0f), tem = (double)(ruh * rvh * rmh);
         const double rt = (double)rho * tem, rq = rt * (1.0 + qtot);
-        const float wm = 0.5f * (w1 + w2);
-        if (moe) {                     // calcmoe (misclibs.F:3488-3502), umove = vmove = 0; vr = 0 drops a term
+        // the reference's terms with a factor 0 (vr, qi) are added to a factor of the
+        // others: zero, or not a number where a value in them is not finite
+        const float wm = __fmaf_rn(0.0f, ql * rho, 0.5f * (w1 + w2));
+        if (moe) {                     // calcmoe (misclibs.F:3488-3502), umove = vmove = 0
           acc[5] = acc[5] + rq * (double)ua;
           acc[6] = acc[6] + rq * (double)va;
           acc[7] = acc[7] + rq * (double)wm;
         }
-        if (ener) {                    // calcener (misclibs.F:3374-3393), umove = vmove = 0; qi = vr = 0 drop two terms
-          const float ke = (0.5f * (u1 * u1 + u2 * u2) + 0.5f * (v1 * v1 + v2 * v2)) + 0.5f * (w1 * w1 + w2 * w2);
+        if (ener) {                    // calcener (misclibs.F:3374-3393), umove = vmove = 0
+          const float ke = __fmaf_rn(0.0f, wm, (0.5f * (u1 * u1 + u2 * u2) + 0.5f * (v1 * v1 + v2 * v2)) + 0.5f * (w1 * w1 + w2 * w2));
           acc[8] = acc[8] + rq * 0.5 * (double)ke;
           const double tmp = (double)tx;
           acc[9] = acc[9] + rt * (double)(s.cv + s.cvv * qv) * tmp;
           acc[10] = acc[10] + rq * (double)s.g * (double)zh;
-          if (liquid) acc[11] = acc[11] + rt * (double)ql * ((double)s.cpl * tmp - (double)s.lv1);
+          const float qz = __fmaf_rn(0.0f, rho, __fmaf_rn(0.0f, tx, ql));
+          acc[11] = acc[11] + (liquid ? rt * (double)qz * ((double)s.cpl * tmp - (double)s.lv1) : (double)qz);
         }
       }
     }

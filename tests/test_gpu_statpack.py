@@ -147,3 +147,35 @@ def test_statpack_with_kessler_liquid(cm1g, oracle_lib):
     v = dict(zip(names, got))
     assert v["qctop"] > v["qcbot"] > 0.0 and v["le"] != 0.0 and v["pratemax"] > 0.0
     ctx.close()
+
+
+@pytest.mark.parametrize("name", ["dry_bubble", "kessler"])
+def test_statpack_of_infinite_values(name, cm1g, oracle_lib):
+    """One infinite or not-a-number value in a field: the statistics that become
+    infinite, of either sign, and not a number are the oracle's (among them the
+    budgets' terms whose factor is zero), the others still agree."""
+    _torch()
+    case = make_case(name, ni=20, nj=12, nk=44)
+    kw_o = dict(qnames=("qv", "qc", "qr"), nql=(2, 3), cloud=(1,)) if name == "kessler" else {}
+    o, keep = stat_opts(case, off=("stat_pcn", "stat_qsrc"), **kw_o)
+    ctx = cm1g.Context(case.cfg, case.grid)
+    names = ctx.stat_setup(o)
+    K, J, I = case.lay.kx(9), case.lay.jx(5), case.lay.ix(7)
+    fields = ["ua", "va", "wa", "ppi", "tha", "prs", "rho"] + (["qa"] if name == "kessler" else [])
+    for field in fields:
+        for value in (np.inf, -np.inf, np.nan):
+            for q in ((0, 1) if field == "qa" else (0,)):
+                st = case.copy_state()
+                a = st[field][q] if field == "qa" else st[field]
+                a[K, J, I] = value
+                with np.errstate(all="ignore"):
+                    ref = oracle_lib.statpack(case, o, st, mtime=3.0, prate=st["prate"] if name == "kessler" else None)
+                f, kw = _args(case, st)
+                if name == "kessler":
+                    kw["prate"] = st["prate"]
+                got = ctx.statpack(3.0, case.dt, *f, **kw)
+                for n, x, y in zip(names, got, ref):
+                    assert np.isnan(x) == np.isnan(y) and (not np.isinf(x) and not np.isinf(y) or x == y), (field, value, n, x, y)
+                fin = [k for k, y in enumerate(ref) if np.isfinite(y)]
+                _compare([names[k] for k in fin], got[fin], ref[fin])
+    ctx.close()
