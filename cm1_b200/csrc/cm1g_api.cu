@@ -139,24 +139,29 @@ static int set_err(int code, const char *fmt, ...) {
   return code;
 }
 
+// Arithmetic only: the entries call it before their first launch (297 tiles of 80
+// levels: 0.7 us; stepping through the blocks' schedule took 7, and 460 for 36,572
+// tiles of 128).
 int cm1g::tile_levels(long tiles, int nk, int slots, int over, int kcmax) {
+  const auto up = [](long a, long b) { return (a + b - 1) / b; };
   int best = 0;
   long best_end = 0;
   for (int kc = 4; kc <= kcmax; kc += kc < 16 ? 1 : kc < 32 ? 2 : 4) {
     const int nch = (nk + kc - 1) / kc;
-    // the full chunks in whole rounds of the slots, then the last chunk of every
-    // tile on the slots as they come free (end of a slot's last block -> slots)
-    const long len = over + kc, full = tiles * (nch - 1), rounds = full / slots, rest = full % slots;
-    std::map<long, long> free_at{{rounds * len, slots - rest}};
-    if (rest) free_at[(rounds + 1) * len] = rest;
-    long end = free_at.rbegin()->first;
-    for (long n = tiles; n > 0;) {
-      const auto it = free_at.begin();
-      const long t = it->first + over + nk - (nch - 1) * kc, m = std::min(n, it->second);
-      if ((it->second -= m) == 0) free_at.erase(it);
-      free_at[t] += m;
-      end = std::max(end, t);
-      n -= m;
+    // the full chunks in whole rounds of the slots: `late` slots come free a block
+    // later than the others
+    const long len = over + kc, full = tiles * (nch - 1), early = slots - full % slots, late = slots - early;
+    const long t0 = full / slots * len, t1 = t0 + len;
+    // then the last chunk of every tile, all of length q, on the slots as they come
+    // free: the first time by which that many have ended, at the end of an early or
+    // of a late slot's block
+    const long q = over + nk - (long)(nch - 1) * kc, c = up(len, q), f = len / q;
+    long i = up(tiles, early);
+    if (late && i > c) i = up(tiles + late * c, slots);
+    long end = t0 + i * q;
+    if (late) {
+      const long j = std::max(1L, up(std::max(0L, tiles - early * f), slots));
+      end = std::max(t1, std::min(end, t1 + j * q));
     }
     if (!best || end < best_end) { best = kc; best_end = end; }
     if (kc >= nk) break;
