@@ -33,6 +33,7 @@
 // expressions keep the reference's operand order and kinds (binary32 where
 // the Fortran is real, binary64 where it declares double precision); the
 // library is compiled with --fmad=false.
+#include <algorithm>
 #include "cm1g_common.cuh"
 #include "k_stat.cuh"
 
@@ -113,10 +114,18 @@ struct StatFlow {
   int m[FM_N], s[FS_N], the_nlev;
 };
 
-// grid: x = chunk of rows, y = level (nk+1: w only).  A warp walks rows, its
-// lanes the points of a row.
-__global__ void __launch_bounds__(ST_NT, 3) k_stat_flow(DGrid g, StatFields f, StatConsts s, StatFlow F, StatLev *lev,
-                                                     int maxlev, int nch) {
+// grid: x = chunk of rows, y = level (nk+1: w only).  wpr of the block's warps (1, 2,
+// 4 or 8) share a row, so that few long rows occupy all of them.  SUMS: 2 with the
+// momentum or energy budgets, 1 with others, 0 with none; EXT: with extrema.  The
+// registers of those left out hold one or two more blocks an SM.  Quantities that are
+// off cost their branch only; PLAIN (most are on, a row a warp) goes without the
+// branches.  256x256x80: w alone 42 us (66 with everything always formed and a row
+// always a warp's), dry mass alone 26 (70), momentum alone 68 (122), everything 154
+// (158); 1100x960x20: w and the Courant number 302 us a call (686), everything 586
+// (875).
+template <int SUMS, bool EXT, bool PLAIN>
+__global__ void __launch_bounds__(ST_NT, 6 - SUMS - EXT) k_stat_flow(DGrid g, StatFields f, StatConsts s, StatFlow F, StatLev *lev,
+                                                            int maxlev, int nch, int wpr) {
   __shared__ float red[2 * FM_N][ST_NW];
   __shared__ double rsum[FS_ACC][ST_NW];
   const int lane = (int)(threadIdx.x & 31), w = (int)(threadIdx.x >> 5);
@@ -125,7 +134,7 @@ __global__ void __launch_bounds__(ST_NT, 3) k_stat_flow(DGrid g, StatFields f, S
   const int pl = g.NI * g.NJ, NI = g.NI;      // < 2^31 points (cm1g_init)
   const bool top = k == nk + 1;
   const bool the = F.m[FM_THE] >= 0 && k <= F.the_nlev, rhs = F.m[FM_RH] >= 0 || the;
-  const bool moe = F.s[FS_MOE] >= 0, ener = F.s[FS_ENER] >= 0;
+  const bool moe = SUMS == 2 && F.s[FS_MOE] >= 0, ener = SUMS == 2 && F.s[FS_ENER] >= 0, wsp = PLAIN || F.m[FM_WSP] >= 0;
   const bool liquid = s.imoist && s.nql1 >= 0;
   float mx[FM_N], mn[FM_N];
   double acc[FS_ACC];
@@ -133,18 +142,20 @@ __global__ void __launch_bounds__(ST_NT, 3) k_stat_flow(DGrid g, StatFields f, S
   for (int q = 0; q < FM_N; q++) { mx[q] = -1.0e30f; mn[q] = 1.0e30f; }
 #pragma unroll
   for (int q = 0; q < FS_ACC; q++) acc[q] = 0.0;
-  auto put = [&](int q, float v) { mx[q] = fmaxf(mx[q], v); mn[q] = fminf(mn[q], v); };
+  auto put = [&](int q, float v) { if (EXT) { mx[q] = fmaxf(mx[q], v); mn[q] = fminf(mn[q], v); } };
 
   const int kk = min(k, nk);
   const float th0 = LDG(&g.th0[kk]), pi0 = LDG(&g.pi0[kk]), mh = LDG(&g.mh[kk]), rmh = LDG(&g.rmh[kk]);
   const float r0 = LDG(&g.rho0[kk]), r0p = LDG(&g.rho0[kk + 1]), r0m = LDG(&g.rho0[kk - 1]), zh = s.zh[kk];
   const float pbase = F.m[FM_PP] >= 0 ? s.p00 * powf(pi0, s.cpdrd) : 0.0f;   // statpack.F:236-242
-  for (int j = j0 + w; j <= j1; j += ST_NW) {
+  if (PLAIN) wpr = 1;
+  const int rows = ST_NW / wpr, i0 = 1 + 32 * (w & (wpr - 1)) + lane;      // the block's rows at a time; first point
+  for (int j = j0 + w / wpr; j <= j1; j += rows) {
     const float vh = LDG(&g.vh[j - g.jb]), rvh = LDG(&g.rvh[j - g.jb]);
     const int orow = k * pl + NI * (j - g.jb) - g.ib;
     const float *ur = f.ua ? f.ua + (long)k * (NI + 1) * g.NJ + (long)(NI + 1) * (j - g.jb) - g.ib : nullptr;
     const float *vr = f.va ? f.va + (long)k * NI * (g.NJ + 1) + (long)NI * (j - g.jb) - g.ib : nullptr;
-    for (int i = 1 + lane; i <= ni + 1; i += 32) {
+    for (int i = i0; i <= ni + 1; i += 32 * wpr) {
       if (top) {
         if (f.wa && i <= ni && j <= nj) put(FM_W, LDG(&f.wa[orow + i]));
         continue;
@@ -167,39 +178,41 @@ __global__ void __launch_bounds__(ST_NT, 3) k_stat_flow(DGrid g, StatFields f, S
         qv = LDG(&f.qa[(long)s.nqv * f.qstride + o]);
         for (int n = s.nql1; n >= 0 && n <= s.nql2; n++) ql = ql + LDG(&f.qa[(long)n * f.qstride + o]);
       }
-      put(FM_V, v1);
-      put(FM_W, w1);
-      put(FM_PPI, ppi);
-      put(FM_THA, tha);
-      put(FM_QV, qv);
-      put(FM_PP, prs - pbase);
-      if (F.m[FM_DIV] >= 0) {          // statpack.F:297-309 (axisymm = 0)
-        const float ta = 0.5f * ((r0 + r0) * u2 - (r0 + r0) * u1) * g.rdx * uh;
-        const float tb = 0.5f * ((r0 + r0) * v2 - (r0 + r0) * v1) * g.rdy * vh;
-        const float tc = 0.5f * ((r0 + r0p) * w2 - (r0 + r0m) * w1) * g.rdz * mh;
-        put(FM_DIV, (ta + tb) + tc);
-      }
-      const float tx = (th0 + tha) * (pi0 + ppi);
-      if (rhs) {                       // statpack.F:364-371; calcthe (misclibs.F:2300-2336), cpm = cp, l0 = 2.555e6
-        const float qvs = st_rslf(prs, tx, s);
-        const float rh = qv * (1.0f + qvs * s.reps) / (qvs * (1.0f + qv * s.reps));
-        put(FM_RH, rh);
-        if (the) {
-          const float cpm = s.cp;
-          put(FM_THE, tx * powf(s.p00 * (1.0f + qv * s.reps) / prs, s.rd / cpm) * powf(rh, -(qv * s.rv / cpm)) *
-                          expf(2.555e6f * qv / (cpm * tx)));
+      const float ua = 0.0f + 0.5f * (u1 + u2), va = 0.0f + 0.5f * (v1 + v2), tx = (th0 + tha) * (pi0 + ppi);
+      if (EXT) {
+        put(FM_V, v1);
+        put(FM_W, w1);
+        put(FM_PPI, ppi);
+        put(FM_THA, tha);
+        put(FM_QV, qv);
+        put(FM_PP, prs - pbase);
+        if (F.m[FM_DIV] >= 0) {          // statpack.F:297-309 (axisymm = 0)
+          const float ta = 0.5f * ((r0 + r0) * u2 - (r0 + r0) * u1) * g.rdx * uh;
+          const float tb = 0.5f * ((r0 + r0) * v2 - (r0 + r0) * v1) * g.rdy * vh;
+          const float tc = 0.5f * ((r0 + r0p) * w2 - (r0 + r0m) * w1) * g.rdz * mh;
+          put(FM_DIV, (ta + tb) + tc);
+        }
+        if (rhs) {                       // statpack.F:364-371; calcthe (misclibs.F:2300-2336), cpm = cp, l0 = 2.555e6
+          const float qvs = st_rslf(prs, tx, s);
+          const float rh = qv * (1.0f + qvs * s.reps) / (qvs * (1.0f + qv * s.reps));
+          put(FM_RH, rh);
+          if (the) {
+            const float cpm = s.cp;
+            put(FM_THE, tx * powf(s.p00 * (1.0f + qv * s.reps) / prs, s.rd / cpm) * powf(rh, -(qv * s.rv / cpm)) *
+                            expf(2.555e6f * qv / (cpm * tx)));
+          }
+        }
+        if (wsp) put(FM_WSP, sqrtf(ua * ua + va * va));   // statpack.F:437-441 (umove = vmove = 0)
+        if (F.m[FM_CFL] >= 0) {          // calccfl (misclibs.F:2618-2665)
+          const float cu = (u1 + u2) * s.dtdx * uh, cv = (v1 + v2) * s.dtdy * vh, cw = (w1 + w2) * s.dtdz * mh;
+          float c;
+          if (s.nx > 1 && s.ny > 1) c = sqrtf((cu * cu + cv * cv) + cw * cw);
+          else if (s.nx > 1) c = sqrtf(cu * cu + cw * cw);
+          else c = sqrtf(cv * cv + cw * cw);
+          put(FM_CFL, c);
         }
       }
-      const float ua = 0.0f + 0.5f * (u1 + u2), va = 0.0f + 0.5f * (v1 + v2);
-      put(FM_WSP, sqrtf(ua * ua + va * va));           // statpack.F:437-441 (umove = vmove = 0)
-      if (F.m[FM_CFL] >= 0) {          // calccfl (misclibs.F:2618-2665)
-        const float cu = (u1 + u2) * s.dtdx * uh, cv = (v1 + v2) * s.dtdy * vh, cw = (w1 + w2) * s.dtdz * mh;
-        float c;
-        if (s.nx > 1 && s.ny > 1) c = sqrtf((cu * cu + cv * cv) + cw * cw);
-        else if (s.nx > 1) c = sqrtf(cu * cu + cw * cw);
-        else c = sqrtf(cv * cv + cw * cw);
-        put(FM_CFL, c);
-      }
+      if (!SUMS) continue;
       // ---- FP64 budgets, in the reference's operand kinds
       if (F.s[FS_MASS] >= 0) acc[0] = acc[0] + (double)(rho * ruh * rvh * rmh);                          // misclibs.F:3160-3166
       if (F.s[FS_TMOIS] >= 0) acc[1] = acc[1] + (double)(rho * ((qv + ql) + 0.0f) * ruh * rvh * rmh);    // :3224-3230, qi = 0
@@ -233,26 +246,28 @@ __global__ void __launch_bounds__(ST_NT, 3) k_stat_flow(DGrid g, StatFields f, S
     }
   }
 #pragma unroll
-  for (int q = 0; q < FM_N; q++) {
+  for (int q = 0; q < (EXT ? FM_N : 0); q++) {
     if (F.m[q] < 0) continue;
     const float a = warp_max(mx[q]), b = warp_min(mn[q]);
     if (lane == 0) { red[2 * q][w] = a; red[2 * q + 1][w] = b; }
   }
 #pragma unroll
-  for (int q = 0; q < FS_ACC; q++) {
+  for (int q = 0; q < (SUMS == 2 ? FS_ACC : SUMS ? 5 : 0); q++) {
+    const int job = q < 3 ? q : q < 5 ? FS_TMF : q < 8 ? FS_MOE : FS_ENER;   // its sum (fs_first)
+    if (!PLAIN && F.s[job] < 0) continue;
     const double a = warp_sum(acc[q]);
     if (lane == 0) rsum[q][w] = a;
   }
   __syncthreads();
   auto rec = [&](int job) -> StatLev & { return lev[((long)job * maxlev + (k - 1)) * nch + blockIdx.x]; };
   const int t = (int)threadIdx.x;
-  if (t < FM_N && F.m[t] >= 0 && !(top && t != FM_W) && !(t == FM_THE && !the)) {
+  if (EXT && t < FM_N && F.m[t] >= 0 && !(top && t != FM_W) && !(t == FM_THE && !the)) {
     float a = red[2 * t][0], b = red[2 * t + 1][0];
     for (int q = 1; q < ST_NW; q++) { a = fmaxf(a, red[2 * t][q]); b = fminf(b, red[2 * t + 1][q]); }
     rec(F.m[t]).vmax = a;
     rec(F.m[t]).vmin = b;
   }
-  if (t >= 32 && t < 32 + FS_N && F.s[t - 32] >= 0 && !top) {
+  if (SUMS && t >= 32 && t < 32 + FS_N && F.s[t - 32] >= 0 && !top) {
     const int q = t - 32;
     for (int c = 0; c < fs_first(q + 1) - fs_first(q); c++) {
       double a = 0.0;
@@ -521,7 +536,24 @@ void launch_stat(const DGrid &g, const StatFields &f, const StatConsts &s, const
   rest();
   if (flow) {
     dim3 grid((unsigned)nch, (unsigned)(F.m[FM_W] >= 0 ? g.nk + 1 : g.nk));
-    { ProfScope _ps("k_stat_flow", st); k_stat_flow<<<grid, ST_NT, 0, st>>>(g, f, s, F, lev, maxlev, nch); }
+    int sums = 0;
+    for (int q = 0; q < FS_N; q++)
+      if (F.s[q] >= 0) sums = std::max(sums, q == FS_MOE || q == FS_ENER ? 2 : 1);
+    // the sharing of rows whose warps take the fewest turns
+    const int rpc = (g.nj + 1 + nch - 1) / nch, nseg = (g.ni + 32) / 32;
+    int wpr = 1, turns = 0;
+    for (int p = 1; p <= ST_NW; p *= 2) {
+      const int n = (rpc * p + ST_NW - 1) / ST_NW * ((nseg + p - 1) / p);
+      if (p == 1 || n < turns) { wpr = p; turns = n; }
+    }
+    ProfScope _ps("k_stat_flow", st);
+    bool ext = false;
+    for (int q : F.m) ext = ext || q >= 0;
+    const auto flow_pass = sums == 2 && wpr == 1 && F.m[FM_WSP] >= 0 ? k_stat_flow<2, true, true>
+                           : sums == 2 ? (ext ? k_stat_flow<2, true, false> : k_stat_flow<2, false, false>)
+                           : sums == 1 ? (ext ? k_stat_flow<1, true, false> : k_stat_flow<1, false, false>)
+                                       : k_stat_flow<0, true, false>;
+    flow_pass<<<grid, ST_NT, 0, st>>>(g, f, s, F, lev, maxlev, nch, wpr);
     if (nl) *nl += 1;
   }
   if (nops > 0) {

@@ -12,7 +12,7 @@ place of 1e5)."""
 import numpy as np
 import pytest
 
-from cm1_b200.cases import make_case, stat_opts
+from cm1_b200.cases import STAT_SWITCHES, make_case, stat_opts
 
 pytestmark = pytest.mark.gpu
 
@@ -178,4 +178,30 @@ def test_statpack_of_infinite_values(name, cm1g, oracle_lib):
                     assert np.isnan(x) == np.isnan(y) and (not np.isinf(x) and not np.isinf(y) or x == y), (field, value, n, x, y)
                 fin = [k for k, y in enumerate(ref) if np.isfinite(y)]
                 _compare([names[k] for k in fin], got[fin], ref[fin])
+    ctx.close()
+
+
+SETS = {"w": ["stat_w"], "winds": ["stat_u", "stat_v", "stat_w", "stat_wsp", "stat_cfl", "stat_div"],
+        "moist": ["stat_q", "stat_rh", "stat_the"], "masses": ["stat_tmass", "stat_tmois", "stat_qmass"],
+        "flux": ["stat_tmf", "stat_thpert"], "momentum": ["stat_mo"], "energy": ["stat_tenerg", "stat_prspert"]}
+
+
+@pytest.mark.parametrize("which", sorted(SETS))
+@pytest.mark.parametrize("ni,nj,nk", [(700, 20, 7), (300, 100, 7), (280, 110, 20), (64, 64, 20), (5, 4, 6)])
+def test_statpack_of_few_switches(ni, nj, nk, which, cm1g, oracle_lib):
+    """The flow pass without budgets, with light ones, with momentum or energy; a
+    row shared by 8, 4, 2 and 1 of a block's warps, and rows of less than a warp."""
+    _torch()
+    case = make_case("supercell", ni=ni, nj=nj, nk=nk, npt=1)
+    st = case.state
+    rng = np.random.default_rng(ni)
+    for n, amp in (("ua", 3.0), ("va", 3.0), ("wa", 1.0), ("tha", 1.0)):
+        st[n] += rng.normal(0, amp, st[n].shape).astype(np.float32)
+    o, keep = stat_opts(case, off=tuple(s for s in STAT_SWITCHES if s not in SETS[which]))
+    ctx = cm1g.Context(case.cfg, case.grid)
+    names = ctx.stat_setup(o)
+    assert len(names) > 2
+    prate = np.zeros((case.lay.NJ, case.lay.NI), np.float32)
+    f, kw = _args(case, st)
+    _compare(names, ctx.statpack(1.0, case.dt, *f, prate=prate, **kw), oracle_lib.statpack(case, o, st, mtime=1.0, prate=prate))
     ctx.close()
