@@ -196,6 +196,8 @@ __global__ void k_d2_tend(DGrid g, Diff2Args a) {
   const float vf0 = LDG(&g.vf[j - g.jb]), vf1 = LDG(&g.vf[j + 1 - g.jb]);
   const float uh = LDG(&g.uh[i - g.ib]), vh = LDG(&g.vh[j - g.jb]), mh = LDG(&g.mh[k]);
   const float mf0 = LDG(&g.mf[k]), mf1 = LDG(&g.mf[k + 1]);
+  // rolled: 256x256x160 with five scalars 490 us, 530 as the compiler unrolls it
+#pragma unroll 1
   for (int n = 0; n < a.nsc; n++) {
     const float *s = a.s[n];
     const float dxl = 0.5f * (rho[o] + rho[o - 1]) * (s[o] - s[o - 1]) * rdx * uf0;
