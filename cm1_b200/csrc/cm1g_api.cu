@@ -142,11 +142,11 @@ static int set_err(int code, const char *fmt, ...) {
 // Arithmetic only: the entries call it before their first launch (297 tiles of 80
 // levels: 0.7 us; stepping through the blocks' schedule took 7, and 460 for 36,572
 // tiles of 128).
-int cm1g::tile_levels(long tiles, int nk, int slots, int over, int kcmax) {
+int cm1g::tile_levels(long tiles, int nk, int slots, int over, int kcmin, int kcmax) {
   const auto up = [](long a, long b) { return (a + b - 1) / b; };
   int best = 0;
   long best_end = 0;
-  for (int kc = 4; kc <= kcmax; kc += kc < 16 ? 1 : kc < 32 ? 2 : 4) {
+  for (int kc = kcmin; kc <= kcmax; kc += kc < 16 ? 1 : kc < 32 ? 2 : 4) {
     const int nch = (nk + kc - 1) / kc;
     // the full chunks in whole rounds of the slots: `late` slots come free a block
     // later than the others

@@ -306,10 +306,10 @@ struct EnerIn {
   float lv1, ls1;
 };
 
-// Levels that a block of a marching tile kernel owns, at most kcmax: the
+// Levels that a block of a marching tile kernel owns, kcmin to kcmax: the
 // choice whose blocks, handed to `slots` resident blocks in launch order,
 // finish first (a block costs its levels plus `over` for its first ones).
-int tile_levels(long tiles, int nk, int slots, int over, int kcmax);
+int tile_levels(long tiles, int nk, int slots, int over, int kcmin, int kcmax);
 
 // Records a message for cm1g_last_error() and returns code (C++ linkage,
 // not part of the C-ABI).

@@ -846,7 +846,7 @@ void launch_adv_momentum(const DGrid &g, const float *u, const float *v, const f
     ProfScope _ps("k_mom", st);
     // launch shape 0: the levels that end first; the other shapes: their table's levels
     const long tiles = (long)((g.ni + 31) / 31) * ((g.nj + MOM_TY - 1) / (MOM_TY - 1));
-    int kc = g.tile_mom > 0 ? kTileShapes[g.tile_mom][2] : tile_levels(tiles, g.nk, 2 * 148, 3, MOM_KC);
+    int kc = g.tile_mom > 0 ? kTileShapes[g.tile_mom][2] : tile_levels(tiles, g.nk, 2 * 148, 3, 4, MOM_KC);
     if (kc > MOM_KC) kc = MOM_KC;
     const size_t sm = (size_t)(kc + 2) * sizeof(MomLev);
     dim3 blk(32, MOM_TY), grid((g.ni + 31) / 31, (g.nj + MOM_TY - 1) / (MOM_TY - 1), (g.nk + kc - 1) / kc);

@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(32 * D2_TY, 2) k_d2_flow(DGrid g, Diff2Args a,
 template <bool MOM>
 static void d2_flow(const DGrid &g, const Diff2Args &a, int ns, int n0, cudaStream_t st) {
   dim3 blk(32, D2_TY), grid((g.ni + 1 + 29) / 30, (g.nj + 1 + D2_TY - 3) / (D2_TY - 2));
-  const int kc = tile_levels((long)grid.x * grid.y, g.nk, 2 * 148, 3, 128);
+  const int kc = tile_levels((long)grid.x * grid.y, g.nk, 2 * 148, 3, 4, 128);
   grid.z = (g.nk + kc - 1) / kc;
   ProfScope _ps("k_d2_flow", st);
   switch (ns) {

@@ -521,12 +521,13 @@ __global__ void __launch_bounds__(256) k_pdef_fix(const __grid_constant__ DGrid 
 // The host entry's single field takes at most 16: its second pass walks a chunk
 // level by level (251x187x79, the one grid measured: 95 us with 20 levels, 76 with
 // 12).  A step's passes keep the rule's choice: one launch's rule serves both, and
-// their words name few levels where tracers are sparse.
+// their words name few levels where tracers are sparse.  Without a second pass (a
+// word holds 4 levels at least) it takes as few as one: 16x16x20 40 to 35 us.
 constexpr int SC_OVER = 2;
 template <int TX, int TY, int PDEF, int RAW>
 static void scal_shape(const DGrid &g, ScalPass P, int kc, int weno, cudaStream_t st, int64_t *nl) {
   dim3 blk(TX, TY + 1), grid((g.ni + TX - 1) / TX, (g.nj + TY - 1) / TY, 1);
-  if (!kc) kc = tile_levels((long)grid.x * grid.y, g.nk, 3 * 148, SC_OVER, RAW ? 16 : SC_KMAX);
+  if (!kc) kc = tile_levels((long)grid.x * grid.y, g.nk, 3 * 148, SC_OVER, RAW && !PDEF ? 1 : 4, RAW ? 16 : SC_KMAX);
   P.kc = kc;
   grid.z = (g.nk + kc - 1) / kc;
   {

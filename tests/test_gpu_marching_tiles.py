@@ -51,7 +51,8 @@ def test_momentum_matches_oracle(ni, nj, nk, bc, cm1g, oracle_lib):
     ctx.close()
 
 
-@pytest.mark.parametrize("ni,nj,nk,npt", [(29, 9, 6, 0), (30, 10, 9, 2), (31, 15, 33, 3), (61, 16, 12, 6)])
+@pytest.mark.parametrize("ni,nj,nk,npt", [(29, 9, 6, 0), (30, 10, 9, 2), (31, 15, 33, 3), (61, 16, 12, 6),
+                                          (152, 91, 41, 2), (180, 130, 33, 1)])
 def test_turbsmag_matches_oracle(ni, nj, nk, npt, cm1g, oracle_lib):
     """At the bar of test_gpu_turb (the log of N^2 is the only difference)."""
     torch = _torch()

@@ -1,9 +1,9 @@
 """The scalar tile chooses the levels of a block by the grid's size, and the
 positive-definite pass names its levels in words of at most 32: grids whose choice
-is the smallest (4), some between and the largest that the advs entry takes (16),
-with level counts that end a chunk and one past it, columns one past a word and
-rows one past a tile; and words of 16 and 32 levels that are named by the next
-chunk's alone.
+is the smallest (4; 1 for the advs entry without the positive-definite pass), some
+between and the largest that the entry takes (16), with level counts that end a
+chunk and one past it, columns one past a word and rows one past a tile; and words
+of 16 and 32 levels that are named by the next chunk's alone.
 The advs entry and a step's tracers are the oracle's bit for bit (binary32 in the
 reference's order on both sides)."""
 import ctypes as C
@@ -24,11 +24,11 @@ def _torch():
     return torch
 
 
-def _levels(cm1g, ni, nj, nk, most):
+def _levels(cm1g, ni, nj, nk, most, fewest=4):
     """The library's own choice for 32 x 7 cells a block, three blocks an SM."""
-    f = cm1g.lib()._ZN4cm1g11tile_levelsEliiii
-    f.argtypes, f.restype = [C.c_long] + [C.c_int] * 4, C.c_int
-    return f(-(-ni // 32) * -(-nj // 7), nk, 3 * 148, 2, most)
+    f = cm1g.lib()._ZN4cm1g11tile_levelsEliiiii
+    f.argtypes, f.restype = [C.c_long] + [C.c_int] * 5, C.c_int
+    return f(-(-ni // 32) * -(-nj // 7), nk, 3 * 148, 2, fewest, most)
 
 
 @pytest.mark.parametrize("ni,nj,nk,bc,kc", [(4, 4, 6, 1, 4), (33, 8, 8, 2, 4), (65, 15, 9, 1, 4), (161, 113, 33, 2, 8),
@@ -126,7 +126,7 @@ def test_advs_across_words_of_16_levels(up, cm1g, oracle_lib):
                                             (225, 163, 33, 2, 16)])
 def test_advs_bitwise(ni, nj, nk, bc, kc, pdef, cm1g, oracle_lib):
     _torch()
-    assert _levels(cm1g, ni, nj, nk, 16) == kc
+    assert _levels(cm1g, ni, nj, nk, 16) == kc and _levels(cm1g, ni, nj, nk, 16, 1) == (1 if kc == 4 else kc)
     case = make_case("dry_bubble", ni=ni, nj=nj, nk=nk, bc=bc, advwenos=1)
     lay = case.lay
     rng = np.random.default_rng(nk)

@@ -11,8 +11,8 @@ from cm1_b200 import binding
 
 
 def _levels():
-    f = binding.lib()._ZN4cm1g11tile_levelsEliiii
-    f.argtypes, f.restype = [C.c_long] + [C.c_int] * 4, C.c_int
+    f = binding.lib()._ZN4cm1g11tile_levelsEliiiii
+    f.argtypes, f.restype = [C.c_long] + [C.c_int] * 5, C.c_int
     return f
 
 
@@ -26,9 +26,9 @@ def _end(tiles, nk, slots, over, kc):
     return max(free)
 
 
-def _simulated(tiles, nk, slots, over, kcmax):
+def _simulated(tiles, nk, slots, over, kcmin, kcmax):
     best = None
-    kc = 4
+    kc = kcmin
     while kc <= kcmax:
         end = _end(tiles, nk, slots, over, kc)
         if best is None or end < best[0]:
@@ -45,11 +45,12 @@ def test_choice_is_the_simulated_one(seed):
     for _ in range(60):
         slots = rng.choice((1, 2, 3, 7, 12, 37))          # any number of slots; the kernels have 296 and 444
         tiles = rng.choice((1, 2, slots, slots + 1, rng.randint(1, 4 * slots)))
-        a = (tiles, rng.randint(5, 70), slots, rng.choice((2, 3)), rng.choice((16, 32, 64, 128)))
+        a = (tiles, rng.randint(5, 70), slots, rng.choice((2, 3)), rng.choice((1, 4)), rng.choice((16, 32, 64, 128)))
         assert f(*a) == _simulated(*a), a
 
 
-@pytest.mark.parametrize("a", [(1, 6, 444, 2, 16), (297, 80, 296, 3, 64), (234, 128, 296, 3, 128), (216, 79, 444, 2, 16),
-                               (296, 40, 444, 2, 32), (444, 64, 444, 2, 32), (445, 65, 444, 2, 32)])
+@pytest.mark.parametrize("a", [(1, 6, 444, 2, 1, 16), (297, 80, 296, 3, 4, 64), (234, 128, 296, 3, 1, 128),
+                               (216, 79, 444, 2, 4, 16), (296, 40, 444, 2, 4, 32), (444, 64, 444, 2, 4, 32),
+                               (445, 65, 444, 2, 1, 32)])
 def test_choice_at_the_kernels_slots(a):
     assert _levels()(*a) == _simulated(*a)
