@@ -58,8 +58,9 @@ void launch_sound(const DGrid &g, int nsound, int nrk, float dt, const float *ua
                   const float *ppi, float *pp3d, const float *piadv, const float *ppten, float *ppx,
                   const float *thv, const float *ppterm, float *rru, float *rrv, float *rrw, float *radbcw,
                   float *radbce, float *radbcs, float *radbcn, float *su, float *sv, float *su2,
-                  float *sv2, float *d1, float *d2, float *lu, float *rbnd, cudaStream_t st, int64_t *nl);
+                  float *sv2, float *d1, float *d2, float *lu, float *rbnd, cudaStream_t st, int64_t *nl, long beside = 0);
 int sound_max_nk();
+long sound_tiles(const DGrid &g);
 cudaError_t sound_init();
 void launch_stage_prep(const DGrid &g, const float *th3d, const float *pp3d, const float *qv, const LiquidIn &liq,
                        int imoist, int eqtset, float *t11, float *t22, float *thterm, float *piadv, int ring, cudaStream_t st,
@@ -657,9 +658,11 @@ static void closure_phi(cm1g_ctx *c, const float *th, float dt, cudaStream_t st,
   }
 }
 
+// beside: 0, or for the members of an ensemble the acoustic tiles of all of them.
 // merge: fill halos in one launch, and rings where their array is formed (the
 // members of an ensemble fill them as launches of their own, k_bc.cu)
-static void run_solve2(cm1g_ctx *c, const cm1g_state_t *d, float dt, double mass1, bool merge = true) {
+static void run_solve2(cm1g_ctx *c, const cm1g_state_t *d, float dt, double mass1, long beside = 0) {
+  const bool merge = beside == 0;
   const DGrid &g = c->g;
   const cm1g_config_t &cf = c->cfg;
   cudaStream_t st = c->stream;
@@ -708,7 +711,8 @@ static void run_solve2(cm1g_ctx *c, const cm1g_state_t *d, float dt, double mass
                         th_in, qv_in, c->mdivx, st, nl, diffit ? &df : nullptr, liq.b8);
     launch_sound(g, cf.nsound, nrk, dt, d->ua, d->u3d, c->uten, d->va, d->v3d, c->vten, d->wa, d->w3d, c->wten,
                  d->ppi, d->pp3d, c->piadv, d->ppten, d->ppx, c->t11, c->t22, c->rru, c->rrv, c->rrw,
-                 d->radbcw, d->radbce, d->radbcs, d->radbcn, c->su, c->sv, c->su2, c->sv2, c->d1, c->d2, c->lu, c->rbnd, st, nl);
+                 d->radbcw, d->radbce, d->radbcs, d->radbcn, c->su, c->sv, c->su2, c->sv2, c->d1, c->d2, c->lu, c->rbnd, st, nl,
+                 beside);
     if (nrk == 3) launch_cfl(g, d->u3d, d->v3d, d->w3d, dt, c->cflbits, st, nl);
     if (openrad) launch_radbc4(g, d->ua, d->u3d, d->va, d->v3d, d->radbcw, d->radbce, d->radbcs, d->radbcn, dttmp, st, nl);
     const int weno = (cf.advwenos == 1 || (cf.advwenos == 2 && nrk == 3)) ? 1 : 0;
@@ -889,14 +893,14 @@ static void run_kessler(cm1g_ctx *c, const cm1g_state_t *d, float dt) {
   launch_kessler(g, a, c->mp_part, c->mp_colbud, c->mp_qbud, c->stream, &c->nlaunch);
 }
 
-static void run_step(cm1g_ctx *c, const cm1g_state_t *d, float dt, double mass1, bool merge = true) {
-  run_solve2(c, d, dt, mass1, merge);
+static void run_step(cm1g_ctx *c, const cm1g_state_t *d, float dt, double mass1, long beside = 0) {
+  run_solve2(c, d, dt, mass1, beside);
   if (c->cfg.imoist && c->cfg.ptype == 1)   // cm1.F:3421-3431 (mp_driver)
     run_kessler(c, d, dt);
   else if (c->cfg.imoist)                   // cm1.F:3410-3415 (ptype=0)
     launch_pdefq(c->g, 0.0f, d->rho, d->q3d + (long)(c->cfg.nqv - 1) * nS(c->g), nullptr, nullptr, c->stream,
                  &c->nlaunch);
-  run_solve3(c, d, merge);
+  run_solve3(c, d, beside == 0);
 }
 
 static int fetch_scalars(cm1g_ctx *c, double *mass2, float *cflmax) {
@@ -1274,6 +1278,7 @@ extern "C" int cm1g_autotune(cm1g_ctx_t *c, float dt, double mass1, const cm1g_s
 // ---------------------------------------------------------------------
 struct cm1g_ens {
   std::vector<cm1g_ctx *> m;
+  long tiles = 0;                             // acoustic tiles of all members
   cudaStream_t stream = nullptr;
   cudaEvent_t fork = nullptr;
   std::vector<cudaEvent_t> join;
@@ -1305,6 +1310,7 @@ extern "C" int cm1g_ensemble_create(cm1g_ctx_t **members, int32_t n, cm1g_ens_t 
   cm1g_ens *e = new cm1g_ens();
   e->m.assign(members, members + n);
   e->join.resize(n);
+  for (cm1g_ctx *c : e->m) e->tiles += sound_tiles(c->g);
   bool ok = cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking) == cudaSuccess &&
             cudaEventCreateWithFlags(&e->fork, cudaEventDisableTiming) == cudaSuccess;
   for (int q = 0; q < n && ok; q++) ok = cudaEventCreateWithFlags(&e->join[q], cudaEventDisableTiming) == cudaSuccess;
@@ -1330,7 +1336,7 @@ static void ens_enqueue(cm1g_ens *e, const cm1g_state_t *st, const float *dt, co
   for (size_t q = 0; q < e->m.size(); q++) {
     cm1g_ctx *c = e->m[q];
     cudaStreamWaitEvent(c->stream, e->fork, 0);
-    run_step(c, &st[q], dt[q], mass1[q], false);
+    run_step(c, &st[q], dt[q], mass1[q], e->tiles);
     cudaEventRecord(e->join[q], c->stream);
     cudaStreamWaitEvent(e->stream, e->join[q], 0);
   }

@@ -740,14 +740,18 @@ static bool sound_tall(const DGrid &g) { return g.nk > SND_MAXNK || nU(g) >= (1L
 // when the grid has no more than one tile for each of the 148 SMs, 16 explicit
 // warps shorten the one wave.  Times of the final stage's substeps (6), one
 // B200: 256x256x80 0.85 ms (7 warps) against 0.89 (10) and 1.29 (16);
-// 512x512x128 5.16 ms (10); 64x64x40 0.104 ms (16) against 0.121 (7).
+// 512x512x128 5.16 ms (10); 64x64x40 0.104 ms (16) against 0.121 (7).  The members
+// of an ensemble run side by side, so the rule counts the tiles of all, up to two for
+// each SM as their acoustic steps do not all fall together (a step of 40 members of
+// 48 to 64 columns: 9.2 ms with each member's own count, 7.7 so; 24 of 48 to 80: 6.0,
+// 5.2; two of 48x48: 0.45, 0.45, and 0.47 with one tile for each SM).
 typedef void (*SoundTileFn)(DGrid, SoundIO, SoundStep);
 struct SoundTile { SoundTileFn fn; int nw, kpt; };
 static const SoundTile kSoundTiles[3] = {
     {k_sound_tile<7, 12, 3>, 7, 12}, {k_sound_tile<10, 13, 2>, 10, 13}, {k_sound_tile<16, 8, 1>, 16, 8}};
-static int sound_tile_of(const DGrid &g, int cfg) {
-  const long tiles = (long)((g.ni + SND_TX - 1) / SND_TX) * g.nj;
-  if (cfg == 1 || tiles <= 148) return 2;
+long sound_tiles(const DGrid &g) { return (long)((g.ni + SND_TX - 1) / SND_TX) * g.nj; }
+static int sound_tile_of(const DGrid &g, int cfg, long beside) {
+  if (cfg == 1 || (beside ? beside <= 2 * 148 : sound_tiles(g) <= 148)) return 2;
   return g.nk <= kSoundTiles[0].nw * kSoundTiles[0].kpt ? 0 : 1;
 }
 
@@ -767,14 +771,15 @@ cudaError_t sound_init() {
 // u3d/v3d/w3d/pp3d receive the result; su/sv/su2/sv2 are scratch for the
 // u/v double buffer, d1/d2 for ppd, lu (scalar-shaped) for the column
 // sweep's LU factors, rbnd (2 NJ*NK + 2 NI*NK floats; roflux = 1 only) for
-// the restricted boundary velocities.  rru/rrv/rrw receive the averages.
+// the restricted boundary velocities.  rru/rrv/rrw receive the averages.  beside: the
+// tiles of all grids that are advanced at the same time (0: this one's).
 void launch_sound(const DGrid &g, int nsound, int nrk, float dt,
                   const float *ua, float *u3d, const float *uten, const float *va, float *v3d, const float *vten,
                   const float *wa, float *w3d, const float *wten, const float *ppi, float *pp3d,
                   const float *piadv, const float *ppten, float *ppx, const float *thv, const float *ppterm,
                   float *rru, float *rrv, float *rrw, float *radbcw, float *radbce,
                   float *radbcs, float *radbcn, float *su, float *sv, float *su2, float *sv2,
-                  float *d1, float *d2, float *lu, float *rbnd, cudaStream_t st, int64_t *nl) {
+                  float *d1, float *d2, float *lu, float *rbnd, cudaStream_t st, int64_t *nl, long beside) {
   int nloop;
   float dts;
   sound_nloop(nsound, nrk, dt, &nloop, &dts);
@@ -794,7 +799,7 @@ void launch_sound(const DGrid &g, int nsound, int nrk, float dt,
   const bool restrict_open = g.roflux && ((g.wbc == 2 && g.ibw) || (g.ebc == 2 && g.ibe) ||
                                           (g.sbc == 2 && g.ibs) || (g.nbc == 2 && g.ibn));
   const int cty = (cfg == 3) ? 2 : 4;
-  const SoundTile &T = kSoundTiles[sound_tile_of(g, cfg)];
+  const SoundTile &T = kSoundTiles[sound_tile_of(g, cfg, beside)];
   const int nw = T.nw + 1;
   const bool col = cfg >= 2;
   dim3 blk = col ? dim3(SNC_TX, cty) : dim3(SND_TX, nw);

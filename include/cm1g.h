@@ -534,8 +534,8 @@ int cm1g_pdefq_noalloc(const cm1g_config_t *cfg, float rmax, double *asq,
  * the levels that the shape functions report for it are those of the passes
  * that do not choose.  sound_form selects the acoustic kernel: -1 automatic,
  * 0 tile form of 32 columns with the warps over the levels chosen by the
- * grid's size (16 where there are at most 148 tiles, else 7 up to 84 levels
- * and 10 above), 1 the same with 16 of them, 2 column sweep with 32 x 4
+ * grid's size (16 where there are at most 148 tiles, or 296 of all members
+ * of an ensemble, else 7 up to 84 levels and 10 above), 1 the same with 16 of them, 2 column sweep with 32 x 4
  * columns per block, 3 column sweep with 32 x 2.  step_ms is the measured
  * large-step time of the configuration (cm1g_autotune; 0 when not measured). */
 typedef struct cm1g_tune {
